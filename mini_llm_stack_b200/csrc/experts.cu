@@ -23,14 +23,16 @@
 //   tensor, or the float32 K-parts of its product, shared_stride apart, added in their order); with a
 //   gate (float32, one number a token) the shared addend is multiplied by sigmoid(gate[t]).
 //
-// The products run with float32 accumulation over k ascending (bfloat16 rows of whole
-// 16-byte pieces on the tensor cores, everything else on CUDA cores), one row
+// The products run with float32 accumulation over k ascending: bfloat16 rows of whole
+// 16-byte pieces on the tensor cores (experts_tc.cu), everything else on CUDA cores, one row
 // tile of one expert a CTA; every row is computed by itself, so a token's result does
 // not depend on the batch, on its place in the sorted order or on the other tokens of
 // its expert.
 #include "common.cuh"
+#include "experts.h"
 
 namespace {
+using namespace mls_experts;
 constexpr int BM = 32, BN = 64, BK = 32, TM = 2, TN = 4;   // 256 threads
 
 constexpr int MAX_GROUPS = 256;
@@ -231,19 +233,6 @@ __device__ __forceinline__ void fill_tile(float (*tile)[ROWS + PAD], int k0, int
     }
 }
 
-// The gated unit on the two products' float32 sums.
-__device__ __forceinline__ float gated_unit(float g, float u, float alpha, float limit) {
-    if (limit > 0.f) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return (g / (1.0f + expf(-alpha * g))) * (u + 1.0f);
-    }
-    return (g / (1.0f + expf(-g))) * u;
-}
-
-// What a product does: the experts' down projection, or an up projection with a unit on its sums.
-enum { DOWN = 0, GATED = 1, RELU2 = 2 };
-
 // GATED: A row = h[slot / top] (* weight[slot] if scale), W = [gate rows | up rows] of
 // expert e ([2F, K]), out y[p, n] = silu(gate) * up in T.
 // RELU2: the same A row, W = Wu[e] ([F, K]), y[p, n] = relu(up)^2.
@@ -342,181 +331,6 @@ expert_gemm_kernel(const T* __restrict__ A, const T* __restrict__ W, void* __res
     }
 }
 
-// The same products for bfloat16 on the tensor cores (mma.sync m16n8k16, float32
-// accumulators): a CTA takes up to four of the same tiles of 32 sorted rows x 64 output
-// columns, its eight warps 32 x 32 each; operands go through shared memory in rows of 32 + 8 values, so that
-// the fragment loads (one 32-bit word a lane) meet no bank twice.  Every output element is
-// its own dot product over k ascending in steps of 16, whatever else is in the tile.  With
-// input scaling the row is rounded to bfloat16 once more after the weight is applied.
-constexpr int MK = 32, MKP = MK + 8;
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-        "{%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// A CTA walks RT consecutive entries of the tile list; entries of one expert that follow each
-// other (a prompt gives an expert many rows) are taken together, up to RT * 32 = 128 rows
-// against one load of every weight tile; rows that are not there are zeros.
-// RT = 1 (few rows an expert: decoding) keeps one entry a CTA, so that as many CTAs as
-// possible stream weights.
-template <int UNIT, int RT>
-__global__ void __launch_bounds__(256)
-expert_mma_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W,
-                  void* __restrict__ out, const int* __restrict__ order,
-                  const int* __restrict__ offsets, const int* __restrict__ tile_expert,
-                  const int* __restrict__ tile_row0, int max_tiles,
-                  const float* __restrict__ weight, int top, int scale, int N, int K,
-                  float alpha, float limit) {
-    constexpr bool GLU = UNIT == GATED, UP = UNIT != DOWN;
-    chain_release();
-    chain_wait();
-    constexpr int MROWS = RT * BM;
-    // RT 4: 4 x 2 warps of 32 rows x 32 columns; RT 1: 2 x 4 warps of 16 x 16
-    constexpr int MF = RT == 4 ? 2 : 1, NF = RT == 4 ? 4 : 2, WARPS_N = RT == 4 ? 2 : 4;
-    constexpr int LOADS = (MROWS * 4 + 255) / 256;            // 16-byte pieces of A a thread loads
-    __shared__ __align__(16) __nv_bfloat16 As[MROWS][MKP];
-    __shared__ __align__(16) __nv_bfloat16 Ws[BN][MKP];
-    __shared__ __align__(16) __nv_bfloat16 Us[GLU ? BN : 1][MKP];
-    __shared__ int slot_s[MROWS];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n0 = blockIdx.x * BN;
-    const int wm = warp / WARPS_N, wn = warp % WARPS_N;
-    const int g = lane >> 2, c = (lane & 3) * 2;
-    const int lrow = tid >> 2, lk = (tid & 3) * 8;            // who loads what: 16 bytes a thread
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    const int t_end = min(max_tiles, (int)(blockIdx.y + 1) * RT);   // every output element is the same sum for either RT
-    int t = blockIdx.y * RT;
-    while (t < t_end) {
-        const int e = tile_expert[t];
-        if (e < 0) break;                                     // the list's unused tail
-        int run = 1;
-        while (t + run < t_end && tile_expert[t + run] == e) ++run;
-        const int p0 = tile_row0[t], p_end = offsets[e + 1];
-        t += run;
-        __syncthreads();                                      // the last run's slot_s is read no more
-        if (tid < MROWS) slot_s[tid] = (tid < run * BM && p0 + tid < p_end) ? order[p0 + tid] : -1;
-        __syncthreads();
-        const __nv_bfloat16* We = W + (size_t)e * (GLU ? 2 : 1) * N * K;
-        float acc[MF][NF][4], acu[GLU ? MF : 1][NF][4];
-#pragma unroll
-        for (int i = 0; i < MF; ++i)
-#pragma unroll
-            for (int j = 0; j < NF; ++j)
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    acc[i][j][x] = 0.f;
-                    if (GLU) acu[i][j][x] = 0.f;
-                }
-        const __nv_bfloat16* a_src[LOADS];
-        float a_scale[LOADS];
-#pragma unroll
-        for (int h2 = 0; h2 < LOADS; ++h2) {
-            const int r = lrow + 64 * h2;
-            const int slot = r < MROWS ? slot_s[r] : -1;
-            a_src[h2] = nullptr;
-            a_scale[h2] = 1.f;
-            if (slot >= 0) {
-                if (UP) {
-                    a_src[h2] = A + (size_t)(slot / top) * K;
-                    if (scale) a_scale[h2] = weight[slot];
-                } else {
-                    a_src[h2] = A + (size_t)(p0 + r) * K;
-                }
-            }
-        }
-        const bool w_ok = n0 + lrow < N;
-        const __nv_bfloat16* w_src = We + (size_t)(n0 + lrow) * K;
-        const __nv_bfloat16* u_src = We + (size_t)(N + n0 + lrow) * K;
-        for (int k0 = 0; k0 < K; k0 += MK) {
-            const bool k_ok = k0 + lk < K;
-#pragma unroll
-            for (int h2 = 0; h2 < LOADS; ++h2) {
-                if (lrow + 64 * h2 >= MROWS) continue;
-                uint4 v = (a_src[h2] && k_ok) ? *reinterpret_cast<const uint4*>(a_src[h2] + k0 + lk) : zero;
-                if (UP && scale && a_src[h2]) {
-                    __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const float2 f2 = __bfloat1622float2(p2[x]);
-                        p2[x] = __floats2bfloat162_rn(f2.x * a_scale[h2], f2.y * a_scale[h2]);
-                    }
-                }
-                *reinterpret_cast<uint4*>(&As[lrow + 64 * h2][lk]) = v;
-            }
-            *reinterpret_cast<uint4*>(&Ws[lrow][lk]) =
-                (w_ok && k_ok) ? *reinterpret_cast<const uint4*>(w_src + k0 + lk) : zero;
-            if (GLU)
-                *reinterpret_cast<uint4*>(&Us[lrow][lk]) =
-                    (w_ok && k_ok) ? *reinterpret_cast<const uint4*>(u_src + k0 + lk) : zero;
-            __syncthreads();
-            if (16 * MF * wm < run * BM) {                    // a warp whose rows are not there idles
-#pragma unroll
-                for (int kk = 0; kk < MK; kk += 16) {
-                    uint32_t a[MF][4];
-#pragma unroll
-                    for (int mf = 0; mf < MF; ++mf) {
-                        const int r = 16 * MF * wm + 16 * mf + g;
-                        a[mf][0] = *reinterpret_cast<const uint32_t*>(&As[r][kk + c]);
-                        a[mf][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + c]);
-                        a[mf][2] = *reinterpret_cast<const uint32_t*>(&As[r][kk + c + 8]);
-                        a[mf][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + c + 8]);
-                    }
-#pragma unroll
-                    for (int nf = 0; nf < NF; ++nf) {
-                        const int n = 8 * NF * wn + 8 * nf + g;
-                        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&Ws[n][kk + c]);
-                        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&Ws[n][kk + c + 8]);
-#pragma unroll
-                        for (int mf = 0; mf < MF; ++mf) mma_bf16(acc[mf][nf], a[mf], b0, b1);
-                        if (GLU) {
-                            const uint32_t u0 = *reinterpret_cast<const uint32_t*>(&Us[n][kk + c]);
-                            const uint32_t u1 = *reinterpret_cast<const uint32_t*>(&Us[n][kk + c + 8]);
-#pragma unroll
-                            for (int mf = 0; mf < MF; ++mf) mma_bf16(acu[mf][nf], a[mf], u0, u1);
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int mf = 0; mf < MF; ++mf)
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int r = 16 * MF * wm + 16 * mf + g + 8 * half;
-                const int slot = slot_s[r];
-                if (slot < 0) continue;
-#pragma unroll
-                for (int nf = 0; nf < NF; ++nf)
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const int n = n0 + 8 * NF * wn + 8 * nf + c + x;
-                        if (n >= N) continue;
-                        const float v = acc[mf][nf][2 * half + x];
-                        if (GLU)
-                            ((__nv_bfloat16*)out)[(size_t)(p0 + r) * N + n] = __float2bfloat16_rn(
-                                gated_unit(v, acu[mf][nf][2 * half + x], alpha, limit));
-                        else if (UP)
-                            ((__nv_bfloat16*)out)[(size_t)(p0 + r) * N + n] =
-                                __float2bfloat16_rn(fmaxf(v, 0.f) * fmaxf(v, 0.f));
-                        else
-                            ((float*)out)[(size_t)slot * N + n] = scale ? v * weight[slot] : v;
-                    }
-            }
-    }
-}
-
-// bfloat16 rows of whole 16-byte pieces at 16-byte addresses: the tensor-core kernel's.
-static inline bool takes_mma(int dtype, const void* a, const void* w, int K) {
-    return dtype == MLS_BF16 && K % 8 == 0 &&
-           (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
-}
-
 template <typename T>
 __global__ void expert_combine_kernel(const float* __restrict__ per_slot, int top,
                                       const void* __restrict__ shared, int shared_dtype,
@@ -576,23 +390,32 @@ MLS_API int mls_route_sort(const int* idx, int n_slots, int n_experts, int n_rea
     return launch_status();
 }
 
-// One of the experts' products over the sorted slots: N outputs of K inputs an expert.
+// Whether the products of these operands run on the tensor cores.
+MLS_API int mls_expert_takes_tc(int dtype, const void* a, const void* w, int K, int n_experts) {
+    return takes_tc(dtype, a, w, K, n_experts) ? 1 : 0;
+}
+
+// One of the experts' products over the sorted slots: N outputs of K inputs an expert.  `rows`:
+// scratch of n_slots x K bfloat16 for the sorted rows where the product runs on the tensor cores
+// (unused otherwise, and by the down product, whose rows are sorted).
 template <int UNIT>
 static int expert_product(const void* A, const void* W, void* out, int dtype, const int* order,
                           const int* offsets, const int* tile_expert, const int* tile_row0,
-                          int max_tiles, const float* weight, int top, int scale, int N, int K,
-                          int many_rows, float alpha, float limit, cudaStream_t stream) {
+                          int max_tiles, const float* weight, int top, int scale, int n_slots,
+                          int n_experts, int N, int K, void* rows, float alpha, float limit,
+                          int* status, cudaStream_t stream) {
     if (max_tiles <= 0) return 0;
-    dim3 grid((N + BN - 1) / BN, max_tiles);
-    if (takes_mma(dtype, A, W, K) && many_rows)
-        MLS_LAUNCH((expert_mma_kernel<UNIT, 4>), dim3(grid.x, (max_tiles + 3) / 4), dim3(256), 0,
-                   stream, (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, out, order, offsets,
-                   tile_expert, tile_row0, max_tiles, weight, top, scale, N, K, alpha, limit);
-    else if (takes_mma(dtype, A, W, K))
-        MLS_LAUNCH((expert_mma_kernel<UNIT, 1>), dim3(grid), dim3(256), 0, stream,
-                   (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, out, order, offsets,
-                   tile_expert, tile_row0, max_tiles, weight, top, scale, N, K, alpha, limit);
-    else if (dtype == MLS_BF16)
+    if (takes_tc(dtype, A, W, K, n_experts)) {
+        if (UNIT != DOWN) {
+            if (!rows) return MLS_ERR_UNSUPPORTED;
+            const int rc = gather_tc(A, order, weight, top, scale, n_slots, K, rows, stream);
+            if (rc) return rc;
+        }
+        return product_tc(UNIT, UNIT == DOWN ? A : rows, W, out, order, offsets, weight, scale,
+                          n_slots, n_experts, N, K, alpha, limit, status, stream);
+    }
+    const dim3 grid((N + BN - 1) / BN, max_tiles);
+    if (dtype == MLS_BF16)
         MLS_LAUNCH((expert_gemm_kernel<__nv_bfloat16, UNIT>), dim3(grid), dim3(256), 0, stream,
                    (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, out, order, offsets,
                    tile_expert, tile_row0, weight, top, scale, N, K, alpha, limit);
@@ -606,26 +429,31 @@ static int expert_product(const void* A, const void* W, void* out, int dtype, co
 MLS_API int mls_expert_glu(const void* h, const void* w_gate_up, void* y, int dtype,
                            const int* order, const int* offsets, const int* tile_expert,
                            const int* tile_row0, int max_tiles, const float* weight, int top,
-                           int scale_in, int F, int K, int many_rows, float alpha, float limit,
-                           cudaStream_t stream) {
+                           int scale_in, int n_slots, int n_experts, int F, int K, void* rows,
+                           float alpha, float limit, int* status, cudaStream_t stream) {
     return expert_product<GATED>(h, w_gate_up, y, dtype, order, offsets, tile_expert, tile_row0,
-                                 max_tiles, weight, top, scale_in, F, K, many_rows, alpha, limit, stream);
+                                 max_tiles, weight, top, scale_in, n_slots, n_experts, F, K, rows,
+                                 alpha, limit, status, stream);
 }
 
 MLS_API int mls_expert_relu2(const void* h, const void* w_up, void* y, int dtype, const int* order,
                              const int* offsets, const int* tile_expert, const int* tile_row0,
-                             int max_tiles, const float* weight, int top, int scale_in, int F, int K,
-                             int many_rows, cudaStream_t stream) {
+                             int max_tiles, const float* weight, int top, int scale_in, int n_slots,
+                             int n_experts, int F, int K, void* rows, int* status,
+                             cudaStream_t stream) {
     return expert_product<RELU2>(h, w_up, y, dtype, order, offsets, tile_expert, tile_row0, max_tiles,
-                                 weight, top, scale_in, F, K, many_rows, 0.f, 0.f, stream);
+                                 weight, top, scale_in, n_slots, n_experts, F, K, rows, 0.f, 0.f,
+                                 status, stream);
 }
 
 MLS_API int mls_expert_down(const void* y, const void* w_down, float* per_slot, int dtype,
                             const int* order, const int* offsets, const int* tile_expert,
                             const int* tile_row0, int max_tiles, const float* weight, int top,
-                            int scale_out, int D, int F, int many_rows, cudaStream_t stream) {
+                            int scale_out, int n_slots, int n_experts, int D, int F, int* status,
+                            cudaStream_t stream) {
     return expert_product<DOWN>(y, w_down, per_slot, dtype, order, offsets, tile_expert, tile_row0,
-                                max_tiles, weight, top, scale_out, D, F, many_rows, 0.f, 0.f, stream);
+                                max_tiles, weight, top, scale_out, n_slots, n_experts, D, F, nullptr,
+                                0.f, 0.f, status, stream);
 }
 
 MLS_API int mls_expert_combine(const float* per_slot, int top, const void* shared,

@@ -792,13 +792,16 @@ class Ops:
                                  [_P, _I, _I, _I, _I, _I, _I, _P, _F, _I, _I, _P, _P, _P]),
                    "sort": _decl(lib, "mls_route_sort",
                                  [_P, _I, _I, _I, _P, _P, _P, _P, _I, _P, _P]),
+                   "takes_tc": _decl(lib, "mls_expert_takes_tc", [_I, _P, _P, _I, _I]),
                    "glu": _decl(lib, "mls_expert_glu",
-                                [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F,
-                                 _P]),
+                                [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P,
+                                 _F, _F, _P, _P]),
                    "relu2": _decl(lib, "mls_expert_relu2",
-                                  [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P]),
+                                  [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
+                                   _P, _P, _P]),
                    "down": _decl(lib, "mls_expert_down",
-                                 [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P]),
+                                 [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
+                                  _P, _P]),
                    "combine": _decl(lib, "mls_expert_combine",
                                     [_P, _I, _P, _I, _I, _LL, _P, _P, _I, _P, _P, _I, _P, _I, _I, _I,
                                      _P])}
@@ -1081,12 +1084,14 @@ class Ops:
         rows = int(self._part_lib("experts")["tile_rows"]())
         return (n_slots + rows - 1) // rows + n_experts
 
-    @staticmethod
-    def _many_rows(n_slots: int, n_experts: int) -> int:
-        """Whether an expert has, on average, rows for more than two 32-row tiles: a CTA of
-        the tensor-core kernel then takes four tiles of an expert against one load of its
-        weights (the sums are the same either way)."""
-        return 1 if n_slots >= 64 * n_experts else 0
+    def _expert_rows(self, h, w, n_slots: int):
+        """Scratch for the sorted rows of an experts' first product where it runs on the tensor
+        cores, else None; counts the kernel that fills it."""
+        n_experts, k = w.shape[0], w.shape[2]
+        if not self._part_lib("experts")["takes_tc"](_code(h.dtype), _ptr(h), _ptr(w), k, n_experts):
+            return None
+        self.launches += 1
+        return self.scratch("expert_rows", (n_slots * k + 1) // 2)
 
     def expert_glu(self, h, w_gate_up, y, work: dict, top: int, scale_in: bool,
                    alpha: float = 1.0, limit: float = 0.0) -> None:
@@ -1097,13 +1102,14 @@ class Ops:
         _need(h.dtype == w_gate_up.dtype == y.dtype and h.is_contiguous() and y.is_contiguous()
               and w_gate_up.is_contiguous() and h.shape[1] == k and y.shape[1] == f2 // 2,
               "expert_glu: operands")
+        rows = self._expert_rows(h, w_gate_up, y.shape[0])
         self.launches += 1
         _check(self._part_lib("experts")["glu"](
             _ptr(h), _ptr(w_gate_up), _ptr(y), _code(h.dtype), _ptr(work["order"]),
             _ptr(work["offsets"]), _ptr(work["tile_expert"]), _ptr(work["tile_row0"]),
-            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_in else 0, f2 // 2, k,
-            self._many_rows(y.shape[0], n_experts), float(alpha), float(limit), self._stream()),
-            "expert_glu")
+            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_in else 0, y.shape[0],
+            n_experts, f2 // 2, k, _ptr(rows), float(alpha), float(limit), _ptr(self.status),
+            self._stream()), "expert_glu")
 
     def expert_relu_squared(self, h, w_up, y, work: dict, top: int, scale_in: bool) -> None:
         """``y[p] = relu(Wu[e] a)^2`` for the sorted slots; ``w_up [E, F, K]``."""
@@ -1111,12 +1117,13 @@ class Ops:
         _need(h.dtype == w_up.dtype == y.dtype and h.is_contiguous() and y.is_contiguous()
               and w_up.is_contiguous() and h.shape[1] == k and y.shape[1] == f,
               "expert_relu_squared: operands")
+        rows = self._expert_rows(h, w_up, y.shape[0])
         self.launches += 1
         _check(self._part_lib("experts")["relu2"](
             _ptr(h), _ptr(w_up), _ptr(y), _code(h.dtype), _ptr(work["order"]),
             _ptr(work["offsets"]), _ptr(work["tile_expert"]), _ptr(work["tile_row0"]),
-            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_in else 0, f, k,
-            self._many_rows(y.shape[0], n_experts), self._stream()), "expert_relu_squared")
+            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_in else 0, y.shape[0],
+            n_experts, f, k, _ptr(rows), _ptr(self.status), self._stream()), "expert_relu_squared")
 
     def expert_down(self, y, w_down, per_slot, work: dict, top: int, scale_out: bool) -> None:
         """``per_slot[slot] = Wd[e] y[p]`` (float32); ``w_down [E, D, F]``."""
@@ -1128,8 +1135,8 @@ class Ops:
         _check(self._part_lib("experts")["down"](
             _ptr(y), _ptr(w_down), _ptr(per_slot), _code(y.dtype), _ptr(work["order"]),
             _ptr(work["offsets"]), _ptr(work["tile_expert"]), _ptr(work["tile_row0"]),
-            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_out else 0, d, f,
-            self._many_rows(y.shape[0], n_experts), self._stream()), "expert_down")
+            work["max_tiles"], _ptr(work["weight"]), top, 1 if scale_out else 0, y.shape[0],
+            n_experts, d, f, _ptr(self.status), self._stream()), "expert_down")
 
     def expert_combine(self, per_slot, top: int, shared, delta, work=None, n_real=None,
                        h=None, shared_gate=None) -> None:

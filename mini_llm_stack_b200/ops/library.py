@@ -46,7 +46,7 @@ MODULES = {
     "tanhnorm": ["tanh_norm.cu"],
     "latent": ["latent.cu"],
     "mlstm": ["mlstm.cu"],
-    "experts": ["experts.cu"],
+    "experts": ["experts.cu", "experts_tc.cu"],
     "shortconv": ["short_conv.cu"],
     "scan": ["linear_scan.cu"],
     "headprep": ["head_prep.cu"],

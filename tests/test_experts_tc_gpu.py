@@ -1,0 +1,100 @@
+"""The experts' products on the tensor cores against float64, at the edges of their tiles: rows of
+an expert around 16, 32, 128 and 256, outputs and inputs that fill no tile, experts without rows,
+all rows at one expert, outputs that stand for no expert."""
+
+import pytest
+import torch
+
+from mini_llm_stack_b200.ops.kernels import Runtime
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    o = Runtime("cuda:0", torch.bfloat16).ops
+    o.require_part("experts")
+    return o
+
+
+def routed(ops, idx, weight, experts, n_real):
+    """The arrays of a step in which token t takes the outputs idx[t] (weights for combining)."""
+    t, top = idx.shape
+    n, i32 = t * top, dict(dtype=torch.int32, device="cuda")
+    tiles = ops.expert_max_tiles(n, experts)
+    work = {"idx": torch.empty(n, **i32), "weight": torch.empty(n, device="cuda"),
+            "order": torch.empty(n, **i32), "offsets": torch.empty(experts + 1, **i32),
+            "cursor": torch.empty(experts, **i32), "tile_expert": torch.empty(tiles, **i32),
+            "tile_row0": torch.empty(tiles, **i32), "max_tiles": tiles}
+    logits = torch.full((t, experts), -50.0)
+    logits.scatter_(1, idx, (torch.arange(top, 0, -1).float() + 3.0).expand(t, top))
+    ops.route(logits.cuda(), top, False, work, n_real=n_real)
+    assert torch.equal(work["idx"].cpu().view(t, top).long(), idx)
+    work["weight"].copy_(weight.reshape(-1))
+    return work
+
+
+def choices(t, experts, top, spread, g):
+    if spread == "one":                      # every token's first choice is the same expert
+        idx = torch.stack([torch.randperm(experts - 1, generator=g)[:top] + 1 for _ in range(t)])
+        idx[:, 0] = 0
+        return idx
+    return torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(t)])
+
+
+CASES = [  # tokens, experts, identity outputs, top, d, f, spread
+    (1, 3, 0, 1, 64, 16, "even"), (16, 4, 0, 1, 72, 40, "one"), (17, 4, 1, 2, 136, 128, "one"),
+    (33, 5, 0, 2, 64, 136, "one"), (40, 2, 0, 1, 200, 129, "even"), (129, 3, 0, 2, 64, 96, "one"),
+    (127, 2, 0, 2, 320, 264, "even"), (257, 3, 1, 2, 128, 72, "one"), (600, 4, 0, 1, 64, 130, "even"),
+    (515, 2, 0, 1, 256, 384, "one"), (70, 300, 0, 3, 64, 32, "even")]
+
+
+@pytest.mark.parametrize("t, experts, identity, top, d, f, spread", CASES)
+@pytest.mark.parametrize("unit", ["silu", "clamped", "relu2"])
+def test_products_of_sorted_rows(ops, t, experts, identity, top, d, f, spread, unit):
+    g = torch.Generator().manual_seed(t + experts)
+    outputs = experts + identity
+    idx = choices(t, outputs, top, spread, g)
+    weight = torch.rand(t, top, generator=g) + 0.1
+    work = routed(ops, idx, weight, outputs, experts)
+    h = torch.randn(t, d, generator=g).bfloat16()
+    mats = 1 if unit == "relu2" else 2
+    w1 = (torch.randn(experts, mats * f, d, generator=g) * d ** -0.5).bfloat16()
+    w2 = (torch.randn(experts, d, f, generator=g) * f ** -0.5).bfloat16()
+    n = t * top
+    y = torch.full((n, f), float("nan"), dtype=torch.bfloat16, device="cuda")
+    out = torch.full((n, d), float("nan"), device="cuda")
+    scale_in = unit == "silu"
+    if unit == "relu2":
+        ops.expert_relu_squared(h.cuda(), w1.cuda(), y, work, top, scale_in)
+    else:
+        ops.expert_glu(h.cuda(), w1.cuda(), y, work, top, scale_in, alpha=1.702,
+                       limit=0.5 if unit == "clamped" else 0.0)
+    ops.expert_down(y, w2.cuda(), out, work, top, not scale_in)
+    ops.check_status()
+    order = work["order"].cpu().long()
+    place = torch.empty(n, dtype=torch.long)
+    place[order] = torch.arange(n)
+    y, out = y.cpu(), out.cpu()
+    for tok in range(t):
+        for j in range(top):
+            slot, e = tok * top + j, int(idx[tok, j])
+            if e >= experts:
+                continue
+            a = h[tok].float() * weight[tok, j] if scale_in else h[tok].float()
+            z = w1[e].double() @ a.bfloat16().double()
+            if unit == "relu2":
+                want = z.clamp(min=0) ** 2
+            else:
+                gate, up = z[:f], z[f:]
+                if unit == "clamped":
+                    gate, up = gate.clamp(max=0.5), up.clamp(-0.5, 0.5)
+                    want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+                else:
+                    want = gate * torch.sigmoid(gate) * up
+            row = y[place[slot]].double()
+            # one rounding to 8 bits behind float32 sums of d products
+            assert (row - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 1e-5, (tok, j)
+            down = w2[e].double() @ row * (1.0 if scale_in else float(weight[tok, j]))
+            # float32 sums of f products of unit size
+            assert (out[slot].double() - down).abs().max() <= 1e-5 * max(1.0, float(row.norm())), (tok, j)
