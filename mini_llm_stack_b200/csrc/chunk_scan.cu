@@ -1,0 +1,851 @@
+// Recurrences over a matrix state per head, S <- decay S + k v^T, chunk by chunk for prompts.
+//
+// Token by token the state's chain of updates leaves most of an SM idle (0.16 to 0.9 us a token,
+// whatever the arithmetic).  Within a chunk of 64 tokens that starts from state S0 the outputs are
+//
+//     o_t = (decay from the chunk's start to t) q_t S0 + sum_s P_ts v_s
+//     P_ts = (decay from s to t) q_t . k_s           s <= t
+//     S0'  = (the chunk's decay) S0 + sum_s (decay from s to the chunk's end) k_s v_s^T
+//
+// so that everything but the hand-over of states between chunks is matrix products, for all
+// chunks, heads and requests at once:
+//
+//   scores   P of every chunk and head [64, 64]
+//   update   U = sum_s (..) k_s v_s^T of every chunk and head [e, f]
+//   carry    walks the chunks: leaves each chunk's S0 where its U was, and the last state in the slot
+//   output   [q | P] x [S0; v], a product over e + 64
+//
+// All of it float32 on CUDA cores as in the token-by-token kernels (fma.rn.f32x2; the operands as
+// they are or scaled by factors <= 1, never by the reciprocal of a decay), so that nothing is
+// rounded that was not rounded there; the sums run over s in another order.  Chunks are counted
+// from a request's first token of the step.
+//
+// Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,824 ->
+// 400 us, mLSTM of 4 heads of 256 x 512 1,296 -> 235; 1,501 tokens of wkv, 32 heads of 64 x 64,
+// 306 -> 97 (the products run at 35 to 40 TFLOP/s: a tile's loads are not all hidden by the other
+// blocks' arithmetic, and wkv's weights of pairs take 42 us).
+//
+// A value that is not a number reaches the earlier tokens of its chunk too (0 x NaN), as it does in
+// the prompt attention's tiles; requests never share a chunk.
+//
+// Bound by the FFMA pipe: T H (2 e f + 64 (e + f)) multiply-adds (retention, 2,048 tokens of 32 heads
+// of 128 x 256: 5.9 G, 0.16 ms at 74 TFLOP/s), and the states' way through memory (U written,
+// read and written by carry, read: 134 MB each there).  Chunks of 64 balance the two: half the
+// length doubles the states, twice the length doubles the products within chunks.
+#include "chunk_scan.h"
+#include "common.cuh"
+
+namespace {
+using namespace mls_chunk;
+constexpr int C = CHUNK;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 twice(float a) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ float4 load4(const void* base, int dtype, size_t i) {
+    if (dtype == MLS_BF16) {
+        const uint2 raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)base + i);
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return *reinterpret_cast<const float4*>((const float*)base + i);
+}
+__device__ __forceinline__ float silu1(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float4 times(float4 v, float f) {
+    return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+}
+
+// Where a block's chunk lies.
+struct Where {
+    int r, c;                        // request, chunk of the request
+    int t0, n;                       // first token, tokens
+    int chunks;                      // the request's chunks of this window
+    size_t idx;                      // place among the window's chunks
+};
+
+// Block z of the grid: request z / span, chunk first + z % span.  Every thread calls; false: none.
+__device__ __forceinline__ bool locate(const Args& a, int first, int span, int z, Where& w) {
+    __shared__ int before_s;
+    w.r = z / span;
+    const int j = z - w.r * span;
+    w.c = first + j;
+    if (threadIdx.x < 32) {
+        // chunks of the window in the requests before this one
+        int sum = 0;
+        for (int r = threadIdx.x; r < w.r; r += 32) {
+            const int all = (a.cu_q[r + 1] - a.cu_q[r] + C - 1) / C;
+            sum += min(max(all - first, 0), span);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (threadIdx.x == 0) before_s = sum;
+    }
+    __syncthreads();
+    const int t = a.cu_q[w.r], len = a.cu_q[w.r + 1] - t;
+    w.chunks = min(max((len + C - 1) / C - first, 0), span);
+    w.idx = (size_t)before_s + j;
+    w.t0 = t + w.c * C;
+    w.n = min(C, len - w.c * C);
+    return j < w.chunks;
+}
+
+// ------------------------------------------------------------------ tiles in shared memory
+// 64 rows of K-contiguous values become T[k][row ^ 4 (k / 4 % 8)]: neither the stores (four rows,
+// eight quads of k a warp) nor the reads of four rows at a time meet a bank twice.
+__device__ __forceinline__ int turn(int k) { return 4 * ((k >> 2) & 7); }
+
+template <int THREADS, typename Get>
+__device__ __forceinline__ void fill_transposed(float (*T)[C], Get get) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 8
+    for (int u = threadIdx.x >> 5; u < 32; u += THREADS / 32) {
+        const int r = 4 * (u & 15) + (lane & 3), q = (lane >> 2) + 8 * (u >> 4);
+        const float4 v = get(r, 4 * q);
+        const int col = r ^ (4 * (q & 7));
+        T[4 * q][col] = v.x;
+        T[4 * q + 1][col] = v.y;
+        T[4 * q + 2][col] = v.z;
+        T[4 * q + 3][col] = v.w;
+    }
+}
+// 64 rows (of k) of W values, as they are.
+template <int THREADS, int W, typename Get>
+__device__ __forceinline__ void fill_rows(float (*T)[W], Get get) {
+#pragma unroll 8
+    for (int u = threadIdx.x; u < C * (W / 4); u += THREADS) {
+        const int k = u / (W / 4), x = 4 * (u % (W / 4));
+        *reinterpret_cast<float4*>(&T[k][x]) = get(k, x);
+    }
+}
+
+// acc += A x B over 64 of k: thread (ty, tx) owns rows 4 ty .. + 3 and 32 further on, columns
+// 4 tx .. + 3 and BN / 2 further on.
+template <int BN, bool TURN_A, bool TURN_B>
+__device__ __forceinline__ void multiply(f32x2 (&acc)[8][4], const float (*A)[C], const float (*B)[BN],
+                                         int tx, int ty) {
+#pragma unroll 8
+    for (int k = 0; k < C; ++k) {
+        const int ra = TURN_A ? (4 * ty) ^ turn(k) : 4 * ty;
+        const int cb = TURN_B ? (4 * tx) ^ turn(k) : 4 * tx;
+        float v[8];
+        *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(&A[k][ra]);
+        *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<const float4*>(&A[k][ra + 32]);
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&B[k][cb]);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&B[k][cb + BN / 2]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const f32x2 two = twice(v[i]);
+            fma2(acc[i][0], two, b0.x);
+            fma2(acc[i][1], two, b0.y);
+            fma2(acc[i][2], two, b1.x);
+            fma2(acc[i][3], two, b1.y);
+        }
+    }
+}
+// Sums of several blocks of 64 are kept apart from the block being multiplied: chains of 64
+// roundings and one a block, not one chain of e + 64.
+template <int N>
+__device__ __forceinline__ void settle(f32x2 (&sum)[N], f32x2 (&acc)[N]) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[j]) : "l"(acc[j]));
+        acc[j] = 0ull;
+    }
+}
+__device__ __forceinline__ void clear(f32x2 (&acc)[8][4]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+}
+
+// Four entries of operand row t (zeros past the chunk and past the head's size).
+struct Reader {
+    const void* base;
+    size_t row, at;                  // elements between tokens; the head's first entry
+    int dtype, silu, n, size;
+    __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head)
+        : base(r.base), row(r.row), at((size_t)w.t0 * r.row + r.off + (size_t)head * r.width),
+          dtype(r.dtype), silu(silu_), n(w.n), size(r.width) {}
+    __device__ __forceinline__ float4 operator()(int t, int i) const {
+        if (t >= n || i >= size) return make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v = load4(base, dtype, at + (size_t)t * row + i);
+        if (silu) v = make_float4(silu1(v.x), silu1(v.y), silu1(v.z), silu1(v.w));
+        return v;
+    }
+};
+
+// What scores and gates leave for the products: a factor of q and of k for every token and head
+// (HEAD_DECAY works them out itself), and the chunk's decay.
+struct Scratch {
+    float* states;                   // [chunks, H, e f (+ e)]
+    float* scores;                   // [chunks, H, 64, 64]
+    float* rows_q;                   // TOKEN_DECAY: [T, H e]; MLSTM: factors [T, H]
+    float* rows_k;
+    float* whole;                    // TOKEN_DECAY: [chunks, H, e]; MLSTM: [chunks, H]
+    double* log_gates;               // MLSTM: [T, H, 2]
+};
+__host__ __device__ inline int state_floats(int mode, int e, int f) {
+    return e * f + (mode == MLSTM ? e : 0);
+}
+
+// ------------------------------------------------------------------------------- scores
+// 4 x 4 scores a thread (the tile is small: warps count); the warps whose rows all lie before
+// their columns have nothing to multiply.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+chunk_scores_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    Where w;
+    const int head = blockIdx.y;
+    if (!locate(a, first, span, blockIdx.z, w)) return;
+    __shared__ __align__(16) float A[C][C], B[C][C];
+    __shared__ float power[C];
+    __shared__ double la[C], lb[C];
+    if (threadIdx.x < C) {
+        if (MODE == HEAD_DECAY) power[threadIdx.x] = powf(a.decay[head], (float)threadIdx.x);
+        if (MODE == MLSTM && threadIdx.x < w.n) {
+            const double* lg = s.log_gates + ((size_t)(w.t0 + threadIdx.x) * a.n_heads + head) * 2;
+            la[threadIdx.x] = lg[0];
+            lb[threadIdx.x] = lg[1];
+        }
+    }
+    const Reader q(a.q, a.silu, w, head), k(a.k, a.silu, w, head);
+    // warps of 16 rows x 32 columns, threads of 4 x 4
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = (warp >> 1) * 16 + (lane >> 3) * 4, c0 = (warp & 1) * 32 + (lane & 7) * 4;
+    const bool idle = (warp >> 1) * 16 + 15 < (warp & 1) * 32;
+    f32x2 acc[4][2], sum[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = sum[i][0] = sum[i][1] = 0ull;
+    for (int i0 = 0; i0 < a.e; i0 += C) {
+        __syncthreads();
+        fill_transposed<256>(A, [&](int r, int i) { return q(r, i0 + i); });
+        fill_transposed<256>(B, [&](int r, int i) { return k(r, i0 + i); });
+        __syncthreads();
+        if (idle) continue;
+#pragma unroll 16
+        for (int x = 0; x < C; ++x) {
+            const float4 v = *reinterpret_cast<const float4*>(&A[x][r0 ^ turn(x)]);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&B[x][c0 ^ turn(x)]);
+            const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const f32x2 two = twice(vs[i]);
+                fma2(acc[i][0], two, b.x);
+                fma2(acc[i][1], two, b.y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) settle(sum[i], acc[i]);
+    }
+    float* P = s.scores + (w.idx * a.n_heads + head) * C * C;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = r0 + i;
+        const float2 lo = halves(sum[i][0]), hi = halves(sum[i][1]);
+        float v[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int j = c0 + x;
+            if (j > t || t >= w.n) v[x] = 0.f;
+            else if (MODE == HEAD_DECAY) v[x] *= power[t - j];
+            else v[x] *= a.q_scale * expf((float)(la[t] + lb[j]));
+        }
+        *reinterpret_cast<float4*>(&P[t * C + c0]) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// A decay per token and channel.  The 64 tokens are four runs of 16, a run four steps of 4.  Inside
+// a step the decays between two tokens are multiplied one by one; between steps of a run, and
+// between runs, the weight of a pair is the product of the decays from its step's (run's) start
+// to t, over whole steps (runs) between, and from s to its step's (run's) end, each at most 1: a
+// thread takes a pair, no decay is ever divided by.
+constexpr int RUN = 16, RUNS = C / RUN, STEP = 4, STEPS = C / STEP;
+__device__ __forceinline__ float4 mul4(float4 x, float4 y) {
+    return make_float4(x.x * y.x, x.y * y.y, x.z * y.z, x.w * y.w);
+}
+__device__ __forceinline__ float dot4(float4 x, float4 y, float v) {
+    v = fmaf(x.x, y.x, v);
+    v = fmaf(x.y, y.y, v);
+    v = fmaf(x.z, y.z, v);
+    return fmaf(x.w, y.w, v);
+}
+// Weights of four queries (from row t) and two keys (from row j) whose factors carry the decays up
+// to the gap between them; `gap`: rows of decays between (gaps of them, e apart).
+__device__ __forceinline__ void pairs_4x2(const float* r, const float* k, int pad, const float* gap, int gaps,
+                                          int e, float (&v)[4][2]) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) v[x][0] = v[x][1] = 0.f;
+#pragma unroll 2
+    for (int i = 0; i < e; i += 4) {
+        float4 y0 = *reinterpret_cast<const float4*>(k + i);
+        float4 y1 = *reinterpret_cast<const float4*>(k + pad + i);
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+            if (g < gaps) {
+                const float4 d = *reinterpret_cast<const float4*>(gap + g * e + i);
+                y0 = mul4(y0, d);
+                y1 = mul4(y1, d);
+            }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const float4 q = *reinterpret_cast<const float4*>(r + x * pad + i);
+            v[x][0] = dot4(q, y0, v[x][0]);
+            v[x][1] = dot4(q, y1, v[x][1]);
+        }
+    }
+}
+
+// QUADS: e / 4 where it is known (heads of 64), else 0.
+template <int QUADS>
+__global__ void __launch_bounds__(256)
+chunk_scores_token_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    Where w;
+    const int quads = QUADS ? QUADS : a.e / 4, e = 4 * quads, pad = e + 4;
+    const int head = blockIdx.y;
+    if (!locate(a, first, span, blockIdx.z, w)) return;
+    extern __shared__ __align__(16) float sm[];
+    float* r_s = sm;                                     // [64][pad]
+    float* k_s = r_s + C * pad;                          // [64][pad]
+    float* w_s = k_s + C * pad;                          // [64][pad]
+    float* step_s = w_s + C * pad;                       // [STEPS][e]: a step's decay
+    float* run_s = step_s + STEPS * e;                   // [RUNS][e]: a run's
+    float* bonus_s = run_s + RUNS * e;                   // [e]
+    const int tid = threadIdx.x;
+    const Reader q(a.q, a.silu, w, head), k(a.k, a.silu, w, head);
+    float* P = s.scores + (w.idx * a.n_heads + head) * C * C;
+#pragma unroll 4
+    for (int u = tid; u < C * quads; u += 256) {
+        const int t = u / quads, i = 4 * (u - t * quads);
+        float4 d = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (t < w.n)
+            d = *reinterpret_cast<const float4*>(a.decay + ((size_t)(w.t0 + t) * a.n_heads + head) * e + i);
+        *reinterpret_cast<float4*>(r_s + t * pad + i) = q(t, i);
+        *reinterpret_cast<float4*>(k_s + t * pad + i) = k(t, i);
+        *reinterpret_cast<float4*>(w_s + t * pad + i) = d;
+    }
+    for (int i = tid; i < e; i += 256)
+        bonus_s[i] = a.bonus ? load_as_float(a.bonus, (size_t)head * e + i, a.bonus_dtype) : 0.f;
+    for (int u = tid; u < C * C / 4; u += 256)           // keys of later steps
+        if (u % (C / 4) > u / (C / 4) / STEP) reinterpret_cast<float4*>(P)[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    auto at4 = [&](const float* base, int t, int i) {
+        return *reinterpret_cast<const float4*>(base + t * pad + i);
+    };
+    // inside the steps: thread (t, s of the same step)
+    {
+        const int t = tid >> 2, j = (t & ~3) + (tid & 3), gap = t - j - 1;
+        float v = 0.f;
+        if (j <= t) {
+#pragma unroll 2
+            for (int i = 0; i < e; i += 4) {
+                float4 y = at4(k_s, j, i);
+                if (j == t) y = mul4(y, *reinterpret_cast<const float4*>(bonus_s + i));
+                if (gap > 0) y = mul4(y, at4(w_s, j + 1, i));
+                if (gap > 1) y = mul4(y, at4(w_s, j + 2, i));
+                v = dot4(at4(r_s, t, i), y, v);
+            }
+        }
+        P[t * C + j] = v;
+    }
+    __syncthreads();
+    // q from its step's start on, k up to its step's end
+    for (int u = tid; u < STEPS * quads; u += 256) {
+        const int g = u / quads, i = 4 * (u - g * quads), t = g * STEP;
+        const float4 w0 = at4(w_s, t, i), w1 = at4(w_s, t + 1, i), w2 = at4(w_s, t + 2, i),
+                     w3 = at4(w_s, t + 3, i);
+        const float4 w01 = mul4(w0, w1), w23 = mul4(w2, w3);
+        auto scale = [&](float* base, int x, float4 f) {
+            float4* p = reinterpret_cast<float4*>(base + x * pad + i);
+            *p = mul4(*p, f);
+        };
+        scale(r_s, t + 1, w0);
+        scale(r_s, t + 2, w01);
+        scale(r_s, t + 3, mul4(w01, w2));
+        scale(k_s, t + 2, w3);
+        scale(k_s, t + 1, w23);
+        scale(k_s, t, mul4(w1, w23));
+        *reinterpret_cast<float4*>(step_s + g * e + i) = mul4(w01, w23);
+    }
+    __syncthreads();
+    // between the steps of a run: a thread takes a step's four queries and two keys before them
+    if (tid < RUNS * 12) {
+        const int run = tid / 12, x = tid % 12;          // steps 1, 2, 3 have 2, 4, 6 pairs of keys
+        const int ga = x < 2 ? 1 : (x < 6 ? 2 : 3), pair = x - (ga == 1 ? 0 : (ga == 2 ? 2 : 6));
+        const int t = run * RUN + ga * STEP, j = run * RUN + 2 * pair, gb = pair / 2;
+        float v[4][2];
+        pairs_4x2(r_s + t * pad, k_s + j * pad, pad, step_s + (run * (RUN / STEP) + gb + 1) * e,
+                  ga - gb - 1, e, v);
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+            *reinterpret_cast<float2*>(P + (t + y) * C + j) = make_float2(v[y][0], v[y][1]);
+    }
+    __syncthreads();
+    // q from its run's start on, k up to its run's end
+    for (int u = tid; u < C * quads; u += 256) {
+        const int t = u / quads, i = 4 * (u - t * quads), g = t / STEP, g0 = g & ~(RUN / STEP - 1);
+        float4 x = at4(r_s, t, i), y = at4(k_s, t, i);
+#pragma unroll
+        for (int h = 0; h < RUN / STEP; ++h) {
+            const float4 d = *reinterpret_cast<const float4*>(step_s + (g0 + h) * e + i);
+            if (g0 + h < g) x = mul4(x, d);
+            if (g0 + h > g) y = mul4(y, d);
+        }
+        *reinterpret_cast<float4*>(r_s + t * pad + i) = x;
+        *reinterpret_cast<float4*>(k_s + t * pad + i) = y;
+    }
+    for (int u = tid; u < RUNS * quads; u += 256) {
+        const int g = u / quads, i = 4 * (u - g * quads);
+        const float4* p = reinterpret_cast<const float4*>(step_s + g * (RUN / STEP) * e + i);
+        *reinterpret_cast<float4*>(run_s + g * e + i) =
+            mul4(mul4(p[0], p[quads]), mul4(p[2 * quads], p[3 * quads]));
+    }
+    __syncthreads();
+    // between runs: a warp takes a pair of them (six), a thread four queries and two keys
+    if (tid < 6 * 32) {
+        const int x = tid >> 5, lane = tid & 31;
+        const int ga = x == 0 ? 1 : (x < 3 ? 2 : 3), gb = x == 0 ? 0 : (x < 3 ? x - 1 : x - 3);
+        const int t = ga * RUN + 4 * (lane >> 3), j = gb * RUN + 2 * (lane & 7);
+        float v[4][2];
+        pairs_4x2(r_s + t * pad, k_s + j * pad, pad, run_s + (gb + 1) * e, ga - gb - 1, e, v);
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+            *reinterpret_cast<float2*>(P + (t + y) * C + j) = make_float2(v[y][0], v[y][1]);
+    }
+    // q from the chunk's start on, k up to the chunk's end, the whole chunk
+#pragma unroll 2
+    for (int u = tid; u < w.n * quads; u += 256) {
+        const int t = u / quads, i = 4 * (u - t * quads), g = t / RUN;
+        float4 x = at4(r_s, t, i), y = at4(k_s, t, i);
+#pragma unroll
+        for (int h = 0; h < RUNS; ++h) {
+            const float4 d = *reinterpret_cast<const float4*>(run_s + h * e + i);
+            if (h < g) x = mul4(x, d);
+            if (h > g) y = mul4(y, d);
+        }
+        const size_t at = ((size_t)(w.t0 + t) * a.n_heads + head) * e + i;
+        *reinterpret_cast<float4*>(s.rows_q + at) = x;
+        *reinterpret_cast<float4*>(s.rows_k + at) = y;
+    }
+    for (int u = tid; u < quads; u += 256) {
+        const float4* p = reinterpret_cast<const float4*>(run_s + 4 * u);
+        *reinterpret_cast<float4*>(s.whole + (w.idx * a.n_heads + head) * e + 4 * u) =
+            mul4(mul4(p[0], p[quads]), mul4(p[2 * quads], p[3 * quads]));
+    }
+}
+
+// mLSTM's gates, a block a head and request, a warp a chunk, two neighbouring tokens a lane.  With F
+// the sums of the log forget gates since the chunk's start (float64, so that differences of long
+// sums lose nothing) the stabiliser m <- max(f + m, i) is F_t + max(m_0, max over s <= t of
+// (i_s - F_s)): a chunk takes two scans over the lanes, and from chunk to chunk goes one number.
+// What follows from it:
+//   factor of q:  exp(F_t + m_0 - m_t) e^-1/2      factor of k:  exp(F_n - F_t + i_t - m_n)
+//   of a pair:    exp((F_t - m_t) + (i_s - F_s))   of the state: exp(F_n + m_0 - m_n)
+constexpr int GATE_WARPS = 16;
+__global__ void __launch_bounds__(32 * GATE_WARPS)
+chunk_gates_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    __shared__ double whole_s[GATE_WARPS], top_s[GATE_WARPS];
+    __shared__ float m_s[GATE_WARPS + 1];
+    const int head = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Where w;
+    if (!locate(a, first, span, blockIdx.y * span, w)) return;
+    float* m_slot = a.state + (size_t)a.state_slot[w.r] * a.slot_stride + (size_t)head * a.head_stride +
+                    state_floats(MLSTM, a.e, a.f);
+    const float bi = load_as_float(a.bias_i, head, a.bias_dtype),
+                bf = load_as_float(a.bias_f, head, a.bias_dtype);
+    const int t_end = a.cu_q[w.r + 1];
+    if (threadIdx.x == 0) m_s[GATE_WARPS] = m_slot[0];
+    for (int c0 = 0; c0 < w.chunks; c0 += GATE_WARPS) {
+        const int c = c0 + warp, t0 = w.t0 + c * C, n = min(C, t_end - t0);
+        double ig[2], F[2], top[2], earlier = -INFINITY;
+        if (c < w.chunks) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                // past the chunk's end: nothing is forgotten, nothing enters
+                const bool there = 2 * lane + x < n;
+                const float* g = a.gates + (size_t)(t0 + min(2 * lane + x, n - 1)) * 2 * a.n_heads;
+                const float z = a.cap * tanhf((g[a.n_heads + head] + bf) / a.cap);
+                F[x] = there ? fminf(z, 0.f) - log1pf(expf(-fabsf(z))) : 0.f;
+                ig[x] = there ? a.cap * tanhf((g[head] + bi) / a.cap) : -INFINITY;
+            }
+            F[1] += F[0];
+            double sum = F[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double x = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += x;
+            }
+            F[0] += sum - F[1];
+            F[1] = sum;
+            top[0] = ig[0] - F[0];
+            top[1] = fmax(top[0], ig[1] - F[1]);
+            double most = top[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double x = __shfl_up_sync(0xffffffffu, most, o);
+                if (lane >= o) most = fmax(most, x);
+            }
+            const double before = __shfl_up_sync(0xffffffffu, most, 1);
+            if (lane) earlier = before;
+            if (lane == 31) {
+                whole_s[warp] = F[1];
+                top_s[warp] = most;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            // m_s[x]: the stabiliser before the chunk of warp x; the last one: behind them all
+            float m = m_s[GATE_WARPS];
+            for (int x = 0; x < GATE_WARPS && c0 + x < w.chunks; ++x) {
+                m_s[x] = m;
+                m = (float)(whole_s[x] + fmax((double)m, top_s[x]));
+                if (x + 1 < GATE_WARPS) m_s[x + 1] = m;
+            }
+            m_s[GATE_WARPS] = m;
+        }
+        __syncthreads();
+        if (c < w.chunks) {
+            const float m0 = m_s[warp];
+            const float m_end = warp + 1 < GATE_WARPS ? m_s[warp + 1] : m_s[GATE_WARPS];
+            const double whole = whole_s[warp];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int j = 2 * lane + x;
+                if (j >= n) continue;
+                const float m = (float)(F[x] + fmax((double)m0, fmax(earlier, top[x])));
+                const size_t at = (size_t)(t0 + j) * a.n_heads + head;
+                s.log_gates[2 * at] = F[x] - m;
+                s.log_gates[2 * at + 1] = ig[x] - F[x];
+                s.rows_q[at] = a.q_scale * expf((float)(F[x] + m0 - m));
+                s.rows_k[at] = expf((float)(whole - F[x] + ig[x] - m_end));
+                a.den[at] = expf(-m);                    // the output kernel adds n . q to it
+            }
+            if (lane == 0) s.whole[(w.idx + c) * a.n_heads + head] = expf((float)(whole + m0 - m_end));
+        }
+        __syncthreads();
+    }
+    for (int g = threadIdx.x; g < a.n_groups; g += blockDim.x) m_slot[g] = m_s[GATE_WARPS];
+}
+
+// Factors of the tokens' rows of q and k in this chunk.
+template <int MODE>
+__device__ __forceinline__ float row_factor(const Args& a, const float* factors, const Where& w, int head,
+                                            int t, int power) {
+    if (t >= w.n) return 0.f;
+    if (MODE == HEAD_DECAY) return powf(a.decay[head], (float)power);
+    if (MODE == MLSTM) return factors[(size_t)(w.t0 + t) * a.n_heads + head];
+    return 1.f;
+}
+
+// ------------------------------------------------------------------------------- update
+// U[i, j] = sum_s factor_s k_s[i] v_s[j]; MLSTM: and n[i] = sum_s factor_s k_s[i].
+template <int MODE, int BN>
+__global__ void __launch_bounds__(BN, BN == 128 ? 4 : 6)
+chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    Where w;
+    const int head = blockIdx.y;
+    if (!locate(a, first, span, blockIdx.z, w)) return;
+    extern __shared__ __align__(16) float tiles[];
+    float(*A)[C] = reinterpret_cast<float(*)[C]>(tiles);
+    float(*B)[BN] = reinterpret_cast<float(*)[BN]>(tiles + C * C);
+    __shared__ float factor[C];
+    const int f_tiles = (a.f + BN - 1) / BN;
+    const int i0 = (blockIdx.x / f_tiles) * C, j0 = (blockIdx.x % f_tiles) * BN;
+    if (threadIdx.x < C)
+        factor[threadIdx.x] = row_factor<MODE>(a, s.rows_k, w, head, threadIdx.x, w.n - 1 - (int)threadIdx.x);
+    __syncthreads();
+    Rows kr = a.k;
+    if (MODE == TOKEN_DECAY) kr = Rows{s.rows_k, MLS_F32, a.n_heads * a.e, 0, a.e};
+    const Reader k(kr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head), v(a.v, a.silu, w, head);
+    fill_rows<BN, C>(A, [&](int t, int i) { return times(k(t, i0 + i), factor[t]); });
+    fill_rows<BN, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
+    __syncthreads();
+    const int tx = threadIdx.x % (BN / 8), ty = threadIdx.x / (BN / 8);
+    f32x2 acc[8][4];
+    clear(acc);
+    multiply<BN, false, false>(acc, A, B, tx, ty);
+    float* U = s.states + (w.idx * a.n_heads + head) * state_floats(MODE, a.e, a.f);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const int i = i0 + 4 * ty + (x & 3) + 32 * (x >> 2);
+        if (i >= a.e) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = j0 + 4 * tx + (BN / 2) * h;
+            const float2 lo = halves(acc[x][2 * h]), hi = halves(acc[x][2 * h + 1]);
+            if (j < a.f)
+                *reinterpret_cast<float4*>(U + (size_t)i * a.f + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    }
+    if (MODE == MLSTM && j0 == 0 && threadIdx.x < C && i0 + threadIdx.x < a.e) {
+        float n = 0.f;
+#pragma unroll 16
+        for (int t = 0; t < C; ++t) n += A[t][threadIdx.x];
+        U[(size_t)a.e * a.f + i0 + threadIdx.x] = n;
+    }
+}
+
+// -------------------------------------------------------------------------------- carry
+// Four neighbouring entries of a head's state a thread, chunk after chunk; the loads of four
+// chunks are under way together.
+template <int MODE>
+__global__ void __launch_bounds__(128)
+chunk_carry_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    Where w;
+    const int head = blockIdx.y;
+    if (!locate(a, first, span, blockIdx.z * span, w)) return;
+    const int size = state_floats(MODE, a.e, a.f);
+    const int at = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (at >= size) return;
+    float4* slot = reinterpret_cast<float4*>(a.state + (size_t)a.state_slot[w.r] * a.slot_stride +
+                                             (size_t)head * a.head_stride + at);
+    const size_t step = (size_t)a.n_heads * size;
+    float* U = s.states + (w.idx * a.n_heads + head) * size + at;
+    const int len = a.cu_q[w.r + 1] - a.cu_q[w.r];
+    const float g = MODE == HEAD_DECAY ? a.decay[head] : 0.f;
+    const float g_whole = MODE == HEAD_DECAY ? powf(g, (float)C) : 0.f;
+    float4 st = *slot;
+    constexpr int AHEAD = 4;
+    for (int c0 = 0; c0 < w.chunks; c0 += AHEAD) {
+        float4 u[AHEAD];
+        float d[AHEAD];
+#pragma unroll
+        for (int x = 0; x < AHEAD; ++x) {
+            const int c = c0 + x;
+            if (c >= w.chunks) continue;
+            u[x] = *reinterpret_cast<const float4*>(U + c * step);
+            if (MODE == HEAD_DECAY) {
+                const int n = len - (w.c + c) * C;
+                d[x] = n >= C ? g_whole : powf(g, (float)n);
+            } else if (MODE == MLSTM) {
+                d[x] = s.whole[(w.idx + c) * a.n_heads + head];
+            } else {
+                d[x] = s.whole[((w.idx + c) * a.n_heads + head) * a.e + at / a.f];   // f % 4 == 0
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < AHEAD; ++x) {
+            const int c = c0 + x;
+            if (c >= w.chunks) continue;
+            *reinterpret_cast<float4*>(U + c * step) = st;
+            st = make_float4(fmaf(d[x], st.x, u[x].x), fmaf(d[x], st.y, u[x].y),
+                             fmaf(d[x], st.z, u[x].z), fmaf(d[x], st.w, u[x].w));
+        }
+    }
+    *slot = st;
+}
+
+// ------------------------------------------------------------------------------- output
+// o = [factor q | P] x [S0; v]; MLSTM: and den_t = max(|[factor q | P] x [n; 1]|, exp(-m_t)) + 1e-6.
+template <int MODE, int BN>
+__global__ void __launch_bounds__(BN, BN == 128 ? 3 : 5)
+chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
+    chain_release();
+    chain_wait();
+    Where w;
+    const int head = blockIdx.y, j0 = blockIdx.x * BN;
+    if (!locate(a, first, span, blockIdx.z, w)) return;
+    extern __shared__ __align__(16) float tiles[];
+    float(*A)[C] = reinterpret_cast<float(*)[C]>(tiles);
+    float(*B)[BN] = reinterpret_cast<float(*)[BN]>(tiles + C * C);
+    __shared__ float factor[C], n_s[C];
+    if (threadIdx.x < C)
+        factor[threadIdx.x] = row_factor<MODE>(a, s.rows_q, w, head, threadIdx.x, threadIdx.x + 1);
+    Rows qr = a.q;
+    if (MODE == TOKEN_DECAY) qr = Rows{s.rows_q, MLS_F32, a.n_heads * a.e, 0, a.e};
+    const Reader q(qr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head), v(a.v, a.silu, w, head);
+    const size_t unit = w.idx * a.n_heads + head;
+    const float* S = s.states + unit * state_floats(MODE, a.e, a.f);
+    const float* P = s.scores + unit * C * C;
+    const int tx = threadIdx.x % (BN / 8), ty = threadIdx.x / (BN / 8);
+    const bool with_n = MODE == MLSTM && j0 == 0;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    f32x2 acc[8][4], sum[8][4];
+    clear(acc);
+    clear(sum);
+    float nq[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // short chains: the sum may nearly vanish
+    for (int i0 = 0; i0 < a.e + C; i0 += C) {            // the last block is [P] x [v]
+        const bool inner = i0 >= a.e;
+        __syncthreads();
+        if (inner) {
+            fill_transposed<BN>(A, [&](int t, int x) {
+                return *reinterpret_cast<const float4*>(P + t * C + x);
+            });
+            fill_rows<BN, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
+        } else {
+            fill_transposed<BN>(A, [&](int t, int x) { return times(q(t, i0 + x), factor[t]); });
+            fill_rows<BN, BN>(B, [&](int i, int j) {
+                return (i0 + i < a.e && j0 + j < a.f)
+                           ? *reinterpret_cast<const float4*>(S + (size_t)(i0 + i) * a.f + j0 + j) : zero;
+            });
+        }
+        if (with_n && threadIdx.x < C)
+            n_s[threadIdx.x] = inner ? 1.f
+                : (i0 + (int)threadIdx.x < a.e ? S[(size_t)a.e * a.f + i0 + threadIdx.x] : 0.f);
+        __syncthreads();
+        multiply<BN, true, false>(acc, A, B, tx, ty);
+#pragma unroll
+        for (int x = 0; x < 8; ++x) settle(sum[x], acc[x]);
+        if (with_n && threadIdx.x < C) {
+#pragma unroll 8
+            for (int x = 0; x < C; ++x) nq[x & 7] = fmaf(A[x][threadIdx.x ^ turn(x)], n_s[x], nq[x & 7]);
+        }
+        if (inner) break;
+    }
+    if (with_n && threadIdx.x < w.n) {
+        float* den = a.den + (size_t)(w.t0 + threadIdx.x) * a.n_heads + head;
+        const float all = ((nq[0] + nq[4]) + (nq[2] + nq[6])) + ((nq[1] + nq[5]) + (nq[3] + nq[7]));
+        *den = fmaxf(fabsf(all), *den) + 1e-6f;
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const int t = 4 * ty + (x & 3) + 32 * (x >> 2);
+        if (t >= w.n) continue;
+        float* dst = a.out + ((size_t)(w.t0 + t) * a.n_heads + head) * a.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = j0 + 4 * tx + (BN / 2) * h;
+            const float2 lo = halves(sum[x][2 * h]), hi = halves(sum[x][2 * h + 1]);
+            if (j < a.f) *reinterpret_cast<float4*>(dst + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    }
+}
+
+template <int MODE, int BN>
+int products(const Args& a, const Scratch& s, int first, int span, bool update, cudaStream_t stream) {
+    const int smem = C * (C + BN) * (int)sizeof(float);
+    static bool configured = false;                      // (with the static arrays over 48 KB at 128)
+    if (!configured) {
+        int rc = (int)cudaFuncSetAttribute(chunk_update_kernel<MODE, BN>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (!rc)
+            rc = (int)cudaFuncSetAttribute(chunk_output_kernel<MODE, BN>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (rc) return rc;
+        configured = true;
+    }
+    const dim3 grid(update ? ((a.e + C - 1) / C) * ((a.f + BN - 1) / BN) : (a.f + BN - 1) / BN, a.n_heads,
+                    a.n_requests * span);
+    if (update)
+        MLS_LAUNCH((chunk_update_kernel<MODE, BN>), grid, dim3(BN), smem, stream, a, s, first, span);
+    else
+        MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(BN), smem, stream, a, s, first, span);
+    return launch_status();
+}
+
+size_t token_smem(int e) {
+    return (size_t)(3 * C * (e + 4) + (STEPS + RUNS + 1) * e) * sizeof(float);
+}
+
+template <int MODE>
+int window(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
+    if (MODE == TOKEN_DECAY) {
+        const size_t smem = token_smem(a.e);
+        auto kernel = a.e == 64 ? chunk_scores_token_kernel<16> : chunk_scores_token_kernel<0>;
+        const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (rc) return rc;
+        MLS_LAUNCH(kernel, dim3(1, a.n_heads, a.n_requests * span), dim3(256), smem,
+                   stream, a, s, first, span);
+    } else {
+        if (MODE == MLSTM)
+            MLS_LAUNCH((chunk_gates_kernel), dim3(a.n_heads, a.n_requests), dim3(32 * GATE_WARPS), 0,
+                       stream, a, s, first, span);
+        MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, a.n_requests * span), dim3(256), 0,
+                   stream, a, s, first, span);
+    }
+    // tiles of 64 x 128 where the values fill them, else of 64 x 64
+    const bool wide = a.f % 128 == 0 || a.f > 192;
+    int rc = wide ? products<MODE, 128>(a, s, first, span, true, stream)
+                  : products<MODE, 64>(a, s, first, span, true, stream);
+    if (rc) return rc;
+    const int quads = state_floats(MODE, a.e, a.f) / 4;
+    MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, a.n_requests), dim3(128),
+               0, stream, a, s, first, span);
+    rc = launch_status();
+    if (rc) return rc;
+    return wide ? products<MODE, 128>(a, s, first, span, false, stream)
+                : products<MODE, 64>(a, s, first, span, false, stream);
+}
+}  // namespace
+
+namespace mls_chunk {
+bool fits(const Args& a) {
+    auto rows_fit = [](const Rows& r) {
+        const size_t bytes = r.dtype == MLS_BF16 ? 8 : 16;
+        return ((r.row | r.off | r.width) & 3) == 0 && reinterpret_cast<uintptr_t>(r.base) % bytes == 0;
+    };
+    if (!rows_fit(a.q) || !rows_fit(a.k) || !rows_fit(a.v) || (a.slot_stride & 3) || (a.head_stride & 3) ||
+        reinterpret_cast<uintptr_t>(a.state) % 16 || reinterpret_cast<uintptr_t>(a.out) % 16)
+        return false;
+    if (a.mode == TOKEN_DECAY && (a.e > 128 || reinterpret_cast<uintptr_t>(a.decay) % 16)) return false;
+    return a.n_heads <= 65535;
+}
+
+// (the float64 logarithms first, then sizes that are multiples of four floats)
+long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long long chunks) {
+    const long long units = chunks * n_heads, tokens = (long long)n_tokens * n_heads;
+    long long n = units * (state_floats(mode, e, f) + C * C);
+    if (mode == TOKEN_DECAY) n += 2 * tokens * e + units * e;
+    if (mode == MLSTM) n += 4 * tokens + 2 * ((tokens + 3) / 4 * 4) + (units + 3) / 4 * 4;
+    return n;
+}
+
+int scan(const Args& a, int most, int window_chunks, long long chunks, float* scratch, cudaStream_t stream) {
+    if (a.n_requests <= 0 || most <= 0) return 0;
+    if ((long long)a.n_requests * window_chunks > 65535) return MLS_ERR_UNSUPPORTED;
+    const long long units = chunks * a.n_heads, tokens = (long long)a.n_tokens * a.n_heads;
+    Scratch s{};
+    float* at = scratch;
+    if (a.mode == MLSTM) {
+        s.log_gates = reinterpret_cast<double*>(at);
+        at += 4 * tokens;
+    }
+    s.states = at;
+    at += units * state_floats(a.mode, a.e, a.f);
+    s.scores = at;
+    at += units * C * C;
+    const long long per = a.mode == TOKEN_DECAY ? tokens * a.e : (tokens + 3) / 4 * 4;
+    if (a.mode != HEAD_DECAY) {
+        s.rows_q = at;
+        s.rows_k = at + per;
+        s.whole = at + 2 * per;
+    }
+    for (int first = 0; first < most; first += window_chunks) {
+        const int span = most - first < window_chunks ? most - first : window_chunks;
+        int rc;
+        if (a.mode == HEAD_DECAY) rc = window<HEAD_DECAY>(a, s, first, span, stream);
+        else if (a.mode == TOKEN_DECAY) rc = window<TOKEN_DECAY>(a, s, first, span, stream);
+        else rc = window<MLSTM>(a, s, first, span, stream);
+        if (rc) return rc;
+    }
+    return 0;
+}
+}  // namespace mls_chunk
+
+// Floats of scratch that the chunk-wise scan of a window of so many chunks (of all requests) takes.
+MLS_API long long mls_chunk_scratch_floats(int mode, int n_tokens, int n_heads, int e, int f,
+                                           long long chunks) {
+    return scratch_floats(mode, n_tokens, n_heads, e, f, chunks);
+}

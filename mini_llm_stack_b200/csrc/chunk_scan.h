@@ -1,0 +1,51 @@
+// The chunk-wise form of the recurrences over a matrix state per head (chunk_scan.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace mls_chunk {
+constexpr int CHUNK = 64;            // tokens of a chunk
+
+// Rows of an operand: element (t, head, i) lies at base[t * row + off + head * width + i].
+struct Rows {
+    const void* base;
+    int dtype, row, off, width;
+};
+
+// How the state decays: one constant a head; a decay per token and key channel, the token read
+// before it enters (with a bonus); mLSTM's gates with their stabiliser.
+enum { HEAD_DECAY = 0, TOKEN_DECAY = 1, MLSTM = 2 };
+
+struct Args {
+    int mode;
+    Rows q, k, v;
+    int silu;                        // q, k and v pass through z * sigmoid(z) as they are read
+    float q_scale;                   // MLSTM: what q is multiplied by
+    const float* decay;              // HEAD_DECAY: [H]; TOKEN_DECAY: [T, H * e]
+    const void* bonus;               // TOKEN_DECAY: [H * e] or null
+    int bonus_dtype;
+    // MLSTM
+    const float* gates;              // [T, 2H]: input and forget pre-activations
+    const void* bias_i;
+    const void* bias_f;
+    int bias_dtype;
+    float cap;
+    int n_groups;                    // copies of the stabiliser in a head's state
+    float* den;                      // [T, H]
+
+    const int* cu_q;
+    const int* state_slot;
+    float* state;
+    long long slot_stride;           // floats between slots
+    int head_stride;                 // floats between the heads of a slot
+    int n_requests, n_tokens, n_heads, e, f;
+    float* out;                      // [T, H * f]
+};
+
+// Whether the chunk-wise kernels take these operands (alignment, sizes).
+bool fits(const Args& a);
+// Floats of scratch for windows of so many chunks in all.
+long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long long chunks);
+// The scan of `most` chunks at most a request, `window` of them at a time.
+int scan(const Args& a, int most, int window, long long chunks_a_window, float* scratch,
+         cudaStream_t stream);
+}  // namespace mls_chunk

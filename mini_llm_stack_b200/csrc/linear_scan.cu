@@ -28,6 +28,7 @@
 // State, decays, exponentials, angles' cosines and sines, norms and sums are float32 (the
 // angles themselves float64: position * frequency); a, k, v come from the projections, with
 // `act` = 1 through silu (z * sigmoid(z), float32) as they are loaded.
+#include "chunk_scan.h"
 #include "common.cuh"
 
 namespace {
@@ -377,6 +378,48 @@ MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off
     if (rpt <= 16) LS_GO(16);
     LS_GO(32);
 #undef LS_GO
+}
+
+// The same for prompts, chunk by chunk (chunk_scan.cu): a decay per token with the token read first,
+// or one decay a head with the token taken in first and no bonus.  `most`: the most chunks of a
+// request; `window` chunks of every request at a time, `chunks` in all requests together.
+MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, int a_off,
+                                    const void* k_src, int k_dtype, int k_row, int k_off,
+                                    const void* v_src, int v_dtype, int v_row, int v_off,
+                                    const float* decay_tok, const float* decay_head,
+                                    const void* bonus, int bonus_dtype, int read_first,
+                                    const int* cu_q, const int* state_slot, float* state,
+                                    long long state_stride, int n_requests, int n_tokens,
+                                    int n_heads, int e, int f, float* out, int act, int most,
+                                    int window, long long chunks, float* scratch,
+                                    cudaStream_t stream) {
+    using namespace mls_chunk;
+    if (n_requests <= 0) return 0;
+    if (e <= 0 || f <= 0 || (!decay_tok == !decay_head) || (decay_tok && !read_first) ||
+        (decay_head && (read_first || bonus)))
+        return MLS_ERR_UNSUPPORTED;
+    Args a{};
+    a.mode = decay_tok ? TOKEN_DECAY : HEAD_DECAY;
+    a.q = Rows{a_src, a_dtype, a_row, a_off, e};
+    a.k = Rows{k_src, k_dtype, k_row, k_off, e};
+    a.v = Rows{v_src, v_dtype, v_row, v_off, f};
+    a.silu = act;
+    a.decay = decay_tok ? decay_tok : decay_head;
+    a.bonus = bonus;
+    a.bonus_dtype = bonus_dtype;
+    a.cu_q = cu_q;
+    a.state_slot = state_slot;
+    a.state = state;
+    a.slot_stride = state_stride;
+    a.head_stride = e * f;
+    a.n_requests = n_requests;
+    a.n_tokens = n_tokens;
+    a.n_heads = n_heads;
+    a.e = e;
+    a.f = f;
+    a.out = out;
+    if (!fits(a)) return MLS_ERR_UNSUPPORTED;
+    return scan(a, most, window, chunks, scratch, stream);
 }
 
 MLS_API int mls_scan_finish(const float* o, const void* gate, int gate_dtype, int gate_row,

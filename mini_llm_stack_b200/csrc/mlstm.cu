@@ -26,6 +26,7 @@
 // arithmetic, the state and the sums are float32; q, k, v and the gate pre-activations
 // come from the projections.  A token's result depends on the tokens before it only
 // through the state, never on the batch or on how the sequence was cut into steps.
+#include "chunk_scan.h"
 #include "common.cuh"
 
 namespace {
@@ -335,6 +336,47 @@ MLS_API int mls_mlstm_scan(const void* qkvg, int dtype, int row_w, int q_off, in
     return pick_scan<float>(maxr, qkvg, row_w, q_off, k_off, v_off, gates, bias_i, bias_f, b_dtype,
                             cap, cu_q, state_slot, state, slot_stride, n_requests, n_heads, e, f,
                             fc, n_groups, num, den, stream);
+}
+
+// The same for prompts, chunk by chunk (chunk_scan.cu).  `most`: the most chunks of a request;
+// `window` chunks of every request at a time, `chunks` in all requests together.
+MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q_off, int k_off,
+                                   int v_off, const float* gates, const void* bias_i,
+                                   const void* bias_f, int b_dtype, float cap, const int* cu_q,
+                                   const int* state_slot, float* state, long long slot_stride,
+                                   int n_requests, int n_tokens, int n_heads, int e, int f, float* num,
+                                   float* den, int most, int window, long long chunks, float* scratch,
+                                   cudaStream_t stream) {
+    using namespace mls_chunk;
+    if (n_requests <= 0) return 0;
+    if (e <= 0 || f <= 0 || n_heads <= 0) return MLS_ERR_UNSUPPORTED;
+    const int fc = mls_mlstm_columns(e, f);
+    Args a{};
+    a.mode = MLSTM;
+    a.q = Rows{qkvg, dtype, row_w, q_off, e};
+    a.k = Rows{qkvg, dtype, row_w, k_off, e};
+    a.v = Rows{qkvg, dtype, row_w, v_off, f};
+    a.q_scale = 1.0f / sqrtf((float)e);
+    a.gates = gates;
+    a.bias_i = bias_i;
+    a.bias_f = bias_f;
+    a.bias_dtype = b_dtype;
+    a.cap = cap;
+    a.n_groups = (f + fc - 1) / fc;
+    a.den = den;
+    a.cu_q = cu_q;
+    a.state_slot = state_slot;
+    a.state = state;
+    a.slot_stride = slot_stride;
+    a.head_stride = e * f + e + a.n_groups;
+    a.n_requests = n_requests;
+    a.n_tokens = n_tokens;
+    a.n_heads = n_heads;
+    a.e = e;
+    a.f = f;
+    a.out = num;
+    if (!fits(a)) return MLS_ERR_UNSUPPORTED;
+    return scan(a, most, window, chunks, scratch, stream);
 }
 
 MLS_API int mls_mlstm_finish(const float* num, const float* den, const void* gate, int gate_row,

@@ -784,6 +784,11 @@ class Ops:
                    "scan": _decl(lib, "mls_mlstm_scan",
                                  [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
                                   _I, _I, _I, _I, _P, _P, _P]),
+                   "chunked": _decl(lib, "mls_mlstm_scan_chunked",
+                                    [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
+                                     _I, _I, _I, _I, _I, _P, _P, _I, _I, _LL, _P, _P]),
+                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
+                                    restype=ctypes.c_longlong),
                    "finish": _decl(lib, "mls_mlstm_finish",
                                    [_P, _P, _P, _I, _I, _P, _I, _F, _P, _I, _I, _I, _I, _P])}
         elif name == "experts":
@@ -835,6 +840,12 @@ class Ops:
             fns = {"scan": _decl(lib, "mls_linear_scan",
                                  [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _P, _P,
                                   _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _P]),
+                   "chunked": _decl(lib, "mls_linear_scan_chunked",
+                                    [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _P, _P,
+                                     _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _I, _I, _I,
+                                     _LL, _P, _P]),
+                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
+                                    restype=ctypes.c_longlong),
                    "finish_row": _decl(lib, "mls_scan_finish_row",
                                        [_P, _P, _I, _I, _I, _P, _F, _F, _P, _LL, _I, _I, _P]),
                    "finish": _decl(lib, "mls_scan_finish",
@@ -1005,6 +1016,58 @@ class Ops:
             _ptr(src), src.shape[1], src_width, _ptr(w), _ptr(dst), dst.shape[1], dst_width,
             _code(w.dtype), n_tokens, heads, n, k, self._stream()), "headwise_linear")
 
+    CHUNK = 64                    # tokens of a chunk of the chunk-wise scans
+    # Tokens of the longest request from which on a step's scans run chunk by chunk: where the five
+    # short kernels of the one take as long as the other takes token by token (measured at the 1b
+    # and 8b sizes: 40-60 us, 56 tokens of retention, 120 of wkv, 125 of mLSTM); half as many where
+    # the token-by-token kernel runs in several rounds of blocks (four prompts at the 8b sizes: 28,
+    # 45 and 45).
+    CHUNKED_FROM = {"head": 64, "token": 128, "mlstm": 128}
+    CHUNKED_BLOCKS = 1024         # ... blocks of 16 columns of a state
+    # Every chunk's state passes through memory four times, a request's twice token by token: steps
+    # of a prompt among many decoded tokens stay there (64 requests of which one brings 256 tokens,
+    # 8b retention: about 310 us either way).
+    CHUNK_TOKENS = 8              # tokens a chunk holds on average at least
+    CHUNK_SCRATCH = 1 << 27       # floats of scratch that a window of chunks may take
+
+    def _chunk_plan(self, part: str, mode: int, step, operands: list, whole: tuple, strides: tuple,
+                    n_heads: int, e: int, f: int):
+        """How a scan over a matrix state runs chunk by chunk: (the most chunks of a request, chunks
+        of a request a window, chunks of a window in all, scratch), or None: token by token.
+
+        Chunk by chunk is for prompts of bfloat16 models (a float32 model's results do not depend
+        on how a prompt is cut, which chunks counted from a step's first token would change) whose
+        rows can be read four entries at a time.  ``operands``: (tensor, first column, head's size);
+        ``whole``: tensors that are read and written 16 bytes at a time; ``strides``: floats
+        between the states of slots and of heads."""
+        lens = getattr(step, "q_lens", None)
+        if self.act_dtype != torch.bfloat16 or not lens:
+            return None
+        least = self.CHUNKED_FROM[("head", "token", "mlstm")[mode]]
+        if len(lens) * n_heads * -(-f // 16) >= self.CHUNKED_BLOCKS:
+            least //= 2
+        each = [-(-n // self.CHUNK) for n in lens]
+        if max(lens) < least or step.n_tokens < self.CHUNK_TOKENS * sum(each):
+            return None
+        if any((t.shape[1] | off | size) & 3 or t.data_ptr() % (4 * t.element_size())
+               for t, off, size in operands) or any(t.data_ptr() % 16 for t in whole) \
+                or any(s & 3 for s in strides) or n_heads > 65535:
+            return None
+        most = window = max(each)
+        floats_of = self._part_lib(part)["scratch"]
+
+        def size(w):
+            chunks = sum(min(c, w) for c in each)
+            return chunks, floats_of(mode, step.n_tokens, n_heads, e, f, chunks)
+
+        chunks, floats = size(window)
+        while window > 1 and (floats > self.CHUNK_SCRATCH or len(lens) * window > 65535):
+            window = (window + 1) // 2
+            chunks, floats = size(window)
+        if len(lens) * window > 65535:
+            return None
+        return most, window, chunks, self.scratch("chunk_scan", floats)
+
     def mlstm_state_width(self, e: int, f: int) -> int:
         """Floats of one head's state: the memory [e, f], the normaliser [e] and one
         stabiliser per group of columns a CTA owns."""
@@ -1026,6 +1089,18 @@ class Ops:
               and num.dtype == den.dtype == torch.float32, "mlstm_scan: bad buffers")
         _need(bias_i.shape == (n_heads,) and bias_f.dtype == bias_i.dtype, "mlstm_scan: bad biases")
         q_off, k_off, v_off = offsets
+        plan = self._chunk_plan("mlstm", 2, step, [(qkvg, o, w) for o, w in zip(offsets, (e, e, f))],
+                                (state, num), (width, width // n_heads), n_heads, e, f)
+        if plan is not None:
+            most, window, chunks, scratch = plan
+            self.launches += 5 * (-(-most // window))
+            _check(self._part_lib("mlstm")["chunked"](
+                _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
+                _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
+                _ptr(step.state_slot), _ptr(state), width, step.n_requests, t, n_heads, e, f,
+                _ptr(num), _ptr(den), most, window, chunks, _ptr(scratch), self._stream()),
+                "mlstm_scan_chunked")
+            return
         self.launches += 1
         _check(self._part_lib("mlstm")["scan"](
             _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
@@ -1392,6 +1467,25 @@ class Ops:
                                      and decay_head.dtype == torch.float32), "linear_scan: decay")
         _need(bonus is None or (bonus.numel() == n_heads * e and bonus.is_contiguous()),
               "linear_scan: bad bonus")
+        plan = None
+        if (decay_tok is not None and read_first and e <= 128 and decay_tok.data_ptr() % 16 == 0) or \
+                (decay_head is not None and not read_first and bonus is None):
+            plan = self._chunk_plan("scan", 0 if decay_tok is None else 1, step,
+                                    [(*a, e), (*k, e), (*v, f)], (state, out),
+                                    (state.stride(0), e * f), n_heads, e, f)
+        if plan is not None:
+            most, window, chunks, scratch = plan
+            self.launches += 4 * (-(-most // window))
+            _check(self._part_lib("scan")["chunked"](
+                _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],
+                _ptr(k[0]), _code(k[0].dtype), k[0].shape[1], k[1],
+                _ptr(v[0]), _code(v[0].dtype), v[0].shape[1], v[1],
+                _ptr(decay_tok), _ptr(decay_head), _ptr(bonus),
+                _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
+                _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
+                step.n_requests, t, n_heads, e, f, _ptr(out), 1 if silu else 0, most, window, chunks,
+                _ptr(scratch), self._stream()), "linear_scan_chunked")
+            return
         self.launches += 1
         _check(self._part_lib("scan")["scan"](
             _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],

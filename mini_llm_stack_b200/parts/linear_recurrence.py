@@ -3,8 +3,9 @@ attention and the gated delta rule.
 
 Both keep ``S [e, f]`` per head (key size e, value size f) in the request's state slot
 (``FixedState``, float32, zero when the slot is claimed) and walk a step's tokens through
-it with the same scan kernel; a portion of a prompt continues from the slot's state, so
-cutting a prompt changes no bit.
+it with the same scan; a portion of a prompt continues from the slot's state.  In a float32
+run cutting a prompt changes no bit; a bfloat16 run takes longer portions chunk by chunk, with
+the sums over a chunk's tokens in another order.
 
 wkv (e = f), with h' the previous token's h (zeros before the first; kept in the slot):
     mix_s = h + (h' - h) * mu_s          for s in r, k, v, g, w
@@ -177,7 +178,7 @@ class LightningAttention(Mixer):
         out = W_o (rms_norm(o over all heads together) * w * sigmoid(W_g h)) * out_scale
 
     The state lives in the request's state slot (float32, zero when claimed) and is carried
-    from token to token, so cutting a prompt changes no bit.  Activations enter the scan in
+    from token to token (cuts as above).  Activations enter the scan in
     float32; decays, state, sums and the norm are float32 in both run types.  With
     ``project=False`` the mixer has no output projection: ``heads(h, step, cache, out)``
     leaves the normed, gated and scaled heads in ``out`` (which may be a block of columns of

@@ -1,0 +1,178 @@
+"""Recurrences over a matrix state chunk by chunk, at the edges of chunks, heads and windows:
+against float64 token by token, and no further from it than the token-by-token kernels."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from mini_llm_stack_b200.ops.kernels import Runtime
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    o = Runtime("cuda:0", torch.bfloat16).ops
+    o.require_part("scan")
+    o.require_part("mlstm")
+    return o
+
+
+def a_step(lens, chunked):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    slots = [(3 * r + 1) % len(lens) if len(lens) % 3 else r for r in range(len(lens))]
+    i32 = dict(dtype=torch.int32, device="cuda")
+    return SimpleNamespace(n_tokens=cu[-1], n_requests=len(lens), cu_q=torch.tensor(cu, **i32),
+                           state_slot=torch.tensor(slots, **i32), q_lens=lens if chunked else []), cu, slots
+
+
+def closer(got, other, want, chain, what):
+    """``got`` lies no further from ``want`` than one and a half times ``other`` (both float32), or
+    than a walk of ``chain`` roundings of 2^-24 takes a sum (one chunk's sums are one chain, the
+    token-by-token kernels add eight shorter ones)."""
+    scale = want.abs().max()
+    mine, theirs = (got.double() - want).norm(), (other.double() - want).norm()
+    assert torch.isfinite(got).all(), what
+    assert mine <= max(1.5 * theirs, 2.0 ** -24 * chain ** 0.5 * want.norm()), (what, float(mine / want.norm()), float(theirs / want.norm()))
+    assert (got.double() - want).abs().max() <= 2e-5 * scale, what
+
+
+@pytest.fixture
+def always(ops, monkeypatch):
+    monkeypatch.setattr(ops, "CHUNKED_FROM", {"head": 1, "token": 1, "mlstm": 1}, raising=False)
+    monkeypatch.setattr(ops, "CHUNK_TOKENS", 0, raising=False)
+    return monkeypatch
+
+
+LENS = [[1], [63, 64, 65], [130, 1, 7, 128], [300]]
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("e, f, heads", [(16, 16, 2), (64, 64, 3), (96, 200, 2), (128, 256, 2), (68, 132, 1), (256, 36, 1)])
+@pytest.mark.parametrize("kind", ["head", "head_silu", "token", "token_plain"])
+def test_linear_scan(ops, always, lens, e, f, heads, kind):
+    if kind.startswith("token") and e > 128:
+        pytest.skip("token by token")
+    g = torch.Generator().manual_seed(e + f + sum(lens))
+    t = sum(lens)
+    q, k = (torch.randn(t, heads * e, generator=g) * e ** -0.5 for _ in range(2))
+    v = torch.randn(t, heads * f, generator=g).bfloat16()
+    if kind == "head_silu":
+        q, k = q.bfloat16(), k.bfloat16()
+    state0 = torch.randn(len(lens), heads * e * f, generator=g)
+    # decays from nothing at all to everything, most of them close to one
+    every = torch.cat([torch.tensor([0.0, 1.0, 1e-30, 0.5]), 1 - 2.0 ** -(1 + 7 * torch.rand(4096, generator=g))])
+    head = kind.startswith("head")
+    decay_head = every[torch.randint(0, 8 if heads > 1 else 4096, (heads,), generator=g)]
+    decay_tok = every[torch.randint(0, 400, (t, heads * e), generator=g)].contiguous()
+    bonus = torch.randn(heads, e, generator=g).bfloat16() if kind == "token" else None
+    act = torch.nn.functional.silu if kind == "head_silu" else (lambda x: x)
+    outs = {}
+    for chunked in (True, False):
+        step, cu, slots = a_step(lens, chunked)
+        state = state0.cuda()
+        out = torch.full((t, heads * f), float("nan"), device="cuda")
+        before = ops.launches
+        ops.linear_scan((q.cuda(), 0), (k.cuda(), 0), (v.cuda(), 0), state, step, heads, e, f, out,
+                        decay_tok=None if head else decay_tok.cuda(),
+                        decay_head=decay_head.cuda() if head else None,
+                        bonus=None if bonus is None else bonus.cuda(), read_first=not head,
+                        silu=kind == "head_silu")
+        assert (ops.launches - before > 1) == chunked
+        outs[chunked] = out.cpu(), state.cpu()
+    want, last = torch.zeros(t, heads, f, dtype=torch.float64), torch.zeros(len(lens), heads, e, f, dtype=torch.float64)
+    qd, kd, vd = (act(x.double()).view(t, heads, -1) for x in (q, k, v))
+    for r, n in enumerate(lens):
+        s = state0[slots[r]].double().view(heads, e, f)
+        for i in range(cu[r], cu[r] + n):
+            kv = kd[i][:, :, None] * vd[i][:, None, :]
+            if head:
+                s = decay_head.double()[:, None, None] * s + kv
+                want[i] = torch.einsum("hef,he->hf", s, qd[i])
+            else:
+                u = bonus.double()[:, :, None] if bonus is not None else 0.0
+                want[i] = torch.einsum("hef,he->hf", s + u * kv, qd[i])
+                s = decay_tok[i].double().view(heads, e, 1) * s + kv
+        last[slots[r]] = s
+    closer(outs[True][0], outs[False][0], want.view(t, -1), e + 64, "outputs")
+    closer(outs[True][1], outs[False][1], last.view(len(lens), -1), 64, "states")
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("e, f, heads", [(16, 64, 2), (64, 192, 2), (96, 192, 1), (256, 512, 1)])
+@pytest.mark.parametrize("forget", [3.0, -4.0])
+def test_mlstm(ops, always, lens, e, f, heads, forget):
+    g = torch.Generator().manual_seed(e + f + sum(lens))
+    t, width = sum(lens), ops.mlstm_state_width(e, f)
+    qkv = torch.randn(t, heads * (2 * e + f), generator=g).bfloat16()
+    gates = torch.randn(t, 2 * heads, generator=g) * 4.0
+    bi, bf = torch.randn(heads, generator=g), torch.randn(heads, generator=g) + forget
+    state0 = torch.randn(len(lens), heads, width, generator=g) * 0.3
+    state0[:, :, e * f + e:] = state0[:, :, e * f + e:e * f + e + 1]
+    outs = {}
+    for chunked in (True, False):
+        step, cu, slots = a_step(lens, chunked)
+        state, num, den = state0.cuda(), torch.empty(t, heads * f, device="cuda"), torch.empty(t, heads, device="cuda")
+        before = ops.launches
+        ops.mlstm_scan(qkv.cuda(), (0, heads * e, 2 * heads * e), gates.cuda(), bi.cuda(), bf.cuda(), 15.0, step,
+                       state, heads, e, f, num, den)
+        assert (ops.launches - before > 1) == chunked
+        outs[chunked] = num.cpu(), den.cpu(), state.cpu()
+    q, k, v = (x.double().view(t, heads, -1) for x in qkv.split([heads * e, heads * e, heads * f], 1))
+    q = q * e ** -0.5
+    ig = 15 * torch.tanh((gates[:, :heads].double() + bi.double()) / 15)
+    fg = torch.nn.functional.logsigmoid(15 * torch.tanh((gates[:, heads:].double() + bf.double()) / 15))
+    want, last = torch.zeros(t, heads, f, dtype=torch.float64), state0.double().clone()
+    want_den = torch.zeros(t, heads, dtype=torch.float64)
+    for r, n in enumerate(lens):
+        st = state0[slots[r]].double()
+        c, norm, m = st[:, :e * f].reshape(heads, e, f).clone(), st[:, e * f:e * f + e].clone(), st[:, e * f + e].clone()
+        for i in range(cu[r], cu[r] + n):
+            new = torch.maximum(fg[i] + m, ig[i])
+            keep, take = torch.exp(fg[i] + m - new), torch.exp(ig[i] - new)
+            m = new
+            c = keep[:, None, None] * c + (take[:, None] * k[i])[:, :, None] * v[i][:, None, :]
+            norm = keep[:, None] * norm + take[:, None] * k[i]
+            want_den[i] = torch.maximum((norm * q[i]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+            want[i] = torch.einsum("hef,he->hf", c, q[i])
+        last[slots[r], :, :e * f] = c.reshape(heads, -1)
+        last[slots[r], :, e * f:e * f + e] = norm
+        last[slots[r], :, e * f + e:] = m[:, None]
+    # (a stabiliser of up to 16 is rounded to float32, which scales both by up to 16 * 2^-24)
+    for got, other, exact in zip(outs[True], outs[False], (want.view(t, -1), want_den, last)):
+        closer(got, other, exact, e + 64 + 16 ** 2, "numerators, denominators, states")
+
+
+def test_windows_of_chunks_and_portions_go_on_from_the_slot(ops, always):
+    """Scratch for one chunk a request at a time, and a prompt in two steps: the same states."""
+    g = torch.Generator().manual_seed(5)
+    lens, heads, e, f = [200, 70, 3], 2, 64, 64
+    t = sum(lens)
+    q, k, v = (torch.randn(t, heads * e, generator=g).bfloat16().cuda() for _ in range(3))
+    decay = torch.tensor([0.97, 0.6]).cuda()
+
+    def walk(lens, rows, state):
+        step, _, _ = a_step(lens, True)
+        step.state_slot = torch.arange(len(lens), dtype=torch.int32, device="cuda")
+        out = torch.empty(sum(lens), heads * f, device="cuda")
+        ops.linear_scan(*(((x[rows].contiguous(), 0)) for x in (q, k, v)), state, step, heads, e, f, out,
+                        decay_head=decay)
+        return out
+
+    every = torch.arange(t, device="cuda")
+    whole = torch.zeros(3, heads * e * f, device="cuda")
+    out = walk(lens, every, whole)
+    always.setattr(ops, "CHUNK_SCRATCH", 1, raising=False)
+    cut = torch.zeros(3, heads * e * f, device="cuda")
+    assert torch.equal(walk(lens, every, cut), out) and torch.equal(cut, whole)
+    first, second = [100, 64, 1], [100, 6, 2]
+    starts = [0, 200, 270]
+    two = torch.zeros(3, heads * e * f, device="cuda")
+    a = torch.cat([torch.arange(s, s + n) for s, n in zip(starts, first)]).cuda()
+    b = torch.cat([torch.arange(s + m, s + m + n) for s, m, n in zip(starts, first, second)]).cuda()
+    got = torch.empty_like(out)
+    got[a], got[b] = walk(first, a, two), walk(second, b, two)
+    assert (got - out).abs().max() <= 1e-5 * out.abs().max() and (two - whole).abs().max() <= 1e-5 * whole.abs().max()
