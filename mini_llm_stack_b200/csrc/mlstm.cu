@@ -55,6 +55,19 @@ __device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&out)[8]) 
     }
 }
 
+// Four neighbouring entries.
+__device__ __forceinline__ float4 load_quad(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_quad(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void store_quad(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store_quad(__nv_bfloat16* p, float4 v) {
+    *reinterpret_cast<uint2*>(p) = pack_bf16x4(v);
+}
+
 // MAXR: most rows of C a thread holds.
 template <typename T, int MAXR>
 __global__ void __launch_bounds__(SCAN_THREADS, MAXR <= 16 ? 2 : 1)
@@ -264,6 +277,56 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ num, const float* 
     }
 }
 
+// The same where rows can be read four entries at a time (f up to 128 * QUADS): a lane keeps its
+// quads in registers, and all loads are under way before the sum is taken (30 -> 12 us for 2,048
+// tokens of 4 heads of 512).
+template <typename T, int QUADS>
+__global__ void __launch_bounds__(256)
+mlstm_finish_quads_kernel(const float* __restrict__ num, const float* __restrict__ den,
+                          const T* __restrict__ gate, int gate_row, int g_off,
+                          const void* __restrict__ w, int w_dtype, float eps, T* __restrict__ out,
+                          long long units, int n_heads, int f) {
+    chain_release();
+    chain_wait();
+    const int lane = threadIdx.x & 31;
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= units) return;
+    const int t = (int)(unit / n_heads), head = (int)(unit % n_heads);
+    const float d = den[unit];
+    const T* g = gate + (size_t)t * gate_row + g_off + head * f;
+    float4 o[QUADS], z[QUADS];
+    float ss = 0.f;
+#pragma unroll
+    for (int x = 0; x < QUADS; ++x) {
+        const int j = 4 * (lane + 32 * x);
+        if (j >= f) continue;
+        o[x] = *reinterpret_cast<const float4*>(num + (size_t)unit * f + j);
+        z[x] = load_quad(g + j);
+    }
+#pragma unroll
+    for (int x = 0; x < QUADS; ++x) {
+        if (4 * (lane + 32 * x) >= f) continue;
+        o[x] = make_float4(o[x].x / d, o[x].y / d, o[x].z / d, o[x].w / d);
+        ss = fmaf(o[x].x, o[x].x, ss);
+        ss = fmaf(o[x].y, o[x].y, ss);
+        ss = fmaf(o[x].z, o[x].z, ss);
+        ss = fmaf(o[x].w, o[x].w, ss);
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)f + eps);
+#pragma unroll
+    for (int x = 0; x < QUADS; ++x) {
+        const int j = 4 * (lane + 32 * x);
+        if (j >= f) continue;
+        const float4 m = w_dtype == MLS_BF16 ? load_quad((const __nv_bfloat16*)w + (size_t)head * f + j)
+                                             : load_quad((const float*)w + (size_t)head * f + j);
+        store_quad(out + (size_t)unit * f + j,
+                   make_float4(o[x].x * inv * m.x / (1.0f + expf(-z[x].x)),
+                               o[x].y * inv * m.y / (1.0f + expf(-z[x].y)),
+                               o[x].z * inv * m.z / (1.0f + expf(-z[x].z)),
+                               o[x].w * inv * m.w / (1.0f + expf(-z[x].w))));
+    }
+}
+
 template <typename T, int MAXR>
 int launch_scan(const void* qkvg, int row_w, int q_off, int k_off, int v_off, const float* gates,
                 const void* bi, const void* bf, int b_dtype, float cap, const int* cu_q,
@@ -388,6 +451,26 @@ MLS_API int mls_mlstm_finish(const float* num, const float* den, const void* gat
     // past the end, so blocks of one warp when it does not divide
     const int warps = units % 4 == 0 ? 4 : 1;
     const int blocks = (int)(units / warps);
+    const uintptr_t bytes = dtype == MLS_BF16 ? 8 : 16;
+    if (((f | gate_row | g_off) & 3) == 0 && f <= 512 && reinterpret_cast<uintptr_t>(num) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(gate) % bytes == 0 && reinterpret_cast<uintptr_t>(out) % bytes == 0 &&
+        reinterpret_cast<uintptr_t>(w) % (w_dtype == MLS_BF16 ? 8 : 16) == 0) {
+#define QUADS_GO(T, N)                                                                             \
+    MLS_LAUNCH((mlstm_finish_quads_kernel<T, N>), dim3((unsigned)((units + 7) / 8)), dim3(256), 0, \
+               stream, num, den, (const T*)gate, gate_row, g_off, w, w_dtype, eps, (T*)out, units, \
+               n_heads, f)
+        if (dtype == MLS_BF16) {
+            if (f <= 128) QUADS_GO(__nv_bfloat16, 1);
+            else if (f <= 256) QUADS_GO(__nv_bfloat16, 2);
+            else QUADS_GO(__nv_bfloat16, 4);
+        } else {
+            if (f <= 128) QUADS_GO(float, 1);
+            else if (f <= 256) QUADS_GO(float, 2);
+            else QUADS_GO(float, 4);
+        }
+#undef QUADS_GO
+        return launch_status();
+    }
     if (dtype == MLS_BF16)
         MLS_LAUNCH((mlstm_finish_kernel<__nv_bfloat16>), dim3(blocks), dim3(32 * warps), 0, stream,
                    num, den, (const __nv_bfloat16*)gate, gate_row, g_off, w, w_dtype, eps,
