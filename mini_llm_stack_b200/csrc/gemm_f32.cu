@@ -168,6 +168,72 @@ gemm_f32_kernel(const T* __restrict__ A, const float* __restrict__ W, float* __r
     }
 }
 
+// Up to FEW_M rows (decoding): what is read is W alone, and an output's sum is one chain over K
+// (4 cycles a step).  Blocks of 64 of K come by asynchronous copies, STAGES of them under way.  With
+// few columns a thread takes one output and a block 16 columns, so that every SM has a block; with
+// many, whose reads of shared memory would bound it (426 us for 3 x 128,256 x 2,048), a thread
+// takes four rows of a column and a block 64 columns.  Against the tiles of 32 x 64 above:
+// 1 x 2,048 x 2,048 64 -> 17 us, 1 x 2,048 x 8,192 245 -> 55, 8 x 128,256 x 2,048 428 -> 391.  Rows of
+// whole 16-byte pieces; the same bits.
+constexpr int FEW_M = 8, FEW_K = 64, FEW_KP = FEW_K + 4;
+template <int BN, int ROWS, int STAGES>
+__global__ void __launch_bounds__(BN * (FEW_M / ROWS))
+gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out,
+                    int M, int N, int K) {
+    chain_release();
+    extern __shared__ __align__(16) float stages[];          // [STAGES][BN + FEW_M][FEW_KP]
+    constexpr int THREADS = BN * (FEW_M / ROWS), STAGE = (BN + FEW_M) * FEW_KP,
+                  UNITS = (BN + FEW_M) * (FEW_K / 4);
+    const int n0 = blockIdx.x * BN, n = threadIdx.x % BN, m0 = threadIdx.x / BN * ROWS;
+    chain_wait();
+    auto fetch = [&](int b) {                                // block b of K into its stage
+        const int k0 = b * FEW_K;
+        if (k0 < K) {
+            float* st = stages + (b % STAGES) * STAGE;
+#pragma unroll 4
+            for (int u = threadIdx.x; u < UNITS; u += THREADS) {
+                const int r = u / (FEW_K / 4), k = 4 * (u % (FEW_K / 4));
+                const bool w = r < BN;
+                const bool there = k0 + k < K && (w ? n0 + r < N : r - BN < M);
+                const float* src = !there ? W : (w ? W + (size_t)(n0 + r) * K : A + (size_t)(r - BN) * K) + k0 + k;
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(st + r * FEW_KP + k);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                             ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int b = 0; b < STAGES - 1; ++b) fetch(b);
+    float acc[ROWS];
+#pragma unroll
+    for (int y = 0; y < ROWS; ++y) acc[y] = 0.f;
+    const int blocks = (K + FEW_K - 1) / FEW_K;
+    for (int b = 0; b < blocks; ++b) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                                     // block b is there, block b - 1 is read
+        fetch(b + STAGES - 1);
+        const float* st = stages + (b % STAGES) * STAGE;
+        const float* w = st + n * FEW_KP;
+        const float* a = st + (BN + m0) * FEW_KP;
+#pragma unroll
+        for (int k = 0; k < FEW_K; k += 4) {
+            const float4 y = load4(w + k);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                const float4 x = load4(a + r * FEW_KP + k);
+                acc[r] = fmaf(x.x, y.x, acc[r]);
+                acc[r] = fmaf(x.y, y.y, acc[r]);
+                acc[r] = fmaf(x.z, y.z, acc[r]);
+                acc[r] = fmaf(x.w, y.w, acc[r]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+        if (m0 + r < M && n0 + n < N) out[(size_t)(m0 + r) * N + n0 + n] = acc[r];
+}
+
 // Few output columns (a router's or a gate's scores: N <= SKINNY_N): the tile kernel above
 // would leave all but a few SMs idle.  Here a warp owns SK_ROWS rows and COLS neighbouring
 // columns; its lanes walk K four entries at a time with a stride of 128 (one entry at a time
@@ -339,6 +405,26 @@ int tiled(const T* A, const float* W, float* out, int M, int N, int K, cudaStrea
 #undef TILES
 }
 
+template <int BN, int ROWS, int STAGES>
+int few_of(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
+    constexpr int smem = STAGES * (BN + FEW_M) * FEW_KP * (int)sizeof(float);
+    static bool configured = false;
+    if (!configured) {
+        const int rc = (int)cudaFuncSetAttribute(gemm_f32_few_kernel<BN, ROWS, STAGES>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (rc) return rc;
+        configured = true;
+    }
+    MLS_LAUNCH((gemm_f32_few_kernel<BN, ROWS, STAGES>), dim3((N + BN - 1) / BN), dim3(BN * (FEW_M / ROWS)),
+               smem, stream, A, W, out, M, N, K);
+    return launch_status();
+}
+int few(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
+    if (N >= 64 * 2 * sm_count()) return few_of<64, 4, 5>(A, W, out, M, N, K, stream);
+    return few_of<16, 1, 8>(A, W, out, M, N, K, stream);
+}
+int few(const __nv_bfloat16*, const float*, float*, int, int, int, cudaStream_t) { return MLS_ERR_UNSUPPORTED; }
+
 template <typename T>
 int product(const T* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
     const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
@@ -353,6 +439,7 @@ int product(const T* A, const float* W, float* out, int M, int N, int K, cudaStr
         if (vec_w) return skinny<T, true, false>(A, W, out, M, N, K, stream);
         return skinny<T, false, false>(A, W, out, M, N, K, stream);
     }
+    if (vec_w && vec_a && M <= FEW_M && sizeof(T) == 4) return few(A, W, out, M, N, K, stream);
     if (vec_w && vec_a) return tiled<T, true>(A, W, out, M, N, K, stream);
     return tiled<T, false>(A, W, out, M, N, K, stream);
 }

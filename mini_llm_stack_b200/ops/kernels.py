@@ -134,7 +134,7 @@ class Ops:
                                   _LL, _I, _P, _I, _LL, _P, _P])
         self._attention_simt = _decl(core, "mls_attention_simt",
                                      [_P, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I,
-                                      _I, _F, _I, _F, _LL, _P, _P, _I, _LL, _I, _P])
+                                      _I, _F, _I, _F, _LL, _P, _P, _I, _LL, _I, _P, _I, _I, _P])
         self._swiglu = _decl(core, "mls_swiglu", [_P, _P, _I, _I, _I, _P])
         self._clamped_glu = _decl(core, "mls_clamped_glu", [_P, _P, _I, _I, _I, _F, _F, _P])
         self._unary_act = _decl(core, "mls_unary_act", [_P, _I, _P, _I, _LL, _I, _P, _I, _I, _P])
@@ -654,13 +654,15 @@ class Ops:
                       _ptr(slopes), keep_first, out.stride(0), int(chunk), plan.share, self._stream()),
                    "attention_mma")
             return
-        self.launches += 1
+        # requests of several tokens share their keys by tiles, the others take a warp a row
+        lens = getattr(step, "q_lens", None) or [0]
+        self.launches += 2 if max(lens) >= 8 > min(lens) and hd % 4 == 0 and hd <= 128 else 1
         _check(self._attention_simt(
             _ptr(qkv), _ptr(out), _code(qkv.dtype), _ptr(cache.k_pool), _ptr(cache.v_pool),
             _ptr(g.block_table), g.max_blocks, _ptr(step.positions), _ptr(step.req_of_token),
             t, n_heads, n_kv, hd, g.block_size, float(scale), int(window), float(softcap),
             cache.k_pool.shape[1], _ptr(sink), _ptr(slopes), keep_first, out.stride(0), int(chunk),
-            self._stream()), "attention_simt")
+            _ptr(step.cu_q), max(lens), min(lens), self._stream()), "attention_simt")
 
     def _split_launches(self, n_split: int, tma: bool, n_ctas: int) -> int:
         """Kernels the context-split attention launches: two to eight splits merge inside
