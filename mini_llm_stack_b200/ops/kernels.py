@@ -147,6 +147,7 @@ class Ops:
         self._attention_lib_handles: dict = {}
         self._split_ctas_per_sm: dict = {}       # head size -> CTAs of the split kernel an SM holds
         self._attention_fused: dict = {}         # head size -> decode attention that also rotates
+        self._attention_shared: dict = {}        # head size -> (pages taken, tcgen05 kernel for shared keys and values)
         self._tc_rows: dict = {}                 # head size -> rows of a tile of the tcgen05 kernel
         self._scratch: dict = {}
         self._transposed: dict = {}              # id(weight) -> (weight, its transposed view)
@@ -537,6 +538,11 @@ class Ops:
                           [_P, _I, _LL, _P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _I, _P, _P, _I, _I,
                            _I, _I, _F, _I, _I, _P, _P, _LL, _P, _P])
             self._attention_fused[hd] = fused
+            self._attention_shared[hd] = (
+                _decl(lib, "mls_attention_shared_tc_takes", [_I]),
+                _decl(lib, "mls_attention_shared_tc",
+                      [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _LL, _P, _P, _LL,
+                       _I, _I, _P]))
             rows_fn = lib.mls_attention_tc_rows
             rows_fn.restype = ctypes.c_int
             self._tc_rows[hd] = int(rows_fn()) or 128
@@ -632,6 +638,20 @@ class Ops:
                           float(softcap), n_tiles_tc, plan.n_tiles_tc_wide, n_small, cache.k_pool.shape[1],
                           _ptr(self.status), _ptr(sink), out.stride(0), _ptr(slopes), keep_first,
                           int(chunk), plan.share, self._stream()), "attention_tc")
+                n_tiles = 0
+                if not n_small:
+                    return
+            if (n_tiles and self.attention_impl == "auto" and plain and not softcap
+                    and cache.k_pool.data_ptr() == cache.v_pool.data_ptr()
+                    and self._attention_shared[hd][0](g.block_size)):
+                # the same where one cached row is key and value (attention over a latent)
+                self.launches += 1
+                _check(self._attention_shared[hd][1](
+                    _ptr(qkv), _ptr(out), _ptr(cache.k_pool), _ptr(g.block_table), g.max_blocks,
+                    _ptr(step.cu_q), _ptr(step.ctx_len), step.n_requests, n_heads, n_kv, g.block_size,
+                    float(scale), int(window), n_tiles_tc, n_small, cache.k_pool.shape[1],
+                    _ptr(self.status), _ptr(sink), out.stride(0), int(chunk), plan.share,
+                    self._stream()), "attention_shared_tc")
                 n_tiles = 0
                 if not n_small:
                     return

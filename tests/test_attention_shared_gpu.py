@@ -1,0 +1,72 @@
+"""Prompt attention where one cached row is key and value, on the tensor cores: against the kernel
+of one warp a row, at the edges of key tiles (96), row tiles (128), pages, windows and chunks."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from mini_llm_stack_b200.ops.kernels import Runtime
+from mini_llm_stack_b200.parts.attention import plan_paged_attention
+from mini_llm_stack_b200.parts.base import GroupView
+
+pytestmark = pytest.mark.gpu
+HD = 256
+
+
+@pytest.fixture(scope="module")
+def ops():
+    o = Runtime("cuda:0", torch.bfloat16).ops
+    o.require_attention(HD)
+    return o
+
+
+@pytest.mark.parametrize("heads, block", [(16, 16), (32, 8), (3, 32), (5, 64)])
+@pytest.mark.parametrize("lens, before, scattered", [
+    ([1, 95, 2, 130], [95, 0, 300, 0], True), ([300], [0], False), ([33, 64], [700, 96], True),
+    ([96, 97], [0, 95], False)])
+@pytest.mark.parametrize("args", [dict(window=0), dict(window=100), dict(window=0, chunk=70), dict(window=33)])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_against_a_warp_a_row(ops, monkeypatch, heads, block, lens, before, scattered, args, sinks):
+    g = torch.Generator(device="cuda").manual_seed(heads + sum(lens))
+    t, r = sum(lens), len(lens)
+    ctx = [b + n for b, n in zip(before, lens)]
+    width = -(-max(ctx) // block)
+    order = (torch.randperm(r * width, generator=torch.Generator().manual_seed(1)) if scattered
+             else torch.arange(r * width)).int()
+    table = order.view(r, width).clone()
+    for i, c in enumerate(ctx):
+        table[i, -(-c // block):] = -1                   # pages that the request does not hold
+        if args["window"]:                               # and those that a window has given back
+            table[i, :max(0, before[i] - args["window"] + 1) // block] = -1
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    step = SimpleNamespace(
+        n_tokens=t, n_requests=r, q_lens=lens, ctx_lens=ctx, max_ctx_len=max(ctx), attn_tiles={},
+        positions=torch.cat([torch.arange(b, c) for b, c in zip(before, ctx)]).to(**i32),
+        cu_q=torch.tensor(cu, **i32), ctx_len=torch.tensor([*ctx, max(ctx)], **i32),
+        req_of_token=torch.repeat_interleave(torch.arange(r), torch.tensor(lens)).to(**i32),
+        groups={0: GroupView(table.cuda(), None, block, width)})
+    pool = torch.randn(1, r * width, block, HD, device="cuda", generator=g).bfloat16()
+    for i, c in enumerate(ctx):                          # the rest of a request's last page is cleared
+        if c % block:
+            pool[0, int(order[i * width + c // block]), c % block:] = 0.0
+    cache = SimpleNamespace(group=0, k_pool=pool, v_pool=pool)
+    qkv = torch.randn(t, (heads + 2) * HD, device="cuda", generator=g).bfloat16()
+    qkv[:, :HD] *= 4.0                                   # a head whose softmax is nearly one key
+    sink = torch.randn(heads, device="cuda", generator=g) * 2 if sinks else None
+    facts = dict(ops.attention_facts(HD))
+    plan = plan_paged_attention(step, facts, heads, 1, HD)
+    got = {}
+    for impl in ("auto", "simt"):
+        monkeypatch.setattr(ops, "attention_impl", impl)
+        out = torch.full((t, heads * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(qkv, out, cache, step, heads, 1, HD, HD ** -0.5, plan=plan, sink=sink, **args)
+        ops.check_status()
+        got[impl] = out.float()
+    assert torch.isfinite(got["auto"]).all()
+    # outputs are averages of unit rows: P is rounded to 8 bits (2^-9 of a sum of weights at most 1,
+    # times values of up to some 4), the result once more
+    assert (got["auto"] - got["simt"]).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * got["simt"].abs().max()
