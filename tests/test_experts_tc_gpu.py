@@ -98,3 +98,65 @@ def test_products_of_sorted_rows(ops, t, experts, identity, top, d, f, spread, u
             down = w2[e].double() @ row * (1.0 if scale_in else float(weight[tok, j]))
             # float32 sums of f products of unit size
             assert (out[slot].double() - down).abs().max() <= 1e-5 * max(1.0, float(row.norm())), (tok, j)
+
+
+@pytest.mark.parametrize("experts, groups", [(5, None), (64, (8, 3)), (65, None), (256, (4, 1)), (257, None), (9000, None)])
+def test_choice_and_order(ops, experts, groups):
+    """Choices against a stable sort (scores of few distinct values, numbers that are none), and the
+    slots in the order of their experts."""
+    g = torch.Generator().manual_seed(experts)
+    t, top = 37, min(5, experts)
+    logits = torch.randint(-6, 7, (t, experts), generator=g).float()
+    logits[3, 1] = float("nan")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    n, tiles = t * top, ops.expert_max_tiles(t * top, experts)
+    work = {"idx": torch.empty(n, **i32), "weight": torch.empty(n, device="cuda"), "order": torch.empty(n, **i32),
+            "offsets": torch.empty(experts + 1, **i32), "cursor": torch.empty(experts, **i32),
+            "tile_expert": torch.empty(tiles, **i32), "tile_row0": torch.empty(tiles, **i32), "max_tiles": tiles}
+    ops.route(logits.cuda(), top, False, work, n_real=experts - 1, groups=groups)
+    idx = work["idx"].cpu().view(t, top).long()
+    for i in range(t):
+        allowed = set(range(experts))
+        if i == 3:
+            allowed.discard(1)
+        elif groups:
+            size = experts // groups[0]
+            best = logits[i].view(groups[0], size).sigmoid().topk(2, -1).values.sum(-1)
+            keep = sorted(range(groups[0]), key=lambda k: (-float(best[k]), k))[:groups[1]]
+            allowed = {e for e in allowed if e // size in keep}
+        if i == 3 and groups:
+            continue
+        want = sorted(allowed, key=lambda e: (-float(logits[i, e]), e))[:top]
+        assert idx[i].tolist() == want + [0] * (top - len(want)), i      # (no number left: output 0)
+    offsets, order = work["offsets"].cpu(), work["order"].cpu().long()
+    counts = torch.bincount(idx.reshape(-1), minlength=experts)
+    assert torch.equal(offsets[1:] - offsets[:-1], counts.int()) and offsets[0] == 0
+    assert torch.equal(order.sort().values, torch.arange(n))
+    assert torch.equal(idx.reshape(-1)[order], torch.repeat_interleave(torch.arange(experts), counts))
+    want = [(e, int(offsets[e]) + r) for e in range(experts - 1) for r in range(0, int(counts[e]), 32)]
+    got = list(zip(work["tile_expert"].tolist(), work["tile_row0"].tolist()))
+    assert got[:len(want)] == want and all(e == -1 for e, _ in got[len(want):])
+
+
+@pytest.mark.parametrize("d", [4, 30, 64, 1028])
+@pytest.mark.parametrize("top", [1, 6, 9])
+@pytest.mark.parametrize("shared", [None, "rows", "gated"])
+def test_combination(ops, d, top, shared):
+    g = torch.Generator().manual_seed(d + top)
+    t, n_real = 11, 7
+    per_slot = torch.randn(t * top, d, generator=g)
+    h = torch.randn(t, d, generator=g).bfloat16()
+    idx = torch.randint(0, n_real + 2, (t, top), generator=g)
+    weight = torch.rand(t, top, generator=g)
+    rows = torch.randn(t, d, generator=g).bfloat16()
+    gate = torch.randn(t, 3, generator=g)
+    delta = torch.full((t, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    work = {"idx": idx.int().reshape(-1).cuda(), "weight": weight.reshape(-1).cuda()}
+    ops.expert_combine(per_slot.cuda(), top, rows.cuda() if shared else None, delta, work=work, n_real=n_real,
+                       h=h.cuda(), shared_gate=gate.cuda()[:, 2] if shared == "gated" else None)
+    own = (idx >= n_real)[..., None]
+    want = torch.where(own, weight.double()[..., None] * h.double()[:, None], per_slot.double().view(t, top, d)).sum(1)
+    if shared:
+        want = want + rows.double() * (torch.sigmoid(gate[:, 2:].double()) if shared == "gated" else 1.0)
+    # float32 sums of `top` values, one rounding to 8 bits
+    assert ((delta.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
