@@ -21,8 +21,8 @@
 // from a request's first token of the step.
 //
 // Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,824 ->
-// 400 us, mLSTM of 4 heads of 256 x 512 1,296 -> 235; 1,501 tokens of wkv, 32 heads of 64 x 64,
-// 306 -> 97 (the products run at 35 to 40 TFLOP/s: a tile's loads are not all hidden by the other
+// 365 us, mLSTM of 4 heads of 256 x 512 1,296 -> 215; 1,501 tokens of wkv, 32 heads of 64 x 64,
+// 306 -> 95 (the products run at 38 to 40 TFLOP/s: the updates' loads are not all hidden by the other
 // blocks' arithmetic, and wkv's weights of pairs take 42 us).
 //
 // A value that is not a number reaches the earlier tokens of its chunk too (0 x NaN), as it does in
@@ -131,26 +131,28 @@ __device__ __forceinline__ void fill_rows(float (*T)[W], Get get) {
 }
 
 // acc += A x B over 64 of k: thread (ty, tx) owns rows 4 ty .. + 3 and 32 further on, columns
-// 4 tx .. + 3 and BN / 2 further on.
-template <int BN, bool TURN_A, bool TURN_B>
-__device__ __forceinline__ void multiply(f32x2 (&acc)[8][4], const float (*A)[C], const float (*B)[BN],
+// 4 tx .. + 3 and, with eight columns a thread (TN), BN / 2 further on.
+template <int BN, int TN, bool TURN_A>
+__device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*A)[C], const float (*B)[BN],
                                          int tx, int ty) {
 #pragma unroll 8
     for (int k = 0; k < C; ++k) {
         const int ra = TURN_A ? (4 * ty) ^ turn(k) : 4 * ty;
-        const int cb = TURN_B ? (4 * tx) ^ turn(k) : 4 * tx;
         float v[8];
         *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(&A[k][ra]);
         *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<const float4*>(&A[k][ra + 32]);
-        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&B[k][cb]);
-        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&B[k][cb + BN / 2]);
+        f32x2 b[TN / 2];
+#pragma unroll
+        for (int h = 0; h < TN / 4; ++h) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&B[k][4 * tx + h * (BN / 2)]);
+            b[2 * h] = q.x;
+            b[2 * h + 1] = q.y;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const f32x2 two = twice(v[i]);
-            fma2(acc[i][0], two, b0.x);
-            fma2(acc[i][1], two, b0.y);
-            fma2(acc[i][2], two, b1.x);
-            fma2(acc[i][3], two, b1.y);
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], two, b[j]);
         }
     }
 }
@@ -164,11 +166,12 @@ __device__ __forceinline__ void settle(f32x2 (&sum)[N], f32x2 (&acc)[N]) {
         acc[j] = 0ull;
     }
 }
-__device__ __forceinline__ void clear(f32x2 (&acc)[8][4]) {
+template <int N>
+__device__ __forceinline__ void clear(f32x2 (&acc)[8][N]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < N; ++j) acc[i][j] = 0ull;
 }
 
 // Four entries of operand row t (zeros past the chunk and past the head's size).
@@ -557,17 +560,19 @@ __device__ __forceinline__ float row_factor(const Args& a, const float* factors,
 
 // ------------------------------------------------------------------------------- update
 // U[i, j] = sum_s factor_s k_s[i] v_s[j]; MLSTM: and n[i] = sum_s factor_s k_s[i].
-template <int MODE, int BN>
-__global__ void __launch_bounds__(BN, BN == 128 ? 4 : 6)
+// Tiles of 64 x 64, 8 x 4 a thread: the loads of a tile are hidden by the other blocks' arithmetic only,
+// and more, smaller blocks hide them better (112 us against 116 at tiles of 64 x 128 for 2,048 tokens of
+// 32 heads of 128 x 256; 16 against 28 for 1,501 tokens of 32 heads of 64 x 64).
+template <int MODE>
+__global__ void __launch_bounds__(128, 5)
 chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
     if (!locate(a, first, span, blockIdx.z, w)) return;
-    extern __shared__ __align__(16) float tiles[];
-    float(*A)[C] = reinterpret_cast<float(*)[C]>(tiles);
-    float(*B)[BN] = reinterpret_cast<float(*)[BN]>(tiles + C * C);
+    constexpr int BN = C, TN = 4, THREADS = 128;
+    __shared__ __align__(16) float A[C][C], B[C][BN];
     __shared__ float factor[C];
     const int f_tiles = (a.f + BN - 1) / BN;
     const int i0 = (blockIdx.x / f_tiles) * C, j0 = (blockIdx.x % f_tiles) * BN;
@@ -577,20 +582,20 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     Rows kr = a.k;
     if (MODE == TOKEN_DECAY) kr = Rows{s.rows_k, MLS_F32, a.n_heads * a.e, 0, a.e};
     const Reader k(kr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head), v(a.v, a.silu, w, head);
-    fill_rows<BN, C>(A, [&](int t, int i) { return times(k(t, i0 + i), factor[t]); });
-    fill_rows<BN, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
+    fill_rows<THREADS, C>(A, [&](int t, int i) { return times(k(t, i0 + i), factor[t]); });
+    fill_rows<THREADS, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
     __syncthreads();
-    const int tx = threadIdx.x % (BN / 8), ty = threadIdx.x / (BN / 8);
-    f32x2 acc[8][4];
+    const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
+    f32x2 acc[8][TN / 2];
     clear(acc);
-    multiply<BN, false, false>(acc, A, B, tx, ty);
+    multiply<BN, TN, false>(acc, A, B, tx, ty);
     float* U = s.states + (w.idx * a.n_heads + head) * state_floats(MODE, a.e, a.f);
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
         const int i = i0 + 4 * ty + (x & 3) + 32 * (x >> 2);
         if (i >= a.e) continue;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < TN / 4; ++h) {
             const int j = j0 + 4 * tx + (BN / 2) * h;
             const float2 lo = halves(acc[x][2 * h]), hi = halves(acc[x][2 * h + 1]);
             if (j < a.f)
@@ -658,19 +663,23 @@ chunk_carry_kernel(const Args a, const Scratch s, int first, int span) {
 }
 
 // ------------------------------------------------------------------------------- output
-// o = [factor q | P] x [S0; v]; MLSTM: and den_t = max(|[factor q | P] x [n; 1]|, exp(-m_t)) + 1e-6.
+// o = [P | factor q] x [v; S0]; MLSTM: and den_t = max(|[P | factor q] x [1; n]|, exp(-m_t)) + 1e-6.
+// The first block of 64 is [P] x [v]; while a block is multiplied the next one's rows of S0 come by
+// asynchronous copies and its rows of q into registers (without that, 2,048 tokens of 32 heads of
+// 128 x 256: 200 us, now 166; 4 heads of 256 x 512: 113, now 85).
 template <int MODE, int BN>
-__global__ void __launch_bounds__(BN, BN == 128 ? 3 : 5)
+__global__ void __launch_bounds__(2 * BN, BN == 128 ? 2 : 3)
 chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y, j0 = blockIdx.x * BN;
     if (!locate(a, first, span, blockIdx.z, w)) return;
+    constexpr int THREADS = 2 * BN, TN = 4, QA = C * (C / 4) / THREADS;      // quads of A a thread brings in
     extern __shared__ __align__(16) float tiles[];
-    float(*A)[C] = reinterpret_cast<float(*)[C]>(tiles);
-    float(*B)[BN] = reinterpret_cast<float(*)[BN]>(tiles + C * C);
-    __shared__ float factor[C], n_s[C];
+    float(*A)[C][C] = reinterpret_cast<float(*)[C][C]>(tiles);
+    float(*B)[C][BN] = reinterpret_cast<float(*)[C][BN]>(tiles + 2 * C * C);
+    __shared__ float factor[C], n_s[2][C];
     if (threadIdx.x < C)
         factor[threadIdx.x] = row_factor<MODE>(a, s.rows_q, w, head, threadIdx.x, threadIdx.x + 1);
     Rows qr = a.q;
@@ -679,79 +688,103 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
     const size_t unit = w.idx * a.n_heads + head;
     const float* S = s.states + unit * state_floats(MODE, a.e, a.f);
     const float* P = s.scores + unit * C * C;
-    const int tx = threadIdx.x % (BN / 8), ty = threadIdx.x / (BN / 8);
+    const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool with_n = MODE == MLSTM && j0 == 0;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    f32x2 acc[8][4], sum[8][4];
+    const int blocks = 1 + (a.e + C - 1) / C;
+    // rows i0 .. of S0 into buffer x (what is not there as zeros)
+    auto ask_rows = [&](int i0, int x) {
+#pragma unroll
+        for (int u = threadIdx.x; u < C * (BN / 4); u += THREADS) {
+            const int i = u / (BN / 4), j = 4 * (u % (BN / 4));
+            const bool there = i0 + i < a.e && j0 + j < a.f;
+            const float* src = there ? S + (size_t)(i0 + i) * a.f + j0 + j : S;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                         ::"r"((uint32_t)__cvta_generic_to_shared(&B[x][i][j])), "l"(src), "r"(there ? 16 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    float4 next[QA];
+    fill_transposed<THREADS>(A[0], [&](int t, int x) { return *reinterpret_cast<const float4*>(P + t * C + x); });
+    fill_rows<THREADS, BN>(B[0], [&](int t, int j) { return v(t, j0 + j); });
+    if (with_n && threadIdx.x < C) n_s[0][threadIdx.x] = 1.f;
+    f32x2 acc[8][TN / 2], sum[8][TN / 2];
     clear(acc);
     clear(sum);
     float nq[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // short chains: the sum may nearly vanish
-    for (int i0 = 0; i0 < a.e + C; i0 += C) {            // the last block is [P] x [v]
-        const bool inner = i0 >= a.e;
-        __syncthreads();
-        if (inner) {
-            fill_transposed<BN>(A, [&](int t, int x) {
-                return *reinterpret_cast<const float4*>(P + t * C + x);
-            });
-            fill_rows<BN, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
-        } else {
-            fill_transposed<BN>(A, [&](int t, int x) { return times(q(t, i0 + x), factor[t]); });
-            fill_rows<BN, BN>(B, [&](int i, int j) {
-                return (i0 + i < a.e && j0 + j < a.f)
-                           ? *reinterpret_cast<const float4*>(S + (size_t)(i0 + i) * a.f + j0 + j) : zero;
-            });
-        }
-        if (with_n && threadIdx.x < C)
-            n_s[threadIdx.x] = inner ? 1.f
-                : (i0 + (int)threadIdx.x < a.e ? S[(size_t)a.e * a.f + i0 + threadIdx.x] : 0.f);
-        __syncthreads();
-        multiply<BN, true, false>(acc, A, B, tx, ty);
+    __syncthreads();
+    for (int b = 0; b < blocks; ++b) {
+        const int x = b & 1, i0 = b * C;                       // i0: first row of the next block's S0
+        const bool more = b + 1 < blocks;
+        float n_next = 0.f;
+        if (more) {
+            ask_rows(i0, x ^ 1);
 #pragma unroll
-        for (int x = 0; x < 8; ++x) settle(sum[x], acc[x]);
+            for (int y = 0; y < QA; ++y) {
+                const int u = warp + y * (THREADS / 32);
+                next[y] = q(4 * (u & 15) + (lane & 3), i0 + 4 * ((lane >> 2) + 8 * (u >> 4)));
+            }
+            if (with_n && threadIdx.x < C && i0 + (int)threadIdx.x < a.e)
+                n_next = S[(size_t)a.e * a.f + i0 + threadIdx.x];
+        }
+        multiply<BN, TN, true>(acc, A[x], B[x], tx, ty);
+#pragma unroll
+        for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
         if (with_n && threadIdx.x < C) {
 #pragma unroll 8
-            for (int x = 0; x < C; ++x) nq[x & 7] = fmaf(A[x][threadIdx.x ^ turn(x)], n_s[x], nq[x & 7]);
+            for (int y = 0; y < C; ++y) nq[y & 7] = fmaf(A[x][y][threadIdx.x ^ turn(y)], n_s[x][y], nq[y & 7]);
         }
-        if (inner) break;
+        if (more) {
+#pragma unroll
+            for (int y = 0; y < QA; ++y) {
+                const int u = warp + y * (THREADS / 32), r = 4 * (u & 15) + (lane & 3),
+                          k = 4 * ((lane >> 2) + 8 * (u >> 4)), col = r ^ turn(k);
+                const float4 z = times(next[y], factor[r]);
+                A[x ^ 1][k][col] = z.x;
+                A[x ^ 1][k + 1][col] = z.y;
+                A[x ^ 1][k + 2][col] = z.z;
+                A[x ^ 1][k + 3][col] = z.w;
+            }
+            if (with_n && threadIdx.x < C) n_s[x ^ 1][threadIdx.x] = n_next;
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
     }
     if (with_n && threadIdx.x < w.n) {
         float* den = a.den + (size_t)(w.t0 + threadIdx.x) * a.n_heads + head;
         const float all = ((nq[0] + nq[4]) + (nq[2] + nq[6])) + ((nq[1] + nq[5]) + (nq[3] + nq[7]));
         *den = fmaxf(fabsf(all), *den) + 1e-6f;
     }
+    const int j = j0 + 4 * tx;
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
         const int t = 4 * ty + (x & 3) + 32 * (x >> 2);
-        if (t >= w.n) continue;
-        float* dst = a.out + ((size_t)(w.t0 + t) * a.n_heads + head) * a.f;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int j = j0 + 4 * tx + (BN / 2) * h;
-            const float2 lo = halves(sum[x][2 * h]), hi = halves(sum[x][2 * h + 1]);
-            if (j < a.f) *reinterpret_cast<float4*>(dst + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
-        }
+        if (t >= w.n || j >= a.f) continue;
+        const float2 lo = halves(sum[x][0]), hi = halves(sum[x][1]);
+        *reinterpret_cast<float4*>(a.out + ((size_t)(w.t0 + t) * a.n_heads + head) * a.f + j) =
+            make_float4(lo.x, lo.y, hi.x, hi.y);
     }
 }
 
+template <int MODE>
+int update(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
+    const dim3 grid(((a.e + C - 1) / C) * ((a.f + C - 1) / C), a.n_heads, a.n_requests * span);
+    MLS_LAUNCH((chunk_update_kernel<MODE>), grid, dim3(128), 0, stream, a, s, first, span);
+    return launch_status();
+}
 template <int MODE, int BN>
-int products(const Args& a, const Scratch& s, int first, int span, bool update, cudaStream_t stream) {
-    const int smem = C * (C + BN) * (int)sizeof(float);
-    static bool configured = false;                      // (with the static arrays over 48 KB at 128)
+int output(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
+    constexpr int smem = 2 * C * (C + BN) * (int)sizeof(float);
+    static bool configured = false;
     if (!configured) {
-        int rc = (int)cudaFuncSetAttribute(chunk_update_kernel<MODE, BN>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (!rc)
-            rc = (int)cudaFuncSetAttribute(chunk_output_kernel<MODE, BN>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const int rc = (int)cudaFuncSetAttribute(chunk_output_kernel<MODE, BN>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (rc) return rc;
         configured = true;
     }
-    const dim3 grid(update ? ((a.e + C - 1) / C) * ((a.f + BN - 1) / BN) : (a.f + BN - 1) / BN, a.n_heads,
-                    a.n_requests * span);
-    if (update)
-        MLS_LAUNCH((chunk_update_kernel<MODE, BN>), grid, dim3(BN), smem, stream, a, s, first, span);
-    else
-        MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(BN), smem, stream, a, s, first, span);
+    const dim3 grid((a.f + BN - 1) / BN, a.n_heads, a.n_requests * span);
+    MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(2 * BN), smem, stream, a, s, first, span);
     return launch_status();
 }
 
@@ -775,18 +808,15 @@ int window(const Args& a, const Scratch& s, int first, int span, cudaStream_t st
         MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, a.n_requests * span), dim3(256), 0,
                    stream, a, s, first, span);
     }
-    // tiles of 64 x 128 where the values fill them, else of 64 x 64
-    const bool wide = a.f % 128 == 0 || a.f > 192;
-    int rc = wide ? products<MODE, 128>(a, s, first, span, true, stream)
-                  : products<MODE, 64>(a, s, first, span, true, stream);
+    int rc = update<MODE>(a, s, first, span, stream);
     if (rc) return rc;
     const int quads = state_floats(MODE, a.e, a.f) / 4;
     MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, a.n_requests), dim3(128),
                0, stream, a, s, first, span);
     rc = launch_status();
     if (rc) return rc;
-    return wide ? products<MODE, 128>(a, s, first, span, false, stream)
-                : products<MODE, 64>(a, s, first, span, false, stream);
+    // (a width of 64 leaves half of a wider tile empty)
+    return a.f <= C ? output<MODE, 64>(a, s, first, span, stream) : output<MODE, 128>(a, s, first, span, stream);
 }
 }  // namespace
 
