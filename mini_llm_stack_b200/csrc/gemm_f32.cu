@@ -241,9 +241,10 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
 // of a block share rows, so all but the first read of a row meets L1.  The 32 partial sums are
 // added by a fixed tree.  The order of the additions depends on K alone (never on M, on COLS or
 // on the row's place), and which kernel runs depends on N alone, so a token's result still does
-// not depend on its batch: many rows take eight or nine columns a warp, few rows one.  Measured
-// against blocks of eight rows in shared memory, whose loads bounded it: 2,048 x 65 x 4,096 from
-// bfloat16 rows 115 -> 45 us, 300 x 64 x 4,096 46 -> 19, 2,048 x 8 x 2,048 25 -> 12.
+// not depend on its batch: many rows take eight or nine columns a warp, fewer rows two, a decode
+// step's one.  Measured against blocks of eight rows in shared memory, whose loads bounded it:
+// 2,048 x 65 x 4,096 from bfloat16 rows 115 -> 45 us, 300 x 64 x 4,096 46 -> 16,
+// 2,048 x 8 x 2,048 25 -> 8.
 constexpr int SKINNY_N = 256, SK_ROWS = 8;
 
 // BY4: four entries of a row of W at a time; VEC: of A as well.
@@ -270,7 +271,7 @@ gemm_f32_skinny_kernel(const T* __restrict__ A, const float* __restrict__ W, flo
     const float* w_row = W + (size_t)n0 * K;
     const int last = N - 1 - n0;
     if (BY4) {
-#pragma unroll (COLS == 1 ? 4 : 2)
+#pragma unroll 2
         for (int k = lane * 4; k < K; k += 128) {
             float4 a[SK_ROWS];
 #pragma unroll
@@ -375,11 +376,15 @@ int skinny(const T* A, const float* W, float* out, int M, int N, int K, cudaStre
                    dim3(256), 0, stream, A, W, out, M, N, K);                                      \
         return launch_status();                                                                    \
     } while (0)
-    // columns a warp: eight, or nine where that saves a group (64 router outputs and a gate's
-    // column), while that leaves four warps an SM; else four
-    const int cols = (N + 8) / 9 < (N + 7) / 8 ? 9 : 8;
-    if ((long long)groups * ((N + cols - 1) / cols) < 4LL * sm_count()) SKINNY(4);
-    if (cols == 9) SKINNY(9);
+    // Two columns a warp while those blocks are one wave (two an SM fit their registers): it is
+    // then a warp's own chain of loads that counts, and a third of the registers lets more of them
+    // be under way (512 x 64 x 4,096 from bfloat16 rows, after a flush of L2: 39 us with four
+    // columns, 32 with eight, 23 with two; 128 x 128 x 2,048: 23, 19, 15).  Past that, A is read
+    // once for eight columns (2,048 x 64 x 4,096: 102, 56, 62), or nine where that saves a group
+    // (64 router outputs and a gate's column).  With float32 rows nine is the faster of the two
+    // throughout (1,500 x 64 x 2,048: 45 us with eight, 36 with nine).
+    if ((long long)groups * ((N + 1) / 2) <= 8LL * 2 * sm_count()) SKINNY(2);
+    if (sizeof(T) == 4 || (N + 8) / 9 < (N + 7) / 8) SKINNY(9);
     SKINNY(8);
 #undef SKINNY
 }

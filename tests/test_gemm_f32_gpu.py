@@ -17,7 +17,8 @@ def ops():
 @pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("m, n, k", [
     (1, 257, 16), (31, 300, 17), (33, 5120, 40), (65, 19000, 64), (97, 9473, 33), (64, 9472, 4),
-    (1, 1, 1), (3, 1000, 132), (8, 260, 64), (5, 19001, 72), (63, 65, 130), (64, 65, 132), (65, 9, 36), (700, 65, 256), (130, 256, 1028), (2100, 8, 24)])
+    (1, 1, 1), (3, 1000, 132), (8, 260, 64), (5, 19001, 72), (63, 65, 130), (64, 65, 132), (65, 9, 36), (700, 65, 256), (130, 256, 1028), (2100, 8, 24),
+    (1501, 64, 132), (1200, 64, 65)])
 def test_product(ops, a_type, m, n, k):
     g = torch.Generator(device="cuda").manual_seed(m * n + k)
     a = torch.randn(m, k, device="cuda", generator=g).to(a_type)
