@@ -130,13 +130,13 @@ __device__ __forceinline__ void fill_rows(float (*T)[W], Get get) {
     }
 }
 
-// acc += A x B over 64 of k: thread (ty, tx) owns rows 4 ty .. + 3 and 32 further on, columns
+// acc += A x B over DEPTH of k, from k0: thread (ty, tx) owns rows 4 ty .. + 3 and 32 further on, columns
 // 4 tx .. + 3 and, with eight columns a thread (TN), BN / 2 further on.
-template <int BN, int TN, bool TURN_A>
+template <int BN, int TN, bool TURN_A, int DEPTH = C>
 __device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*A)[C], const float (*B)[BN],
-                                         int tx, int ty) {
+                                         int tx, int ty, int k0 = 0) {
 #pragma unroll 8
-    for (int k = 0; k < C; ++k) {
+    for (int k = k0; k < k0 + DEPTH; ++k) {
         const int ra = TURN_A ? (4 * ty) ^ turn(k) : 4 * ty;
         float v[8];
         *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(&A[k][ra]);
@@ -156,8 +156,10 @@ __device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*
         }
     }
 }
-// Sums of several blocks of 64 are kept apart from the block being multiplied: chains of 64
-// roundings and one a block, not one chain of e + 64.
+// Outputs and scores add up over runs of 16 of k, kept apart from the run being multiplied: chains of
+// 16 roundings and one a run, as exact as the token-by-token kernels' sums (chains of 64: 1.2 times
+// their error at 130 tokens).
+constexpr int SUMS = 16;
 template <int N>
 __device__ __forceinline__ void settle(f32x2 (&sum)[N], f32x2 (&acc)[N]) {
 #pragma unroll
@@ -251,9 +253,10 @@ chunk_scores_kernel(const Args a, const Scratch s, int first, int span) {
                 fma2(acc[i][0], two, b.x);
                 fma2(acc[i][1], two, b.y);
             }
-        }
+            if (x % SUMS == SUMS - 1)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) settle(sum[i], acc[i]);
+                for (int y = 0; y < 4; ++y) settle(sum[y], acc[y]);
+        }
     }
     float* P = s.scores + (w.idx * a.n_heads + head) * C * C;
 #pragma unroll
@@ -728,9 +731,12 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
             if (with_n && threadIdx.x < C && i0 + (int)threadIdx.x < a.e)
                 n_next = S[(size_t)a.e * a.f + i0 + threadIdx.x];
         }
-        multiply<BN, TN, true>(acc, A[x], B[x], tx, ty);
+#pragma unroll 1
+        for (int k0 = 0; k0 < C; k0 += SUMS) {
+            multiply<BN, TN, true, SUMS>(acc, A[x], B[x], tx, ty, k0);
 #pragma unroll
-        for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
+            for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
+        }
         if (with_n && threadIdx.x < C) {
 #pragma unroll 8
             for (int y = 0; y < C; ++y) nq[y & 7] = fmaf(A[x][y][threadIdx.x ^ turn(y)], n_s[x][y], nq[y & 7]);
