@@ -284,11 +284,10 @@ constexpr int RUN = 16, RUNS = C / RUN, STEP = 4, STEPS = C / STEP;
 __device__ __forceinline__ float4 mul4(float4 x, float4 y) {
     return make_float4(x.x * y.x, x.y * y.y, x.z * y.z, x.w * y.w);
 }
+// Four products added up by themselves first: chains of e / 4 of them stay as exact as the
+// token-by-token kernel's.
 __device__ __forceinline__ float dot4(float4 x, float4 y, float v) {
-    v = fmaf(x.x, y.x, v);
-    v = fmaf(x.y, y.y, v);
-    v = fmaf(x.z, y.z, v);
-    return fmaf(x.w, y.w, v);
+    return v + fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, x.x * y.x)));
 }
 // Weights of four queries (from row t) and two keys (from row j) whose factors carry the decays up
 // to the gap between them; `gap`: rows of decays between (gaps of them, e apart).
@@ -589,9 +588,20 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     fill_rows<THREADS, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
     __syncthreads();
     const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
-    f32x2 acc[8][TN / 2];
-    clear(acc);
-    multiply<BN, TN, false>(acc, A, B, tx, ty);
+    f32x2 sum[8][TN / 2];
+    clear(sum);
+    if (MODE == TOKEN_DECAY) {                             // its factors are rounded already: short chains
+        f32x2 acc[8][TN / 2];
+        clear(acc);
+#pragma unroll 1
+        for (int k0 = 0; k0 < C; k0 += SUMS) {
+            multiply<BN, TN, false, SUMS>(acc, A, B, tx, ty, k0);
+#pragma unroll
+            for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
+        }
+    } else {
+        multiply<BN, TN, false>(sum, A, B, tx, ty);
+    }
     float* U = s.states + (w.idx * a.n_heads + head) * state_floats(MODE, a.e, a.f);
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
@@ -600,7 +610,7 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
 #pragma unroll
         for (int h = 0; h < TN / 4; ++h) {
             const int j = j0 + 4 * tx + (BN / 2) * h;
-            const float2 lo = halves(acc[x][2 * h]), hi = halves(acc[x][2 * h + 1]);
+            const float2 lo = halves(sum[x][2 * h]), hi = halves(sum[x][2 * h + 1]);
             if (j < a.f)
                 *reinterpret_cast<float4*>(U + (size_t)i * a.f + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
