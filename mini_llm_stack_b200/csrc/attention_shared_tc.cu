@@ -48,7 +48,8 @@ constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.0f;             // log2: P stays below 2^8
 
 constexpr int B_K_FULL = 0, B_K_EMPTY = STAGES, B_S_FULL = 2 * STAGES, B_P_FULL = B_S_FULL + 2,
-              B_O_REST = B_P_FULL + 2, B_Q_FULL = B_O_REST + 1, N_BARS = B_Q_FULL + 1;
+              B_O_REST = B_P_FULL + 2, B_O_LAST = B_O_REST + 1, B_Q_FULL = B_O_LAST + 1,
+              N_BARS = B_Q_FULL + 1;
 constexpr int SMEM_BYTES = Q_BYTES + STAGES * K_STAGE + 8 * N_BARS + 16;
 
 struct Params {
@@ -120,6 +121,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
             mbar_init(bar(B_P_FULL + b), ROWS);
         }
         mbar_init(bar(B_O_REST), 1);
+        mbar_init(bar(B_O_LAST), 1);
         mbar_init(bar(B_Q_FULL), ROWS);
         fence_barrier_init();
     }
@@ -222,7 +224,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 for (int kk = 0; kk < BN / 16; ++kk)
                     umma_ts(tmem + COL_O, tmem + (i & 1) * 128 + kk * 8,
                             umma_desc_mn(v_src + kk * 16 * 128, KBLOCK), idesc_o, (i | kk) ? 1u : 0u);
-                umma_commit(bar(B_O_REST));                    // O holds step i
+                umma_commit(bar(i + 1 < steps ? B_O_REST : B_O_LAST));   // O holds step i
                 umma_commit(bar(B_K_EMPTY + i % STAGES));      // the tile has been read both ways
                 if (i + 2 < steps && !issue_s(i + 2)) timed_out = true;
             }
@@ -342,9 +344,10 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
             tc_fence_before();
             mbar_arrive(bar(B_P_FULL + (i & 1)));
         }
-        // the last two products, in order: the last scores were ready before either of them
-        if (!timed_out && steps > 1 && !mbar_wait(bar(B_O_REST), (steps - 2) & 1)) timed_out = true;
-        if (!timed_out && !mbar_wait(bar(B_O_REST), (steps - 1) & 1)) timed_out = true;
+        // All products are done once the last one is (they run in order).  It has a barrier of its own:
+        // behind this thread's last arrival two phases of O_REST could end before it looks, and a parity
+        // cannot tell a phase from the one two further on.
+        if (!timed_out && !mbar_wait(bar(B_O_LAST), 0)) timed_out = true;
         tc_fence_after();
         if (P.sink && live && m_used != -INFINITY)
             l += exp2f(P.sink[kvh * P.group + g] * LOG2E - m_used);

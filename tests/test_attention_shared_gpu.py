@@ -70,3 +70,33 @@ def test_against_a_warp_a_row(ops, monkeypatch, heads, block, lens, before, scat
     # outputs are averages of unit rows: P is rounded to 8 bits (2^-9 of a sum of weights at most 1,
     # times values of up to some 4), the result once more
     assert (got["auto"] - got["simt"]).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * got["simt"].abs().max()
+
+
+def test_every_tile_ends(ops):
+    """Tiles of one to eight steps, many times over: the end of a tile is told by a barrier of its own,
+    so that no wait looks for a phase that two later ones have passed.  The same bits every time."""
+    lens, heads, block = [96 * n - 3 for n in range(1, 9)], 8, 16
+    t, r = sum(lens), len(lens)
+    width = -(-max(lens) // block)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    step = SimpleNamespace(
+        n_tokens=t, n_requests=r, q_lens=lens, ctx_lens=lens, max_ctx_len=max(lens), attn_tiles={},
+        positions=torch.cat([torch.arange(n) for n in lens]).to(**i32),
+        cu_q=torch.tensor(cu, **i32), ctx_len=torch.tensor([*lens, max(lens)], **i32),
+        req_of_token=torch.repeat_interleave(torch.arange(r), torch.tensor(lens)).to(**i32),
+        groups={0: GroupView(torch.arange(r * width, **i32).view(r, width), None, block, width)})
+    g = torch.Generator(device="cuda").manual_seed(3)
+    pool = torch.randn(1, r * width, block, HD, device="cuda", generator=g).bfloat16()
+    cache = SimpleNamespace(group=0, k_pool=pool, v_pool=pool)
+    qkv = torch.randn(t, (heads + 2) * HD, device="cuda", generator=g).bfloat16()
+    plan = plan_paged_attention(step, dict(ops.attention_facts(HD)), heads, 1, HD)
+    first = None
+    for _ in range(200):
+        out = torch.full((t, heads * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(qkv, out, cache, step, heads, 1, HD, HD ** -0.5, 0, plan=plan)
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    ops.check_status()
