@@ -6,18 +6,27 @@
 // tile of keys is brought in once and read twice, as the K-major operand of S = Q K^T and as the
 // MN-major one of O += P V, and one chain of 128 rows keeps two score buffers, so that the
 // tensor cores work on step i + 2's scores and step i's outputs while the softmax takes step i + 1.
-// Tiles of 96 keys: three of them fit beside Q (48 KB each and 64 KB), and a step's products (16
-// instructions of 128 x 96 and 6 of 128 x 256, some 3,800 cycles) outlast the softmax of its
-// 96 scores a thread.
+// Tiles of 96 keys: three of them fit beside Q (48 KB each and 64 KB).
+//
+// The running maximum that the weights are taken against may lag behind by up to 2^8, so the largest
+// weights of a row are not 1 but any number, and one bfloat16 would round each of them: on peaked rows
+// two to three times the error of kernels that rescale at every new maximum.  A weight is therefore
+// two bfloat16, the number rounded and what that left (16 bits together), and O += P V twice the
+// instructions.  Distance from float64, 700 tokens of 8 heads, the output's own rounding included, for scores
+// of deviation 1, 2 and 5: 1.58e-3, 1.64e-3, 1.65e-3; with one bfloat16 a weight 1.95e-3 and more; the
+// mma.sync tiles 1.90e-3, 1.80e-3, 1.70e-3.
 //
 //   warp 0      brings the tiles in with TMA, one copy per page and 64-wide quarter (one per quarter
 //               for a run of consecutive pages);
 //   warp 1      issues the products (tcgen05.mma);
-//   warps 2..5  softmax, one thread a row: read S, mask, exponentiate, write P over it as bfloat16,
+//   warps 2..5  softmax, one thread a row: read S, mask, exponentiate, write P over it as two bfloat16,
 //               rescale O when the running maximum has grown by more than 2^8, store O at the end.
 //
 // Measured against the mma.sync tiles (attention_mma.cu) on 32 heads over one latent of 256, prompts
-// of 682 and 1,366 tokens: 230 -> 70 us (545 TFLOP/s of causal arithmetic).
+// of 682 and 1,366 tokens: 230 -> 82 us (70 with one bfloat16 a weight: a step's products then were
+// 12.6 MFLOP and are 18.9 now, half as much again for 16 % of the time, so it is the softmax, one warp a
+// scheduler, that most of a step waits for; at the measured 1.65 PFLOP/s the products of a step take
+// about 3,100 cycles).
 // Every wait is bounded and reports MLS_STATUS_TIMEOUT.
 #include "common.cuh"
 #include "tma.cuh"
@@ -221,9 +230,10 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 tc_fence_after();
                 const uint32_t v_src = k_smem + (i % STAGES) * K_STAGE;
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; ++kk)
+                for (int kk = 0; kk < 2 * (BN / 16); ++kk)     // the weights' upper halves, then the rest
                     umma_ts(tmem + COL_O, tmem + (i & 1) * 128 + kk * 8,
-                            umma_desc_mn(v_src + kk * 16 * 128, KBLOCK), idesc_o, (i | kk) ? 1u : 0u);
+                            umma_desc_mn(v_src + kk % (BN / 16) * 16 * 128, KBLOCK), idesc_o,
+                            (i | kk) ? 1u : 0u);
                 umma_commit(bar(i + 1 < steps ? B_O_REST : B_O_LAST));   // O holds step i
                 umma_commit(bar(B_K_EMPTY + i % STAGES));      // the tile has been read both ways
                 if (i + 2 < steps && !issue_s(i + 2)) timed_out = true;
@@ -328,7 +338,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
             float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c0 = 0; c0 < BN; c0 += 32) {
-                uint32_t pk[16];
+                uint32_t pk[16], rest[16];
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
                     const float p0 = fast_exp2(fmaf(sc[c0 + 2 * u], P.scale_log2, neg_m));
@@ -336,8 +346,11 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                     part[u & 3] += p0 + p1;
                     __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
                     pk[u] = *reinterpret_cast<uint32_t*>(&h);
+                    h = __floats2bfloat162_rn(p0 - __low2float(h), p1 - __high2float(h));
+                    rest[u] = *reinterpret_cast<uint32_t*>(&h);
                 }
                 tmem_st16(s_addr + c0 / 2, pk);
+                tmem_st16(s_addr + (BN + c0) / 2, rest);
             }
             l += (part[0] + part[1]) + (part[2] + part[3]);
             tmem_st_wait();                      // P and a rescaled O are in place

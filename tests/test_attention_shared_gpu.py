@@ -100,3 +100,48 @@ def test_every_tile_ends(ops):
         first = out if first is None else first
         assert torch.equal(out, first)
     ops.check_status()
+
+
+@pytest.mark.parametrize("peak", [1.0, 2.0, 5.0])
+@pytest.mark.parametrize("heads, kv", [(8, 1), (6, 2)])
+def test_no_further_from_float64_than_the_tiles_it_replaces(ops, monkeypatch, peak, heads, kv):
+    """Flat and peaked weights (scores of deviation ``peak``), beside the mma.sync tiles."""
+    lens, block = [700, 45], 16
+    t, r = sum(lens), len(lens)
+    width = -(-max(lens) // block)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    order = torch.randperm(r * width, generator=torch.Generator().manual_seed(2)).view(r, width)
+    step = SimpleNamespace(
+        n_tokens=t, n_requests=r, q_lens=lens, ctx_lens=lens, max_ctx_len=max(lens), attn_tiles={},
+        positions=torch.cat([torch.arange(n) for n in lens]).to(**i32),
+        cu_q=torch.tensor([0, lens[0], t], **i32), ctx_len=torch.tensor([*lens, max(lens)], **i32),
+        req_of_token=torch.repeat_interleave(torch.arange(r), torch.tensor(lens)).to(**i32),
+        groups={0: GroupView(order.to(**i32), None, block, width)})
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    rows = torch.randn(kv, t, HD, device="cuda", generator=g).bfloat16()
+    pool = torch.zeros(kv, r * width, block, HD, dtype=torch.bfloat16, device="cuda")
+    at = 0
+    for i, n in enumerate(lens):
+        for j in range(n):
+            pool[:, int(order[i, j // block]), j % block] = rows[:, at + j]
+        at += n
+    cache = SimpleNamespace(group=0, k_pool=pool, v_pool=pool)
+    qkv = torch.randn(t, (heads + 2 * kv) * HD, device="cuda", generator=g).mul_(peak).bfloat16()
+    plan = plan_paged_attention(step, dict(ops.attention_facts(HD)), heads, kv, HD)
+    want, at = torch.empty(t, heads, HD, dtype=torch.float64, device="cuda"), 0
+    for n in lens:
+        hidden = torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1)
+        for h in range(heads):
+            k = rows[h // (heads // kv), at:at + n].double()
+            s = qkv[at:at + n, h * HD:(h + 1) * HD].double() @ k.T * HD ** -0.5
+            want[at:at + n, h] = torch.softmax(s.masked_fill(hidden, float("-inf")), -1) @ k
+        at += n
+    far = {}
+    for impl in ("auto", "mma"):
+        monkeypatch.setattr(ops, "attention_impl", impl)
+        out = torch.full((t, heads * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(qkv, out, cache, step, heads, kv, HD, HD ** -0.5, 0, plan=plan)
+        far[impl] = float((out.double().view_as(want) - want).norm() / want.norm())
+    ops.check_status()
+    print(heads, kv, peak, far)
+    assert far["auto"] <= 1.01 * far["mma"], far          # both are rounded to 8 bits once, which is most of it
