@@ -13,8 +13,8 @@
 // two to three times the error of kernels that rescale at every new maximum.  A weight is therefore
 // two bfloat16, the number rounded and what that left (16 bits together), and O += P V twice the
 // instructions.  Distance from float64, 700 tokens of 8 heads, the output's own rounding included, for scores
-// of deviation 1, 2 and 5: 1.58e-3, 1.64e-3, 1.65e-3; with one bfloat16 a weight 1.95e-3 and more; the
-// mma.sync tiles 1.90e-3, 1.80e-3, 1.70e-3.
+// of deviation 1, 2 and 5: 1.58e-3, 1.64e-3, 1.65e-3; with one bfloat16 a weight 1.93e-3, 1.95e-3, 1.96e-3;
+// the mma.sync tiles 1.90e-3, 1.80e-3, 1.70e-3.
 //
 //   warp 0      brings the tiles in with TMA, one copy per page and 64-wide quarter (one per quarter
 //               for a run of consecutive pages);
@@ -439,7 +439,9 @@ MLS_API int mls_attention_shared_tc(const void* qkv, void* out, const void* pool
                                     cudaStream_t stream) {
 #if MLS_HEAD_DIM == 256
     if (n_tiles <= 0 || n_req <= 0) return 0;
-    if (n_heads % n_kv || share < 1 || !mls_attention_shared_tc_takes(block_size) || out_stride % 8)
+    if (n_heads % n_kv || share < 1 || !mls_attention_shared_tc_takes(block_size) || out_stride % 8 ||
+        (reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) |
+         reinterpret_cast<uintptr_t>(pool)) % 16)
         return MLS_ERR_UNSUPPORTED;
     static bool configured = false;
     if (!configured) {

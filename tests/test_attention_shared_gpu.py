@@ -145,3 +145,61 @@ def test_no_further_from_float64_than_the_tiles_it_replaces(ops, monkeypatch, pe
     ops.check_status()
     print(heads, kv, peak, far)
     assert far["auto"] <= 1.01 * far["mma"], far          # both are rounded to 8 bits once, which is most of it
+
+
+def prompts(ops, heads=4, kv=1, lens=(130, 40), block=16):
+    """A step of whole prompts over pages in order: (step, cache, qkv, plan)."""
+    t, r = sum(lens), len(lens)
+    width = -(-max(lens) // block)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    step = SimpleNamespace(
+        n_tokens=t, n_requests=r, q_lens=list(lens), ctx_lens=list(lens), max_ctx_len=max(lens), attn_tiles={},
+        positions=torch.cat([torch.arange(n) for n in lens]).to(**i32),
+        cu_q=torch.tensor(cu, **i32), ctx_len=torch.tensor([*lens, max(lens)], **i32),
+        req_of_token=torch.repeat_interleave(torch.arange(r), torch.tensor(lens)).to(**i32),
+        groups={0: GroupView(torch.arange(r * width, **i32).view(r, width), None, block, width)})
+    g = torch.Generator(device="cuda").manual_seed(11)
+    pool = torch.randn(kv, r * width, block, HD, device="cuda", generator=g).bfloat16()
+    qkv = torch.randn(t, (heads + 2 * kv) * HD, device="cuda", generator=g).bfloat16()
+    plan = plan_paged_attention(step, dict(ops.attention_facts(HD)), heads, kv, HD)
+    return step, SimpleNamespace(group=0, k_pool=pool, v_pool=pool), qkv, plan
+
+
+@pytest.fixture
+def taken(ops, monkeypatch):
+    """Calls that the kernel for shared rows took."""
+    takes, fn = ops._attention_shared[HD]
+    calls = []
+
+    def counted(*args):
+        calls.append(args)
+        return fn(*args)
+
+    monkeypatch.setitem(ops._attention_shared, HD, (takes, counted))
+    return calls
+
+
+def by_warps(ops, monkeypatch, step, cache, qkv, heads, kv, scale):
+    with monkeypatch.context() as m:
+        m.setattr(ops, "attention_impl", "simt")
+        out = torch.empty(step.n_tokens, heads * HD, dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(qkv, out, cache, step, heads, kv, HD, scale, 0)
+    return out.float()
+
+
+@pytest.mark.parametrize("first", [0, 4, 8, 12])
+def test_columns_of_a_wider_buffer(ops, monkeypatch, taken, first):
+    """Output rows that start between 16-byte addresses are the mma.sync tiles'."""
+    heads, scale = 4, HD ** -0.5
+    step, cache, qkv, plan = prompts(ops, heads)
+    wide = torch.full((step.n_tokens, heads * HD + 16), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = wide[:, first:first + heads * HD]
+    ops.paged_attention(qkv, out, cache, step, heads, 1, HD, scale, 0, plan=plan)
+    ops.check_status()
+    assert len(taken) == (1 if first % 8 == 0 else 0)
+    want = by_warps(ops, monkeypatch, step, cache, qkv, heads, 1, scale)
+    assert (out.float() - want).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * want.abs().max()
+    assert (wide[:, :first] == 7.0).all() and (wide[:, first + heads * HD:] == 7.0).all()
