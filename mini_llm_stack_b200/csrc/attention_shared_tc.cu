@@ -440,6 +440,7 @@ MLS_API int mls_attention_shared_tc(const void* qkv, void* out, const void* pool
 #if MLS_HEAD_DIM == 256
     if (n_tiles <= 0 || n_req <= 0) return 0;
     if (n_heads % n_kv || share < 1 || !mls_attention_shared_tc_takes(block_size) || out_stride % 8 ||
+        !(scale > 0.f) ||
         (reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) |
          reinterpret_cast<uintptr_t>(pool)) % 16)
         return MLS_ERR_UNSUPPORTED;

@@ -644,9 +644,10 @@ class Ops:
             if (n_tiles and self.attention_impl == "auto" and plain and not softcap
                     and cache.k_pool.data_ptr() == cache.v_pool.data_ptr()
                     and (out.data_ptr() | qkv.data_ptr() | cache.k_pool.data_ptr()) % 16 == 0
-                    and self._attention_shared[hd][0](g.block_size)):
+                    and scale > 0 and self._attention_shared[hd][0](g.block_size)):
                 # the same where one cached row is key and value (attention over a latent); rows are
-                # read and written 16 bytes at a time (the mma.sync tiles write four)
+                # read and written 16 bytes at a time (the mma.sync tiles write four), and the
+                # largest score is looked for before the scale is applied
                 self.launches += 1
                 _check(self._attention_shared[hd][1](
                     _ptr(qkv), _ptr(out), _ptr(cache.k_pool), _ptr(g.block_table), g.max_blocks,

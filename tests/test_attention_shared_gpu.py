@@ -203,3 +203,15 @@ def test_columns_of_a_wider_buffer(ops, monkeypatch, taken, first):
     want = by_warps(ops, monkeypatch, step, cache, qkv, heads, 1, scale)
     assert (out.float() - want).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * want.abs().max()
     assert (wide[:, :first] == 7.0).all() and (wide[:, first + heads * HD:] == 7.0).all()
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.0625])
+def test_scales_that_are_not_positive(ops, monkeypatch, taken, scale):
+    """The kernel takes the maximum of scores before they are scaled: such calls are the tiles'."""
+    step, cache, qkv, plan = prompts(ops)
+    out = torch.full((step.n_tokens, 4 * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(qkv, out, cache, step, 4, 1, HD, scale, 0, plan=plan)
+    ops.check_status()
+    want = by_warps(ops, monkeypatch, step, cache, qkv, 4, 1, scale)
+    assert (out.float() - want).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * want.abs().max()
+    assert not taken
