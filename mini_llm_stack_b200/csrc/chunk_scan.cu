@@ -75,27 +75,48 @@ struct Where {
     size_t idx;                      // place among the window's chunks
 };
 
-// Block z of the grid: request z / span, chunk first + z % span.  Every thread calls; false: none.
+// Chunk z of the window's chunks, or (REQUEST) the first one of request z of those that go chunk by
+// chunk: a request's length alone says whether it does.  Every thread calls; false: none.
+template <bool REQUEST>
 __device__ __forceinline__ bool locate(const Args& a, int first, int span, int z, Where& w) {
-    __shared__ int before_s;
-    w.r = z / span;
-    const int j = z - w.r * span;
-    w.c = first + j;
+    __shared__ int at_s[2];          // request, place of its first chunk
     if (threadIdx.x < 32) {
-        // chunks of the window in the requests before this one
-        int sum = 0;
-        for (int r = threadIdx.x; r < w.r; r += 32) {
-            const int all = (a.cu_q[r + 1] - a.cu_q[r] + C - 1) / C;
-            sum += min(max(all - first, 0), span);
-        }
+        const int lane = threadIdx.x;
+        int taken = 0, before = 0;   // requests that go chunk by chunk and chunks before these 32
+        if (lane == 0) at_s[0] = -1;
+        __syncwarp();
+        for (int r0 = 0; r0 < a.n_requests; r0 += 32) {
+            const int r = r0 + lane;
+            const int len = r < a.n_requests ? a.cu_q[r + 1] - a.cu_q[r] : 0;
+            const bool in = len >= a.least;
+            const unsigned all = __ballot_sync(0xffffffffu, in);
+            const int k = taken + __popc(all & ((1u << lane) - 1u));
+            const int count = in ? min(max((len + C - 1) / C - first, 0), span) : 0;
+            int sum = count;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (threadIdx.x == 0) before_s = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += x;
+            }
+            const int start = before + sum - count;
+            const bool here = REQUEST ? in && k == z : z >= start && z < start + count;
+            if (here) {
+                at_s[0] = r;
+                at_s[1] = start;
+            }
+            if (__any_sync(0xffffffffu, here)) break;
+            taken += __popc(all);
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
     }
     __syncthreads();
+    w.r = at_s[0];
+    if (w.r < 0) return false;
+    const int j = REQUEST ? 0 : z - at_s[1];
+    w.c = first + j;
     const int t = a.cu_q[w.r], len = a.cu_q[w.r + 1] - t;
     w.chunks = min(max((len + C - 1) / C - first, 0), span);
-    w.idx = (size_t)before_s + j;
+    w.idx = (size_t)(at_s[1] + j);
     w.t0 = t + w.c * C;
     w.n = min(C, len - w.c * C);
     return j < w.chunks;
@@ -216,7 +237,7 @@ chunk_scores_kernel(const Args a, const Scratch s, int first, int span) {
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
     __shared__ __align__(16) float A[C][C], B[C][C];
     __shared__ float power[C];
     __shared__ double la[C], lb[C];
@@ -324,7 +345,7 @@ chunk_scores_token_kernel(const Args a, const Scratch s, int first, int span) {
     Where w;
     const int quads = QUADS ? QUADS : a.e / 4, e = 4 * quads, pad = e + 4;
     const int head = blockIdx.y;
-    if (!locate(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
     extern __shared__ __align__(16) float sm[];
     float* r_s = sm;                                     // [64][pad]
     float* k_s = r_s + C * pad;                          // [64][pad]
@@ -471,7 +492,7 @@ chunk_gates_kernel(const Args a, const Scratch s, int first, int span) {
     __shared__ float m_s[GATE_WARPS + 1];
     const int head = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Where w;
-    if (!locate(a, first, span, blockIdx.y * span, w)) return;
+    if (!locate<true>(a, first, span, blockIdx.y, w)) return;
     float* m_slot = a.state + (size_t)a.state_slot[w.r] * a.slot_stride + (size_t)head * a.head_stride +
                     state_floats(MLSTM, a.e, a.f);
     const float bi = load_as_float(a.bias_i, head, a.bias_dtype),
@@ -572,7 +593,7 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
     constexpr int BN = C, TN = 4, THREADS = 128;
     __shared__ __align__(16) float A[C][C], B[C][BN];
     __shared__ float factor[C];
@@ -633,7 +654,7 @@ chunk_carry_kernel(const Args a, const Scratch s, int first, int span) {
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate(a, first, span, blockIdx.z * span, w)) return;
+    if (!locate<true>(a, first, span, blockIdx.z, w)) return;
     const int size = state_floats(MODE, a.e, a.f);
     const int at = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (at >= size) return;
@@ -687,7 +708,7 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
     chain_wait();
     Where w;
     const int head = blockIdx.y, j0 = blockIdx.x * BN;
-    if (!locate(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
     constexpr int THREADS = 2 * BN, TN = 4, QA = C * (C / 4) / THREADS;      // quads of A a thread brings in
     extern __shared__ __align__(16) float tiles[];
     float(*A)[C][C] = reinterpret_cast<float(*)[C][C]>(tiles);
@@ -784,13 +805,13 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
 }
 
 template <int MODE>
-int update(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
-    const dim3 grid(((a.e + C - 1) / C) * ((a.f + C - 1) / C), a.n_heads, a.n_requests * span);
+int update(const Args& a, const Scratch& s, int chunks, int first, int span, cudaStream_t stream) {
+    const dim3 grid(((a.e + C - 1) / C) * ((a.f + C - 1) / C), a.n_heads, chunks);
     MLS_LAUNCH((chunk_update_kernel<MODE>), grid, dim3(128), 0, stream, a, s, first, span);
     return launch_status();
 }
 template <int MODE, int BN>
-int output(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
+int output(const Args& a, const Scratch& s, int chunks, int first, int span, cudaStream_t stream) {
     constexpr int smem = 2 * C * (C + BN) * (int)sizeof(float);
     static bool configured = false;
     if (!configured) {
@@ -799,7 +820,7 @@ int output(const Args& a, const Scratch& s, int first, int span, cudaStream_t st
         if (rc) return rc;
         configured = true;
     }
-    const dim3 grid((a.f + BN - 1) / BN, a.n_heads, a.n_requests * span);
+    const dim3 grid((a.f + BN - 1) / BN, a.n_heads, chunks);
     MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(2 * BN), smem, stream, a, s, first, span);
     return launch_status();
 }
@@ -809,30 +830,31 @@ size_t token_smem(int e) {
 }
 
 template <int MODE>
-int window(const Args& a, const Scratch& s, int first, int span, cudaStream_t stream) {
+int window(const Args& a, const Scratch& s, int taken, int chunks, int first, int span, cudaStream_t stream) {
     if (MODE == TOKEN_DECAY) {
         const size_t smem = token_smem(a.e);
         auto kernel = a.e == 64 ? chunk_scores_token_kernel<16> : chunk_scores_token_kernel<0>;
         const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (rc) return rc;
-        MLS_LAUNCH(kernel, dim3(1, a.n_heads, a.n_requests * span), dim3(256), smem,
+        MLS_LAUNCH(kernel, dim3(1, a.n_heads, chunks), dim3(256), smem,
                    stream, a, s, first, span);
     } else {
         if (MODE == MLSTM)
-            MLS_LAUNCH((chunk_gates_kernel), dim3(a.n_heads, a.n_requests), dim3(32 * GATE_WARPS), 0,
+            MLS_LAUNCH((chunk_gates_kernel), dim3(a.n_heads, taken), dim3(32 * GATE_WARPS), 0,
                        stream, a, s, first, span);
-        MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, a.n_requests * span), dim3(256), 0,
+        MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, chunks), dim3(256), 0,
                    stream, a, s, first, span);
     }
-    int rc = update<MODE>(a, s, first, span, stream);
+    int rc = update<MODE>(a, s, chunks, first, span, stream);
     if (rc) return rc;
     const int quads = state_floats(MODE, a.e, a.f) / 4;
-    MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, a.n_requests), dim3(128),
+    MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, taken), dim3(128),
                0, stream, a, s, first, span);
     rc = launch_status();
     if (rc) return rc;
     // (a width of 64 leaves half of a wider tile empty)
-    return a.f <= C ? output<MODE, 64>(a, s, first, span, stream) : output<MODE, 128>(a, s, first, span, stream);
+    return a.f <= C ? output<MODE, 64>(a, s, chunks, first, span, stream)
+                    : output<MODE, 128>(a, s, chunks, first, span, stream);
 }
 }  // namespace
 
@@ -858,9 +880,10 @@ long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long
     return n;
 }
 
-int scan(const Args& a, int most, int window_chunks, long long chunks, float* scratch, cudaStream_t stream) {
-    if (a.n_requests <= 0 || most <= 0) return 0;
-    if ((long long)a.n_requests * window_chunks > 65535) return MLS_ERR_UNSUPPORTED;
+int scan(const Args& a, int taken, int most, int window_chunks, long long chunks, float* scratch,
+         cudaStream_t stream) {
+    if (taken <= 0 || most <= 0) return 0;
+    if (chunks > 65535 || taken > 65535 || a.least < 1) return MLS_ERR_UNSUPPORTED;
     const long long units = chunks * a.n_heads, tokens = (long long)a.n_tokens * a.n_heads;
     Scratch s{};
     float* at = scratch;
@@ -881,9 +904,9 @@ int scan(const Args& a, int most, int window_chunks, long long chunks, float* sc
     for (int first = 0; first < most; first += window_chunks) {
         const int span = most - first < window_chunks ? most - first : window_chunks;
         int rc;
-        if (a.mode == HEAD_DECAY) rc = window<HEAD_DECAY>(a, s, first, span, stream);
-        else if (a.mode == TOKEN_DECAY) rc = window<TOKEN_DECAY>(a, s, first, span, stream);
-        else rc = window<MLSTM>(a, s, first, span, stream);
+        if (a.mode == HEAD_DECAY) rc = window<HEAD_DECAY>(a, s, taken, (int)chunks, first, span, stream);
+        else if (a.mode == TOKEN_DECAY) rc = window<TOKEN_DECAY>(a, s, taken, (int)chunks, first, span, stream);
+        else rc = window<MLSTM>(a, s, taken, (int)chunks, first, span, stream);
         if (rc) return rc;
     }
     return 0;

@@ -38,6 +38,7 @@ struct Args {
     long long slot_stride;           // floats between slots
     int head_stride;                 // floats between the heads of a slot
     int n_requests, n_tokens, n_heads, e, f;
+    int least;                       // requests of at least so many tokens (>= 1); the others are left out
     float* out;                      // [T, H * f]
 };
 
@@ -45,7 +46,7 @@ struct Args {
 bool fits(const Args& a);
 // Floats of scratch for windows of so many chunks in all.
 long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long long chunks);
-// The scan of `most` chunks at most a request, `window` of them at a time.
-int scan(const Args& a, int most, int window, long long chunks_a_window, float* scratch,
+// The scan of `taken` requests, `most` chunks of one at the most, `window` of them at a time.
+int scan(const Args& a, int taken, int most, int window, long long chunks_a_window, float* scratch,
          cudaStream_t stream);
 }  // namespace mls_chunk

@@ -30,6 +30,7 @@
 // `act` = 1 through silu (z * sigmoid(z), float32) as they are loaded.
 #include "chunk_scan.h"
 #include "common.cuh"
+#include <limits.h>
 
 namespace {
 constexpr int LS_COLS = 16;         // columns of S a CTA owns
@@ -71,12 +72,13 @@ linear_scan_kernel(const void* __restrict__ a_src, int a_dtype, int a_row, int a
                    const void* __restrict__ bonus, int bonus_dtype, int read_first,
                    const int* __restrict__ cu_q, const int* __restrict__ state_slot,
                    float* __restrict__ state, long long state_stride,
-                   int n_heads, int e, int f, int tokens_a_pass, float* __restrict__ out, int act) {
+                   int n_heads, int e, int f, int tokens_a_pass, float* __restrict__ out, int act,
+                   int chunked_from) {
     chain_release();
     chain_wait();
     const int r = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * LS_COLS;
     const int t0 = cu_q[r], n = cu_q[r + 1] - t0;
-    if (n <= 0) return;
+    if (n <= 0 || n >= chunked_from) return;              // (longer requests: chunk_scan.cu's)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int grp = lane & (LS_GROUPS - 1);               // row group: the low three lane bits
     const int my_col = warp * 4 + (lane >> 3);
@@ -470,7 +472,7 @@ int launch_scan(dim3 grid, size_t smem, cudaStream_t stream, const void* a_src, 
                 int decay_row, const float* decay_head, const void* bonus, int bonus_dtype,
                 int read_first, const int* cu_q, const int* state_slot, float* state,
                 long long state_stride, int n_heads, int e, int f, int tokens_a_pass, float* out,
-                int act) {
+                int act, int chunked_from) {
     auto kernel = decay_tok ? linear_scan_kernel<RPT, true> : linear_scan_kernel<RPT, false>;
     if (smem > 48 * 1024) {
         const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -480,11 +482,13 @@ int launch_scan(dim3 grid, size_t smem, cudaStream_t stream, const void* a_src, 
     MLS_LAUNCH(kernel, grid, dim3(LS_THREADS), smem, stream, a_src, a_dtype, a_row, a_off, k_src,
                k_dtype, k_row, k_off, v_src, v_dtype, v_row, v_off, decay_tok, decay_row,
                decay_head, bonus, bonus_dtype, read_first, cu_q, state_slot, state, state_stride,
-               n_heads, e, f, tokens_a_pass, out, act);
+               n_heads, e, f, tokens_a_pass, out, act, chunked_from);
     return launch_status();
 }
 }  // namespace
 
+// `chunked_from`: requests of at least so many tokens are left out (mls_linear_scan_chunked takes
+// them); 0: none.
 MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off,
                             const void* k_src, int k_dtype, int k_row, int k_off,
                             const void* v_src, int v_dtype, int v_row, int v_off,
@@ -492,7 +496,7 @@ MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off
                             const void* bonus, int bonus_dtype, int read_first, const int* cu_q,
                             const int* state_slot, float* state, long long state_stride,
                             int n_requests, int n_heads, int e, int f, float* out, int act,
-                            cudaStream_t stream) {
+                            int chunked_from, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (e <= 0 || f <= 0 || e > 32 * LS_GROUPS || (!decay_tok == !decay_head))
         return MLS_ERR_UNSUPPORTED;
@@ -504,7 +508,8 @@ MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off
     return launch_scan<R>(grid, smem, stream, a_src, a_dtype, a_row, a_off, k_src, k_dtype, k_row, \
                           k_off, v_src, v_dtype, v_row, v_off, decay_tok, decay_row, decay_head,  \
                           bonus, bonus_dtype, read_first, cu_q, state_slot, state, state_stride,  \
-                          n_heads, e, f, tokens_a_pass, out, act)
+                          n_heads, e, f, tokens_a_pass, out, act,                                 \
+                          chunked_from > 0 ? chunked_from : INT_MAX)
     if (rpt <= 2) LS_GO(2);
     if (rpt <= 4) LS_GO(4);
     if (rpt <= 8) LS_GO(8);
@@ -514,8 +519,9 @@ MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off
 }
 
 // The same for prompts, chunk by chunk (chunk_scan.cu): a decay per token with the token read first,
-// or one decay a head with the token taken in first and no bonus.  `most`: the most chunks of a
-// request; `window` chunks of every request at a time, `chunks` in all requests together.
+// or one decay a head with the token taken in first and no bonus.  It takes the requests of at least
+// `least` tokens, `taken` of them: `most` chunks of one at the most, `window` of every one at a time,
+// `chunks` in all of them together.
 MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, int a_off,
                                     const void* k_src, int k_dtype, int k_row, int k_off,
                                     const void* v_src, int v_dtype, int v_row, int v_off,
@@ -523,8 +529,8 @@ MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, i
                                     const void* bonus, int bonus_dtype, int read_first,
                                     const int* cu_q, const int* state_slot, float* state,
                                     long long state_stride, int n_requests, int n_tokens,
-                                    int n_heads, int e, int f, float* out, int act, int most,
-                                    int window, long long chunks, float* scratch,
+                                    int n_heads, int e, int f, float* out, int act, int least,
+                                    int taken, int most, int window, long long chunks, float* scratch,
                                     cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
@@ -550,9 +556,10 @@ MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, i
     a.n_heads = n_heads;
     a.e = e;
     a.f = f;
+    a.least = least;
     a.out = out;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
-    return scan(a, most, window, chunks, scratch, stream);
+    return scan(a, taken, most, window, chunks, scratch, stream);
 }
 
 MLS_API int mls_scan_finish(const float* o, const void* gate, int gate_dtype, int gate_row,

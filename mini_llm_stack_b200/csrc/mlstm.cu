@@ -25,9 +25,12 @@
 // are added up once a block, in a fixed order.  All gate
 // arithmetic, the state and the sums are float32; q, k, v and the gate pre-activations
 // come from the projections.  A token's result depends on the tokens before it only
-// through the state, never on the batch or on how the sequence was cut into steps.
+// through the state, never on the batch, and in this kernel not on how the sequence was cut
+// into steps either.  Longer portions of bfloat16 runs go chunk by chunk (chunk_scan.cu), with
+// sums over a chunk's tokens: a request's own portions then say in which order it is added up.
 #include "chunk_scan.h"
 #include "common.cuh"
+#include <limits.h>
 
 namespace {
 constexpr int SCAN_THREADS = 256;
@@ -76,7 +79,7 @@ mlstm_scan_kernel(const T* __restrict__ qkvg, int row_w, int q_off, int k_off, i
                   const void* __restrict__ bias_i, const void* __restrict__ bias_f, int b_dtype,
                   float cap, const int* __restrict__ cu_q, const int* __restrict__ state_slot,
                   float* __restrict__ state, long long slot_stride, int n_heads, int e, int f,
-                  int fc, int n_groups, float* __restrict__ num, float* __restrict__ den) {
+                  int fc, int n_groups, float* __restrict__ num, float* __restrict__ den, int chunked_from) {
     chain_release();
     chain_wait();
     extern __shared__ float sm[];
@@ -121,6 +124,8 @@ mlstm_scan_kernel(const T* __restrict__ qkvg, int row_w, int q_off, int k_off, i
     const bool vload = e % V == 0 && row_w % V == 0 && q_off % V == 0 && k_off % V == 0 &&
                        reinterpret_cast<uintptr_t>(qkvg) % 16 == 0;
 
+    // (longer requests are chunk_scan.cu's; asked here, the state's loads need not wait for the lengths)
+    if (t1 - t0 >= chunked_from) return;
     for (int tb = t0; tb < t1; tb += TB) {
         const int nb = min(TB, t1 - tb);
         // ---- the block's inputs (16 bytes a load where the layout allows)
@@ -332,7 +337,7 @@ int launch_scan(const void* qkvg, int row_w, int q_off, int k_off, int v_off, co
                 const void* bi, const void* bf, int b_dtype, float cap, const int* cu_q,
                 const int* state_slot, float* state, long long slot_stride, int n_requests,
                 int n_heads, int e, int f, int fc, int n_groups, float* num, float* den,
-                cudaStream_t stream) {
+                int chunked_from, cudaStream_t stream) {
     const int eg_count = SCAN_THREADS / fc;
     const size_t smem = (size_t)(2 * TB * e + TB * fc + TB * eg_count * fc + 2 * TB + TB * 8 + TB) *
                         sizeof(float);
@@ -346,7 +351,7 @@ int launch_scan(const void* qkvg, int row_w, int q_off, int k_off, int v_off, co
     MLS_LAUNCH((mlstm_scan_kernel<T, MAXR>), dim3(n_groups, n_heads, n_requests),
                dim3(SCAN_THREADS), smem, stream, (const T*)qkvg, row_w, q_off, k_off, v_off, gates,
                bi, bf, b_dtype, cap, cu_q, state_slot, state, slot_stride, n_heads, e, f, fc,
-               n_groups, num, den);
+               n_groups, num, den, chunked_from);
     return launch_status();
 }
 
@@ -355,11 +360,11 @@ int pick_scan(int maxr, const void* qkvg, int row_w, int q_off, int k_off, int v
               const float* gates, const void* bi, const void* bf, int b_dtype, float cap,
               const int* cu_q, const int* state_slot, float* state, long long slot_stride,
               int n_requests, int n_heads, int e, int f, int fc, int n_groups, float* num,
-              float* den, cudaStream_t stream) {
+              float* den, int chunked_from, cudaStream_t stream) {
 #define MLS_SCAN(R)                                                                            \
     return launch_scan<T, R>(qkvg, row_w, q_off, k_off, v_off, gates, bi, bf, b_dtype, cap,    \
                              cu_q, state_slot, state, slot_stride, n_requests, n_heads, e, f,  \
-                             fc, n_groups, num, den, stream)
+                             fc, n_groups, num, den, chunked_from, stream)
     if (maxr <= 4) MLS_SCAN(4);
     if (maxr <= 8) MLS_SCAN(8);
     if (maxr <= 16) MLS_SCAN(16);
@@ -379,12 +384,15 @@ MLS_API int mls_mlstm_columns(int e, int f) {
     return fc;
 }
 
+// `chunked_from`: requests of at least so many tokens are left out (mls_mlstm_scan_chunked takes
+// them); 0: none.
 MLS_API int mls_mlstm_scan(const void* qkvg, int dtype, int row_w, int q_off, int k_off, int v_off,
                            const float* gates, const void* bias_i, const void* bias_f, int b_dtype,
                            float cap, const int* cu_q, const int* state_slot, float* state,
                            long long slot_stride, int n_requests, int n_heads, int e, int f,
-                           float* num, float* den, cudaStream_t stream) {
+                           float* num, float* den, int chunked_from, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
+    if (chunked_from <= 0) chunked_from = INT_MAX;
     if (e <= 0 || e > MAXN * SCAN_THREADS || f <= 0 || n_heads <= 0 || n_heads > 65535 ||
         n_requests > 65535)
         return MLS_ERR_UNSUPPORTED;
@@ -395,21 +403,23 @@ MLS_API int mls_mlstm_scan(const void* qkvg, int dtype, int row_w, int q_off, in
     if (dtype == MLS_BF16)
         return pick_scan<__nv_bfloat16>(maxr, qkvg, row_w, q_off, k_off, v_off, gates, bias_i,
                                         bias_f, b_dtype, cap, cu_q, state_slot, state, slot_stride,
-                                        n_requests, n_heads, e, f, fc, n_groups, num, den, stream);
+                                        n_requests, n_heads, e, f, fc, n_groups, num, den, chunked_from,
+                                        stream);
     return pick_scan<float>(maxr, qkvg, row_w, q_off, k_off, v_off, gates, bias_i, bias_f, b_dtype,
                             cap, cu_q, state_slot, state, slot_stride, n_requests, n_heads, e, f,
-                            fc, n_groups, num, den, stream);
+                            fc, n_groups, num, den, chunked_from, stream);
 }
 
-// The same for prompts, chunk by chunk (chunk_scan.cu).  `most`: the most chunks of a request;
-// `window` chunks of every request at a time, `chunks` in all requests together.
+// The same for prompts, chunk by chunk (chunk_scan.cu): the requests of at least `least` tokens, `taken`
+// of them; `most` chunks of one at the most, `window` of every one at a time, `chunks` in all of them
+// together.
 MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q_off, int k_off,
                                    int v_off, const float* gates, const void* bias_i,
                                    const void* bias_f, int b_dtype, float cap, const int* cu_q,
                                    const int* state_slot, float* state, long long slot_stride,
                                    int n_requests, int n_tokens, int n_heads, int e, int f, float* num,
-                                   float* den, int most, int window, long long chunks, float* scratch,
-                                   cudaStream_t stream) {
+                                   float* den, int least, int taken, int most, int window, long long chunks,
+                                   float* scratch, cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
     if (e <= 0 || f <= 0 || n_heads <= 0) return MLS_ERR_UNSUPPORTED;
@@ -437,9 +447,10 @@ MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q
     a.n_heads = n_heads;
     a.e = e;
     a.f = f;
+    a.least = least;
     a.out = num;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
-    return scan(a, most, window, chunks, scratch, stream);
+    return scan(a, taken, most, window, chunks, scratch, stream);
 }
 
 MLS_API int mls_mlstm_finish(const float* num, const float* den, const void* gate, int gate_row,

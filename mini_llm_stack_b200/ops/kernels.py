@@ -808,10 +808,10 @@ class Ops:
             fns = {"columns": _decl(lib, "mls_mlstm_columns", [_I, _I]),
                    "scan": _decl(lib, "mls_mlstm_scan",
                                  [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
-                                  _I, _I, _I, _I, _P, _P, _P]),
+                                  _I, _I, _I, _I, _P, _P, _I, _P]),
                    "chunked": _decl(lib, "mls_mlstm_scan_chunked",
                                     [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
-                                     _I, _I, _I, _I, _I, _P, _P, _I, _I, _LL, _P, _P]),
+                                     _I, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _LL, _P, _P]),
                    "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish": _decl(lib, "mls_mlstm_finish",
@@ -864,11 +864,11 @@ class Ops:
         elif name == "scan":
             fns = {"scan": _decl(lib, "mls_linear_scan",
                                  [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _P, _P,
-                                  _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _P]),
+                                  _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _I, _P]),
                    "chunked": _decl(lib, "mls_linear_scan_chunked",
                                     [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _P, _P,
                                      _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _I, _I, _I,
-                                     _LL, _P, _P]),
+                                     _I, _I, _LL, _P, _P]),
                    "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish_row": _decl(lib, "mls_scan_finish_row",
@@ -1042,23 +1042,19 @@ class Ops:
             _code(w.dtype), n_tokens, heads, n, k, self._stream()), "headwise_linear")
 
     CHUNK = 64                    # tokens of a chunk of the chunk-wise scans
-    # Tokens of the longest request from which on a step's scans run chunk by chunk: where the five
-    # short kernels of the one take as long as the other takes token by token (measured at the 1b
-    # and 8b sizes: 40-60 us, 56 tokens of retention, 120 of wkv, 125 of mLSTM); half as many where
-    # the token-by-token kernel runs in several rounds of blocks (four prompts at the 8b sizes: 28,
-    # 45 and 45).
+    # Tokens of a request from which on its scans run chunk by chunk: where the five short kernels of
+    # the one take as long as the other takes token by token (one prompt at the 1b and 8b sizes: 40-60
+    # us, 56 tokens of retention, 120 of wkv, 125 of mLSTM).  A request's own length decides and
+    # nothing else of the step, so that its bits do not depend on the requests beside it.
     CHUNKED_FROM = {"head": 64, "token": 128, "mlstm": 128}
-    CHUNKED_BLOCKS = 1024         # ... blocks of 16 columns of a state
-    # Every chunk's state passes through memory four times, a request's twice token by token: steps
-    # of a prompt among many decoded tokens stay there (64 requests of which one brings 256 tokens,
-    # 8b retention: about 310 us either way).
-    CHUNK_TOKENS = 8              # tokens a chunk holds on average at least
     CHUNK_SCRATCH = 1 << 27       # floats of scratch that a window of chunks may take
 
     def _chunk_plan(self, part: str, mode: int, step, operands: list, whole: tuple, strides: tuple,
                     n_heads: int, e: int, f: int):
-        """How a scan over a matrix state runs chunk by chunk: (the most chunks of a request, chunks
-        of a request a window, chunks of a window in all, scratch), or None: token by token.
+        """How the scans over a matrix state of a step's longer requests run chunk by chunk: (tokens
+        from which on a request does, such requests, the most chunks of one, chunks of each a window,
+        chunks of a window in all, scratch, whether other requests are left), or None: all token by
+        token.
 
         Chunk by chunk is for prompts of bfloat16 models (a float32 model's results do not depend
         on how a prompt is cut, which chunks counted from a step's first token would change) whose
@@ -1069,15 +1065,13 @@ class Ops:
         if self.act_dtype != torch.bfloat16 or not lens:
             return None
         least = self.CHUNKED_FROM[("head", "token", "mlstm")[mode]]
-        if len(lens) * n_heads * -(-f // 16) >= self.CHUNKED_BLOCKS:
-            least //= 2
-        each = [-(-n // self.CHUNK) for n in lens]
-        if max(lens) < least or step.n_tokens < self.CHUNK_TOKENS * sum(each):
+        if max(lens) < least:
             return None
         if any((t.shape[1] | off | size) & 3 or t.data_ptr() % (4 * t.element_size())
                for t, off, size in operands) or any(t.data_ptr() % 16 for t in whole) \
                 or any(s & 3 for s in strides) or n_heads > 65535:
             return None
+        each = [-(-n // self.CHUNK) for n in lens if n >= least]
         most = window = max(each)
         floats_of = self._part_lib(part)["scratch"]
 
@@ -1086,12 +1080,13 @@ class Ops:
             return chunks, floats_of(mode, step.n_tokens, n_heads, e, f, chunks)
 
         chunks, floats = size(window)
-        while window > 1 and (floats > self.CHUNK_SCRATCH or len(lens) * window > 65535):
+        while window > 1 and (floats > self.CHUNK_SCRATCH or chunks > 65535):
             window = (window + 1) // 2
             chunks, floats = size(window)
-        if len(lens) * window > 65535:
+        if chunks > 65535:
             return None
-        return most, window, chunks, self.scratch("chunk_scan", floats)
+        return (least, len(each), most, window, chunks, self.scratch("chunk_scan", floats),
+                len(each) < len(lens))
 
     def mlstm_state_width(self, e: int, f: int) -> int:
         """Floats of one head's state: the memory [e, f], the normaliser [e] and one
@@ -1116,22 +1111,24 @@ class Ops:
         q_off, k_off, v_off = offsets
         plan = self._chunk_plan("mlstm", 2, step, [(qkvg, o, w) for o, w in zip(offsets, (e, e, f))],
                                 (state, num), (width, width // n_heads), n_heads, e, f)
+        chunked_from = 0
         if plan is not None:
-            most, window, chunks, scratch = plan
+            chunked_from, taken, most, window, chunks, scratch, others = plan
             self.launches += 5 * (-(-most // window))
             _check(self._part_lib("mlstm")["chunked"](
                 _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
                 _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
                 _ptr(step.state_slot), _ptr(state), width, step.n_requests, t, n_heads, e, f,
-                _ptr(num), _ptr(den), most, window, chunks, _ptr(scratch), self._stream()),
-                "mlstm_scan_chunked")
-            return
+                _ptr(num), _ptr(den), chunked_from, taken, most, window, chunks, _ptr(scratch),
+                self._stream()), "mlstm_scan_chunked")
+            if not others:
+                return
         self.launches += 1
         _check(self._part_lib("mlstm")["scan"](
             _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
             _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
             _ptr(step.state_slot), _ptr(state), width, step.n_requests, n_heads, e, f, _ptr(num),
-            _ptr(den), self._stream()), "mlstm_scan")
+            _ptr(den), chunked_from, self._stream()), "mlstm_scan")
 
     def mlstm_finish(self, num, den, qkvg, g_off: int, weight, eps: float, out, n_heads: int,
                      f: int) -> None:
@@ -1498,8 +1495,9 @@ class Ops:
             plan = self._chunk_plan("scan", 0 if decay_tok is None else 1, step,
                                     [(*a, e), (*k, e), (*v, f)], (state, out),
                                     (state.stride(0), e * f), n_heads, e, f)
+        chunked_from = 0
         if plan is not None:
-            most, window, chunks, scratch = plan
+            chunked_from, taken, most, window, chunks, scratch, others = plan
             self.launches += 4 * (-(-most // window))
             _check(self._part_lib("scan")["chunked"](
                 _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],
@@ -1508,9 +1506,10 @@ class Ops:
                 _ptr(decay_tok), _ptr(decay_head), _ptr(bonus),
                 _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
                 _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
-                step.n_requests, t, n_heads, e, f, _ptr(out), 1 if silu else 0, most, window, chunks,
-                _ptr(scratch), self._stream()), "linear_scan_chunked")
-            return
+                step.n_requests, t, n_heads, e, f, _ptr(out), 1 if silu else 0, chunked_from, taken,
+                most, window, chunks, _ptr(scratch), self._stream()), "linear_scan_chunked")
+            if not others:
+                return
         self.launches += 1
         _check(self._part_lib("scan")["scan"](
             _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],
@@ -1519,8 +1518,8 @@ class Ops:
             _ptr(decay_tok), n_heads * e, _ptr(decay_head), _ptr(bonus),
             _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
             _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
-            step.n_requests, n_heads, e, f, _ptr(out), 1 if silu else 0, self._stream()),
-            "linear_scan")
+            step.n_requests, n_heads, e, f, _ptr(out), 1 if silu else 0, chunked_from,
+            self._stream()), "linear_scan")
 
     def scan_finish(self, o, gate, gate_off: int, weight, eps: float, out, n_heads: int,
                     f: int) -> None:

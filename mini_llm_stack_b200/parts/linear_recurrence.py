@@ -4,8 +4,10 @@ attention and the gated delta rule.
 Both keep ``S [e, f]`` per head (key size e, value size f) in the request's state slot
 (``FixedState``, float32, zero when the slot is claimed) and walk a step's tokens through
 it with the same scan; a portion of a prompt continues from the slot's state.  In a float32
-run cutting a prompt changes no bit; a bfloat16 run takes longer portions chunk by chunk, with
-the sums over a chunk's tokens in another order.
+run cutting a prompt changes no bit; a bfloat16 run takes portions of many tokens chunk by chunk
+(wkv and lightning attention; the delta rule walks every token), with the sums over a chunk's
+tokens in another order.  A portion's own length decides which: the bits of a request do not
+depend on the requests beside it.
 
 wkv (e = f), with h' the previous token's h (zeros before the first; kept in the slot):
     mix_s = h + (h' - h) * mu_s          for s in r, k, v, g, w

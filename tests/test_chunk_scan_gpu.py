@@ -176,3 +176,52 @@ def test_windows_of_chunks_and_portions_go_on_from_the_slot(ops, always):
     got = torch.empty_like(out)
     got[a], got[b] = walk(first, a, two), walk(second, b, two)
     assert (got - out).abs().max() <= 1e-5 * out.abs().max() and (two - whole).abs().max() <= 1e-5 * whole.abs().max()
+
+
+@pytest.mark.parametrize("kind", ["head", "token", "mlstm"])
+def test_a_requests_bits_do_not_depend_on_its_neighbours(ops, kind):
+    """Requests on both sides of the line between the kernels, more of them than a warp's lanes, beside
+    each other and alone: a request's own length says which kernel takes it."""
+    lens = [1] * 30 + [63, 64, 1, 200, 127, 128, 5, 65, 1]
+    heads, e, f = 2, 64, 128
+    t, r = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(7)
+    rows = torch.randn(t, heads * (2 * e + f), generator=g).bfloat16().cuda()
+    decay_head = torch.tensor([0.97, 0.8]).cuda()
+    decay_tok = (1 - 0.2 * torch.rand(t, heads * e, generator=g)).cuda()
+    gates = torch.randn(t, 2 * heads, generator=g).cuda()
+    bias = torch.randn(2, heads, generator=g).cuda()
+    width = ops.mlstm_state_width(e, f) if kind == "mlstm" else e * f
+    state0 = torch.randn(r, heads * width, generator=g).cuda()
+    if kind == "mlstm":
+        state0.view(r, heads, width)[:, :, e * f + e:] = 0.5
+
+    def walk(lens, at, slots):
+        n = sum(lens)
+        x, step = rows[at:at + n].contiguous(), a_step(lens, True)[0]
+        step.state_slot = torch.arange(len(lens), dtype=torch.int32, device="cuda")
+        state = state0[slots].clone()
+        out = torch.full((n, heads * f), float("nan"), device="cuda")
+        den = torch.zeros(n, heads, device="cuda")
+        before = ops.launches
+        if kind == "mlstm":
+            ops.mlstm_scan(x, (0, heads * e, 2 * heads * e), gates[at:at + n].contiguous(), bias[0], bias[1], 15.0,
+                           step, state.view(len(lens), heads, width), heads, e, f, out, den)
+        else:
+            ops.linear_scan((x, 0), (x, heads * e), (x, 2 * heads * e), state, step, heads, e, f, out,
+                            decay_tok=decay_tok[at:at + n].contiguous() if kind == "token" else None,
+                            decay_head=decay_head if kind == "head" else None, read_first=kind == "token")
+        return out, den, state, ops.launches - before
+
+    whole, at = walk(lens, 0, slice(0, r)), 0
+    assert torch.isfinite(whole[0]).all()
+    short = 1 if kind == "mlstm" else 0
+    assert whole[3] == 5 + short                       # the chunks' kernels and one for the other requests
+    least = ops.CHUNKED_FROM[kind]
+    for i, n in enumerate(lens):
+        alone = walk([n], at, slice(i, i + 1))
+        assert alone[3] == (4 + short if n >= least else 1)
+        for x, y in zip(whole[:2], alone[:2]):
+            assert torch.equal(x[at:at + n], y), (i, n)
+        assert torch.equal(whole[2][i], alone[2][0]), (i, n)
+        at += n
