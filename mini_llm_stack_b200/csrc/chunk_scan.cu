@@ -15,9 +15,10 @@
 //   carry    walks the chunks: leaves each chunk's S0 where its U was, and the last state in the slot
 //   output   [q | P] x [S0; v], a product over e + 64
 //
-// All of it float32 on CUDA cores as in the token-by-token kernels (fma.rn.f32x2; the operands as
-// they are or scaled by factors <= 1, never by the reciprocal of a decay), so that nothing is
-// rounded that was not rounded there; the sums run over s in another order.  Chunks are counted
+// All of it float32 on CUDA cores as in the token-by-token kernels (fma.rn.f32x2).  Decays enter only as
+// factors <= 1, never as the reciprocal of one.  Scores, the rows of q and k times their factors and each
+// chunk's U are rounded to float32 once more than there; what a chunk saves is the state's own rounding a
+// token.  Ops.CHUNKED_FROM says from where on that leaves outputs and states no further from float64.  Chunks are counted
 // from a request's first token of the step.
 //
 // Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,824 ->
@@ -177,9 +178,9 @@ __device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*
         }
     }
 }
-// Outputs and scores add up over runs of 16 of k, kept apart from the run being multiplied: chains of
-// 16 roundings and one a run, as exact as the token-by-token kernels' sums (chains of 64: 1.2 times
-// their error at 130 tokens).
+// Every product adds up over runs of 16 of k, kept apart from the run being multiplied: chains of 16
+// roundings and one a run.  With chains of 64 outputs had 1.2 times the token-by-token kernels' error at
+// 130 tokens and states 1.02 times at 64; with runs of 16 both lie below it from Ops.CHUNKED_FROM on.
 constexpr int SUMS = 16;
 template <int N>
 __device__ __forceinline__ void settle(f32x2 (&sum)[N], f32x2 (&acc)[N]) {
@@ -609,19 +610,14 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     fill_rows<THREADS, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
     __syncthreads();
     const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
-    f32x2 sum[8][TN / 2];
+    f32x2 sum[8][TN / 2], acc[8][TN / 2];                  // (the factors are rounded already: short chains)
     clear(sum);
-    if (MODE == TOKEN_DECAY) {                             // its factors are rounded already: short chains
-        f32x2 acc[8][TN / 2];
-        clear(acc);
+    clear(acc);
 #pragma unroll 1
-        for (int k0 = 0; k0 < C; k0 += SUMS) {
-            multiply<BN, TN, false, SUMS>(acc, A, B, tx, ty, k0);
+    for (int k0 = 0; k0 < C; k0 += SUMS) {
+        multiply<BN, TN, false, SUMS>(acc, A, B, tx, ty, k0);
 #pragma unroll
-            for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
-        }
-    } else {
-        multiply<BN, TN, false>(sum, A, B, tx, ty);
+        for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
     }
     float* U = s.states + (w.idx * a.n_heads + head) * state_floats(MODE, a.e, a.f);
 #pragma unroll

@@ -1042,11 +1042,14 @@ class Ops:
             _code(w.dtype), n_tokens, heads, n, k, self._stream()), "headwise_linear")
 
     CHUNK = 64                    # tokens of a chunk of the chunk-wise scans
-    # Tokens of a request from which on its scans run chunk by chunk: where the five short kernels of
-    # the one take as long as the other takes token by token (one prompt at the 1b and 8b sizes: 40-60
-    # us, 56 tokens of retention, 120 of wkv, 125 of mLSTM).  A request's own length decides and
-    # nothing else of the step, so that its bits do not depend on the requests beside it.
-    CHUNKED_FROM = {"head": 64, "token": 128, "mlstm": 128}
+    # Tokens of a request from which on its scans run chunk by chunk: where one prompt's four or five
+    # short kernels take no longer than the other kernel token by token, and lie no further from
+    # float64.  Retention, 16 and 32 heads of 128 x 256: 38 and 43 us against 40 and 47 at 48 tokens, errors
+    # 0.94 (outputs) and 0.74 (states) of its.  wkv, 32 and 64 heads of 64 x 64: 40 and 48 against 57 and 72 at
+    # 200 tokens, 0.97 and 0.85 at 192, but 1.02 and 0.88 at 128.  mLSTM, 4 and 8 heads of 256 x 512: 86 and 77
+    # against 87 and 96 at 128, 0.81 (numerators), 0.84 (denominators) and 0.68.  A request's own length decides and nothing else of the
+    # step, so that its bits do not depend on the requests beside it.
+    CHUNKED_FROM = {"head": 48, "token": 192, "mlstm": 128}
     CHUNK_SCRATCH = 1 << 27       # floats of scratch that a window of chunks may take
 
     def _chunk_plan(self, part: str, mode: int, step, operands: list, whole: tuple, strides: tuple,

@@ -182,7 +182,7 @@ def test_windows_of_chunks_and_portions_go_on_from_the_slot(ops, always):
 def test_a_requests_bits_do_not_depend_on_its_neighbours(ops, kind):
     """Requests on both sides of the line between the kernels, more of them than a warp's lanes, beside
     each other and alone: a request's own length says which kernel takes it."""
-    lens = [1] * 30 + [63, 64, 1, 200, 127, 128, 5, 65, 1]
+    lens = [1] * 30 + [47, 48, 1, 200, 127, 128, 5, 65, 1, 191, 192]
     heads, e, f = 2, 64, 128
     t, r = sum(lens), len(lens)
     g = torch.Generator().manual_seed(7)
@@ -225,3 +225,59 @@ def test_a_requests_bits_do_not_depend_on_its_neighbours(ops, kind):
             assert torch.equal(x[at:at + n], y), (i, n)
         assert torch.equal(whole[2][i], alone[2][0]), (i, n)
         at += n
+
+
+@pytest.mark.parametrize("kind, heads, e, f", [("head", 16, 128, 256), ("token", 32, 64, 64), ("mlstm", 4, 256, 512)])
+@pytest.mark.parametrize("more", [0, 17, 300])
+def test_no_further_from_float64_than_token_by_token(ops, kind, heads, e, f, more):
+    """From the shortest request that goes chunk by chunk on, at the sizes and decays of real layers.
+    Norms of two sets of n independent errors of the same size differ by chance by 1 / sqrt(n) of
+    themselves or so (each varies by 1 / sqrt(2n)): twice that is allowed, which counts for the
+    denominators only (4 a token), and a hundredth for errors that are not independent."""
+    t = ops.CHUNKED_FROM[kind] + more
+    g = torch.Generator(device="cuda").manual_seed(t)
+    q, k, v = (torch.randn(t, heads * w, device="cuda", generator=g).bfloat16() for w in (e, e, f))
+    head = torch.tensor([1 - 2.0 ** (-5 - 3 * i / heads) for i in range(heads)], device="cuda")
+    pace = torch.rand(heads * e, device="cuda", generator=g) * 5 - 6
+    tok = torch.exp(-torch.exp(pace + 0.3 * torch.randn(t, heads * e, device="cuda", generator=g)))
+    bonus = (torch.randn(heads, e, device="cuda", generator=g) * 0.5).bfloat16()
+    gates = torch.randn(t, 2 * heads, device="cuda", generator=g)
+    bi, bf = torch.randn(heads, device="cuda", generator=g), torch.randn(heads, device="cuda", generator=g) + 3
+    got = {}
+    for chunked in (True, False):
+        step = a_step([t], chunked)[0]
+        out, den = torch.empty(t, heads * f, device="cuda"), torch.empty(t, heads, device="cuda")
+        if kind == "mlstm":
+            state = torch.zeros(1, heads, ops.mlstm_state_width(e, f), device="cuda")
+            ops.mlstm_scan(torch.cat([q, k, v], 1), (0, heads * e, 2 * heads * e), gates, bi, bf, 15.0, step, state,
+                           heads, e, f, out, den)
+            got[chunked] = out, state[0, :, :e * f + e], den
+        else:
+            state = torch.zeros(1, heads * e * f, device="cuda")
+            ops.linear_scan((q, 0), (k, 0), (v, 0), state, step, heads, e, f, out,
+                            decay_tok=tok if kind == "token" else None, decay_head=head if kind == "head" else None,
+                            bonus=bonus if kind == "token" else None, read_first=kind == "token")
+            got[chunked] = out, state.view(heads, -1)
+    q, k, v = (x.double().view(t, heads, -1) for x in (q, k, v))
+    s, n, m = (torch.zeros(*x, dtype=torch.float64, device="cuda") for x in ((heads, e, f), (heads, e), (heads,)))
+    ig = 15 * torch.tanh((gates[:, :heads].double() + bi.double()) / 15)
+    fg = torch.nn.functional.logsigmoid(15 * torch.tanh((gates[:, heads:].double() + bf.double()) / 15))
+    outs, dens = [], []
+    for i in range(t):
+        kv = k[i][:, :, None] * v[i][:, None, :]
+        if kind == "head":
+            s = head.double()[:, None, None] * s + kv
+            outs.append(torch.einsum("hef,he->hf", s, q[i]))
+        elif kind == "token":
+            outs.append(torch.einsum("hef,he->hf", s + bonus.double()[:, :, None] * kv, q[i]))
+            s = tok[i].double().view(heads, e, 1) * s + kv
+        else:
+            new = torch.maximum(fg[i] + m, ig[i])
+            keep, take = torch.exp(fg[i] + m - new), torch.exp(ig[i] - new)
+            m, s, n = new, keep[:, None, None] * s + take[:, None, None] * kv, keep[:, None] * n + take[:, None] * k[i]
+            outs.append(torch.einsum("hef,he->hf", s, q[i]) * e ** -0.5)
+            dens.append(torch.maximum((n * q[i]).sum(-1).abs() * e ** -0.5, torch.exp(-m)) + 1e-6)
+    last = torch.cat([s.reshape(heads, -1), n], 1) if kind == "mlstm" else s.reshape(heads, -1)
+    for i, want in enumerate([torch.stack(outs).view(t, -1), last] + ([torch.stack(dens)] if dens else [])):
+        mine, theirs = ((got[x][i].double() - want).norm() / want.norm() for x in (True, False))
+        assert mine <= (1.01 + 2 * want.numel() ** -0.5) * theirs, (i, float(mine), float(theirs))
