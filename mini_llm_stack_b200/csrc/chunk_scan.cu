@@ -72,18 +72,18 @@ __device__ __forceinline__ float4 times(float4 v, float f) {
 struct Where {
     int r, c;                        // request, chunk of the request
     int t0, n;                       // first token, tokens
-    int chunks;                      // the request's chunks of this window
-    size_t idx;                      // place among the window's chunks
+    int chunks;                      // the request's chunks of this part
+    size_t idx;                      // place among the part's chunks
 };
 
-// Chunk z of the window's chunks, or (REQUEST) the first one of request z of those that go chunk by
-// chunk: a request's length alone says whether it does.  Every thread calls; false: none.
+// Chunk z of the part's chunks, or (REQUEST) the first one of its request z.  A request's length alone
+// says whether it goes chunk by chunk.  Every thread calls; false: none.
 template <bool REQUEST>
-__device__ __forceinline__ bool locate(const Args& a, int first, int span, int z, Where& w) {
+__device__ __forceinline__ bool locate(const Args& a, const Part& p, int z, Where& w) {
     __shared__ int at_s[2];          // request, place of its first chunk
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
-        int taken = 0, before = 0;   // requests that go chunk by chunk and chunks before these 32
+        int taken = -p.from, before = 0;   // the part's requests and chunks before these 32
         if (lane == 0) at_s[0] = -1;
         __syncwarp();
         for (int r0 = 0; r0 < a.n_requests; r0 += 32) {
@@ -92,7 +92,7 @@ __device__ __forceinline__ bool locate(const Args& a, int first, int span, int z
             const bool in = len >= a.least;
             const unsigned all = __ballot_sync(0xffffffffu, in);
             const int k = taken + __popc(all & ((1u << lane) - 1u));
-            const int count = in ? min(max((len + C - 1) / C - first, 0), span) : 0;
+            const int count = in && k >= 0 && k < p.count ? min(max((len + C - 1) / C - p.first, 0), p.span) : 0;
             int sum = count;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -114,9 +114,9 @@ __device__ __forceinline__ bool locate(const Args& a, int first, int span, int z
     w.r = at_s[0];
     if (w.r < 0) return false;
     const int j = REQUEST ? 0 : z - at_s[1];
-    w.c = first + j;
+    w.c = p.first + j;
     const int t = a.cu_q[w.r], len = a.cu_q[w.r + 1] - t;
-    w.chunks = min(max((len + C - 1) / C - first, 0), span);
+    w.chunks = min(max((len + C - 1) / C - p.first, 0), p.span);
     w.idx = (size_t)(at_s[1] + j);
     w.t0 = t + w.c * C;
     w.n = min(C, len - w.c * C);
@@ -204,7 +204,9 @@ struct Reader {
     size_t row, at;                  // elements between tokens; the head's first entry
     int dtype, silu, n, size;
     __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head)
-        : base(r.base), row(r.row), at((size_t)w.t0 * r.row + r.off + (size_t)head * r.width),
+        : Reader(r, silu_, w, head, (size_t)w.t0) {}
+    __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head, size_t t0)
+        : base(r.base), row(r.row), at(t0 * r.row + r.off + (size_t)head * r.width),
           dtype(r.dtype), silu(silu_), n(w.n), size(r.width) {}
     __device__ __forceinline__ float4 operator()(int t, int i) const {
         if (t >= n || i >= size) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -215,14 +217,15 @@ struct Reader {
 };
 
 // What scores and gates leave for the products: a factor of q and of k for every token and head
-// (HEAD_DECAY works them out itself), and the chunk's decay.
+// (HEAD_DECAY works them out itself), and the chunk's decay.  All of it by chunks, so that its size does
+// not depend on the step's other tokens.
 struct Scratch {
+    double* log_gates;               // MLSTM: [chunks, 64, H, 2]
     float* states;                   // [chunks, H, e f (+ e)]
     float* scores;                   // [chunks, H, 64, 64]
-    float* rows_q;                   // TOKEN_DECAY: [T, H e]; MLSTM: factors [T, H]
+    float* rows_q;                   // TOKEN_DECAY: [chunks, 64, H e]; MLSTM: factors [chunks, 64, H]
     float* rows_k;
     float* whole;                    // TOKEN_DECAY: [chunks, H, e]; MLSTM: [chunks, H]
-    double* log_gates;               // MLSTM: [T, H, 2]
 };
 __host__ __device__ inline int state_floats(int mode, int e, int f) {
     return e * f + (mode == MLSTM ? e : 0);
@@ -233,19 +236,19 @@ __host__ __device__ inline int state_floats(int mode, int e, int f) {
 // their columns have nothing to multiply.
 template <int MODE>
 __global__ void __launch_bounds__(256)
-chunk_scores_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_scores_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, part, blockIdx.z, w)) return;
     __shared__ __align__(16) float A[C][C], B[C][C];
     __shared__ float power[C];
     __shared__ double la[C], lb[C];
     if (threadIdx.x < C) {
         if (MODE == HEAD_DECAY) power[threadIdx.x] = powf(a.decay[head], (float)threadIdx.x);
         if (MODE == MLSTM && threadIdx.x < w.n) {
-            const double* lg = s.log_gates + ((size_t)(w.t0 + threadIdx.x) * a.n_heads + head) * 2;
+            const double* lg = s.log_gates + ((w.idx * C + threadIdx.x) * a.n_heads + head) * 2;
             la[threadIdx.x] = lg[0];
             lb[threadIdx.x] = lg[1];
         }
@@ -340,13 +343,13 @@ __device__ __forceinline__ void pairs_4x2(const float* r, const float* k, int pa
 // QUADS: e / 4 where it is known (heads of 64), else 0.
 template <int QUADS>
 __global__ void __launch_bounds__(256)
-chunk_scores_token_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_scores_token_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     Where w;
     const int quads = QUADS ? QUADS : a.e / 4, e = 4 * quads, pad = e + 4;
     const int head = blockIdx.y;
-    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, part, blockIdx.z, w)) return;
     extern __shared__ __align__(16) float sm[];
     float* r_s = sm;                                     // [64][pad]
     float* k_s = r_s + C * pad;                          // [64][pad]
@@ -466,7 +469,7 @@ chunk_scores_token_kernel(const Args a, const Scratch s, int first, int span) {
             if (h < g) x = mul4(x, d);
             if (h > g) y = mul4(y, d);
         }
-        const size_t at = ((size_t)(w.t0 + t) * a.n_heads + head) * e + i;
+        const size_t at = ((w.idx * C + t) * a.n_heads + head) * e + i;
         *reinterpret_cast<float4*>(s.rows_q + at) = x;
         *reinterpret_cast<float4*>(s.rows_k + at) = y;
     }
@@ -486,14 +489,14 @@ chunk_scores_token_kernel(const Args a, const Scratch s, int first, int span) {
 //   of a pair:    exp((F_t - m_t) + (i_s - F_s))   of the state: exp(F_n + m_0 - m_n)
 constexpr int GATE_WARPS = 16;
 __global__ void __launch_bounds__(32 * GATE_WARPS)
-chunk_gates_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_gates_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     __shared__ double whole_s[GATE_WARPS], top_s[GATE_WARPS];
     __shared__ float m_s[GATE_WARPS + 1];
     const int head = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Where w;
-    if (!locate<true>(a, first, span, blockIdx.y, w)) return;
+    if (!locate<true>(a, part, blockIdx.y, w)) return;
     float* m_slot = a.state + (size_t)a.state_slot[w.r] * a.slot_stride + (size_t)head * a.head_stride +
                     state_floats(MLSTM, a.e, a.f);
     const float bi = load_as_float(a.bias_i, head, a.bias_dtype),
@@ -558,12 +561,12 @@ chunk_gates_kernel(const Args a, const Scratch s, int first, int span) {
                 const int j = 2 * lane + x;
                 if (j >= n) continue;
                 const float m = (float)(F[x] + fmax((double)m0, fmax(earlier, top[x])));
-                const size_t at = (size_t)(t0 + j) * a.n_heads + head;
+                const size_t at = ((w.idx + c) * C + j) * a.n_heads + head;
                 s.log_gates[2 * at] = F[x] - m;
                 s.log_gates[2 * at + 1] = ig[x] - F[x];
                 s.rows_q[at] = a.q_scale * expf((float)(F[x] + m0 - m));
                 s.rows_k[at] = expf((float)(whole - F[x] + ig[x] - m_end));
-                a.den[at] = expf(-m);                    // the output kernel adds n . q to it
+                a.den[(size_t)(t0 + j) * a.n_heads + head] = expf(-m);   // the output kernel adds n . q to it
             }
             if (lane == 0) s.whole[(w.idx + c) * a.n_heads + head] = expf((float)(whole + m0 - m_end));
         }
@@ -578,7 +581,7 @@ __device__ __forceinline__ float row_factor(const Args& a, const float* factors,
                                             int t, int power) {
     if (t >= w.n) return 0.f;
     if (MODE == HEAD_DECAY) return powf(a.decay[head], (float)power);
-    if (MODE == MLSTM) return factors[(size_t)(w.t0 + t) * a.n_heads + head];
+    if (MODE == MLSTM) return factors[(w.idx * C + t) * a.n_heads + head];
     return 1.f;
 }
 
@@ -589,12 +592,12 @@ __device__ __forceinline__ float row_factor(const Args& a, const float* factors,
 // 32 heads of 128 x 256; 16 against 28 for 1,501 tokens of 32 heads of 64 x 64).
 template <int MODE>
 __global__ void __launch_bounds__(128, 5)
-chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_update_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, part, blockIdx.z, w)) return;
     constexpr int BN = C, TN = 4, THREADS = 128;
     __shared__ __align__(16) float A[C][C], B[C][BN];
     __shared__ float factor[C];
@@ -605,7 +608,8 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
     __syncthreads();
     Rows kr = a.k;
     if (MODE == TOKEN_DECAY) kr = Rows{s.rows_k, MLS_F32, a.n_heads * a.e, 0, a.e};
-    const Reader k(kr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head), v(a.v, a.silu, w, head);
+    const Reader k(kr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head, MODE == TOKEN_DECAY ? w.idx * C : (size_t)w.t0);
+    const Reader v(a.v, a.silu, w, head);
     fill_rows<THREADS, C>(A, [&](int t, int i) { return times(k(t, i0 + i), factor[t]); });
     fill_rows<THREADS, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
     __syncthreads();
@@ -645,12 +649,12 @@ chunk_update_kernel(const Args a, const Scratch s, int first, int span) {
 // chunks are under way together.
 template <int MODE>
 __global__ void __launch_bounds__(128)
-chunk_carry_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_carry_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
-    if (!locate<true>(a, first, span, blockIdx.z, w)) return;
+    if (!locate<true>(a, part, blockIdx.z, w)) return;
     const int size = state_floats(MODE, a.e, a.f);
     const int at = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (at >= size) return;
@@ -699,12 +703,12 @@ chunk_carry_kernel(const Args a, const Scratch s, int first, int span) {
 // 128 x 256: 200 us, now 166; 4 heads of 256 x 512: 113, now 85).
 template <int MODE, int BN>
 __global__ void __launch_bounds__(2 * BN, BN == 128 ? 2 : 3)
-chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
+chunk_output_kernel(const Args a, const Scratch s, const Part part) {
     chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y, j0 = blockIdx.x * BN;
-    if (!locate<false>(a, first, span, blockIdx.z, w)) return;
+    if (!locate<false>(a, part, blockIdx.z, w)) return;
     constexpr int THREADS = 2 * BN, TN = 4, QA = C * (C / 4) / THREADS;      // quads of A a thread brings in
     extern __shared__ __align__(16) float tiles[];
     float(*A)[C][C] = reinterpret_cast<float(*)[C][C]>(tiles);
@@ -714,7 +718,8 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
         factor[threadIdx.x] = row_factor<MODE>(a, s.rows_q, w, head, threadIdx.x, threadIdx.x + 1);
     Rows qr = a.q;
     if (MODE == TOKEN_DECAY) qr = Rows{s.rows_q, MLS_F32, a.n_heads * a.e, 0, a.e};
-    const Reader q(qr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head), v(a.v, a.silu, w, head);
+    const Reader q(qr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head, MODE == TOKEN_DECAY ? w.idx * C : (size_t)w.t0);
+    const Reader v(a.v, a.silu, w, head);
     const size_t unit = w.idx * a.n_heads + head;
     const float* S = s.states + unit * state_floats(MODE, a.e, a.f);
     const float* P = s.scores + unit * C * C;
@@ -801,13 +806,13 @@ chunk_output_kernel(const Args a, const Scratch s, int first, int span) {
 }
 
 template <int MODE>
-int update(const Args& a, const Scratch& s, int chunks, int first, int span, cudaStream_t stream) {
-    const dim3 grid(((a.e + C - 1) / C) * ((a.f + C - 1) / C), a.n_heads, chunks);
-    MLS_LAUNCH((chunk_update_kernel<MODE>), grid, dim3(128), 0, stream, a, s, first, span);
+int update(const Args& a, const Scratch& s, const Part& part, cudaStream_t stream) {
+    const dim3 grid(((a.e + C - 1) / C) * ((a.f + C - 1) / C), a.n_heads, part.chunks);
+    MLS_LAUNCH((chunk_update_kernel<MODE>), grid, dim3(128), 0, stream, a, s, part);
     return launch_status();
 }
 template <int MODE, int BN>
-int output(const Args& a, const Scratch& s, int chunks, int first, int span, cudaStream_t stream) {
+int output(const Args& a, const Scratch& s, const Part& part, cudaStream_t stream) {
     constexpr int smem = 2 * C * (C + BN) * (int)sizeof(float);
     static bool configured = false;
     if (!configured) {
@@ -816,8 +821,8 @@ int output(const Args& a, const Scratch& s, int chunks, int first, int span, cud
         if (rc) return rc;
         configured = true;
     }
-    const dim3 grid((a.f + BN - 1) / BN, a.n_heads, chunks);
-    MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(2 * BN), smem, stream, a, s, first, span);
+    const dim3 grid((a.f + BN - 1) / BN, a.n_heads, part.chunks);
+    MLS_LAUNCH((chunk_output_kernel<MODE, BN>), grid, dim3(2 * BN), smem, stream, a, s, part);
     return launch_status();
 }
 
@@ -826,31 +831,31 @@ size_t token_smem(int e) {
 }
 
 template <int MODE>
-int window(const Args& a, const Scratch& s, int taken, int chunks, int first, int span, cudaStream_t stream) {
+int launch(const Args& a, const Scratch& s, const Part& part, cudaStream_t stream) {
     if (MODE == TOKEN_DECAY) {
         const size_t smem = token_smem(a.e);
         auto kernel = a.e == 64 ? chunk_scores_token_kernel<16> : chunk_scores_token_kernel<0>;
         const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (rc) return rc;
-        MLS_LAUNCH(kernel, dim3(1, a.n_heads, chunks), dim3(256), smem,
-                   stream, a, s, first, span);
+        MLS_LAUNCH(kernel, dim3(1, a.n_heads, part.chunks), dim3(256), smem,
+                   stream, a, s, part);
     } else {
         if (MODE == MLSTM)
-            MLS_LAUNCH((chunk_gates_kernel), dim3(a.n_heads, taken), dim3(32 * GATE_WARPS), 0,
-                       stream, a, s, first, span);
-        MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, chunks), dim3(256), 0,
-                   stream, a, s, first, span);
+            MLS_LAUNCH((chunk_gates_kernel), dim3(a.n_heads, part.count), dim3(32 * GATE_WARPS), 0,
+                       stream, a, s, part);
+        MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, part.chunks), dim3(256), 0,
+                   stream, a, s, part);
     }
-    int rc = update<MODE>(a, s, chunks, first, span, stream);
+    int rc = update<MODE>(a, s, part, stream);
     if (rc) return rc;
     const int quads = state_floats(MODE, a.e, a.f) / 4;
-    MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, taken), dim3(128),
-               0, stream, a, s, first, span);
+    MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, part.count), dim3(128),
+               0, stream, a, s, part);
     rc = launch_status();
     if (rc) return rc;
     // (a width of 64 leaves half of a wider tile empty)
-    return a.f <= C ? output<MODE, 64>(a, s, chunks, first, span, stream)
-                    : output<MODE, 128>(a, s, chunks, first, span, stream);
+    return a.f <= C ? output<MODE, 64>(a, s, part, stream)
+                    : output<MODE, 128>(a, s, part, stream);
 }
 }  // namespace
 
@@ -868,49 +873,41 @@ bool fits(const Args& a) {
 }
 
 // (the float64 logarithms first, then sizes that are multiples of four floats)
-long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long long chunks) {
-    const long long units = chunks * n_heads, tokens = (long long)n_tokens * n_heads;
-    long long n = units * (state_floats(mode, e, f) + C * C);
-    if (mode == TOKEN_DECAY) n += 2 * tokens * e + units * e;
-    if (mode == MLSTM) n += 4 * tokens + 2 * ((tokens + 3) / 4 * 4) + (units + 3) / 4 * 4;
-    return n;
+long long scratch_floats(int mode, int n_heads, int e, int f, long long chunks) {
+    long long n = (long long)state_floats(mode, e, f) + C * C;               // a chunk and head
+    if (mode == TOKEN_DECAY) n += 2LL * C * e + e;
+    if (mode == MLSTM) n += 4 * C + 2 * C + 1;
+    return chunks * n_heads * n;
 }
 
-int scan(const Args& a, int taken, int most, int window_chunks, long long chunks, float* scratch,
-         cudaStream_t stream) {
-    if (taken <= 0 || most <= 0) return 0;
-    if (chunks > 65535 || taken > 65535 || a.least < 1) return MLS_ERR_UNSUPPORTED;
-    const long long units = chunks * a.n_heads, tokens = (long long)a.n_tokens * a.n_heads;
+int scan(const Args& a, const Part& part, float* scratch, cudaStream_t stream) {
+    if (part.count <= 0 || part.span <= 0 || part.chunks <= 0) return 0;
+    if (part.chunks > 65535 || part.count > 65535 || part.from < 0 || part.first < 0 || a.least < 1)
+        return MLS_ERR_UNSUPPORTED;
+    const size_t units = (size_t)part.chunks * a.n_heads, rows = units * C;
     Scratch s{};
     float* at = scratch;
     if (a.mode == MLSTM) {
         s.log_gates = reinterpret_cast<double*>(at);
-        at += 4 * tokens;
+        at += 4 * rows;
     }
     s.states = at;
     at += units * state_floats(a.mode, a.e, a.f);
     s.scores = at;
     at += units * C * C;
-    const long long per = a.mode == TOKEN_DECAY ? tokens * a.e : (tokens + 3) / 4 * 4;
     if (a.mode != HEAD_DECAY) {
+        const size_t per = a.mode == TOKEN_DECAY ? rows * a.e : rows;
         s.rows_q = at;
         s.rows_k = at + per;
         s.whole = at + 2 * per;
     }
-    for (int first = 0; first < most; first += window_chunks) {
-        const int span = most - first < window_chunks ? most - first : window_chunks;
-        int rc;
-        if (a.mode == HEAD_DECAY) rc = window<HEAD_DECAY>(a, s, taken, (int)chunks, first, span, stream);
-        else if (a.mode == TOKEN_DECAY) rc = window<TOKEN_DECAY>(a, s, taken, (int)chunks, first, span, stream);
-        else rc = window<MLSTM>(a, s, taken, (int)chunks, first, span, stream);
-        if (rc) return rc;
-    }
-    return 0;
+    if (a.mode == HEAD_DECAY) return launch<HEAD_DECAY>(a, s, part, stream);
+    if (a.mode == TOKEN_DECAY) return launch<TOKEN_DECAY>(a, s, part, stream);
+    return launch<MLSTM>(a, s, part, stream);
 }
 }  // namespace mls_chunk
 
-// Floats of scratch that the chunk-wise scan of a window of so many chunks (of all requests) takes.
-MLS_API long long mls_chunk_scratch_floats(int mode, int n_tokens, int n_heads, int e, int f,
-                                           long long chunks) {
-    return scratch_floats(mode, n_tokens, n_heads, e, f, chunks);
+// Floats of scratch that so many chunks of a chunk-wise scan take.
+MLS_API long long mls_chunk_scratch_floats(int mode, int n_heads, int e, int f, long long chunks) {
+    return scratch_floats(mode, n_heads, e, f, chunks);
 }

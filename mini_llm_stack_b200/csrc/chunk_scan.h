@@ -37,16 +37,22 @@ struct Args {
     float* state;
     long long slot_stride;           // floats between slots
     int head_stride;                 // floats between the heads of a slot
-    int n_requests, n_tokens, n_heads, e, f;
+    int n_requests, n_heads, e, f;
     int least;                       // requests of at least so many tokens (>= 1); the others are left out
     float* out;                      // [T, H * f]
 };
 
+// Some of the chunks of a step, as many as scratch holds at a time: chunks [first, first + span) of `count`
+// of the requests that go chunk by chunk, from the `from`th of them on; `chunks` in all.
+struct Part {
+    int from, count, first, span, chunks;
+};
+
 // Whether the chunk-wise kernels take these operands (alignment, sizes).
 bool fits(const Args& a);
-// Floats of scratch for windows of so many chunks in all.
-long long scratch_floats(int mode, int n_tokens, int n_heads, int e, int f, long long chunks);
-// The scan of `taken` requests, `most` chunks of one at the most, `window` of them at a time.
-int scan(const Args& a, int taken, int most, int window, long long chunks_a_window, float* scratch,
-         cudaStream_t stream);
+// Floats of scratch for so many chunks.
+long long scratch_floats(int mode, int n_heads, int e, int f, long long chunks);
+// The scan of a part.  A request's parts come one after the other, on one stream: each goes on from the
+// state that the one before it left in the slot.
+int scan(const Args& a, const Part& part, float* scratch, cudaStream_t stream);
 }  // namespace mls_chunk

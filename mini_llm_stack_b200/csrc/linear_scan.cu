@@ -519,19 +519,18 @@ MLS_API int mls_linear_scan(const void* a_src, int a_dtype, int a_row, int a_off
 }
 
 // The same for prompts, chunk by chunk (chunk_scan.cu): a decay per token with the token read first,
-// or one decay a head with the token taken in first and no bonus.  It takes the requests of at least
-// `least` tokens, `taken` of them: `most` chunks of one at the most, `window` of every one at a time,
-// `chunks` in all of them together.
+// or one decay a head with the token taken in first and no bonus.  Of the requests of at least `least`
+// tokens it takes `count` from the `from`th on: their chunks [first, first + span), `chunks` in all.
 MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, int a_off,
                                     const void* k_src, int k_dtype, int k_row, int k_off,
                                     const void* v_src, int v_dtype, int v_row, int v_off,
                                     const float* decay_tok, const float* decay_head,
                                     const void* bonus, int bonus_dtype, int read_first,
                                     const int* cu_q, const int* state_slot, float* state,
-                                    long long state_stride, int n_requests, int n_tokens,
-                                    int n_heads, int e, int f, float* out, int act, int least,
-                                    int taken, int most, int window, long long chunks, float* scratch,
-                                    cudaStream_t stream) {
+                                    long long state_stride, int n_requests, int n_heads,
+                                    int e, int f, float* out, int act, int least,
+                                    int from, int count, int first, int span, int chunks,
+                                    float* scratch, cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
     if (e <= 0 || f <= 0 || (!decay_tok == !decay_head) || (decay_tok && !read_first) ||
@@ -552,14 +551,13 @@ MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, i
     a.slot_stride = state_stride;
     a.head_stride = e * f;
     a.n_requests = n_requests;
-    a.n_tokens = n_tokens;
     a.n_heads = n_heads;
     a.e = e;
     a.f = f;
     a.least = least;
     a.out = out;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
-    return scan(a, taken, most, window, chunks, scratch, stream);
+    return scan(a, Part{from, count, first, span, chunks}, scratch, stream);
 }
 
 MLS_API int mls_scan_finish(const float* o, const void* gate, int gate_dtype, int gate_row,

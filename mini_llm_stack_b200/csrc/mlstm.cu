@@ -410,15 +410,14 @@ MLS_API int mls_mlstm_scan(const void* qkvg, int dtype, int row_w, int q_off, in
                             fc, n_groups, num, den, chunked_from, stream);
 }
 
-// The same for prompts, chunk by chunk (chunk_scan.cu): the requests of at least `least` tokens, `taken`
-// of them; `most` chunks of one at the most, `window` of every one at a time, `chunks` in all of them
-// together.
+// The same for prompts, chunk by chunk (chunk_scan.cu): of the requests of at least `least` tokens, `count`
+// from the `from`th on, their chunks [first, first + span), `chunks` in all.
 MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q_off, int k_off,
                                    int v_off, const float* gates, const void* bias_i,
                                    const void* bias_f, int b_dtype, float cap, const int* cu_q,
                                    const int* state_slot, float* state, long long slot_stride,
-                                   int n_requests, int n_tokens, int n_heads, int e, int f, float* num,
-                                   float* den, int least, int taken, int most, int window, long long chunks,
+                                   int n_requests, int n_heads, int e, int f, float* num,
+                                   float* den, int least, int from, int count, int first, int span, int chunks,
                                    float* scratch, cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
@@ -443,14 +442,13 @@ MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q
     a.slot_stride = slot_stride;
     a.head_stride = e * f + e + a.n_groups;
     a.n_requests = n_requests;
-    a.n_tokens = n_tokens;
     a.n_heads = n_heads;
     a.e = e;
     a.f = f;
     a.least = least;
     a.out = num;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
-    return scan(a, taken, most, window, chunks, scratch, stream);
+    return scan(a, Part{from, count, first, span, chunks}, scratch, stream);
 }
 
 MLS_API int mls_mlstm_finish(const float* num, const float* den, const void* gate, int gate_row,

@@ -811,8 +811,8 @@ class Ops:
                                   _I, _I, _I, _I, _P, _P, _I, _P]),
                    "chunked": _decl(lib, "mls_mlstm_scan_chunked",
                                     [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
-                                     _I, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _LL, _P, _P]),
-                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
+                                     _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P]),
+                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish": _decl(lib, "mls_mlstm_finish",
                                    [_P, _P, _P, _I, _I, _P, _I, _F, _P, _I, _I, _I, _I, _P])}
@@ -867,9 +867,9 @@ class Ops:
                                   _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _I, _P]),
                    "chunked": _decl(lib, "mls_linear_scan_chunked",
                                     [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _P, _P,
-                                     _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _P, _I, _I, _I,
-                                     _I, _I, _LL, _P, _P]),
-                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _I, _LL],
+                                     _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _I, _I, _I,
+                                     _I, _I, _I, _P, _P]),
+                   "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish_row": _decl(lib, "mls_scan_finish_row",
                                        [_P, _P, _I, _I, _I, _P, _F, _F, _P, _LL, _I, _I, _P]),
@@ -1050,14 +1050,33 @@ class Ops:
     # against 87 and 96 at 128, 0.81 (numerators), 0.84 (denominators) and 0.68.  A request's own length decides and nothing else of the
     # step, so that its bits do not depend on the requests beside it.
     CHUNKED_FROM = {"head": 48, "token": 192, "mlstm": 128}
-    CHUNK_SCRATCH = 1 << 27       # floats of scratch that a window of chunks may take
+    CHUNK_SCRATCH = 1 << 27       # floats of scratch that the chunks under way may take (at least one does)
+
+    @staticmethod
+    def _chunk_parts(each: list, most: int) -> list:
+        """Requests of ``each`` so many chunks, cut into parts of at most ``most`` chunks in all: (first
+        request, requests, first chunk of each, chunks of each at the most, chunks in all).  Whole
+        requests, as many as fit, or as many chunks as fit of one that does not."""
+        parts, at, n, longest, total = [], 0, 0, 0, 0
+        for i, c in enumerate(each):
+            if n and total + c > most:
+                parts.append((at, n, 0, longest, total))
+                at, n, longest, total = i, 0, 0, 0
+            if c > most:
+                parts += [(i, 1, k, min(most, c - k), min(most, c - k)) for k in range(0, c, most)]
+                at = i + 1
+            else:
+                n, longest, total = n + 1, max(longest, c), total + c
+        if n:
+            parts.append((at, n, 0, longest, total))
+        return parts
 
     def _chunk_plan(self, part: str, mode: int, step, operands: list, whole: tuple, strides: tuple,
                     n_heads: int, e: int, f: int):
         """How the scans over a matrix state of a step's longer requests run chunk by chunk: (tokens
-        from which on a request does, such requests, the most chunks of one, chunks of each a window,
-        chunks of a window in all, scratch, whether other requests are left), or None: all token by
-        token.
+        from which on a request does, parts of the work, scratch, whether other requests are left), or
+        None: all token by token.  The parts change no bit: a request's chunks go on from the state
+        that the ones before them left in its slot.
 
         Chunk by chunk is for prompts of bfloat16 models (a float32 model's results do not depend
         on how a prompt is cut, which chunks counted from a step's first token would change) whose
@@ -1075,21 +1094,24 @@ class Ops:
                 or any(s & 3 for s in strides) or n_heads > 65535:
             return None
         each = [-(-n // self.CHUNK) for n in lens if n >= least]
-        most = window = max(each)
-        floats_of = self._part_lib(part)["scratch"]
-
-        def size(w):
-            chunks = sum(min(c, w) for c in each)
-            return chunks, floats_of(mode, step.n_tokens, n_heads, e, f, chunks)
-
-        chunks, floats = size(window)
-        while window > 1 and (floats > self.CHUNK_SCRATCH or chunks > 65535):
-            window = (window + 1) // 2
-            chunks, floats = size(window)
-        if chunks > 65535:
-            return None
-        return (least, len(each), most, window, chunks, self.scratch("chunk_scan", floats),
-                len(each) < len(lens))
+        chunk = self._part_lib(part)["scratch"](mode, n_heads, e, f, 1)
+        most = min(65535, max(1, self.CHUNK_SCRATCH // chunk))
+        while True:
+            parts = self._chunk_parts(each, most)
+            # (a power of two of chunks: scratch that grows drops the captured graphs)
+            need = min(most, 1 << (max(p[4] for p in parts) - 1).bit_length())
+            try:
+                scratch = self.scratch("chunk_scan", chunk * need)
+                break
+            except torch.cuda.OutOfMemoryError:
+                # fewer chunks at a time, from now on: what there is already, or half as many
+                held = self._scratch.get("chunk_scan")
+                fits = held.numel() // chunk if held is not None else 0
+                if most == 1:
+                    raise
+                most = fits if 0 < fits < most else most // 2
+                self.CHUNK_SCRATCH = most * chunk
+        return least, parts, scratch, len(each) < len(lens)
 
     def mlstm_state_width(self, e: int, f: int) -> int:
         """Floats of one head's state: the memory [e, f], the normaliser [e] and one
@@ -1116,14 +1138,15 @@ class Ops:
                                 (state, num), (width, width // n_heads), n_heads, e, f)
         chunked_from = 0
         if plan is not None:
-            chunked_from, taken, most, window, chunks, scratch, others = plan
-            self.launches += 5 * (-(-most // window))
-            _check(self._part_lib("mlstm")["chunked"](
-                _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
-                _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
-                _ptr(step.state_slot), _ptr(state), width, step.n_requests, t, n_heads, e, f,
-                _ptr(num), _ptr(den), chunked_from, taken, most, window, chunks, _ptr(scratch),
-                self._stream()), "mlstm_scan_chunked")
+            chunked_from, parts, scratch, others = plan
+            self.launches += 5 * len(parts)
+            for p in parts:
+                _check(self._part_lib("mlstm")["chunked"](
+                    _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
+                    _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
+                    _ptr(step.state_slot), _ptr(state), width, step.n_requests, n_heads, e, f,
+                    _ptr(num), _ptr(den), chunked_from, *p, _ptr(scratch), self._stream()),
+                    "mlstm_scan_chunked")
             if not others:
                 return
         self.launches += 1
@@ -1500,17 +1523,18 @@ class Ops:
                                     (state.stride(0), e * f), n_heads, e, f)
         chunked_from = 0
         if plan is not None:
-            chunked_from, taken, most, window, chunks, scratch, others = plan
-            self.launches += 4 * (-(-most // window))
-            _check(self._part_lib("scan")["chunked"](
-                _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],
-                _ptr(k[0]), _code(k[0].dtype), k[0].shape[1], k[1],
-                _ptr(v[0]), _code(v[0].dtype), v[0].shape[1], v[1],
-                _ptr(decay_tok), _ptr(decay_head), _ptr(bonus),
-                _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
-                _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
-                step.n_requests, t, n_heads, e, f, _ptr(out), 1 if silu else 0, chunked_from, taken,
-                most, window, chunks, _ptr(scratch), self._stream()), "linear_scan_chunked")
+            chunked_from, parts, scratch, others = plan
+            self.launches += 4 * len(parts)
+            for p in parts:
+                _check(self._part_lib("scan")["chunked"](
+                    _ptr(a[0]), _code(a[0].dtype), a[0].shape[1], a[1],
+                    _ptr(k[0]), _code(k[0].dtype), k[0].shape[1], k[1],
+                    _ptr(v[0]), _code(v[0].dtype), v[0].shape[1], v[1],
+                    _ptr(decay_tok), _ptr(decay_head), _ptr(bonus),
+                    _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
+                    _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
+                    step.n_requests, n_heads, e, f, _ptr(out), 1 if silu else 0, chunked_from, *p,
+                    _ptr(scratch), self._stream()), "linear_scan_chunked")
             if not others:
                 return
         self.launches += 1

@@ -281,3 +281,55 @@ def test_no_further_from_float64_than_token_by_token(ops, kind, heads, e, f, mor
     for i, want in enumerate([torch.stack(outs).view(t, -1), last] + ([torch.stack(dens)] if dens else [])):
         mine, theirs = ((got[x][i].double() - want).norm() / want.norm() for x in (True, False))
         assert mine <= (1.01 + 2 * want.numel() ** -0.5) * theirs, (i, float(mine), float(theirs))
+
+
+@pytest.mark.parametrize("kind", ["head", "token", "mlstm"])
+def test_scratch_is_bounded(always, kind):
+    """Three chunks of scratch for 34 requests, and memory that gives out: parts of the work, the same bits."""
+    ops = Runtime("cuda:0", torch.bfloat16).ops        # its own scratch
+    for part in ("scan", "mlstm"):
+        ops.require_part(part)
+    always.setattr(ops, "CHUNKED_FROM", {"head": 2, "token": 2, "mlstm": 2}, raising=False)
+    lens = [200, 70, 1, 600] + [3] * 30
+    heads, e, f, t, r = 2, 64, 64, sum(lens), len(lens)
+    g = torch.Generator().manual_seed(3)
+    rows = torch.randn(t, heads * (2 * e + f), generator=g).bfloat16().cuda()
+    decay = (1 - 0.2 * torch.rand(t, heads * e, generator=g)).cuda()
+    gates, bias = torch.randn(t, 2 * heads, generator=g).cuda(), torch.randn(2, heads, generator=g).cuda()
+    width = ops.mlstm_state_width(e, f) if kind == "mlstm" else e * f
+
+    def walk():
+        step = a_step(lens, True)[0]
+        state = torch.zeros(r, heads * width, device="cuda")
+        out, den = torch.full((t, heads * f), float("nan"), device="cuda"), torch.zeros(t, heads, device="cuda")
+        if kind == "mlstm":
+            ops.mlstm_scan(rows, (0, heads * e, 2 * heads * e), gates, bias[0], bias[1], 15.0, step,
+                           state.view(r, heads, width), heads, e, f, out, den)
+        else:
+            ops.linear_scan((rows, 0), (rows, heads * e), (rows, 2 * heads * e), state, step, heads, e, f, out,
+                            decay_tok=decay if kind == "token" else None,
+                            decay_head=torch.tensor([0.97, 0.8]).cuda() if kind == "head" else None,
+                            read_first=kind == "token")
+        return out, den, state
+
+    part = ops._part_lib("mlstm" if kind == "mlstm" else "scan")
+    chunk = part["scratch"](("head", "token", "mlstm").index(kind), heads, e, f, 1)
+    always.setattr(ops, "CHUNK_SCRATCH", 3 * chunk, raising=False)
+    bounded = walk()
+    assert ops._scratch["chunk_scan"].numel() <= max(3 * chunk, 1 << 16)
+    always.setattr(ops, "CHUNK_SCRATCH", 1 << 27, raising=False)
+    real = ops.scratch
+
+    def short(tag, n):
+        if n > 5 * chunk:
+            raise torch.cuda.OutOfMemoryError("no more")
+        return real(tag, n)
+
+    always.setattr(ops, "scratch", short)
+    given_out = walk()
+    assert chunk <= ops.CHUNK_SCRATCH <= 5 * chunk
+    always.setattr(ops, "scratch", real)
+    always.setattr(ops, "CHUNK_SCRATCH", 1 << 27, raising=False)
+    whole = walk()
+    for x, y, z in zip(bounded, given_out, whole):
+        assert torch.equal(x, z) and torch.equal(y, z) and torch.isfinite(z).all()
