@@ -519,8 +519,8 @@ MLS_API int mls_route_sort(const int* idx, int n_slots, int n_experts, int n_rea
 }
 
 // Whether the products of these operands run on the tensor cores.
-MLS_API int mls_expert_takes_tc(int dtype, const void* a, const void* w, int K, int n_experts) {
-    return takes_tc(dtype, a, w, K, n_experts) ? 1 : 0;
+MLS_API int mls_expert_takes_tc(int dtype, const void* a, const void* w, int K) {
+    return takes_tc(dtype, a, w, K) ? 1 : 0;
 }
 
 // One of the experts' products over the sorted slots: N outputs of K inputs an expert.  `rows`:
@@ -533,7 +533,7 @@ static int expert_product(const void* A, const void* W, void* out, int dtype, co
                           int n_experts, int N, int K, void* rows, float alpha, float limit,
                           int* status, cudaStream_t stream) {
     if (max_tiles <= 0) return 0;
-    if (takes_tc(dtype, A, W, K, n_experts)) {
+    if (takes_tc(dtype, A, W, K)) {
         if (UNIT != DOWN) {
             if (!rows) return MLS_ERR_UNSUPPORTED;
             const int rc = gather_tc(A, order, weight, top, scale, n_slots, K, rows, stream);

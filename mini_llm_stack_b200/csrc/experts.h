@@ -6,7 +6,7 @@ namespace mls_experts {
 // What a product does: the experts' down projection, or an up projection with a unit on its sums.
 enum { DOWN = 0, GATED = 1, RELU2 = 2 };
 
-constexpr int TC_EXPERTS = 4096;     // experts whose table fits beside the stages
+constexpr int TC_EXPERTS = 4096;     // experts of a launch: their table lies beside the stages
 
 // The gated unit on the two products' float32 sums.
 __device__ __forceinline__ float gated_unit(float g, float u, float alpha, float limit) {
@@ -19,7 +19,7 @@ __device__ __forceinline__ float gated_unit(float g, float u, float alpha, float
 }
 
 // bfloat16 rows of whole 16-byte pieces at 16-byte addresses: the tensor cores'.
-bool takes_tc(int dtype, const void* a, const void* w, int K, int n_experts);
+bool takes_tc(int dtype, const void* a, const void* w, int K);
 // The product over sorted rows [n_slots, K], and the rows themselves.
 int product_tc(int unit, const void* rows, const void* W, void* out, const int* order,
                const int* offsets, const float* weight, int scale, int n_slots, int n_experts, int N,

@@ -365,8 +365,8 @@ int launch_nt(const TcParams& p, const void* rows, const void* W, int n_slots, c
 // The lines leave room for experts of twice the average before a second tile is needed at 32;
 // from 96 on average a good part of the experts has more than 128 rows.
 template <int UNIT>
-int launch_unit(const TcParams& p, const void* rows, const void* W, int n_slots, cudaStream_t stream) {
-    const int average = n_slots / p.n_experts;
+int launch_unit(const TcParams& p, const void* rows, const void* W, int n_slots, int average,
+                cudaStream_t stream) {
     if (average >= 96) return launch_nt<UNIT, 256>(p, rows, W, n_slots, stream);
     if (average >= 16) return launch_nt<UNIT, 128>(p, rows, W, n_slots, stream);
     return launch_nt<UNIT, 32>(p, rows, W, n_slots, stream);
@@ -374,8 +374,8 @@ int launch_unit(const TcParams& p, const void* rows, const void* W, int n_slots,
 }  // namespace
 
 namespace mls_experts {
-bool takes_tc(int dtype, const void* a, const void* w, int K, int n_experts) {
-    return dtype == MLS_BF16 && K % 8 == 0 && n_experts <= TC_EXPERTS &&
+bool takes_tc(int dtype, const void* a, const void* w, int K) {
+    return dtype == MLS_BF16 && K % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
 }
 
@@ -383,10 +383,18 @@ int product_tc(int unit, const void* rows, const void* W, void* out, const int* 
                const int* offsets, const float* weight, int scale, int n_slots, int n_experts, int N,
                int K, float alpha, float limit, int* status, cudaStream_t stream) {
     if (n_slots <= 0 || N <= 0) return 0;
-    const TcParams p{out, order, offsets, weight, n_experts, N, K, scale, alpha, limit, status};
-    if (unit == GATED) return launch_unit<GATED>(p, rows, W, n_slots, stream);
-    if (unit == RELU2) return launch_unit<RELU2>(p, rows, W, n_slots, stream);
-    return launch_unit<DOWN>(p, rows, W, n_slots, stream);
+    const int average = n_slots / n_experts;
+    // as many experts a launch as their table has room beside the stages
+    for (int e0 = 0; e0 < n_experts; e0 += TC_EXPERTS) {
+        const int n = n_experts - e0 < TC_EXPERTS ? n_experts - e0 : TC_EXPERTS;
+        const TcParams p{out, order, offsets + e0, weight, n, N, K, scale, alpha, limit, status};
+        const void* w = (const __nv_bfloat16*)W + (size_t)e0 * (unit == GATED ? 2 : 1) * N * K;
+        const int rc = unit == GATED   ? launch_unit<GATED>(p, rows, w, n_slots, average, stream)
+                       : unit == RELU2 ? launch_unit<RELU2>(p, rows, w, n_slots, average, stream)
+                                       : launch_unit<DOWN>(p, rows, w, n_slots, average, stream);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 int gather_tc(const void* h, const int* order, const float* weight, int top, int scale, int n_slots,

@@ -822,7 +822,7 @@ class Ops:
                                  [_P, _I, _I, _I, _I, _I, _I, _P, _F, _I, _I, _P, _P, _P]),
                    "sort": _decl(lib, "mls_route_sort",
                                  [_P, _I, _I, _I, _P, _P, _P, _P, _I, _P, _P]),
-                   "takes_tc": _decl(lib, "mls_expert_takes_tc", [_I, _P, _P, _I, _I]),
+                   "takes_tc": _decl(lib, "mls_expert_takes_tc", [_I, _P, _P, _I]),
                    "glu": _decl(lib, "mls_expert_glu",
                                 [_P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P,
                                  _F, _F, _P, _P]),
@@ -1210,8 +1210,8 @@ class Ops:
     def _expert_rows(self, h, w, n_slots: int):
         """Scratch for the sorted rows of an experts' first product where it runs on the tensor
         cores, else None; counts the kernel that fills it."""
-        n_experts, k = w.shape[0], w.shape[2]
-        if not self._part_lib("experts")["takes_tc"](_code(h.dtype), _ptr(h), _ptr(w), k, n_experts):
+        k = w.shape[2]
+        if not self._part_lib("experts")["takes_tc"](_code(h.dtype), _ptr(h), _ptr(w), k):
             return None
         self.launches += 1
         return self.scratch("expert_rows", (n_slots * k + 1) // 2)

@@ -160,3 +160,37 @@ def test_combination(ops, d, top, shared):
         want = want + rows.double() * (torch.sigmoid(gate[:, 2:].double()) if shared == "gated" else 1.0)
     # float32 sums of `top` values, one rounding to 8 bits
     assert ((delta.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("unit", ["silu", "relu2"])
+def test_more_experts_than_a_launch_takes(ops, unit):
+    """5,000 experts, rows at both ends and on both sides of 4,096, on the tensor cores; a few rows of
+    each against float64."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    experts, t, top, d, f = 5000, 40, 3, 64, 16
+    idx = torch.randint(0, experts, (t, top), generator=torch.Generator().manual_seed(2))
+    idx[:, 1] = (idx[:, 0] + 1) % experts
+    idx[:, 2] = (idx[:, 0] + 2) % experts
+    idx[:8] = torch.tensor([[0, 4095, 4096]] * 4 + [[4999, 4096, 1]] * 4)
+    work = routed(ops, idx, torch.ones(t, top), experts, experts)
+    h = torch.randn(t, d, device="cuda", generator=g).bfloat16()
+    mats = 1 if unit == "relu2" else 2
+    w1 = (torch.randn(experts, mats * f, d, device="cuda", generator=g) * d ** -0.5).bfloat16()
+    w2 = (torch.randn(experts, d, f, device="cuda", generator=g) * f ** -0.5).bfloat16()
+    assert ops._part_lib("experts")["takes_tc"](1, h.data_ptr(), w1.data_ptr(), d)
+    n = t * top
+    y = torch.full((n, f), float("nan"), dtype=torch.bfloat16, device="cuda")
+    out = torch.full((n, d), float("nan"), device="cuda")
+    (ops.expert_relu_squared if unit == "relu2" else ops.expert_glu)(h, w1, y, work, top, False)
+    ops.expert_down(y, w2, out, work, top, False)
+    ops.check_status()
+    rows, e = torch.arange(n, device="cuda") // top, idx.reshape(-1).cuda()
+    z = torch.einsum("nfd,nd->nf", w1[e].double(), h[rows].double())
+    want = z.clamp(min=0) ** 2 if unit == "relu2" else z[:, :f] * torch.sigmoid(z[:, :f]) * z[:, f:]
+    place = torch.empty(n, dtype=torch.long, device="cuda")
+    place[work["order"].long()] = torch.arange(n, device="cuda")
+    got = y[place].double()
+    # one rounding to 8 bits behind float32 sums of d products; float32 sums of f products
+    assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 1e-5
+    down = torch.einsum("ndf,nf->nd", w2[e].double(), got)
+    assert (out.double() - down).abs().max() <= 1e-5 * max(1.0, float(got.norm(dim=1).max()))
