@@ -142,8 +142,20 @@ def test_choice_and_order(ops, experts, groups):
 @pytest.mark.parametrize("top", [1, 6, 9])
 @pytest.mark.parametrize("shared", [None, "rows", "gated"])
 def test_combination(ops, d, top, shared):
+    combination(ops, 11, d, top, shared)
+
+
+@pytest.mark.parametrize("t, d", [(127, 256), (128, 256), (130, 252), (32, 1024), (31, 1024), (64, 516), (64, 514)])
+@pytest.mark.parametrize("top", [1, 9])
+@pytest.mark.parametrize("shared", [None, "rows", "gated"])
+def test_combination_of_more_rows(ops, t, d, top, shared):
+    """Both sides of the line from which on rows are added up four entries at a time."""
+    combination(ops, t, d, top, shared)
+
+
+def combination(ops, t, d, top, shared):
     g = torch.Generator().manual_seed(d + top)
-    t, n_real = 11, 7
+    n_real = 7
     per_slot = torch.randn(t * top, d, generator=g)
     h = torch.randn(t, d, generator=g).bfloat16()
     idx = torch.randint(0, n_real + 2, (t, top), generator=g)
