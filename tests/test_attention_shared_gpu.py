@@ -215,3 +215,24 @@ def test_scales_that_are_not_positive(ops, monkeypatch, taken, scale):
     want = by_warps(ops, monkeypatch, step, cache, qkv, 4, 1, scale)
     assert (out.float() - want).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * want.abs().max()
     assert not taken
+
+
+@pytest.mark.parametrize("block, calls", [(8, 1), (16, 1), (32, 1), (64, 0)])
+@pytest.mark.parametrize("heads, kv", [(4, 1), (6, 2)])
+def test_which_pages_the_kernel_takes(ops, monkeypatch, taken, block, calls, heads, kv):
+    step, cache, qkv, plan = prompts(ops, heads, kv, block=block)
+    out = torch.full((step.n_tokens, heads * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(qkv, out, cache, step, heads, kv, HD, HD ** -0.5, 0, plan=plan)
+    ops.check_status()
+    assert len(taken) == calls
+    want = by_warps(ops, monkeypatch, step, cache, qkv, heads, kv, HD ** -0.5)
+    assert (out.float() - want).abs().max() <= 2.0 ** -9 * 4 + 2.0 ** -8 * want.abs().max()
+
+
+def test_rows_of_keys_and_values_apart_are_not_taken(ops, taken):
+    step, cache, qkv, plan = prompts(ops)
+    cache.v_pool = cache.k_pool.clone()
+    out = torch.empty(step.n_tokens, 4 * HD, dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(qkv, out, cache, step, 4, 1, HD, HD ** -0.5, 0, plan=plan)
+    ops.check_status()
+    assert not taken

@@ -206,3 +206,22 @@ def test_more_experts_than_a_launch_takes(ops, unit):
     assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max() + 1e-5
     down = torch.einsum("ndf,nf->nd", w2[e].double(), got)
     assert (out.double() - down).abs().max() <= 1e-5 * max(1.0, float(got.norm(dim=1).max()))
+
+
+@pytest.mark.parametrize("t, experts, identity, top, d, f, spread", CASES)
+def test_which_products_run_on_the_tensor_cores(ops, t, experts, identity, top, d, f, spread):
+    """The cases above: rows of whole 16-byte pieces do (the gather of the first product is a launch more),
+    the down products of 129 and 130 inputs do not."""
+    idx = choices(t, experts + identity, top, spread, torch.Generator().manual_seed(0))
+    work = routed(ops, idx, torch.ones(t, top), experts + identity, experts)
+    b16 = dict(dtype=torch.bfloat16, device="cuda")
+    h, y, out = torch.zeros(t, d, **b16), torch.zeros(t * top, f, **b16), torch.zeros(t * top, d, device="cuda")
+    w1, w2 = torch.zeros(experts, 2 * f, d, **b16), torch.zeros(experts, d, f, **b16)
+    takes = ops._part_lib("experts")["takes_tc"]
+    assert d % 8 == 0 and takes(1, h.data_ptr(), w1.data_ptr(), d)
+    assert bool(takes(1, y.data_ptr(), w2.data_ptr(), f)) == (f % 8 == 0)
+    before = ops.launches
+    ops.expert_glu(h, w1, y, work, top, True)
+    assert ops.launches - before == 2
+    ops.expert_down(y, w2, out, work, top, False)
+    ops.check_status()
