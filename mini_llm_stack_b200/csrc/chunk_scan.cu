@@ -26,8 +26,9 @@
 // 306 -> 95 (the products run at 38 to 40 TFLOP/s: the updates' loads are not all hidden by the other
 // blocks' arithmetic, and wkv's weights of pairs take 42 us).
 //
-// A value that is not a number reaches the earlier tokens of its chunk too (0 x NaN), as it does in
-// the prompt attention's tiles; requests never share a chunk.
+// A token's value that is infinite or not a number reaches no earlier token: P is lower triangular, and a
+// chunk with such a value multiplies its lower triangle only (0 x inf is not 0).  Requests never share a
+// chunk.
 //
 // Bound by the FFMA pipe: T H (2 e f + 64 (e + f)) multiply-adds (retention, 2,048 tokens of 32 heads
 // of 128 x 256: 5.9 G, 0.16 ms at 74 TFLOP/s), and the states' way through memory (U written,
@@ -153,11 +154,12 @@ __device__ __forceinline__ void fill_rows(float (*T)[W], Get get) {
 }
 
 // acc += A x B over DEPTH of k, from k0: thread (ty, tx) owns rows 4 ty .. + 3 and 32 further on, columns
-// 4 tx .. + 3 and, with eight columns a thread (TN), BN / 2 further on.
-template <int BN, int TN, bool TURN_A, int DEPTH = C>
+// 4 tx .. + 3 and, with eight columns a thread (TN), BN / 2 further on.  LOWER: row r of A ends at k = r,
+// and what follows (zeros) is left out.
+template <int BN, int TN, bool TURN_A, int DEPTH = C, bool LOWER = false>
 __device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*A)[C], const float (*B)[BN],
                                          int tx, int ty, int k0 = 0) {
-#pragma unroll 8
+#pragma unroll (LOWER ? 1 : 8)
     for (int k = k0; k < k0 + DEPTH; ++k) {
         const int ra = TURN_A ? (4 * ty) ^ turn(k) : 4 * ty;
         float v[8];
@@ -172,6 +174,7 @@ __device__ __forceinline__ void multiply(f32x2 (&acc)[8][TN / 2], const float (*
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
+            if (LOWER && 4 * ty + (i & 3) + 32 * (i >> 2) < k) continue;
             const f32x2 two = twice(v[i]);
 #pragma unroll
             for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], two, b[j]);
@@ -742,13 +745,18 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
     };
     float4 next[QA];
     fill_transposed<THREADS>(A[0], [&](int t, int x) { return *reinterpret_cast<const float4*>(P + t * C + x); });
-    fill_rows<THREADS, BN>(B[0], [&](int t, int j) { return v(t, j0 + j); });
+    bool odd = false;                                          // a value that is not a number, or infinite
+    fill_rows<THREADS, BN>(B[0], [&](int t, int j) {
+        const float4 x = v(t, j0 + j);
+        odd |= !((x.x + x.y + x.z + x.w) * 0.f == 0.f);        // (a sum that overflows: no harm)
+        return x;
+    });
     if (with_n && threadIdx.x < C) n_s[0][threadIdx.x] = 1.f;
     f32x2 acc[8][TN / 2], sum[8][TN / 2];
     clear(acc);
     clear(sum);
     float nq[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // short chains: the sum may nearly vanish
-    __syncthreads();
+    odd = __syncthreads_or(odd);
     for (int b = 0; b < blocks; ++b) {
         const int x = b & 1, i0 = b * C;                       // i0: first row of the next block's S0
         const bool more = b + 1 < blocks;
@@ -765,7 +773,8 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
         }
 #pragma unroll 1
         for (int k0 = 0; k0 < C; k0 += SUMS) {
-            multiply<BN, TN, true, SUMS>(acc, A[x], B[x], tx, ty, k0);
+            if (odd && b == 0) multiply<BN, TN, true, SUMS, true>(acc, A[0], B[0], tx, ty, k0);
+            else multiply<BN, TN, true, SUMS>(acc, A[x], B[x], tx, ty, k0);
 #pragma unroll
             for (int y = 0; y < 8; ++y) settle(sum[y], acc[y]);
         }

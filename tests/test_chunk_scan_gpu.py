@@ -333,3 +333,41 @@ def test_scratch_is_bounded(always, kind):
     whole = walk()
     for x, y, z in zip(bounded, given_out, whole):
         assert torch.equal(x, z) and torch.equal(y, z) and torch.isfinite(z).all()
+
+
+@pytest.mark.parametrize("kind", ["head", "token", "mlstm"])
+@pytest.mark.parametrize("what", ["v", "k", "q"])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan")])
+@pytest.mark.parametrize("f", [64, 132])
+def test_no_number_reaches_earlier_tokens_or_other_requests(ops, always, kind, what, odd, f):
+    """One entry of one token that is infinite or not a number: earlier tokens of its chunk and other
+    requests keep their bits, later ones are no numbers where the token-by-token kernel has none."""
+    lens, bad, heads, e = [70, 200, 3], 70 + 100, 2, 64
+    t = sum(lens)
+    g = torch.Generator().manual_seed(5)
+    clean = torch.randn(t, heads * (2 * e + f), generator=g).bfloat16().cuda()
+    spoiled = clean.clone()
+    spoiled[bad, {"q": 0, "k": heads * e, "v": 2 * heads * e}[what] + 5] = odd
+    decay = (1 - 0.2 * torch.rand(t, heads * e, generator=g)).cuda()
+    gates, bias = torch.randn(t, 2 * heads, generator=g).cuda(), torch.randn(2, heads, generator=g).cuda()
+    got = {}
+    for name, rows, chunked in (("clean", clean, True), ("odd", spoiled, True), ("tokens", spoiled, False)):
+        step = a_step(lens, chunked)[0]
+        out, den = torch.empty(t, heads * f, device="cuda"), torch.ones(t, heads, device="cuda")
+        if kind == "mlstm":
+            state = torch.zeros(3, heads, ops.mlstm_state_width(e, f), device="cuda")
+            ops.mlstm_scan(rows, (0, heads * e, 2 * heads * e), gates, bias[0], bias[1], 15.0, step, state, heads,
+                           e, f, out, den)
+        else:
+            state = torch.zeros(3, heads * e * f, device="cuda")
+            ops.linear_scan((rows, 0), (rows, heads * e), (rows, 2 * heads * e), state, step, heads, e, f, out,
+                            decay_tok=decay if kind == "token" else None,
+                            decay_head=torch.tensor([0.97, 0.8]).cuda() if kind == "head" else None,
+                            read_first=kind == "token")
+        got[name] = torch.cat([out, den], 1)
+    untouched = torch.ones(t, dtype=torch.bool, device="cuda")
+    untouched[bad:270] = False
+    assert torch.equal(got["odd"][untouched], got["clean"][untouched])
+    # (a denominator that is no number falls to its floor, in either kernel: the numerators tell)
+    odd, tokens = (got[x][:, :heads * f].isfinite() for x in ("odd", "tokens"))
+    assert torch.equal(odd, tokens) and not odd[bad].all()
