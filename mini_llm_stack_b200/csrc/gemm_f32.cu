@@ -241,14 +241,14 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
 // of a block share rows, so all but the first read of a row meets L1.  The 32 partial sums are
 // added by a fixed tree.  The order of the additions depends on K alone (never on M, on COLS or
 // on the row's place), and which kernel runs depends on N alone, so a token's result still does
-// not depend on its batch: many rows take eight or nine columns a warp, fewer rows two, a decode
-// step's one.  Measured against blocks of eight rows in shared memory, whose loads bounded it:
+// not depend on its batch: many rows take eight or nine columns a warp (or four), fewer rows two, a
+// decode step's one.  Measured against blocks of eight rows in shared memory, whose loads bounded it:
 // 2,048 x 65 x 4,096 from bfloat16 rows 115 -> 45 us, 300 x 64 x 4,096 46 -> 16,
 // 2,048 x 8 x 2,048 25 -> 8.
 constexpr int SKINNY_N = 256, SK_ROWS = 8;
 
-// BY4: four entries of a row of W at a time; VEC: of A as well.
-template <typename T, bool BY4, bool VEC, int COLS>
+// BY4: four entries of a row at a time, of both operands.
+template <typename T, bool BY4, int COLS>
 __global__ void __launch_bounds__(256)
 gemm_f32_skinny_kernel(const T* __restrict__ A, const float* __restrict__ W, float* __restrict__ out,
                        int M, int N, int K) {
@@ -275,7 +275,7 @@ gemm_f32_skinny_kernel(const T* __restrict__ A, const float* __restrict__ W, flo
         for (int k = lane * 4; k < K; k += 128) {
             float4 a[SK_ROWS];
 #pragma unroll
-            for (int r = 0; r < SK_ROWS; ++r) a[r] = fetch4<VEC>(a_row[r], k, K);
+            for (int r = 0; r < SK_ROWS; ++r) a[r] = load4(a_row[r] + k);
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
                 const float4 w = load4(w_row + (size_t)min(c, last) * K + k);
@@ -311,71 +311,97 @@ gemm_f32_skinny_kernel(const T* __restrict__ A, const float* __restrict__ W, flo
         }
 }
 
-// The same for the few rows of a decode step: a block holds SK_ROWS rows of A in shared memory
-// (all its warps' loads at once under way) and each of its warps one column, with the loads of
-// several rounds of W under way.  The same order of additions.
+// The same with a block's SK_ROWS rows of A in shared memory (all its warps' loads at once under way) and
+// COLS columns a warp, with the loads of several rounds of W under way.  The same order of additions.
+// One column a warp for the few rows of a decode step; four for many rows that cannot be read four
+// entries at a time, where the kernel above has more than one wave of two columns a warp.
 constexpr int SK_KC = 1024;
-template <typename T>
+template <int COLS>
 __global__ void __launch_bounds__(256)
-gemm_f32_skinny_few_kernel(const T* __restrict__ A, const float* __restrict__ W,
-                           float* __restrict__ out, int M, int N, int K, int by4) {
+gemm_f32_skinny_shared_kernel(const void* __restrict__ A, int a_dtype, const float* __restrict__ W,
+                              float* __restrict__ out, int M, int N, int K, int by4) {
     chain_release();
     chain_wait();
     __shared__ __align__(16) float As[SK_ROWS][SK_KC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * SK_ROWS, n = blockIdx.y * 8 + warp;
-    float acc[SK_ROWS];
+    const int m0 = blockIdx.x * SK_ROWS;
+    const int n0 = (blockIdx.y * 8 + warp) * COLS;
+    float acc[COLS][SK_ROWS];
 #pragma unroll
-    for (int r = 0; r < SK_ROWS; ++r) acc[r] = 0.f;
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int r = 0; r < SK_ROWS; ++r) acc[c][r] = 0.f;
     for (int k0 = 0; k0 < K; k0 += SK_KC) {
         const int kc = min(SK_KC, K - k0);
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < SK_ROWS; ++r)
             for (int k = threadIdx.x; k < kc; k += 256)
-                As[r][k] = m0 + r < M ? Elem<T>::load(A + (size_t)(m0 + r) * K + k0 + k) : 0.f;
+                As[r][k] = m0 + r < M ? load_as_float(A, (size_t)(m0 + r) * K + k0 + k, a_dtype) : 0.f;
         __syncthreads();
-        if (n >= N) continue;
-        const float* w_row = W + (size_t)n * K + k0;
+        if (n0 >= N) continue;
         if (by4) {
 #pragma unroll 4
             for (int k = lane * 4; k < kc; k += 128) {
-                const float4 w = load4(w_row + k);
+                float4 a[SK_ROWS];
 #pragma unroll
-                for (int r = 0; r < SK_ROWS; ++r) {
-                    const float4 a = *reinterpret_cast<const float4*>(&As[r][k]);
-                    float s = acc[r];
-                    s = fmaf(a.x, w.x, s);
-                    s = fmaf(a.y, w.y, s);
-                    s = fmaf(a.z, w.z, s);
-                    acc[r] = fmaf(a.w, w.w, s);
+                for (int r = 0; r < SK_ROWS; ++r) a[r] = *reinterpret_cast<const float4*>(&As[r][k]);
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) {
+                    if (n0 + c >= N) break;
+                    const float4 w = load4(W + (size_t)(n0 + c) * K + k0 + k);
+#pragma unroll
+                    for (int r = 0; r < SK_ROWS; ++r) {
+                        float s = acc[c][r];
+                        s = fmaf(a[r].x, w.x, s);
+                        s = fmaf(a[r].y, w.y, s);
+                        s = fmaf(a[r].z, w.z, s);
+                        acc[c][r] = fmaf(a[r].w, w.w, s);
+                    }
                 }
             }
         } else {
             for (int k = lane; k < kc; k += 32) {
-                const float w = w_row[k];
 #pragma unroll
-                for (int r = 0; r < SK_ROWS; ++r) acc[r] = fmaf(As[r][k], w, acc[r]);
+                for (int c = 0; c < COLS; ++c) {
+                    if (n0 + c >= N) break;
+                    const float w = W[(size_t)(n0 + c) * K + k0 + k];
+#pragma unroll
+                    for (int r = 0; r < SK_ROWS; ++r) acc[c][r] = fmaf(As[r][k], w, acc[c][r]);
+                }
             }
         }
     }
 #pragma unroll
-    for (int r = 0; r < SK_ROWS; ++r) {
-        const float s = warp_sum(acc[r]);
-        if (lane == 0 && n < N && m0 + r < M) out[(size_t)(m0 + r) * N + n] = s;
-    }
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int r = 0; r < SK_ROWS; ++r) {
+            const float s = warp_sum(acc[c][r]);
+            if (lane == 0 && n0 + c < N && m0 + r < M) out[(size_t)(m0 + r) * N + n0 + c] = s;
+        }
 }
 
-template <typename T, bool BY4, bool VEC>
-int skinny(const T* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
+template <typename T, int COLS>
+int skinny_shared(const T* A, const float* W, float* out, int M, int N, int K, bool by4, cudaStream_t stream) {
+    MLS_LAUNCH((gemm_f32_skinny_shared_kernel<COLS>),
+               dim3((M + SK_ROWS - 1) / SK_ROWS, (N + 8 * COLS - 1) / (8 * COLS)), dim3(256), 0, stream,
+               (const void*)A, sizeof(T) == 2 ? MLS_BF16 : MLS_F32, W, out, M, N, K, by4 ? 1 : 0);
+    return launch_status();
+}
+
+template <typename T>
+int skinny(const T* A, const float* W, float* out, int M, int N, int K, bool vec_a, bool vec_w, cudaStream_t stream) {
     const int groups = (M + SK_ROWS - 1) / SK_ROWS;
-#define SKINNY(C)                                                                                  \
+#define SKINNY(BY4, C)                                                                             \
     do {                                                                                           \
         const long long warps = (long long)groups * ((N + C - 1) / C);                             \
-        MLS_LAUNCH((gemm_f32_skinny_kernel<T, BY4, VEC, C>), dim3((unsigned)((warps + 7) / 8)),    \
+        MLS_LAUNCH((gemm_f32_skinny_kernel<T, BY4, C>), dim3((unsigned)((warps + 7) / 8)),         \
                    dim3(256), 0, stream, A, W, out, M, N, K);                                      \
         return launch_status();                                                                    \
     } while (0)
+    if (M < 64 || vec_a != vec_w)
+        return M < 64 ? skinny_shared<T, 1>(A, W, out, M, N, K, vec_w, stream)
+                      : skinny_shared<T, 4>(A, W, out, M, N, K, vec_w, stream);
     // Two columns a warp while those blocks are one wave (two an SM fit their registers): it is
     // then a warp's own chain of loads that counts, and a third of the registers lets more of them
     // be under way (512 x 64 x 4,096 from bfloat16 rows, after a flush of L2: 39 us with four
@@ -383,9 +409,25 @@ int skinny(const T* A, const float* W, float* out, int M, int N, int K, cudaStre
     // once for eight columns (2,048 x 64 x 4,096: 102, 56, 62), or nine where that saves a group
     // (64 router outputs and a gate's column).  With float32 rows nine is the faster of the two
     // throughout (1,500 x 64 x 2,048: 45 us with eight, 36 with nine).
-    if ((long long)groups * ((N + 1) / 2) <= 8LL * 2 * sm_count()) SKINNY(2);
-    if (sizeof(T) == 4 || (N + 8) / 9 < (N + 7) / 8) SKINNY(9);
-    SKINNY(8);
+    const bool one_wave = (long long)groups * ((N + 1) / 2) <= 8LL * 2 * sm_count();
+    const bool nine = (N + 8) / 9 < (N + 7) / 8;
+    if (vec_a) {
+        if (one_wave) SKINNY(true, 2);
+        if constexpr (sizeof(T) == 2)
+            if (!nine) SKINNY(true, 8);
+        SKINNY(true, 9);
+    }
+    // Entry by entry the wide variants' loads bound them: they wait out fewer than eight warps an SM, and
+    // float32 rows throughout, while shared memory serves four columns a warp (K = 1,023, wide / shared: float32
+    // 1,500 x 33 50 / 25 us, 1,500 x 128 94 / 71; bfloat16 200 x 256 34 / 26, 1,500 x 64 25 / 49).  Two columns a
+    // warp are one too many for one column (64 x 1 x 2,050 27 / 22 us) in float32.
+    if (one_wave && (N > 1 || sizeof(T) == 2)) SKINNY(false, 2);
+    if constexpr (sizeof(T) == 2)
+        if ((long long)groups * ((N + 7) / 8) >= 8LL * sm_count()) {
+            if (nine) SKINNY(false, 9);
+            SKINNY(false, 8);
+        }
+    return skinny_shared<T, 4>(A, W, out, M, N, K, false, stream);
 #undef SKINNY
 }
 
@@ -428,23 +470,14 @@ int few(const float* A, const float* W, float* out, int M, int N, int K, cudaStr
     if (N >= 64 * 2 * sm_count()) return few_of<64, 4, 5>(A, W, out, M, N, K, stream);
     return few_of<16, 1, 8>(A, W, out, M, N, K, stream);
 }
-int few(const __nv_bfloat16*, const float*, float*, int, int, int, cudaStream_t) { return MLS_ERR_UNSUPPORTED; }
 
 template <typename T>
 int product(const T* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
     const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
     const bool vec_w = K % 4 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
-    if (N <= SKINNY_N && M < 64) {
-        MLS_LAUNCH((gemm_f32_skinny_few_kernel<T>), dim3((M + SK_ROWS - 1) / SK_ROWS, (N + 7) / 8),
-                   dim3(256), 0, stream, A, W, out, M, N, K, vec_w ? 1 : 0);
-        return launch_status();
-    }
-    if (N <= SKINNY_N) {
-        if (vec_w && vec_a) return skinny<T, true, true>(A, W, out, M, N, K, stream);
-        if (vec_w) return skinny<T, true, false>(A, W, out, M, N, K, stream);
-        return skinny<T, false, false>(A, W, out, M, N, K, stream);
-    }
-    if (vec_w && vec_a && M <= FEW_M && sizeof(T) == 4) return few(A, W, out, M, N, K, stream);
+    if (N <= SKINNY_N) return skinny(A, W, out, M, N, K, vec_a, vec_w, stream);
+    if constexpr (sizeof(T) == 4)
+        if (vec_w && vec_a && M <= FEW_M) return few(A, W, out, M, N, K, stream);
     if (vec_w && vec_a) return tiled<T, true>(A, W, out, M, N, K, stream);
     return tiled<T, false>(A, W, out, M, N, K, stream);
 }
