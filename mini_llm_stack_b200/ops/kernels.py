@@ -677,15 +677,56 @@ class Ops:
                       _ptr(slopes), keep_first, out.stride(0), int(chunk), plan.share, self._stream()),
                    "attention_mma")
             return
-        # requests of several tokens share their keys by tiles, the others take a warp a row
+        # requests of several tokens share their keys by tiles where that is the faster way, the others
+        # take a warp a row
         lens = getattr(step, "q_lens", None) or [0]
-        self.launches += 2 if max(lens) >= 8 > min(lens) and hd % 4 == 0 and hd <= 128 else 1
+        longest = max(lens) if self._rows_by_tiles(step, lens, n_heads, n_kv,
+                                                   int(window) or int(chunk)) else 0
+        self.launches += 2 if longest >= 8 > min(lens) and hd % 4 == 0 and hd <= 128 else 1
         _check(self._attention_simt(
             _ptr(qkv), _ptr(out), _code(qkv.dtype), _ptr(cache.k_pool), _ptr(cache.v_pool),
             _ptr(g.block_table), g.max_blocks, _ptr(step.positions), _ptr(step.req_of_token),
             t, n_heads, n_kv, hd, g.block_size, float(scale), int(window), float(softcap),
             cache.k_pool.shape[1], _ptr(sink), _ptr(slopes), keep_first, out.stride(0), int(chunk),
-            _ptr(step.cu_q), max(lens), min(lens), self._stream()), "attention_simt")
+            _ptr(step.cu_q), longest, min(lens), self._stream()), "attention_simt")
+
+    # What the two float32 attention kernels take, in keys that a warp walks alone (0.67 us a key with heads
+    # of 64, 1.1 with 128): a tile's warps walk one in 0.3 of that, up to 16,000 (key, row) pairs cost the
+    # GPU's tiles as much, 2,500 its warps; the second kernel's launch as much as ten.
+    TILE_KEY, TILE_PAIRS, ROW_PAIRS, TILE_LAUNCH = 0.3, 16000, 2500, 10
+
+    def _rows_by_tiles(self, step, lens: list, n_heads: int, n_kv: int, span: int) -> bool:
+        """Whether the float32 attention kernels should take a step's requests of eight tokens and more by
+        tiles (the bits are the same).  The tiles run before the rows, so that decoded tokens beside a short
+        portion wait for both (seven decoded at 1,000 tokens and a portion of nine, 8 heads of 80: 892 us
+        with tiles, 676 by rows), and the requests in one block come one after the other (16 prompts of
+        eight tokens, no group: 39 us, 11 by rows), while a portion of 64 at 8,000 tokens takes a quarter.
+        ``span`` > 0: a token reads at most so many keys."""
+        if max(lens) < 8:
+            return False
+        ctx = getattr(step, "ctx_lens", None)
+        if not ctx:
+            return True
+        key = ("rows_by_tiles", n_heads, n_kv, span)
+        known = getattr(step, "attn_tiles", None)
+        if known is not None and key in known:
+            return known[key]
+        tokens = max(1, 32 // min(n_heads // n_kv, 32))          # of a block
+        reads = [(n, min(c, span + n) if span else c) for n, c in zip(lens, ctx)]
+        big, small = [x for x in reads if x[0] >= 8], [x for x in reads if x[0] < 8]
+        pairs = [n_heads * sum(n * (c - n / 2) for n, c in some) for some in (big, small)]
+
+        def longest(some):
+            return max((c for _, c in some), default=0)
+
+        by_rows = max(longest(big), longest(small), sum(pairs) / self.ROW_PAIRS)
+        in_a_block = max(c * min(len(big), -(-tokens // n)) for n, c in big)
+        by_tiles = (max(self.TILE_KEY * in_a_block, pairs[0] / self.TILE_PAIRS) + self.TILE_LAUNCH
+                    + max(longest(small), pairs[1] / self.ROW_PAIRS))
+        if known is None:
+            return by_tiles < by_rows
+        known[key] = by_tiles < by_rows
+        return known[key]
 
     def _split_launches(self, n_split: int, tma: bool, n_ctas: int) -> int:
         """Kernels the context-split attention launches: two to eight splits merge inside
