@@ -50,6 +50,18 @@ def test_finish(ops, act, t, heads, f, weighted):
 @pytest.mark.parametrize("t, heads, e, dims", [(1, 1, 8, 8), (5, 3, 64, 32), (4, 2, 64, 60), (3, 32, 128, 128),
                                                (2, 3, 72, 8), (2, 5, 128, 0), (3, 2, 20, 8)])
 def test_rotation(ops, act, t, heads, e, dims):
+    rotation(ops, act, t, heads, e, dims)
+
+
+@pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("t, heads, e, dims", [(1, 64, 8, 8), (5, 8, 64, 32), (4, 9, 64, 56), (2, 8, 72, 8), (3, 7, 72, 72),
+                                               (2, 4, 128, 0), (2, 26, 20, 8), (1, 1, 512, 256)])
+def test_rotation_of_wide_rows(ops, act, t, heads, e, dims):
+    """Rows on both sides of 512 entries, from which on they go four entries at a time."""
+    rotation(ops, act, t, heads, e, dims)
+
+
+def rotation(ops, act, t, heads, e, dims):
     g = torch.Generator(device="cuda").manual_seed(t + e)
     width = heads * e
     src = torch.randn(t, 3 * width, device="cuda", generator=g).to(act)
