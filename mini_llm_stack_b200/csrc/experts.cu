@@ -594,9 +594,9 @@ MLS_API int mls_expert_combine(const float* per_slot, int top, const void* share
     auto quads = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
     const int act = dtype == MLS_BF16 ? 8 : 16;
     // (Few or narrow rows are one short wave either way, and the loop over single entries ends sooner: 8
-    // tokens of 512 entries, 8 rows each, 1.56 us, 1.81 by quads; 2,048 of 64 1.88, 2.76; 130 of 256 1.70, 1.80;
-    // 300 of 256 2.05, 1.93; 64 of 512 1.82, 1.81.  2,048 of 2,048, 4 rows: 20.0, 11.4.)
-    if (d >= 256 && (long long)n_tokens * d >= 32768 &&
+    // tokens of 512 entries, 8 rows each, 1.56 us, 1.81 by quads; 2,048 of 64 1.88, 2.76; 64 of 512 1.56, 1.69; 33 of
+    // 1,024 1.68, 1.79.  130 of 512 1.93, 1.87; 64 of 2,048, 4 rows, 2.18, 1.77; 2,048 of them 20.0, 11.4.)
+    if (d >= 256 && (long long)n_tokens * d >= 65536 &&
         d % 4 == 0 && shared_stride % 4 == 0 && n_tokens <= 65535 && quads(per_slot, 16) && quads(h, act) &&
         quads(delta, act) && quads(shared, shared_dtype == MLS_BF16 ? 8 : 16)) {
         const int threads = d >= 1024 ? 256 : 64;

@@ -145,7 +145,7 @@ def test_combination(ops, d, top, shared):
     combination(ops, 11, d, top, shared)
 
 
-@pytest.mark.parametrize("t, d", [(127, 256), (128, 256), (130, 252), (32, 1024), (31, 1024), (64, 516), (64, 514)])
+@pytest.mark.parametrize("t, d", [(255, 256), (256, 256), (280, 252), (64, 1024), (63, 1024), (130, 516), (130, 514)])
 @pytest.mark.parametrize("top", [1, 9])
 @pytest.mark.parametrize("shared", [None, "rows", "gated"])
 def test_combination_of_more_rows(ops, t, d, top, shared):

@@ -33,3 +33,17 @@ def test_product(ops, a_type, m, n, k):
     few = torch.empty(len(some), n, device="cuda")
     ops.linear(a[some].contiguous(), w, few)
     assert torch.equal(few, out[some])
+
+
+@pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off_a, off_w", [(1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m, n, k", [(5, 33, 64), (100, 33, 64), (1500, 70, 64), (90, 300, 64)])
+def test_rows_between_addresses(ops, a_type, off_a, off_w, m, n, k):
+    """Operands that cannot be read four entries at a time although their rows are whole quads."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m * k + 1, device="cuda", generator=g).to(a_type)[off_a:][:m * k].view(m, k)
+    w = torch.randn(n * k + 1, device="cuda", generator=g)[off_w:][:n * k].view(n, k)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    ops.linear(a, w, out)
+    bound = 2.0 ** -24 * (k + 2) * (a.double().abs() @ w.double().abs().T)
+    assert ((out.double() - a.double() @ w.double().T).abs() <= bound + 1e-30).all()
