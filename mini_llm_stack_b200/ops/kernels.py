@@ -1085,8 +1085,8 @@ class Ops:
     CHUNK = 64                    # tokens of a chunk of the chunk-wise scans
     # Tokens of a request from which on its scans run chunk by chunk: where one prompt's four or five
     # short kernels take no longer than the other kernel token by token, and lie no further from
-    # float64.  Retention, 16 and 32 heads of 128 x 256: 38 and 43 us against 40 and 47 at 48 tokens, errors
-    # 0.94 (outputs) and 0.74 (states) of its.  wkv, 32 and 64 heads of 64 x 64: 40 and 48 against 57 and 72 at
+    # float64.  Retention, 16 and 32 heads of 128 x 256: 39 and 45 us against 40 and 47 at 48 tokens, errors
+    # 0.94 (outputs) and 0.74 (states) of its.  wkv, 32 and 64 heads of 64 x 64: 41 and 49 against 57 and 72 at
     # 200 tokens, 0.97 and 0.85 at 192, but 1.02 and 0.88 at 128.  mLSTM, 4 and 8 heads of 256 x 512: 86 and 77
     # against 87 and 96 at 128, 0.81 (numerators), 0.84 (denominators) and 0.68.  A request's own length decides and nothing else of the
     # step, so that its bits do not depend on the requests beside it.
