@@ -27,6 +27,8 @@
 // 12.6 MFLOP and are 18.9 now, half as much again for 16 % of the time, so it is the softmax, one warp a
 // scheduler, that most of a step waits for; at the measured 1.65 PFLOP/s the products of a step take
 // about 3,100 cycles).
+// A key or value that is not a number reaches the earlier tokens of its tile of 128 rows, and of a tile whose last
+// page it lies in (0 x NaN), as in attention_tc.cu; requests share no page.
 // Every wait is bounded and reports MLS_STATUS_TIMEOUT.
 #include "common.cuh"
 #include "tma.cuh"

@@ -18,13 +18,13 @@
 // All of it float32 on CUDA cores as in the token-by-token kernels (fma.rn.f32x2).  Decays enter only as
 // factors <= 1, never as the reciprocal of one.  Scores, the rows of q and k times their factors and each
 // chunk's U are rounded to float32 once more than there; what a chunk saves is the state's own rounding a
-// token.  Ops.CHUNKED_FROM says from where on that leaves outputs and states no further from float64.  Chunks are counted
-// from a request's first token of the step.
+// token.  Ops.CHUNKED_FROM says from where on that leaves outputs and states no further from float64.
+// Chunks are counted from a request's first token of the step.
 //
-// Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,824 ->
-// 365 us, mLSTM of 4 heads of 256 x 512 1,296 -> 215; 1,501 tokens of wkv, 32 heads of 64 x 64,
-// 306 -> 95 (the products run at 38 to 40 TFLOP/s: the updates' loads are not all hidden by the other
-// blocks' arithmetic, and wkv's weights of pairs take 42 us).
+// Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,825 ->
+// 398 us, mLSTM of 4 heads of 256 x 512 1,343 -> 238, wkv of 32 heads of 64 x 64 581 -> 126 (the products run at
+// 38 to 40 TFLOP/s: the updates' loads are not all hidden by the other blocks' arithmetic, and wkv's weights of
+// pairs take a third of its time).
 //
 // A token's value that is infinite or not a number reaches no earlier token: P is lower triangular, and a
 // chunk with such a value multiplies its lower triangle only (0 x inf is not 0).  Requests never share a

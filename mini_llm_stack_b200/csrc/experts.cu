@@ -10,7 +10,7 @@
 //   chosen.  A (token, choice) pair is a "slot": slot = t * top + j.  Outputs n_real .. E-1 stand for experts without weights that
 //   return their input: they get no tiles, and mls_expert_combine adds weight * h for them.
 // mls_route_sort: slots ordered by expert: order[p] = slot, offsets[E + 1], and the list
-//   of row tiles (tile_expert, tile_row0) the products below walk.  One CTA.
+//   of row tiles (tile_expert, tile_row0) the CUDA-core products below walk.  One CTA.
 // mls_expert_glu: y[p, :] = unit(Wg[e] a, Wu[e] a) with unit(g, u) = silu(g) * u or, with a
 //   limit > 0, g' * sigmoid(alpha g') * (u' + 1), g' = min(g, limit), u' = clamp(u, +-limit);
 //   a = weight[slot] * h[token]
