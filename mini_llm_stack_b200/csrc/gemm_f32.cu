@@ -1,6 +1,8 @@
 // True 32-bit matrix product for the float32 path: out[M, N] = A[M, K] * W[N, K]^T.
 // A may be held in bfloat16 (a router's input in a 16-bit run): its values are widened as
 // they are loaded, the arithmetic is the same.
+// Long rows of many columns go to the tensor cores (gemm_f32_tc.cu; mls_f32::takes_tc says which); here
+// are the others.
 //
 // FFMA on CUDA cores, two products an instruction where they lie side by side (fma.rn.f32x2
 // rounds each as fmaf does): no tensor cores, no TF32, no reduced-precision mode.
@@ -9,8 +11,10 @@
 // Both operands are K-contiguous (the reference's nn.Linear layout [out, in],
 // train/model.py:79-82,130-132).
 #include "common.cuh"
+#include "gemm_f32.h"
 
 namespace {
+using namespace mls_f32;
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 twice(float a) {
     f32x2 r;
@@ -50,7 +54,8 @@ __device__ __forceinline__ float4 fetch4(const T* row, int k, int K) {
 // in registers, and two tiles in shared memory leave one barrier a block.
 // Measured against 64 x 64 tiles of 4 x 4 a thread, loaded element by element and behind two
 // barriers: 515 x 16,384 x 2,048 1,513 -> 718 us (48 TFLOP/s), 515 x 2,048 x 8,192 910 -> 506,
-// 2,048 x 16,384 x 2,048 5,289 -> 2,551 (54), 64 x 2,048 x 2,048 155 -> 64.  The same bits.
+// 2,048 x 16,384 x 2,048 5,289 -> 2,551 (54), 64 x 2,048 x 2,048 155 -> 64 (sizes that the tensor cores
+// take now).  The same bits.
 constexpr int BK = 16, KQ = BK / 4;
 
 template <typename T, bool VEC, int BM, int BN, int TM, int BLOCKS>
@@ -173,8 +178,8 @@ gemm_f32_kernel(const T* __restrict__ A, const float* __restrict__ W, float* __r
 // few columns a thread takes one output and a block 16 columns, so that every SM has a block; with
 // many, whose reads of shared memory would bound it (426 us for 3 x 128,256 x 2,048), a thread
 // takes four rows of a column and a block 64 columns.  Against the tiles of 32 x 64 above:
-// 1 x 2,048 x 2,048 64 -> 17 us, 1 x 2,048 x 8,192 245 -> 55, 8 x 128,256 x 2,048 428 -> 391.  Rows of
-// whole 16-byte pieces; the same bits.
+// 1 x 2,048 x 2,048 64 -> 17 us, 1 x 2,048 x 8,192 245 -> 55, 8 x 128,256 x 2,048 428 -> 391 (sizes that
+// the tensor cores take now).  Rows of whole 16-byte pieces; the same bits.
 constexpr int FEW_M = 8, FEW_K = 64, FEW_KP = FEW_K + 4;
 template <int BN, int ROWS, int STAGES>
 __global__ void __launch_bounds__(BN * (FEW_M / ROWS))
@@ -245,7 +250,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
 // decode step's one.  Measured against blocks of eight rows in shared memory, whose loads bounded it:
 // 2,048 x 65 x 4,096 from bfloat16 rows 115 -> 45 us, 300 x 64 x 4,096 46 -> 16,
 // 2,048 x 8 x 2,048 25 -> 8.
-constexpr int SKINNY_N = 256, SK_ROWS = 8;
+constexpr int SK_ROWS = 8;
 
 // BY4: four entries of a row at a time, of both operands.
 template <typename T, bool BY4, int COLS>
@@ -472,10 +477,12 @@ int few(const float* A, const float* W, float* out, int M, int N, int K, cudaStr
 }
 
 template <typename T>
-int product(const T* A, const float* W, float* out, int M, int N, int K, cudaStream_t stream) {
+int product(const T* A, int a_dtype, const float* W, float* out, int M, int N, int K, float* scratch, int* status,
+            cudaStream_t stream) {
     const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
     const bool vec_w = K % 4 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
     if (N <= SKINNY_N) return skinny(A, W, out, M, N, K, vec_a, vec_w, stream);
+    if (takes_tc(W, N, K)) return product_tc(A, a_dtype, W, out, M, N, K, scratch, status, stream);
     if constexpr (sizeof(T) == 4)
         if (vec_w && vec_a && M <= FEW_M) return few(A, W, out, M, N, K, stream);
     if (vec_w && vec_a) return tiled<T, true>(A, W, out, M, N, K, stream);
@@ -483,10 +490,17 @@ int product(const T* A, const float* W, float* out, int M, int N, int K, cudaStr
 }
 }  // namespace
 
-MLS_API int mls_gemm_f32(const void* A, int a_dtype, const float* W, float* out, int M, int N,
-                         int K, cudaStream_t stream) {
+// `scratch`: mls_gemm_f32_scratch_floats floats at a 16-byte address.
+MLS_API int mls_gemm_f32(const void* A, int a_dtype, const float* W, float* out, int M, int N, int K,
+                         float* scratch, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (a_dtype == MLS_F32) return product((const float*)A, W, out, M, N, K, stream);
-    if (a_dtype == MLS_BF16) return product((const __nv_bfloat16*)A, W, out, M, N, K, stream);
+    if (a_dtype == MLS_F32)
+        return product((const float*)A, a_dtype, W, out, M, N, K, scratch, status, stream);
+    if (a_dtype == MLS_BF16)
+        return product((const __nv_bfloat16*)A, a_dtype, W, out, M, N, K, scratch, status, stream);
     return MLS_ERR_UNSUPPORTED;
+}
+
+MLS_API long long mls_gemm_f32_scratch_floats(const void* A, int a_dtype, const float* W, int M, int N, int K) {
+    return M > 0 && takes_tc(W, N, K) ? tc_scratch_floats(A, a_dtype, M, N, K) : 0;
 }

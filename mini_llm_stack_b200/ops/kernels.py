@@ -128,7 +128,9 @@ class Ops:
         self._embed = _decl(core, "mls_embed", [_P, _P, _I, _P, _I, _I, _I, _F, _P, _P, _P, _P])
         self._add_rmsnorm = _decl(core, "mls_add_rmsnorm",
                                   [_P, _P, _I, _P, _I, _F, _P, _I, _I, _I, _P, _I, _LL, _P, _P])
-        self._gemm_f32 = _decl(core, "mls_gemm_f32", [_P, _I, _P, _P, _I, _I, _I, _P])
+        self._gemm_f32 = _decl(core, "mls_gemm_f32", [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P])
+        self._gemm_f32_scratch = _decl(core, "mls_gemm_f32_scratch_floats",
+                                       [_P, _I, _P, _I, _I, _I], restype=ctypes.c_longlong)
         self._rope_store = _decl(core, "mls_rope_store",
                                  [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                                   _LL, _I, _P, _I, _LL, _P, _P])
@@ -299,9 +301,12 @@ class Ops:
             _need(a.dtype in (torch.float32, torch.bfloat16), f"linear: input dtype {a.dtype}")
             o32 = out if out.dtype == torch.float32 else torch.empty(
                 (m, n), dtype=torch.float32, device=out.device)
+            # rows as bfloat16 parts, and sums of a product cut along K
+            floats = self._gemm_f32_scratch(_ptr(a), _code(a.dtype), _ptr(w), m, n, k)
+            held = self.scratch("gemm_f32", floats) if floats else None
             self.launches += 1
-            _check(self._gemm_f32(_ptr(a), _code(a.dtype), _ptr(w), _ptr(o32), m, n, k,
-                                  self._stream()), "gemm_f32")
+            _check(self._gemm_f32(_ptr(a), _code(a.dtype), _ptr(w), _ptr(o32), m, n, k, _ptr(held),
+                                  _ptr(self.status), self._stream()), "gemm_f32")
             if o32 is not out:
                 out.copy_(o32)
             return

@@ -47,3 +47,55 @@ def test_rows_between_addresses(ops, a_type, off_a, off_w, m, n, k):
     ops.linear(a, w, out)
     bound = 2.0 ** -24 * (k + 2) * (a.double().abs() @ w.double().abs().T)
     assert ((out.double() - a.double() @ w.double().T).abs() <= bound + 1e-30).all()
+
+
+@pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("m, n, k", [
+    (1, 257, 2048), (16, 300, 2052), (17, 260, 2304), (33, 2048, 2080), (161, 385, 2056), (170, 4100, 2048),
+    (700, 1000, 4100), (5, 16384, 512), (321, 16500, 548)])
+def test_product_on_tensor_cores(ops, a_type, off, m, n, k):
+    """Sizes around the edges of its tiles, blocks and groups: nearer to float64 than a chain over k could
+    be, and the same bits for a row whatever rows it is computed with (cut along K or not)."""
+    g = torch.Generator(device="cuda").manual_seed(m * n + k + off)
+    a = torch.randn(m * k + 1, device="cuda", generator=g).to(a_type)[off:][:m * k].view(m, k)
+    w = torch.randn(n, k, device="cuda", generator=g)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    ops.linear(a, w, out)
+    want = a.double() @ w.double().T
+    # parts left out: 3 of a product's 9, 2^-25 of it together at the most in the root mean square of many;
+    # sums: 2^-23 a step of four cut ones over 64 of k, 2^-24 rounded a block of 64 and a group
+    steps = 4 * 2 + (k + 63) // 64 / 8 + 8
+    size = (a.double().abs() @ w.double().abs().T)
+    assert ((out.double() - want).abs() <= 2.0 ** -24 * (2 + steps) * size).all()
+    assert (out.double() - want).norm() <= 2e-7 * want.norm()
+    some = sorted({0, m // 2, m - 1})
+    few = torch.empty(len(some), n, device="cuda")
+    ops.linear(a[some].contiguous(), w, few)
+    assert torch.equal(few, out[some])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("m", [4, 200])
+def test_odd_values_on_tensor_cores(ops, m):
+    """Infinities, values that are no numbers, and values at both ends of float32's range: what a chain
+    of float32 products and sums gives."""
+    n, k = 300, 2048
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, w = torch.randn(m, k, device="cuda", generator=g), torch.randn(n, k, device="cuda", generator=g)
+    a[0, 5], a[1, 7], a[2, :] = float("inf"), float("nan"), a[2] * 1e37
+    a[3] *= 2.0 ** -60
+    w[4, 9], w[6, 2], w[8] = 3.4e38, float("-inf"), w[8] * 2.0 ** -40
+    out = torch.empty(m, n, device="cuda")
+    ops.linear(a, w, out)
+    want = a.double() @ w.double().T
+    size = a.double().abs() @ w.double().abs().T
+    plain = size < 3e38                                   # no partial sum beyond float32's range
+    assert ((out.double() - want).abs()[plain] <= 2.0 ** -24 * 24 * size[plain]).all()
+    assert (out[0, 0].isinf() or out[0, 0].isnan()) and out[1].isnan().all()
+    # an infinite product decides a sum as in a chain: infinite where no other one is of the other sign
+    sure = torch.ones(m, n, dtype=torch.bool, device="cuda")
+    sure[:, 4] = sure[:, 6] = False
+    sure[1:] = False
+    assert (out[sure] == torch.where(a[0, 5] * w[:, 5] > 0, float("inf"), float("-inf")).expand(m, n)[sure]).all()
+    ops.check_status()
