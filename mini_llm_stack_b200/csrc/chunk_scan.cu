@@ -15,31 +15,28 @@
 //   carry    walks the chunks: leaves each chunk's S0 where its U was, and the last state in the slot
 //   output   [q | P] x [S0; v], a product over e + 64
 //
-// All of it float32 on CUDA cores as in the token-by-token kernels (fma.rn.f32x2).  Decays enter only as
-// factors <= 1, never as the reciprocal of one.  Scores, the rows of q and k times their factors and each
-// chunk's U are rounded to float32 once more than there; what a chunk saves is the state's own rounding a
-// token.  Ops.CHUNKED_FROM says from where on that leaves outputs and states no further from float64.
-// Chunks are counted from a request's first token of the step.
+// All of it float32, on CUDA cores (fma.rn.f32x2) or, updates and outputs of wide heads, as bfloat16 parts on the
+// tensor cores (chunk_scan_tc.cu).  Decays enter only as factors <= 1, never as the reciprocal of one.  Scores,
+// the rows of q and k times their factors and each chunk's U are rounded to float32 once more than token by
+// token; what a chunk saves is the state's own rounding a token.  Ops.CHUNKED_FROM says from where on that
+// leaves outputs and states no further from float64.  Chunks are counted from a request's first token of the step.
 //
-// Measured (2,048 tokens, the scan's launches together): retention of 32 heads of 128 x 256 1,825 ->
-// 398 us, mLSTM of 4 heads of 256 x 512 1,343 -> 238, wkv of 32 heads of 64 x 64 581 -> 126 (the products run at
-// 38 to 40 TFLOP/s: the updates' loads are not all hidden by the other blocks' arithmetic, and wkv's weights of
-// pairs take a third of its time).
+// Measured (2,048 tokens, the scan's launches together, token by token -> all on CUDA cores -> now): retention of
+// 32 heads of 128 x 256 1,825 -> 398 -> 225 us, mLSTM of 4 heads of 256 x 512 1,343 -> 238 -> 126; wkv of 32 heads of
+// 64 x 64 581 -> 126 (its weights of pairs take a third of that).
 //
 // A token's value that is infinite or not a number reaches no earlier token: P is lower triangular, and a
 // chunk with such a value multiplies its lower triangle only (0 x inf is not 0).  Requests never share a
 // chunk.
 //
-// Bound by the FFMA pipe: T H (2 e f + 64 (e + f)) multiply-adds (retention, 2,048 tokens of 32 heads
-// of 128 x 256: 5.9 G, 0.16 ms at 74 TFLOP/s), and the states' way through memory (U written,
-// read and written by carry, read: 134 MB each there).  Chunks of 64 balance the two: half the
-// length doubles the states, twice the length doubles the products within chunks.
-#include "chunk_scan.h"
-#include "common.cuh"
+// Bound by the states' way through memory (retention: U written, read and written by carry, read: 134 MB each, 82 us
+// together), the loads that a block waits for before it multiplies, and where the products run on CUDA cores by
+// the FFMA pipe: T H (2 e f + 64 (e + f)) multiply-adds.  Chunks of 64 balance the two: half the length doubles
+// the states, twice the length doubles the products within chunks.
+#include "chunk_common.cuh"
 
 namespace {
 using namespace mls_chunk;
-constexpr int C = CHUNK;
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 twice(float a) {
@@ -55,75 +52,6 @@ __device__ __forceinline__ float2 halves(f32x2 v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
     return r;
 }
-__device__ __forceinline__ float4 load4(const void* base, int dtype, size_t i) {
-    if (dtype == MLS_BF16) {
-        const uint2 raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)base + i);
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-        return make_float4(lo.x, lo.y, hi.x, hi.y);
-    }
-    return *reinterpret_cast<const float4*>((const float*)base + i);
-}
-__device__ __forceinline__ float silu1(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float4 times(float4 v, float f) {
-    return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
-}
-
-// Where a block's chunk lies.
-struct Where {
-    int r, c;                        // request, chunk of the request
-    int t0, n;                       // first token, tokens
-    int chunks;                      // the request's chunks of this part
-    size_t idx;                      // place among the part's chunks
-};
-
-// Chunk z of the part's chunks, or (REQUEST) the first one of its request z.  A request's length alone
-// says whether it goes chunk by chunk.  Every thread calls; false: none.
-template <bool REQUEST>
-__device__ __forceinline__ bool locate(const Args& a, const Part& p, int z, Where& w) {
-    __shared__ int at_s[2];          // request, place of its first chunk
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int taken = -p.from, before = 0;   // the part's requests and chunks before these 32
-        if (lane == 0) at_s[0] = -1;
-        __syncwarp();
-        for (int r0 = 0; r0 < a.n_requests; r0 += 32) {
-            const int r = r0 + lane;
-            const int len = r < a.n_requests ? a.cu_q[r + 1] - a.cu_q[r] : 0;
-            const bool in = len >= a.least;
-            const unsigned all = __ballot_sync(0xffffffffu, in);
-            const int k = taken + __popc(all & ((1u << lane) - 1u));
-            const int count = in && k >= 0 && k < p.count ? min(max((len + C - 1) / C - p.first, 0), p.span) : 0;
-            int sum = count;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_up_sync(0xffffffffu, sum, o);
-                if (lane >= o) sum += x;
-            }
-            const int start = before + sum - count;
-            const bool here = REQUEST ? in && k == z : z >= start && z < start + count;
-            if (here) {
-                at_s[0] = r;
-                at_s[1] = start;
-            }
-            if (__any_sync(0xffffffffu, here)) break;
-            taken += __popc(all);
-            before += __shfl_sync(0xffffffffu, sum, 31);
-        }
-    }
-    __syncthreads();
-    w.r = at_s[0];
-    if (w.r < 0) return false;
-    const int j = REQUEST ? 0 : z - at_s[1];
-    w.c = p.first + j;
-    const int t = a.cu_q[w.r], len = a.cu_q[w.r + 1] - t;
-    w.chunks = min(max((len + C - 1) / C - p.first, 0), p.span);
-    w.idx = (size_t)(at_s[1] + j);
-    w.t0 = t + w.c * C;
-    w.n = min(C, len - w.c * C);
-    return j < w.chunks;
-}
-
 // ------------------------------------------------------------------ tiles in shared memory
 // 64 rows of K-contiguous values become T[k][row ^ 4 (k / 4 % 8)]: neither the stores (four rows,
 // eight quads of k a warp) nor the reads of four rows at a time meet a bank twice.
@@ -199,39 +127,6 @@ __device__ __forceinline__ void clear(f32x2 (&acc)[8][N]) {
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < N; ++j) acc[i][j] = 0ull;
-}
-
-// Four entries of operand row t (zeros past the chunk and past the head's size).
-struct Reader {
-    const void* base;
-    size_t row, at;                  // elements between tokens; the head's first entry
-    int dtype, silu, n, size;
-    __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head)
-        : Reader(r, silu_, w, head, (size_t)w.t0) {}
-    __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head, size_t t0)
-        : base(r.base), row(r.row), at(t0 * r.row + r.off + (size_t)head * r.width),
-          dtype(r.dtype), silu(silu_), n(w.n), size(r.width) {}
-    __device__ __forceinline__ float4 operator()(int t, int i) const {
-        if (t >= n || i >= size) return make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v = load4(base, dtype, at + (size_t)t * row + i);
-        if (silu) v = make_float4(silu1(v.x), silu1(v.y), silu1(v.z), silu1(v.w));
-        return v;
-    }
-};
-
-// What scores and gates leave for the products: a factor of q and of k for every token and head
-// (HEAD_DECAY works them out itself), and the chunk's decay.  All of it by chunks, so that its size does
-// not depend on the step's other tokens.
-struct Scratch {
-    double* log_gates;               // MLSTM: [chunks, 64, H, 2]
-    float* states;                   // [chunks, H, e f (+ e)]
-    float* scores;                   // [chunks, H, 64, 64]
-    float* rows_q;                   // TOKEN_DECAY: [chunks, 64, H e]; MLSTM: factors [chunks, 64, H]
-    float* rows_k;
-    float* whole;                    // TOKEN_DECAY: [chunks, H, e]; MLSTM: [chunks, H]
-};
-__host__ __device__ inline int state_floats(int mode, int e, int f) {
-    return e * f + (mode == MLSTM ? e : 0);
 }
 
 // ------------------------------------------------------------------------------- scores
@@ -578,16 +473,6 @@ chunk_gates_kernel(const Args a, const Scratch s, const Part part) {
     for (int g = threadIdx.x; g < a.n_groups; g += blockDim.x) m_slot[g] = m_s[GATE_WARPS];
 }
 
-// Factors of the tokens' rows of q and k in this chunk.
-template <int MODE>
-__device__ __forceinline__ float row_factor(const Args& a, const float* factors, const Where& w, int head,
-                                            int t, int power) {
-    if (t >= w.n) return 0.f;
-    if (MODE == HEAD_DECAY) return powf(a.decay[head], (float)power);
-    if (MODE == MLSTM) return factors[(w.idx * C + t) * a.n_heads + head];
-    return 1.f;
-}
-
 // ------------------------------------------------------------------------------- update
 // U[i, j] = sum_s factor_s k_s[i] v_s[j]; MLSTM: and n[i] = sum_s factor_s k_s[i].
 // Tiles of 64 x 64, 8 x 4 a thread: the loads of a tile are hidden by the other blocks' arithmetic only,
@@ -835,6 +720,10 @@ int output(const Args& a, const Scratch& s, const Part& part, cudaStream_t strea
     return launch_status();
 }
 
+// The tensor cores take heads whose columns fill the 128 rows of an instruction (32 heads of 64 x 64 fill half
+// of them: 1,501 tokens' updates 16.4 us either way, outputs 32.8 against 32.6) and whose rows fit shared memory.
+bool takes_tc(const Args& a) { return a.e >= 64 && a.e <= 256 && a.f >= 128; }
+
 size_t token_smem(int e) {
     return (size_t)(3 * C * (e + 4) + (STEPS + RUNS + 1) * e) * sizeof(float);
 }
@@ -855,13 +744,15 @@ int launch(const Args& a, const Scratch& s, const Part& part, cudaStream_t strea
         MLS_LAUNCH((chunk_scores_kernel<MODE>), dim3(1, a.n_heads, part.chunks), dim3(256), 0,
                    stream, a, s, part);
     }
-    int rc = update<MODE>(a, s, part, stream);
+    const bool tensor_cores = takes_tc(a);
+    int rc = tensor_cores ? update_tc<MODE>(a, s, part, stream) : update<MODE>(a, s, part, stream);
     if (rc) return rc;
     const int quads = state_floats(MODE, a.e, a.f) / 4;
     MLS_LAUNCH((chunk_carry_kernel<MODE>), dim3((quads + 127) / 128, a.n_heads, part.count), dim3(128),
                0, stream, a, s, part);
     rc = launch_status();
     if (rc) return rc;
+    if (tensor_cores) return output_tc<MODE>(a, s, part, stream);
     // (a width of 64 leaves half of a wider tile empty)
     return a.f <= C ? output<MODE, 64>(a, s, part, stream)
                     : output<MODE, 128>(a, s, part, stream);

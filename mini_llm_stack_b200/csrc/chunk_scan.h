@@ -40,6 +40,7 @@ struct Args {
     int n_requests, n_heads, e, f;
     int least;                       // requests of at least so many tokens (>= 1); the others are left out
     float* out;                      // [T, H * f]
+    int* status;                     // where a wait that runs out is noted
 };
 
 // Some of the chunks of a step, as many as scratch holds at a time: chunks [first, first + span) of `count`

@@ -35,6 +35,7 @@
 // quarter of the lanes each), 8..15 = sums (two warps a quarter, 16 columns in turn).  Every
 // wait is bounded; one that runs out sets MLS_STATUS_TIMEOUT, and the kernel frees its tensor memory
 // and returns.
+#include "bf16_parts.cuh"
 #include "common.cuh"
 #include "gemm_f32.h"
 #include "tcgen05.cuh"
@@ -77,8 +78,6 @@ __device__ __noinline__ float chain_of(const TcParams& p, int m, int n) {
         s = fmaf(load_as_float(p.A, (size_t)m * p.K + k, p.a_f32 ? MLS_F32 : MLS_BF16), w[k], s);
     return s;
 }
-__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
-
 // Rows of 64 bytes with the 64-byte swizzle; 8-row groups are 512 bytes apart.
 __device__ __forceinline__ uint64_t rows_desc(uint32_t addr) {
     uint64_t d = 0;
@@ -90,26 +89,6 @@ __device__ __forceinline__ uint64_t rows_desc(uint32_t addr) {
     return d;
 }
 
-__device__ __forceinline__ bool elect_one() {
-    uint32_t yes;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(yes));
-    return yes != 0;
-}
-
-// Two neighbouring values as bfloat16 (lower half: the first), and what that leaves of them.
-__device__ __forceinline__ uint32_t part_of(float& x, float& y) {
-    uint32_t two;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(two) : "f"(y), "f"(x));
-    x -= __uint_as_float(two << 16);
-    y -= __uint_as_float(two & 0xffff0000u);
-    return two;
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-                 "r"(r[7]) : "memory");
-}
 template <int N>
 __device__ __forceinline__ void more_registers() {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
@@ -134,7 +113,7 @@ __device__ __forceinline__ Unit unit_of(const TcParams& p, int i) {
 // NT: the most rows of a tile.
 template <int NT>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
+gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ CUtensorMap rows_map,
                    const __grid_constant__ CUtensorMap w_map) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int ACCS = NT > 32 ? 2 : 4;
@@ -309,7 +288,7 @@ gemm_f32_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_ma
                     for (int y = 0; y < 3; ++y) {
                         uint32_t two[8];
 #pragma unroll
-                        for (int x = 0; x < 8; ++x) two[x] = part_of(v[2 * x], v[2 * x + 1]);
+                        for (int x = 0; x < 8; ++x) two[x] = bf16_part(v[2 * x], v[2 * x + 1]);
                         tmem_st8(w + y * (BK / 2) + h * 8, two);
                     }
                 }
@@ -390,7 +369,7 @@ gemm_f32_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_ma
 
 // The groups' sums of a cut product, added up in the groups' order.
 __global__ void __launch_bounds__(256)
-gemm_f32_parts_kernel(const TcParams p, const float* __restrict__ parts, float* __restrict__ out) {
+gemm_f32_parts_kernel(const __grid_constant__ TcParams p, const float* __restrict__ parts, float* __restrict__ out) {
     chain_release();
     chain_wait();
     const size_t size = (size_t)p.M * p.N;
@@ -432,10 +411,10 @@ split_rows_kernel(const T* __restrict__ A, int M, int K, int width, __nv_bfloat1
 #pragma unroll
     for (int y = 0; y < (sizeof(T) == 4 ? 3 : 1); ++y) {
         uint4 out;
-        out.x = part_of(v[0], v[1]);
-        out.y = part_of(v[2], v[3]);
-        out.z = part_of(v[4], v[5]);
-        out.w = part_of(v[6], v[7]);
+        out.x = bf16_part(v[0], v[1]);
+        out.y = bf16_part(v[2], v[3]);
+        out.z = bf16_part(v[4], v[5]);
+        out.w = bf16_part(v[6], v[7]);
         dst[y * apart] = out;
     }
 }

@@ -530,7 +530,7 @@ MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, i
                                     long long state_stride, int n_requests, int n_heads,
                                     int e, int f, float* out, int act, int least,
                                     int from, int count, int first, int span, int chunks,
-                                    float* scratch, cudaStream_t stream) {
+                                    float* scratch, int* status, cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
     if (e <= 0 || f <= 0 || (!decay_tok == !decay_head) || (decay_tok && !read_first) ||
@@ -556,6 +556,7 @@ MLS_API int mls_linear_scan_chunked(const void* a_src, int a_dtype, int a_row, i
     a.f = f;
     a.least = least;
     a.out = out;
+    a.status = status;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
     return scan(a, Part{from, count, first, span, chunks}, scratch, stream);
 }

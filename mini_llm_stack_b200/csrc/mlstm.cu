@@ -418,7 +418,7 @@ MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q
                                    const int* state_slot, float* state, long long slot_stride,
                                    int n_requests, int n_heads, int e, int f, float* num,
                                    float* den, int least, int from, int count, int first, int span, int chunks,
-                                   float* scratch, cudaStream_t stream) {
+                                   float* scratch, int* status, cudaStream_t stream) {
     using namespace mls_chunk;
     if (n_requests <= 0) return 0;
     if (e <= 0 || f <= 0 || n_heads <= 0) return MLS_ERR_UNSUPPORTED;
@@ -447,6 +447,7 @@ MLS_API int mls_mlstm_scan_chunked(const void* qkvg, int dtype, int row_w, int q
     a.f = f;
     a.least = least;
     a.out = num;
+    a.status = status;
     if (!fits(a)) return MLS_ERR_UNSUPPORTED;
     return scan(a, Part{from, count, first, span, chunks}, scratch, stream);
 }

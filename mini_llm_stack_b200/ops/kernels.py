@@ -857,7 +857,7 @@ class Ops:
                                   _I, _I, _I, _I, _P, _P, _I, _P]),
                    "chunked": _decl(lib, "mls_mlstm_scan_chunked",
                                     [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _LL,
-                                     _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P]),
+                                     _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P]),
                    "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish": _decl(lib, "mls_mlstm_finish",
@@ -914,7 +914,7 @@ class Ops:
                    "chunked": _decl(lib, "mls_linear_scan_chunked",
                                     [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _P, _P, _P,
                                      _I, _I, _P, _P, _P, _LL, _I, _I, _I, _I, _P, _I, _I, _I, _I,
-                                     _I, _I, _I, _P, _P]),
+                                     _I, _I, _I, _P, _P, _P]),
                    "scratch": _decl(lib, "mls_chunk_scratch_floats", [_I, _I, _I, _I, _LL],
                                     restype=ctypes.c_longlong),
                    "finish_row": _decl(lib, "mls_scan_finish_row",
@@ -1191,7 +1191,8 @@ class Ops:
                     _ptr(qkvg), _code(qkvg.dtype), qkvg.shape[1], q_off, k_off, v_off, _ptr(gates),
                     _ptr(bias_i), _ptr(bias_f), _code(bias_i.dtype), float(cap), _ptr(step.cu_q),
                     _ptr(step.state_slot), _ptr(state), width, step.n_requests, n_heads, e, f,
-                    _ptr(num), _ptr(den), chunked_from, *p, _ptr(scratch), self._stream()),
+                    _ptr(num), _ptr(den), chunked_from, *p, _ptr(scratch),
+                    _ptr(self.status), self._stream()),
                     "mlstm_scan_chunked")
             if not others:
                 return
@@ -1580,7 +1581,7 @@ class Ops:
                     _code(bonus.dtype) if bonus is not None else 0, 1 if read_first else 0,
                     _ptr(step.cu_q), _ptr(step.state_slot), _ptr(state), state.stride(0),
                     step.n_requests, n_heads, e, f, _ptr(out), 1 if silu else 0, chunked_from, *p,
-                    _ptr(scratch), self._stream()), "linear_scan_chunked")
+                    _ptr(scratch), _ptr(self.status), self._stream()), "linear_scan_chunked")
             if not others:
                 return
         self.launches += 1

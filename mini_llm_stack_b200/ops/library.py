@@ -45,10 +45,10 @@ MODULES = {
     "layernorm": ["layernorm.cu"],
     "tanhnorm": ["tanh_norm.cu"],
     "latent": ["latent.cu"],
-    "mlstm": ["mlstm.cu", "chunk_scan.cu"],
+    "mlstm": ["mlstm.cu", "chunk_scan.cu", "chunk_scan_tc.cu"],
     "experts": ["experts.cu", "experts_tc.cu"],
     "shortconv": ["short_conv.cu"],
-    "scan": ["linear_scan.cu", "chunk_scan.cu"],
+    "scan": ["linear_scan.cu", "chunk_scan.cu", "chunk_scan_tc.cu"],
     "headprep": ["head_prep.cu"],
     "side": ["side_input.cu"],
     "gatednorm": ["gated_norm.cu"],

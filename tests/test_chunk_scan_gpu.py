@@ -371,3 +371,10 @@ def test_no_number_reaches_earlier_tokens_or_other_requests(ops, always, kind, w
     # (a denominator that is no number falls to its floor, in either kernel: the numerators tell)
     odd, tokens = (got[x][:, :heads * f].isfinite() for x in ("odd", "tokens"))
     assert torch.equal(odd, tokens) and not odd[bad].all()
+
+
+@pytest.mark.parametrize("kind", ["head", "head_silu"])
+@pytest.mark.parametrize("e, f, heads", [(64, 128, 2), (160, 300, 1), (252, 516, 1)])
+def test_wide_heads_on_tensor_cores(ops, always, e, f, heads, kind):
+    """Heads of one, two and four groups of 128 columns a block, with remainders of 64 rows and of 128 columns."""
+    test_linear_scan(ops, always, [130, 1, 7, 128], e, f, heads, kind)
