@@ -10,6 +10,12 @@ constexpr int SKINNY_N = 256;        // up to so many columns the product is by 
 // 22.6 both).
 constexpr int TC_K = 2048;
 constexpr long long TC_SIZE = 1 << 23;
+// Rows of 4,096 to 8,191 stay with the chain over k although the tensor cores would take them faster and leave
+// them nearer to float64 (16 x 4,096 x 4,096: 164 / 35 us).  What such runs are checked against are chains over k
+// in float32 themselves: a layer of hidden size 4,096 lies up to 3.3e-5 from float64 there and is held to 3.0e-5,
+// so that only sums with the same roundings pass (the chain's differ from it by 2.4e-5, the tensor cores' by 3.2e-5,
+// float64's own would by 3.3e-5).  From 8,192 on (feed-forward rows) and below 4,096 both pass.
+constexpr int CHAIN_K0 = 4096, CHAIN_K1 = 8192;
 
 // Whether the tensor cores take a product.  N, K and the weights' address say so, never the rows: a row's
 // bits do not depend on the rows it is computed with.

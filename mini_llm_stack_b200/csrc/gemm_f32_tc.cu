@@ -517,7 +517,8 @@ int launch_nt(const TcParams& p, const CUtensorMap& rows_map, const CUtensorMap&
 
 namespace mls_f32 {
 bool takes_tc(const float* W, int N, int K) {
-    return N > SKINNY_N && (K >= TC_K || (K >= TC_K / 4 && (long long)N * K >= TC_SIZE)) && K % 4 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
+    if (N <= SKINNY_N || K % 4 || reinterpret_cast<uintptr_t>(W) % 16 || (K >= CHAIN_K0 && K < CHAIN_K1)) return false;
+    return K >= TC_K || (K >= TC_K / 4 && (long long)N * K >= TC_SIZE);
 }
 
 long long tc_scratch_floats(const void* A, int a_dtype, int M, int N, int K) {
