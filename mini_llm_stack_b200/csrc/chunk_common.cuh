@@ -16,7 +16,7 @@ __device__ __forceinline__ float4 load4(const void* base, int dtype, size_t i) {
     }
     return *reinterpret_cast<const float4*>((const float*)base + i);
 }
-__device__ __forceinline__ float silu1(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu1(float z) { return times_sigmoid(z, z); }
 __device__ __forceinline__ float4 times(float4 v, float f) {
     return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
 }

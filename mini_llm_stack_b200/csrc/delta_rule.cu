@@ -38,8 +38,8 @@
 namespace {
 constexpr float DR_UNIT_EPS = 1e-6f;     // inside the root of the unit vectors
 
-__device__ __forceinline__ float silu1(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float sigmoid1(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu1(float z) { return times_sigmoid(z, z); }
+__device__ __forceinline__ float sigmoid1(float z) { return times_sigmoid(1.0f, z); }
 __device__ __forceinline__ float softplus1(float z) {
     return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
 }

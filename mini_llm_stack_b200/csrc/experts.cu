@@ -405,7 +405,7 @@ __global__ void expert_combine_kernel(const float* __restrict__ per_slot, int to
             float v = load_as_float(shared, i, shared_dtype);
 #pragma unroll 4
             for (int k = 1; k < shared_parts; ++k) v += ((const float*)shared)[i + k * shared_stride];
-            s += gate ? v / (1.0f + expf(-gate[t * gate_stride])) : v;
+            s += gate ? times_sigmoid(v, gate[t * gate_stride]) : v;
         }
         Elem<T>::store(delta + i, s);
     }
@@ -476,7 +476,7 @@ expert_combine_quads_kernel(const float* __restrict__ per_slot, int top, const v
         for (int k = 1; k < shared_parts; ++k) add4(v, quad_of(shared, i + k * shared_stride, MLS_F32));
         if (gate) {
             const float f = 1.0f + expf(-gate[t * gate_stride]);
-            v = make_float4(v.x / f, v.y / f, v.z / f, v.w / f);
+            v = make_float4(over(v.x, f), over(v.y, f), over(v.z, f), over(v.w, f));
         }
         add4(s, v);
     }

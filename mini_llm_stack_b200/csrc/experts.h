@@ -1,6 +1,6 @@
 // What the experts' two source files share.
 #pragma once
-#include <cuda_runtime.h>
+#include "common.cuh"
 
 namespace mls_experts {
 // What a product does: the experts' down projection, or an up projection with a unit on its sums.
@@ -13,9 +13,9 @@ __device__ __forceinline__ float gated_unit(float g, float u, float alpha, float
     if (limit > 0.f) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
-        return (g / (1.0f + expf(-alpha * g))) * (u + 1.0f);
+        return times_sigmoid(g, alpha * g) * (u + 1.0f);
     }
-    return (g / (1.0f + expf(-g))) * u;
+    return times_sigmoid(g, g) * u;
 }
 
 // bfloat16 rows of whole 16-byte pieces at 16-byte addresses: the tensor cores'.

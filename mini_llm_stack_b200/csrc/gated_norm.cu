@@ -36,7 +36,7 @@ struct GatedNormArgs {
     int n_out, d;
 };
 
-__device__ __forceinline__ float sigmoid1(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float sigmoid1(float z) { return times_sigmoid(1.0f, z); }
 
 template <int N>
 __device__ __forceinline__ Pack<N> weight_pack(const float* w, int step, int c) {

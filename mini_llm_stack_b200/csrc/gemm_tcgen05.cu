@@ -83,9 +83,21 @@ __device__ __forceinline__ float gated(float g, float u, float alpha, float limi
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
     }
-    return (g / (1.0f + expf(-alpha * g))) * (u + shift);
+    return times_sigmoid(g, alpha * g) * (u + shift);
 }
 #define GATED(p, g, u) gated(g, u, (p).glu_alpha, (p).glu_limit, (p).glu_shift)
+// Sixteen of them: whether there is a limit is asked once.
+__device__ __forceinline__ void gated16(const GemmParams& p, const uint32_t (&g)[16], const uint32_t (&u)[16],
+                                        float* r) {
+    if (p.glu_limit > 0.f) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) r[e] = GATED(p, __uint_as_float(g[e]), __uint_as_float(u[e]));
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+            r[e] = gated(__uint_as_float(g[e]), __uint_as_float(u[e]), p.glu_alpha, 0.f, p.glu_shift);
+    }
+}
 // An activation without a gate on a finished output (epilogue 2: relu(x)^2; else x).
 __device__ __forceinline__ float ungated(int epilogue, float x) {
     if (epilogue == 2) {
@@ -382,16 +394,18 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
 //   empty[s]      the instructions reading stage s are done: tcgen05.commit arrives on
 //                 both CTAs' barriers at once;
 //   acc_full[a]   accumulator a is complete: commit to both CTAs;
-//   acc_empty[a]  (first CTA) both CTAs' epilogue warps have read accumulator a: four local
-//                 arrivals and four from the second CTA.
+//   acc_empty[a]  (first CTA) both CTAs' epilogue warps have read accumulator a: eight local
+//                 arrivals and eight from the second CTA.
 // Every load lands in the loading CTA's own shared memory only (no multicast).
 //
-// The epilogue (bfloat16 output whose rows are whole 16-byte chunks): the four epilogue
-// warps round 64 output columns of their 128 rows into a swizzled staging tile in shared
-// memory, and one thread hands the tile to TMA, which writes whole 128-byte row pieces and
-// clips at the matrix's edge; two staging tiles alternate.  (Storing from registers, each
-// thread 32 bytes of its own row, cost 7-10 % of the K = 4,096 products.)  Other outputs
-// are stored from registers.
+// The epilogue (bfloat16 output whose rows are whole 16-byte chunks): two sets of four
+// epilogue warps take runs of 64 output columns in turn, round them for their 128 rows into
+// the set's swizzled staging tile in shared memory, and one thread hands the tile to TMA,
+// which writes whole 128-byte row pieces and clips at the matrix's edge.  (Storing from
+// registers, each thread 32 bytes of its own row, cost 7-10 % of the K = 4,096 products.)
+// Other outputs are stored from registers.  A product of one round pays for the last tile's
+// epilogue: with one set and the compiler's division (common.cuh's `over`) 707 x 2,048 x 2,048
+// with SwiGLU took 38 us, now 18; 600 x 16,384 x 2,048 64 -> 43, 2,048 x 5,632 x 4,096 79 -> 74.
 template <int STAGES>
 struct PairSmem {
     static constexpr int A_BYTES = BM * BK * 2;              // this CTA's 128 rows of A
@@ -404,9 +418,10 @@ struct PairSmem {
     static constexpr int TOTAL = TMEM_SLOT + 16 + 1024;
 };
 constexpr int PAIR_BN = 256;
+constexpr int PAIR_SETS = 2, PAIR_THREADS = 64 + 128 * PAIR_SETS;   // sets of four epilogue warps
 
 template <int STAGES>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS)
 gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap,
                          const __grid_constant__ CUtensorMap bmap,
                          const __grid_constant__ CUtensorMap omap,
@@ -441,7 +456,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(acc_full(a), 1);
-            mbar_init(acc_empty(a), 8);
+            mbar_init(acc_empty(a), 8 * PAIR_SETS);
         }
         fence_barrier_init();
     }
@@ -516,9 +531,12 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         // ---------------------------------------------------------------- epilogue
         const int q = warp & 3;
         const int row_in = q * 32 + lane;
-        const bool issuer = q == 0 && lane == 0;
+        const int set = (warp - 2) >> 2;                     // takes every second run of columns
+        const bool issuer = (warp - 2) % 4 == 0 && lane == 0;
+        const uint32_t stage = base + L::OUT + set * L::OUT_TILE;
+        auto set_sync = [&] { asm volatile("bar.sync %0, 128;\n" ::"r"(1 + set) : "memory"); };
         const int acc_cols = p.epilogue == 1 ? 128 : 64;     // accumulator columns behind 64 outputs
-        int it = 0, fills = 0;
+        int it = 0;
         for (int unit = cluster; unit < unit_count; unit += clusters, ++it) {
             const PairUnit w = pair_unit(p, unit, cut, kblocks);
             const int mi = w.tile % m_pairs, ni = w.tile / m_pairs;
@@ -537,10 +555,9 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                 const int part_row0 =
                     ((w.tile - p.tail_full) * p.tail_parts + w.part) * (2 * BM) + (int)rank * BM;
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 32, ++fills) {
-                    const uint32_t stage = base + L::OUT + (fills & 1) * L::OUT_TILE;
-                    if (issuer) tma_store_wait_read<1>();
-                    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                for (int c0 = 32 * set; c0 < BN; c0 += 32 * PAIR_SETS) {
+                    if (issuer) tma_store_wait_read<0>();
+                    set_sync();
                     uint32_t ra[16], rb[16];
                     tmem_ld16(tmem_d + c0, ra);
                     tmem_ld16(tmem_d + c0 + 16, rb);
@@ -556,7 +573,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                                        "r"(rb[4 * ch]), "r"(rb[4 * ch + 1]), "r"(rb[4 * ch + 2]),
                                        "r"(rb[4 * ch + 3]) : "memory");
                     }
-                    if (c0 + 32 >= BN) {
+                    if (c0 + 32 * PAIR_SETS >= BN) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) {
@@ -565,7 +582,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                         }
                     }
                     fence_proxy_async();
-                    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                    set_sync();
                     // the map sees the float32 scratch as rows of 512 two-byte elements
                     if (issuer) tma_store_2d(&pmap, c0 * 2, part_row0, stage);
                 }
@@ -573,11 +590,10 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             }
             if (staged_stores) {
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += acc_cols, ++fills) {
-                    const uint32_t stage = base + L::OUT + (fills & 1) * L::OUT_TILE;
+                for (int c0 = set * acc_cols; c0 < BN; c0 += PAIR_SETS * acc_cols) {
                     // the store that last read this staging tile has read it
-                    if (issuer) tma_store_wait_read<1>();
-                    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                    if (issuer) tma_store_wait_read<0>();
+                    set_sync();
 #pragma unroll
                     for (int part = 0; part < 2; ++part) {   // 32 outputs each
                         float r[32];
@@ -588,9 +604,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                                 tmem_ld16(tmem_d + c0 + part * 64 + b * 32, g);
                                 tmem_ld16(tmem_d + c0 + part * 64 + b * 32 + 16, u);
                                 tmem_ld_wait();
-#pragma unroll
-                                for (int e = 0; e < 16; ++e)
-                                    r[b * 16 + e] = GATED(p, __uint_as_float(g[e]), __uint_as_float(u[e]));
+                                gated16(p, g, u, r + b * 16);
                             }
                         } else {
                             uint32_t a[16], b[16];
@@ -617,7 +631,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                                            "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
                         }
                     }
-                    if (c0 + acc_cols >= BN) {
+                    if (c0 + PAIR_SETS * acc_cols >= BN) {
                         // the accumulator has been read: the MMA thread may fill it again
                         tc_fence_before();
                         __syncwarp();
@@ -627,7 +641,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                         }
                     }
                     fence_proxy_async();
-                    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                    set_sync();
                     if (issuer) {
                         // a box that lies wholly outside the matrix is not handed over at all
                         const int out_col = (ni * BN + c0) / (p.epilogue == 1 ? 2 : 1);
@@ -638,7 +652,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                 continue;
             }
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = 32 * set; c0 < BN; c0 += 32 * PAIR_SETS) {
                 uint32_t ra[16], rb[16];
                 tmem_ld16(tmem_d + c0, ra);
                 tmem_ld16(tmem_d + c0 + 16, rb);
@@ -891,7 +905,7 @@ int launch_pair(const GemmParams& p, const void* a, const void* b, cudaStream_t 
     }
     const long long most = sm_count() / 2;                   // one pair on two SMs
     const int grid = 2 * (int)(units < most ? units : most);
-    MLS_LAUNCH((gemm_tcgen05_pair_kernel<STAGES>), dim3(grid), dim3(THREADS), L::TOTAL, stream, q,
+    MLS_LAUNCH((gemm_tcgen05_pair_kernel<STAGES>), dim3(grid), dim3(PAIR_THREADS), L::TOTAL, stream, q,
                amap, bmap, omap, pmap, staged);
     int rc = launch_status();
     if (rc || q.tail_parts <= 1) return rc;

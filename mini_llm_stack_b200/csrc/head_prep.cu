@@ -531,7 +531,7 @@ head_difference_kernel(const T* __restrict__ o, int hd, float lambda, float mul,
 #pragma unroll
         for (int x = 0; x < V; ++x) {
             d.v[x] = d.v[x] * inv * mul;
-            if (gate) d.v[x] = d.v[x] / (1.0f + expf(-z.v[x]));
+            if (gate) d.v[x] = times_sigmoid(d.v[x], z.v[x]);
         }
         store_pack<V>(out, ((size_t)t * n_heads + h) * f + c, DT, d);
     }

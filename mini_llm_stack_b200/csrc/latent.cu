@@ -296,10 +296,10 @@ sigmoid_gate_kernel(T* __restrict__ o, const RowParts proj, int gate_col, int pe
             }
             T* at = o + (size_t)t * n + c;
             float4 v = load4(at);
-            v.x = v.x / (1.0f + expf(-z.x));
-            v.y = v.y / (1.0f + expf(-z.y));
-            v.z = v.z / (1.0f + expf(-z.z));
-            v.w = v.w / (1.0f + expf(-z.w));
+            v.x = times_sigmoid(v.x, z.x);
+            v.y = times_sigmoid(v.y, z.y);
+            v.z = times_sigmoid(v.z, z.z);
+            v.w = times_sigmoid(v.w, z.w);
             store4(at, v);
         }
         return;
@@ -309,7 +309,7 @@ sigmoid_gate_kernel(T* __restrict__ o, const RowParts proj, int gate_col, int pe
          idx += (size_t)gridDim.x * blockDim.x) {
         const int t = (int)(idx / n), c = (int)(idx - (size_t)t * n);
         const float z = proj.at(t, gate_col + c / per);
-        Elem<T>::store(o + idx, Elem<T>::load(o + idx) / (1.0f + expf(-z)));
+        Elem<T>::store(o + idx, times_sigmoid(Elem<T>::load(o + idx), z));
     }
 }
 

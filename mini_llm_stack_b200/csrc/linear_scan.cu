@@ -55,7 +55,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = pack_bf16x4(v);
 }
 
-__device__ __forceinline__ float silu1(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu1(float z) { return times_sigmoid(z, z); }
 __device__ __forceinline__ float4 silu4(float4 v) {
     return make_float4(silu1(v.x), silu1(v.y), silu1(v.z), silu1(v.w));
 }
@@ -247,7 +247,7 @@ scan_finish_kernel(const float* __restrict__ o, const void* __restrict__ gate, i
         const float z = load_as_float(gate, (size_t)t * gate_row + gate_off + c, gate_dtype);
         float v = row[j] * inv;
         if (w) v *= load_as_float(w, c, w_dtype);
-        Elem<T>::store(out + (size_t)t * n_heads * f + c, v * (z / (1.0f + expf(-z))));
+        Elem<T>::store(out + (size_t)t * n_heads * f + c, v * times_sigmoid(z, z));
     }
 }
 
@@ -313,7 +313,7 @@ scan_finish_row_kernel(const float* __restrict__ o, const T* __restrict__ gate, 
         const float z = Elem<T>::load(gate + (size_t)t * gate_row + gate_off + j);
         float v = row[j] * inv;
         if (w) v *= w[j];
-        Elem<T>::store(out + (size_t)t * out_row + j, v * (1.0f / (1.0f + expf(-z))) * out_scale);
+        Elem<T>::store(out + (size_t)t * out_row + j, v * times_sigmoid(1.0f, z) * out_scale);
     }
 }
 

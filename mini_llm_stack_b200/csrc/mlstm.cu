@@ -278,7 +278,7 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ num, const float* 
         const float o = nr[j] / d;
         const float z = Elem<T>::load(gate + (size_t)t * gate_row + g_off + head * f + j);
         Elem<T>::store(out + (size_t)unit * f + j,
-                       o * inv * load_as_float(w, head * f + j, w_dtype) / (1.0f + expf(-z)));
+                       times_sigmoid(o * inv * load_as_float(w, head * f + j, w_dtype), z));
     }
 }
 
@@ -325,10 +325,10 @@ mlstm_finish_quads_kernel(const float* __restrict__ num, const float* __restrict
         const float4 m = w_dtype == MLS_BF16 ? load_quad((const __nv_bfloat16*)w + (size_t)head * f + j)
                                              : load_quad((const float*)w + (size_t)head * f + j);
         store_quad(out + (size_t)unit * f + j,
-                   make_float4(o[x].x * inv * m.x / (1.0f + expf(-z[x].x)),
-                               o[x].y * inv * m.y / (1.0f + expf(-z[x].y)),
-                               o[x].z * inv * m.z / (1.0f + expf(-z[x].z)),
-                               o[x].w * inv * m.w / (1.0f + expf(-z[x].w))));
+                   make_float4(times_sigmoid(o[x].x * inv * m.x, z[x].x),
+                               times_sigmoid(o[x].y * inv * m.y, z[x].y),
+                               times_sigmoid(o[x].z * inv * m.z, z[x].z),
+                               times_sigmoid(o[x].w * inv * m.w, z[x].w)));
     }
 }
 

@@ -4,7 +4,7 @@
 #include "common.cuh"
 
 namespace {
-__device__ __forceinline__ float silu_mul(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
+__device__ __forceinline__ float silu_mul(float g, float u) { return times_sigmoid(g, g) * u; }
 
 // 16 bytes per thread and operand: I must be a multiple of 8 (bfloat16) or 4 (float32).
 __global__ void swiglu_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu,
@@ -66,7 +66,7 @@ __device__ __forceinline__ float clamped_glu(float g, float u, float alpha, floa
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
     }
-    return (g / (1.0f + expf(-alpha * g))) * (u + 1.0f);
+    return times_sigmoid(g, alpha * g) * (u + 1.0f);
 }
 template <typename T>
 __global__ void clamped_glu_kernel(const T* __restrict__ gu, T* __restrict__ out, int inter,

@@ -779,3 +779,21 @@ def test_bf16_attention_kernels_agree_with_each_other(rts, block, window):
     assert (got["mma"] - got["simt"]).abs().max().item() <= 1.2e-2 * scale
     # the two mma.sync kernels do the same arithmetic on the same tiles
     assert (got["mma"] - got["no_tma"]).abs().max().item() <= 1e-3 * scale
+
+
+def test_gated_sums_at_the_ends_of_their_range(rts):
+    """silu(g) * u for gates from one end of float32 to the other: the value to a few roundings (of the
+    exponential and the quotient), infinities, zeros and values that are no numbers as division has them."""
+    ops = rts[torch.float32].ops
+    g = torch.cat([torch.linspace(-110, 110, 8192), torch.randn(8192) * 3, 10.0 ** torch.linspace(-44, 38.5, 2048),
+                   -10.0 ** torch.linspace(-44, 2, 2040), torch.tensor([0.0, -0.0, float("inf"), -float("inf"),
+                                                                        float("nan"), 88.7, -88.72, -88.73])]).to(DEV)
+    out = torch.empty((1, g.numel()), dtype=torch.float32, device=DEV)
+    ops.swiglu(torch.cat([g, torch.ones_like(g)])[None].contiguous(), out)
+    want = g / (1 + torch.exp(-g))
+    assert torch.equal(out[0].isnan(), want.isnan()) and torch.equal(out[0].isinf(), want.isinf())
+    exact = g.double() / (1 + torch.exp(-g.double()))
+    # where the exponential is finite in float32: 2 ulp of it, a rounding of the sum and an ulp of the quotient
+    sure = g.isfinite() & (g > -88.0)
+    assert ((out[0].double() - exact).abs()[sure] <= 4 * 2.0 ** -23 * exact.abs()[sure] + 2.0 ** -149).all()
+    assert (out[0][g.isfinite() & (g <= -88.0)].abs() <= 1e-36).all()
