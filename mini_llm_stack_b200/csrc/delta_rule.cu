@@ -31,11 +31,15 @@
 // k and q), and multiplies them two at a time (fma.rn.f32x2).  The sum over the rows is the
 // lane's own in a fixed order and three shuffles: a token's bits do not depend on the batch.
 // The scan takes two tokens at a time from a portion's start, which moves the last bits where
-// a cut separates two tokens.  Everything is float32.
+// a cut separates two tokens.  Longer requests of bfloat16 models go chunk by chunk (delta_chunk.cu).
+// Everything is float32.
 #include "common.cuh"
+#include "delta_rule.h"
 #include "tma.cuh"
+#include <limits.h>
 
 namespace {
+using namespace mls_delta;
 constexpr float DR_UNIT_EPS = 1e-6f;     // inside the root of the unit vectors
 
 __device__ __forceinline__ float silu1(float z) { return times_sigmoid(z, z); }
@@ -115,30 +119,6 @@ struct DeltaArgs {
         return state + (size_t)slot * state_stride + ring_at;
     }
 };
-
-// What the scan reads, float32, so that the tokens of a pass are one run of memory each:
-//   [G][T][q: er | k: er]      [H][fr / 16][T][16 values]      [H][T][DR_SCALARS]
-// with the scalars of a value head and token: decay, step, k . q, k' . k, k' . q, 0, 0, 0, where k'
-// is the key of the token before (anything where a request's tokens of the step begin).
-constexpr int DR_SCALARS = 8, DR_COLS = 16;
-struct Prepared {
-    size_t v_at, s_at;                 // where the values and the scalars begin
-    size_t T;
-    int er, fr;
-    __host__ __device__ Prepared(int n_tokens, int H, int G, int er_, int fr_)
-        : v_at((size_t)n_tokens * G * 2 * er_), s_at(v_at + (size_t)n_tokens * H * fr_),
-          T((size_t)n_tokens), er(er_), fr(fr_) {}
-    __host__ __device__ size_t qk(int kv, int t) const { return ((size_t)kv * T + t) * 2 * er; }
-    __host__ __device__ size_t v(int head, int chunk, int t) const {
-        return v_at + (((size_t)head * (fr / DR_COLS) + chunk) * T + t) * DR_COLS;
-    }
-    __host__ __device__ size_t scalars(int head, int t) const {
-        return s_at + ((size_t)head * T + t) * DR_SCALARS;
-    }
-};
-__host__ __device__ inline int prepared_floats(int H, int G, int er, int fr) {      // a token's share
-    return 2 * G * er + H * (fr + DR_SCALARS);
-}
 
 // A head's channels spread over a warp (channel lane + 32 i) with the convolution's weights and
 // its last inputs; TT >= taps, the places before the real taps count as zero.
@@ -321,7 +301,7 @@ constexpr int DS_TOKENS = 16;          // tokens in one of the two buffers
 template <int R4, int C>
 __global__ void __launch_bounds__(128 / C)
 delta_scan_kernel(const DeltaArgs a, const float* __restrict__ rows, float* __restrict__ out,
-                  int* status) {
+                  int* status, int chunked_from) {
     using namespace mls_tma;
     constexpr int ER = 32 * R4, QK = 2 * ER;           // floats of a token's q and k
     constexpr int DS_THREADS = 128 / C;
@@ -337,7 +317,7 @@ delta_scan_kernel(const DeltaArgs a, const float* __restrict__ rows, float* __re
     const int my = warp * 4 * C + (lane >> 3);         // my columns: this one and every fourth behind it
     const Prepared from(a.n_tokens, a.H, a.G, ER, a.fr);
     const int t0 = a.cu_q[r], n = a.cu_q[r + 1] - t0;
-    if (n <= 0) return;
+    if (n <= 0 || n >= chunked_from) return;           // (longer requests: delta_chunk.cu's)
     const int slot = a.state_slot[r];
     if (threadIdx.x == 0) {
         mbar_init((uint32_t)__cvta_generic_to_shared(&full_bars[0]), 1);
@@ -704,7 +684,7 @@ int launch_prep(const DeltaArgs& a, float* out, cudaStream_t stream) {
     return launch_status();
 }
 template <int R4, int C>
-int launch_scan(const DeltaArgs& a, const float* rows, float* out, int* status,
+int launch_scan(const DeltaArgs& a, const float* rows, float* out, int* status, int chunked_from,
                 cudaStream_t stream) {
     constexpr size_t qk = 2 * 32 * R4;
     const size_t smem = (2 * DS_TOKENS * (qk + DS_COLS + DR_SCALARS) + 4 * qk) * sizeof(float);
@@ -714,7 +694,7 @@ int launch_scan(const DeltaArgs& a, const float* rows, float* out, int* status,
         if (rc) return rc;
     }
     MLS_LAUNCH((delta_scan_kernel<R4, C>), dim3(a.fr / DS_COLS, a.H, a.n_requests), dim3(128 / C),
-               smem, stream, a, rows, out, status);
+               smem, stream, a, rows, out, status, chunked_from);
     return launch_status();
 }
 template <int R4, int C>
@@ -778,9 +758,10 @@ MLS_API int mls_delta_prep(const float* proj, int width, int qkv_col, int a_col,
 MLS_API int mls_delta_scan(const float* rows, const float* proj, int width, int qkv_col, int taps,
                            const int* state_slot, const int* cu_q, const int* positions,
                            float* state, long long state_stride, int n_tokens, int n_requests,
-                           int H, int G, int e, int f, float* out, int* status,
+                           int H, int G, int e, int f, float* out, int* status, int chunked_from,
                            cudaStream_t stream) {
     if (n_tokens <= 0 || n_requests <= 0) return 0;
+    if (chunked_from <= 0) chunked_from = INT_MAX;
     const DeltaArgs a = make_args(proj, 1, 0, width, qkv_col, 0, 0, 0, nullptr, 0, taps, nullptr, nullptr,
                                   state_slot, cu_q, nullptr, positions, state, state_stride,
                                   n_tokens, n_requests, H, G, e, f);
@@ -788,7 +769,7 @@ MLS_API int mls_delta_scan(const float* rows, const float* proj, int width, int 
     // one column a lane while every CTA has an SM to itself (more warps to hide the chain of
     // products and sums), two beyond that (half the reads of k and q); the bits are the same
     const bool one = (long long)(a.fr / DS_COLS) * H * n_requests <= sm_count();
-#define DS_GO(R, C) return launch_scan<R, C>(a, rows, out, status, stream)
+#define DS_GO(R, C) return launch_scan<R, C>(a, rows, out, status, chunked_from, stream)
     switch (a.er / 32) {
         case 1: if (one) DS_GO(1, 1); DS_GO(1, 2);
         case 2: if (one) DS_GO(2, 1); DS_GO(2, 2);
@@ -800,6 +781,33 @@ MLS_API int mls_delta_scan(const float* rows, const float* proj, int width, int 
         default: DS_GO(8, 1);
     }
 #undef DS_GO
+}
+
+// Whether requests can go chunk by chunk (delta_chunk.cu): the scratch of a chunk in floats, or 0.
+MLS_API long long mls_delta_chunk_floats(int H, int G, int e, int f) {
+    const int er = (e + 31) / 32 * 32;
+    return chunk_fits(er, (f + 15) / 16 * 16) ? chunk_floats(H, G, er) : 0;
+}
+// The scan of requests of at least `least` tokens chunk by chunk: of those `count` from the `from`th on, their
+// chunks [first, first + span), `chunks` in all; `scratch`: so many chunks' floats at a 16-byte address.
+MLS_API int mls_delta_scan_chunked(const float* rows, const float* proj, int width, int qkv_col, int taps,
+                                   const int* state_slot, const int* cu_q, const int* positions, float* state,
+                                   long long state_stride, int n_tokens, int n_requests, int H, int G, int e, int f,
+                                   float* out, int* status, int least, int from, int count, int first, int span,
+                                   int chunks, float* scratch, cudaStream_t stream) {
+    if (n_tokens <= 0 || n_requests <= 0) return 0;
+    const DeltaArgs a = make_args(proj, 1, 0, width, qkv_col, 0, 0, 0, nullptr, 0, taps, nullptr, nullptr,
+                                  state_slot, cu_q, nullptr, positions, state, state_stride, n_tokens, n_requests,
+                                  H, G, e, f);
+    if (!sizes_ok(a)) return MLS_ERR_UNSUPPORTED;
+    ChunkArgs c{};
+    c.rows = rows, c.out = out, c.state = state, c.state_stride = state_stride, c.cu_q = cu_q;
+    c.state_slot = state_slot, c.n_tokens = n_tokens, c.n_requests = n_requests;
+    c.H = H, c.G = G, c.e = e, c.f = f, c.er = a.er, c.fr = a.fr;
+    c.least = least, c.from = from, c.count = count, c.first = first, c.span = span, c.chunks = chunks;
+    c.status = status, c.proj = proj, c.positions = positions, c.width = width, c.qkv_col = qkv_col;
+    c.taps = taps, c.channels = a.channels, c.ring_at = a.ring_at;
+    return chunk_scan(c, scratch, stream);
 }
 
 // A step of one token a request, to the gated and normed heads: out [T, H f] in `dtype`.

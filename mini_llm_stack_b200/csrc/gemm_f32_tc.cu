@@ -89,15 +89,6 @@ __device__ __forceinline__ uint64_t rows_desc(uint32_t addr) {
     return d;
 }
 
-template <int N>
-__device__ __forceinline__ void more_registers() {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
-}
-template <int N>
-__device__ __forceinline__ void fewer_registers() {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(N));
-}
-
 // Unit i: a tile (tiles of rows fastest, so that a tile of weights leaves memory once), and of K the
 // blocks [from, to).
 struct Unit {

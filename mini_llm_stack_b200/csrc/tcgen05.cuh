@@ -149,4 +149,14 @@ __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
 }
 
+// A warpgroup's registers a thread: all its warps call; the shares add up to what the block was launched with.
+template <int N>
+__device__ __forceinline__ void more_registers() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void fewer_registers() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(N));
+}
+
 }  // namespace mls_tc

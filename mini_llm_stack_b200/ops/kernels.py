@@ -938,7 +938,12 @@ class Ops:
                                   _I, _I, _I, _I, _I, _P, _P]),
                    "scan": _decl(lib, "mls_delta_scan",
                                  [_P, _P, _I, _I, _I, _P, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _I, _P,
-                                  _P, _P]),
+                                  _P, _I, _P]),
+                   "chunk": _decl(lib, "mls_delta_chunk_floats", [_I, _I, _I, _I],
+                                  restype=ctypes.c_longlong),
+                   "chunked": _decl(lib, "mls_delta_scan_chunked",
+                                    [_P, _P, _I, _I, _I, _P, _P, _P, _P, _LL, _I, _I, _I, _I, _I, _I,
+                                     _P, _P, _I, _I, _I, _I, _I, _I, _P, _P]),
                    "step": _decl(lib, "mls_delta_step",
                                  [_P, _I, _LL, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P, _P, _F, _P, _P,
                                   _P, _P, _LL, _I, _I, _I, _I, _I, _P, _I, _P])}
@@ -1096,6 +1101,12 @@ class Ops:
     # against 87 and 96 at 128, 0.81 (numerators), 0.84 (denominators) and 0.68.  A request's own length decides and nothing else of the
     # step, so that its bits do not depend on the requests beside it.
     CHUNKED_FROM = {"head": 48, "token": 192, "mlstm": 128}
+    # The delta rule's: its chunk-wise scan costs 39 us and 4.1 a chunk, however few blocks of a head and 128 columns
+    # there are, the other one a time per token that falls with them.  32 heads of 128 x 128, one request of 256 tokens 56
+    # us against 67 (192: 50 / 52, but errors of outputs 0.98 at 192 and 1.03 at 128 of its); 16 heads 55 / 44, at
+    # 512 79 / 83.
+    DELTA_CHUNKED_FROM = {"few": 512, "many": 256}
+    DELTA_MANY = 32               # blocks of a head and 128 columns
     CHUNK_SCRATCH = 1 << 27       # floats of scratch that the chunks under way may take (at least one does)
 
     @staticmethod
@@ -1116,6 +1127,25 @@ class Ops:
         if n:
             parts.append((at, n, 0, longest, total))
         return parts
+
+    def _chunk_scratch(self, chunk: int, each: list):
+        """Scratch for requests of ``each`` so many chunks of ``chunk`` floats, and the parts in which
+        they are done where it does not hold them all: (parts, scratch)."""
+        most = min(65535, max(1, self.CHUNK_SCRATCH // chunk))
+        while True:
+            parts = self._chunk_parts(each, most)
+            # (a power of two of chunks: scratch that grows drops the captured graphs)
+            need = min(most, 1 << (max(p[4] for p in parts) - 1).bit_length())
+            try:
+                return parts, self.scratch("chunk_scan", chunk * need)
+            except torch.cuda.OutOfMemoryError:
+                # fewer chunks at a time, from now on: what there is already, or half as many
+                held = self._scratch.get("chunk_scan")
+                fits = held.numel() // chunk if held is not None else 0
+                if most == 1:
+                    raise
+                most = fits if 0 < fits < most else most // 2
+                self.CHUNK_SCRATCH = most * chunk
 
     def _chunk_plan(self, part: str, mode: int, step, operands: list, whole: tuple, strides: tuple,
                     n_heads: int, e: int, f: int):
@@ -1140,23 +1170,7 @@ class Ops:
                 or any(s & 3 for s in strides) or n_heads > 65535:
             return None
         each = [-(-n // self.CHUNK) for n in lens if n >= least]
-        chunk = self._part_lib(part)["scratch"](mode, n_heads, e, f, 1)
-        most = min(65535, max(1, self.CHUNK_SCRATCH // chunk))
-        while True:
-            parts = self._chunk_parts(each, most)
-            # (a power of two of chunks: scratch that grows drops the captured graphs)
-            need = min(most, 1 << (max(p[4] for p in parts) - 1).bit_length())
-            try:
-                scratch = self.scratch("chunk_scan", chunk * need)
-                break
-            except torch.cuda.OutOfMemoryError:
-                # fewer chunks at a time, from now on: what there is already, or half as many
-                held = self._scratch.get("chunk_scan")
-                fits = held.numel() // chunk if held is not None else 0
-                if most == 1:
-                    raise
-                most = fits if 0 < fits < most else most // 2
-                self.CHUNK_SCRATCH = most * chunk
+        parts, scratch = self._chunk_scratch(self._part_lib(part)["scratch"](mode, n_heads, e, f, 1), each)
         return least, parts, scratch, len(each) < len(lens)
 
     def mlstm_state_width(self, e: int, f: int) -> int:
@@ -1885,11 +1899,28 @@ class Ops:
               "delta_scan: bad state")
         _need(out.shape == (t, n_heads * f) and out.dtype == torch.float32 and out.is_contiguous(),
               "delta_scan: bad out")
+        lens = getattr(step, "q_lens", None)
+        chunked_from = 0
+        chunk = int(self._part_lib("delta")["chunk"](n_heads, n_kv, e, f))
+        # as the other scans: prompts of bfloat16 models, a request's own length decides
+        least = self.DELTA_CHUNKED_FROM["many" if n_heads * -(-f // 128) >= self.DELTA_MANY else "few"]
+        if chunk and self.act_dtype == torch.bfloat16 and lens and max(lens) >= least:
+            chunked_from = least
+            parts, scratch = self._chunk_scratch(chunk, [-(-n // self.CHUNK) for n in lens if n >= chunked_from])
+            self.launches += 2 * len(parts)
+            for p in parts:
+                _check(self._part_lib("delta")["chunked"](
+                    _ptr(rows), _ptr(proj), proj.shape[1], col, taps, _ptr(step.state_slot),
+                    _ptr(step.cu_q), _ptr(step.positions), _ptr(state), state.stride(0), t,
+                    step.n_requests, n_heads, n_kv, e, f, _ptr(out), _ptr(self.status), chunked_from, *p,
+                    _ptr(scratch), self._stream()), "delta_scan_chunked")
+            if min(lens) >= chunked_from:
+                return
         self.launches += 1
         _check(self._part_lib("delta")["scan"](
             _ptr(rows), _ptr(proj), proj.shape[1], col, taps, _ptr(step.state_slot), _ptr(step.cu_q),
             _ptr(step.positions), _ptr(state), state.stride(0), t, step.n_requests, n_heads, n_kv, e,
-            f, _ptr(out), _ptr(self.status), self._stream()), "delta_scan")
+            f, _ptr(out), _ptr(self.status), chunked_from, self._stream()), "delta_scan")
 
     def delta_step(self, proj, cols: tuple, conv, taps: int, a_exp, dt_bias, norm_w, eps: float,
                    state, step, n_heads: int, n_kv: int, e: int, f: int, out) -> None:

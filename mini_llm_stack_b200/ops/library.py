@@ -52,7 +52,7 @@ MODULES = {
     "headprep": ["head_prep.cu"],
     "side": ["side_input.cu"],
     "gatednorm": ["gated_norm.cu"],
-    "delta": ["delta_rule.cu"],
+    "delta": ["delta_rule.cu", "delta_chunk.cu"],
 }
 
 

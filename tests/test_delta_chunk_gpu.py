@@ -1,0 +1,98 @@
+"""The gated delta rule chunk by chunk: against float64 token by token at the edges of chunks, heads and
+columns, cut into portions and parts, beside other requests, and with values that are no numbers."""
+
+import numpy as np
+import pytest
+import torch
+
+from mini_llm_stack_b200.ops.kernels import Runtime
+from test_nekedra_gpu import DeltaCase, fake_step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def ops(monkeypatch):
+    o = Runtime("cuda:0", torch.bfloat16).ops
+    for part in ("delta", "scan"):
+        o.require_part(part)
+    monkeypatch.setattr(o, "DELTA_CHUNKED_FROM", {"few": 2, "many": 2}, raising=False)
+    return o
+
+
+def walk(ops, case, portions, slots, state, chunked=True):
+    """Scan outputs of ``portions`` [(sequence, from, to)], device tensors."""
+    nh, nk, e, f = case.sizes
+    step = fake_step([b - a for _, a, b in portions], [a for _, a, _ in portions], slots)
+    if not chunked:
+        step.q_lens = []
+    p = case.rows_of(portions)
+    rows = torch.full((step.n_tokens, ops.delta_rows(*case.sizes)), float("nan"), device="cuda")
+    ops.delta_prep(p, case.cols, case.dev["conv"], case.taps, case.dev["a_exp"], case.dev["dt"], state, step, nh, nk, e,
+                   f, rows)
+    out = torch.full((step.n_tokens, nh * f), float("nan"), device="cuda")
+    before = ops.launches
+    ops.delta_scan(rows, p, case.cols[0], case.taps, state, step, nh, nk, e, f, out)
+    ops.check_status()
+    return out, ops.launches - before
+
+
+@pytest.mark.parametrize("sizes", [(4, 2, 64, 64, 4), (2, 2, 96, 100, 3), (6, 2, 100, 72, 1), (3, 1, 128, 200, 4),
+                                   (12, 2, 80, 128, 2)])
+@pytest.mark.parametrize("lens", [(2, 130), (64, 63, 65), (300,)])
+def test_against_float64(ops, sizes, lens):
+    nh, nk, e, f, taps = sizes
+    case = DeltaCase(nh, nk, e, f, taps, lens, seed=sum(lens) + e)
+    portions, slots = [(i, 0, n) for i, n in enumerate(lens)], list(range(len(lens)))[::-1]
+    state, tokens_state = case.new_state(ops, len(lens)), case.new_state(ops, len(lens))
+    out, launches = walk(ops, case, portions, slots, state)
+    tokens, one = walk(ops, case, portions, slots, tokens_state, chunked=False)
+    assert (launches, one) == (2, 1)
+    want = np.concatenate([w[0] for w in case.want])
+    mine, theirs = (np.linalg.norm(x.cpu().double().numpy() - want) / np.linalg.norm(want) for x in (out, tokens))
+    # a chunk rounds P, T, R and U to float32 once each, and adds up runs of 32 or 64 in units of 2^-23 each way
+    assert mine <= max(1.3 * theirs, 4 * 2.0 ** -24), (mine, theirs)
+    matrices = nh * (-(-f // 16) * 16) * (-(-e // 32) * 32)
+    a, b = state[:, :matrices].double(), tokens_state[:, :matrices].double()
+    assert (a - b).norm() <= 1e-6 * b.norm()
+    # the convolution's inputs that the next tokens read: the last taps - 1 positions of each request
+    c = 2 * nk * e + nh * f
+    for i, n in enumerate(lens):
+        for pos in range(max(0, n - taps + 1), n):
+            at = matrices + (pos % taps) * c
+            assert torch.equal(state[slots[i], at:at + c], tokens_state[slots[i], at:at + c])
+
+
+def test_portions_parts_and_neighbours(ops, monkeypatch):
+    """A prompt in two portions (on chunks' edges: the same bits), a little scratch, and other requests beside it."""
+    case = DeltaCase(2, 1, 128, 128, 4, (300, 70, 3), seed=3)
+    state = case.new_state(ops, 3)
+    whole, _ = walk(ops, case, [(0, 0, 300)], [0], state)
+    kept = state[0].clone()
+    state.zero_()
+    first, _ = walk(ops, case, [(0, 0, 192)], [0], state)
+    rest, _ = walk(ops, case, [(0, 192, 300)], [0], state)
+    assert torch.equal(torch.cat([first, rest]), whole)
+    state.zero_()
+    # three requests, the short one token by token, and room for one chunk at a time
+    monkeypatch.setattr(ops, "DELTA_CHUNKED_FROM", {"few": 64, "many": 64}, raising=False)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH", 1, raising=False)
+    mixed, launches = walk(ops, case, [(1, 0, 70), (0, 0, 300), (2, 0, 3)], [2, 0, 1], state)
+    assert launches == 2 * (2 + 5) + 1
+    assert torch.equal(mixed[70:370], whole)
+    matrices = 2 * 128 * 128
+    assert torch.equal(state[0, :matrices], kept[:matrices]) and torch.isfinite(mixed).all()
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "step"])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan")])
+def test_no_number_reaches_earlier_tokens_or_columns(ops, what, odd):
+    case = DeltaCase(2, 1, 64, 80, 1, (200,), seed=5)          # one tap: the token's own inputs alone
+    bad, c0 = 100, case.cols[0]
+    clean, _ = walk(ops, case, [(0, 0, 200)], [0], case.new_state(ops, 1))
+    at = {"q": c0 + 3, "k": c0 + 64 + 3, "v": c0 + 2 * 64 + 80 + 7, "decay": case.cols[1], "step": case.cols[2]}[what]
+    case.proj[0][bad, at] = odd
+    got, _ = walk(ops, case, [(0, 0, 200)], [0], case.new_state(ops, 1))
+    tokens, _ = walk(ops, case, [(0, 0, 200)], [0], case.new_state(ops, 1), chunked=False)
+    assert torch.equal(got[:bad], clean[:bad])
+    assert torch.equal(got.isfinite(), tokens.isfinite())
