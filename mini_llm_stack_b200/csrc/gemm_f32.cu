@@ -481,8 +481,8 @@ int product(const T* A, int a_dtype, const float* W, float* out, int M, int N, i
             cudaStream_t stream) {
     const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
     const bool vec_w = K % 4 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
+    if (takes_tc(a_dtype, W, N, K)) return product_tc(A, a_dtype, W, out, M, N, K, scratch, status, stream);
     if (N <= SKINNY_N) return skinny(A, W, out, M, N, K, vec_a, vec_w, stream);
-    if (takes_tc(W, N, K)) return product_tc(A, a_dtype, W, out, M, N, K, scratch, status, stream);
     if constexpr (sizeof(T) == 4)
         if (vec_w && vec_a && M <= FEW_M) return few(A, W, out, M, N, K, stream);
     if (vec_w && vec_a) return tiled<T, true>(A, W, out, M, N, K, stream);
@@ -502,5 +502,5 @@ MLS_API int mls_gemm_f32(const void* A, int a_dtype, const float* W, float* out,
 }
 
 MLS_API long long mls_gemm_f32_scratch_floats(const void* A, int a_dtype, const float* W, int M, int N, int K) {
-    return M > 0 && takes_tc(W, N, K) ? tc_scratch_floats(A, a_dtype, M, N, K) : 0;
+    return M > 0 && takes_tc(a_dtype, W, N, K) ? tc_scratch_floats(A, a_dtype, M, N, K) : 0;
 }

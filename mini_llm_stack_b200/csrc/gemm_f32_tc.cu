@@ -1,4 +1,4 @@
-// Float32 products of more than 256 columns on the 5th-generation tensor cores:
+// Float32 products of long rows on the 5th-generation tensor cores (gemm_f32.h says which):
 // out[M, N] = A[M, K] * W[N, K]^T, both operands float32 (A may be bfloat16).
 //
 // Every operand is the sum of three bfloat16 (8 + 8 + 8 bits of the 24 that a float32 has; the
@@ -9,7 +9,7 @@
 //
 // each exact, in float32 accumulators.  The tensor cores cut off what an addition cannot hold, so an
 // accumulator takes 64 of K only, the small products first; the sums of 64 are added up in float32
-// registers, rounded to nearest, over a group of K (an eighth of it, 256 at least), and the groups'
+// registers, rounded to nearest, over a group of K (a sixteenth of it, 128 at least), and the groups'
 // sums in their turn.  That order depends on K alone: a row's bits are the same whatever rows it is
 // computed with, and whether a CTA walks all of K or one group (few rows), whose sum it then leaves to
 // gemm_f32_parts_kernel.  Distance from float64 (2-norm over 2-norm, normal values) against one chain of fmaf
@@ -28,8 +28,8 @@
 // single lane takes each cost some 50 cycles to prepare, which bounded every size (851 us for 651, 431 for 235).
 //
 // Measured against FFMA (us): 2,048 x 16,384 x 2,048 2,460 -> 651 (211 TFLOP/s), 515 x 16,384 x 2,048 721 -> 211,
-// 515 x 2,048 x 8,192 510 -> 141, 16 x 2,048 x 8,192 320 -> 33, 3 x 128,256 x 2,048 393 -> 236 (1.05 GB: 4.5 TB/s),
-// 1 x 2,048 x 2,048 20.5 -> 18.4.
+// 515 x 2,048 x 8,192 510 -> 127, 16 x 2,048 x 8,192 250 -> 25, 3 x 128,256 x 2,048 393 -> 236 (1.05 GB: 4.5 TB/s),
+// 1 x 2,048 x 2,048 22.5 -> 10.5; eight groups of K instead of sixteen leave 16 x 64 x 4,096 at 11.3 instead of 7.9.
 //
 // Warp roles: 0 = TMA producer, 1 = tensor memory and instructions, 4..7 = splitting the weights (a
 // quarter of the lanes each), 8..15 = sums (two warps a quarter, 16 columns in turn).  Every
@@ -54,7 +54,7 @@ constexpr int ROW_BYTES = BK * 2;                     // a row of a part's block
 constexpr int THREADS = 512;
 constexpr int SUM_WARPS = 8, SPLIT_WARPS = 4;
 constexpr int W_COLS = 3 * BK / 2, W_BUFS = 4;        // tensor memory of a block's parts; such blocks
-constexpr int GROUPS = 8, GROUP_MIN = 256;
+constexpr int GROUPS = 16, GROUP_MIN = 128;
 constexpr int MAX_STAGES = 12, RING_BYTES = 200 * 1024;
 
 struct TcParams {
@@ -459,8 +459,8 @@ struct Cut {
 Cut cut_of(int M, int N, int K) {
     Cut best{};
     const int blocks = (K + BK - 1) / BK;
-    const int least = GROUP_MIN / BK, eighth = ((blocks + GROUPS - 1) / GROUPS + 1) & ~1;
-    const int group = eighth > least ? eighth : least, groups = (blocks + group - 1) / group;
+    const int least = GROUP_MIN / BK, share = ((blocks + GROUPS - 1) / GROUPS + 1) & ~1;
+    const int group = share > least ? share : least, groups = (blocks + group - 1) / group;
     const long long n_tiles = (N + UMMA_M - 1) / UMMA_M, sms = sm_count();
     double least_cycles = 0;
     for (int most = 16; most <= NT_MANY; most += 16) {
@@ -507,8 +507,11 @@ int launch_nt(const TcParams& p, const CUtensorMap& rows_map, const CUtensorMap&
 }  // namespace
 
 namespace mls_f32 {
-bool takes_tc(const float* W, int N, int K) {
-    if (N <= SKINNY_N || K % 4 || reinterpret_cast<uintptr_t>(W) % 16 || (K >= CHAIN_K0 && K < CHAIN_K1)) return false;
+bool takes_tc(int a_dtype, const float* W, int N, int K) {
+    if (K % 4 || reinterpret_cast<uintptr_t>(W) % 16) return false;
+    if (N <= SKINNY_N) 
+        return N >= FEWEST_N && K >= (a_dtype == MLS_BF16 ? TC_K : 2 * TC_K) && (long long)N * K >= FEWEST_SIZE;
+    if (K >= CHAIN_K0 && K < CHAIN_K1) return false;
     return K >= TC_K || (K >= TC_K / 4 && (long long)N * K >= TC_SIZE);
 }
 
