@@ -27,7 +27,8 @@
 // through shared memory, eight rows a warp, with each row's operations in the same order: the same
 // bits.  It takes the requests of at least TILE_LEN tokens; a warp a row read every key once a
 // row, a key's row a lane, which touches 32 lines a load: 470 us for 515 tokens in three requests
-// of 32 / 8 heads of 64 in float32, 90 us now.
+// of 32 / 8 heads of 64 in float32, 71 us now (90 with the keys loaded between two barriers, 81 with a branch a row around
+// its shuffles).  Bound by the chain of a block's steps: 32 keys' scores, maxima, exponentials and sums behind every barrier.
 #include "common.cuh"
 
 namespace {
@@ -158,10 +159,13 @@ attention_simt_kernel(const T* __restrict__ qkv, T* __restrict__ out,
 
 constexpr int TILE_WARPS = 4, TILE_R = 8, TILE_ROWS = TILE_WARPS * TILE_R, KEYS = 32;
 
-template <int HD>
+// ASYNC (float32): the next 32 keys come by asynchronous copies while these are worked on, into buffers of their
+// own (a block waited for them, and for the page numbers before them, twice in every 32 keys).
+template <int HD, bool ASYNC>
 struct TileSmem {
     static constexpr int KP = HD + 4;                // a lane a key: 16-byte reads that meet no bank twice
-    static constexpr int K = 0, V = K + KEYS * KP, Q = V + KEYS * HD, P = Q + TILE_ROWS * HD;
+    static constexpr int BUF = KEYS * (KP + HD);     // keys, then values
+    static constexpr int Q = (ASYNC ? 2 : 1) * BUF, P = Q + TILE_ROWS * HD;
     static constexpr int FLOATS = P + TILE_ROWS * KEYS;
 };
 
@@ -187,11 +191,12 @@ attention_simt_tile_kernel(const T* __restrict__ qkv, T* __restrict__ out,
                            const int* __restrict__ cu_q, int heads_a_block, int head_blocks) {
     chain_release();
     chain_wait();
-    using L = TileSmem<HD>;
+    constexpr bool ASYNC = sizeof(T) == 4;
+    using L = TileSmem<HD, ASYNC>;
     constexpr int ND = HD / 32;
     extern __shared__ __align__(16) float sm[];
-    float* K_s = sm + L::K;
-    float* V_s = sm + L::V;
+    float* K_s = sm;
+    float* V_s = sm + KEYS * L::KP;
     float* Q_s = sm + L::Q;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quads = hd / 4;
     float* P_s = sm + L::P + warp * TILE_R * KEYS;
@@ -237,26 +242,59 @@ attention_simt_tile_kernel(const T* __restrict__ qkv, T* __restrict__ out,
         const int lo_first = max(0, first_visible(positions[s0], window, chunk));
         const int keep_most = min(keep_first, max(0, first_visible(p_last, window, chunk)));
         const int* table = block_table + (size_t)r * max_blocks;
-        for (int j0 = keep_most > 0 ? 0 : (lo_first / KEYS) * KEYS; j0 <= p_last; j0 += KEYS) {
-            if (j0 >= keep_most && j0 + KEYS <= lo_first) {          // past the kept keys: on to the window
-                j0 = (lo_first / KEYS) * KEYS - KEYS;
-                continue;
-            }
-            __syncthreads();
-#pragma unroll 2
+        // the 32 keys from j on, or where they lie between the kept keys and the window the window's first ones
+        auto tile_at = [&](int j) { return j >= keep_most && j + KEYS <= lo_first ? (lo_first / KEYS) * KEYS : j; };
+        // where this thread's quad u of the keys from j0 on lies in the pools; false: nowhere
+        auto place = [&](int j0, int u, size_t& at) {
+            const int x = u / quads, i = 4 * (u - x * quads), j = j0 + x;
+            const int page = j <= p_last && (j >= lo_first || j < keep_most) ? table[j / block_size] : -1;
+            at = (((size_t)kvh * n_pages + max(page, 0)) * block_size + j % block_size) * hd + i;
+            return page >= 0;
+        };
+        auto ask = [&](int j0, int buf) {
+#pragma unroll 4
             for (int u = threadIdx.x; u < KEYS * quads; u += TILE_WARPS * 32) {
-                const int x = u / quads, i = 4 * (u - x * quads), j = j0 + x;
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-                const int page = j <= p_last && (j >= lo_first || j < keep_most) ? table[j / block_size] : -1;
-                if (page >= 0) {
-                    const size_t at = (((size_t)kvh * n_pages + page) * block_size + j % block_size) * hd + i;
-                    kv = quad(k_pool + at);
-                    vv = quad(v_pool + at);
-                }
-                *reinterpret_cast<float4*>(K_s + x * L::KP + i) = kv;
-                *reinterpret_cast<float4*>(V_s + x * HD + i) = vv;
+                const int x = u / quads, i = 4 * (u - x * quads);
+                size_t at;
+                const bool there = place(j0, u, at);
+                const uint32_t k = (uint32_t)__cvta_generic_to_shared(sm + buf * L::BUF + x * L::KP + i);
+                const uint32_t v = (uint32_t)__cvta_generic_to_shared(sm + buf * L::BUF + KEYS * L::KP + x * HD + i);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                             ::"r"(k), "l"(k_pool + (there ? at : 0)), "r"(there ? 16 : 0) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                             ::"r"(v), "l"(v_pool + (there ? at : 0)), "r"(there ? 16 : 0) : "memory");
             }
-            __syncthreads();
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        int j0 = tile_at(keep_most > 0 ? 0 : (lo_first / KEYS) * KEYS), buf = 0;
+        if (ASYNC) {
+            __syncthreads();                                         // (another request's keys may still be read)
+            if (j0 <= p_last) ask(j0, 0);
+        }
+        for (int j_next; j0 <= p_last; j0 = j_next, buf ^= 1) {
+            j_next = tile_at(j0 + KEYS);
+            if (ASYNC) {
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+                __syncthreads();                                     // these are there, those before are read
+                if (j_next <= p_last) ask(j_next, buf ^ 1);
+                K_s = sm + buf * L::BUF;
+                V_s = K_s + KEYS * L::KP;
+            } else {
+                __syncthreads();
+#pragma unroll 2
+                for (int u = threadIdx.x; u < KEYS * quads; u += TILE_WARPS * 32) {
+                    const int x = u / quads, i = 4 * (u - x * quads);
+                    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+                    size_t at;
+                    if (place(j0, u, at)) {
+                        kv = quad(k_pool + at);
+                        vv = quad(v_pool + at);
+                    }
+                    *reinterpret_cast<float4*>(K_s + x * L::KP + i) = kv;
+                    *reinterpret_cast<float4*>(V_s + x * HD + i) = vv;
+                }
+                __syncthreads();
+            }
             // rows that see some of these keys, and whether all of the warp's rows see all of them
             bool on[TILE_R], any = false, every = true;
 #pragma unroll
@@ -283,28 +321,40 @@ attention_simt_tile_kernel(const T* __restrict__ qkv, T* __restrict__ out,
                     s[y] = fmaf(q4.w, k4.w, s[y]);
                 }
             }
+            // (row beside row, without a branch between them: their shuffles and exponentials overlap)
             const int j = j0 + lane;
+            float top[TILE_R], sum[TILE_R];
+            bool valid[TILE_R];
 #pragma unroll
             for (int y = 0; y < TILE_R; ++y) {
-                const bool valid = on[y] && (j >= lo[y] || j < keep[y]) && j <= p[y];
-                float v = -INFINITY;
-                if (valid) {
-                    v = s[y] * scale;
-                    if (slopes) v -= slope[y] * (float)(p[y] - j);
-                    if (softcap > 0.f) v = softcap * tanhf(v / softcap);
-                }
-                const float top = warp_max(v);
-                if (on[y]) {
-                    const float m_new = fmaxf(m[y], top);
-                    const float pj = valid ? expf(v - m_new) : 0.f;
-                    const float corr = expf(m[y] - m_new);           // (0 on the first chunk)
-                    l[y] = l[y] * corr + warp_sum(pj);
-#pragma unroll
-                    for (int i = 0; i < ND; ++i) acc[y][i] *= corr;
-                    m[y] = m_new;
-                    P_s[y * KEYS + lane] = pj;
-                }
+                valid[y] = on[y] && (j >= lo[y] || j < keep[y]) && j <= p[y];
+                float v = s[y] * scale;
+                if (slopes) v -= slope[y] * (float)(p[y] - j);
+                if (softcap > 0.f) v = softcap * tanhf(v / softcap);
+                top[y] = s[y] = valid[y] ? v : -INFINITY;
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int y = 0; y < TILE_R; ++y) top[y] = fmaxf(top[y], __shfl_xor_sync(0xffffffffu, top[y], o));
+#pragma unroll
+            for (int y = 0; y < TILE_R; ++y) {
+                const float m_new = fmaxf(m[y], top[y]);
+                sum[y] = valid[y] ? expf(s[y] - m_new) : 0.f;
+                P_s[y * KEYS + lane] = sum[y];
+                // (0 on a row's first keys; a row that sees none of these stays as it is)
+                const float corr = on[y] ? expf(m[y] - m_new) : 1.f;
+                top[y] = corr;
+#pragma unroll
+                for (int i = 0; i < ND; ++i) acc[y][i] *= corr;
+                if (on[y]) m[y] = m_new;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int y = 0; y < TILE_R; ++y) sum[y] += __shfl_xor_sync(0xffffffffu, sum[y], o);
+#pragma unroll
+            for (int y = 0; y < TILE_R; ++y) l[y] = fmaf(l[y], top[y], sum[y]);
             __syncwarp();
             if (every) {
 #pragma unroll 2
@@ -374,7 +424,7 @@ int launch_tile(const void* qkv, void* out, const void* k_pool, const void* v_po
                 int n_kv, int hd, int block_size, float scale, int window, float softcap,
                 long long n_pages, const float* sink, const float* slopes, int keep_first,
                 long long out_stride, int chunk, const int* cu_q, cudaStream_t stream) {
-    constexpr int smem = TileSmem<HD>::FLOATS * (int)sizeof(float);
+    constexpr int smem = TileSmem<HD, sizeof(T) == 4>::FLOATS * (int)sizeof(float);
     static bool configured = false;
     if (!configured) {
         const int rc = (int)cudaFuncSetAttribute(attention_simt_tile_kernel<T, HD>,
