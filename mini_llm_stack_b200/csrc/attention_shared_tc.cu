@@ -113,7 +113,9 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
     if (r >= P.n_req) return;
     tile = (rows + ROWS - 1) / ROWS - 1 - tile;
     const int kvh = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from which the
+    // instructions take their operands)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int tok0 = P.cu_q[r], pos0 = P.ctx_len[r] - q_len;
     const int row0 = tile * ROWS;
     const int hi = pos0 + (min(rows, row0 + ROWS) - 1) / P.group;
@@ -204,7 +206,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
             if (!mbar_wait(bar(B_K_FULL + j % STAGES), (j / STAGES) & 1)) timed_out = true;
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issue
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = umma_idesc(BN, 0);
             constexpr uint32_t idesc_o = umma_idesc(HD, 1);
             // S = Q K^T for step i, into the buffer whose P the product of step i - 2 has read
@@ -214,11 +216,14 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 if (!mbar_wait(bar(B_K_FULL + slot), (i / STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint32_t k_src = k_smem + slot * K_STAGE;
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk)
-                    umma(tmem + (i & 1) * 128, umma_desc(q_smem + (kk >> 2) * QBLOCK + (kk & 3) * 32),
-                         umma_desc(k_src + (kk >> 2) * KBLOCK + (kk & 3) * 32), idesc_s, kk ? 1u : 0u);
-                umma_commit(bar(B_S_FULL + (i & 1)));
+                    for (int kk = 0; kk < HD / 16; ++kk)
+                        umma(tmem + (i & 1) * 128, umma_desc(q_smem + (kk >> 2) * QBLOCK + (kk & 3) * 32),
+                             umma_desc(k_src + (kk >> 2) * KBLOCK + (kk & 3) * 32), idesc_s, kk ? 1u : 0u);
+                    umma_commit(bar(B_S_FULL + (i & 1)));
+                }
+                __syncwarp();
                 return true;
             };
             if (!mbar_wait(bar(B_Q_FULL), 0)) timed_out = true;
@@ -231,13 +236,16 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 }
                 tc_fence_after();
                 const uint32_t v_src = k_smem + (i % STAGES) * K_STAGE;
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < 2 * (BN / 16); ++kk)     // the weights' upper halves, then the rest
-                    umma_ts(tmem + COL_O, tmem + (i & 1) * 128 + kk * 8,
-                            umma_desc_mn(v_src + kk % (BN / 16) * 16 * 128, KBLOCK), idesc_o,
-                            (i | kk) ? 1u : 0u);
-                umma_commit(bar(i + 1 < steps ? B_O_REST : B_O_LAST));   // O holds step i
-                umma_commit(bar(B_K_EMPTY + i % STAGES));      // the tile has been read both ways
+                    for (int kk = 0; kk < 2 * (BN / 16); ++kk) // the weights' upper halves, then the rest
+                        umma_ts(tmem + COL_O, tmem + (i & 1) * 128 + kk * 8,
+                                umma_desc_mn(v_src + kk % (BN / 16) * 16 * 128, KBLOCK), idesc_o,
+                                (i | kk) ? 1u : 0u);
+                    umma_commit(bar(i + 1 < steps ? B_O_REST : B_O_LAST));   // O holds step i
+                    umma_commit(bar(B_K_EMPTY + i % STAGES));  // the tile has been read both ways
+                }
+                __syncwarp();
                 if (i + 2 < steps && !issue_s(i + 2)) timed_out = true;
             }
         }

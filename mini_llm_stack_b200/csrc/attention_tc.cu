@@ -142,7 +142,9 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
     if (r >= P.n_req) return;
     tile = (rows + tile_rows - 1) / tile_rows - 1 - tile;
     const int kvh = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from which the
+    // instructions take their operands)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int tok0 = P.cu_q[r], ctx = P.ctx_len[r];
     const int row0 = tile * tile_rows;
     const int pos0 = ctx - q_len;
@@ -289,7 +291,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issue
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = umma_idesc(BN, 0);
             constexpr uint32_t idesc_o = umma_idesc(HD, 1);
             // S_c = Q_c K^T for chain c's step i, over whatever the chain's score columns hold
@@ -301,15 +303,18 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                 tc_fence_after();
                 const uint32_t k_src = k_smem + slot * K_STAGE;
                 const uint32_t q_src = q_smem + (P.two_tiles ? c * Q_BYTES : 0);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * BLOCK + (kk & 3) * 32;
-                    umma(tmem + COL_S + c * BN, umma_desc(q_src + off), umma_desc(k_src + off),
-                         idesc_s, kk ? 1u : 0u);
+                    for (int kk = 0; kk < HD / 16; ++kk) {
+                        const uint32_t off = (kk >> 2) * BLOCK + (kk & 3) * 32;
+                        umma(tmem + COL_S + c * BN, umma_desc(q_src + off), umma_desc(k_src + off),
+                             idesc_s, kk ? 1u : 0u);
+                    }
+                    umma_commit(bar(B_S_FULL + c));
+                    // the keys are done with after the last chain that reads them
+                    if (!P.two_tiles || c == chains - 1) umma_commit(bar(B_K_EMPTY + slot));
                 }
-                umma_commit(bar(B_S_FULL + c));
-                // the keys are done with after the last chain that reads them
-                if (!P.two_tiles || c == chains - 1) umma_commit(bar(B_K_EMPTY + slot));
+                __syncwarp();
                 return true;
             };
             // O_c += P_c V for chain c's step i, P read from tensor memory
@@ -319,12 +324,15 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                 if (!mbar_wait(bar(B_V_FULL + slot), (t / V_STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint32_t v_src = v_smem + slot * V_STAGE;
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; ++kk)
-                    umma_ts(tmem + COL_O + c * BN, tmem + COL_S + c * BN + kk * 8,
-                            umma_desc_mn(v_src + kk * 16 * 128, KBLOCK), idesc_o, (i | kk) ? 1u : 0u);
-                umma_commit(bar(B_O_REST + c));            // O_c holds step i
-                if (!P.two_tiles || c == chains - 1) umma_commit(bar(B_V_EMPTY + slot));
+                    for (int kk = 0; kk < BN / 16; ++kk)
+                        umma_ts(tmem + COL_O + c * BN, tmem + COL_S + c * BN + kk * 8,
+                                umma_desc_mn(v_src + kk * 16 * 128, KBLOCK), idesc_o, (i | kk) ? 1u : 0u);
+                    umma_commit(bar(B_O_REST + c));        // O_c holds step i
+                    if (!P.two_tiles || c == chains - 1) umma_commit(bar(B_V_EMPTY + slot));
+                }
+                __syncwarp();
                 return true;
             };
             if (!mbar_wait(bar(B_Q_FULL), 0)) timed_out = true;

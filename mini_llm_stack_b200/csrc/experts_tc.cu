@@ -112,7 +112,9 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::TMEM_SLOT);
     int* start = reinterpret_cast<int*>(gbase + L::TABLE);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from which the
+    // instructions take their operands)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     chain_release();
     if (threadIdx.x == 0) {
         for (int s = 0; s < L::STAGES; ++s) {
@@ -196,7 +198,7 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- instructions
-        if (lane == 0) {
+        {
             int g = 0, it = 0;
             for (int i = blockIdx.x; i < units && !timed_out; i += gridDim.x, ++it) {
                 const Unit u = unit_of<NT>(i, m_tiles, start, p.n_experts, p.offsets);
@@ -216,15 +218,19 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
                     }
                     tc_fence_after();
                     const uint32_t a = base + slot * L::STAGE, b = a + L::A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int m = 0; m < L::MATS; ++m)
+                        for (int m = 0; m < L::MATS; ++m)
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                            umma(d + m * NT, umma_desc(a + m * (ROWS_W * BK * 2) + kk * UMMA_K * 2),
-                                 umma_desc(b + kk * UMMA_K * 2), idesc, (kb | kk) ? 1u : 0u);
-                    umma_commit(empty(slot));
+                            for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                                umma(d + m * NT, umma_desc(a + m * (ROWS_W * BK * 2) + kk * UMMA_K * 2),
+                                     umma_desc(b + kk * UMMA_K * 2), idesc, (kb | kk) ? 1u : 0u);
+                        umma_commit(empty(slot));
+                    }
+                    __syncwarp();
                 }
-                umma_commit(acc_full(acc));
+                if (elect_one()) umma_commit(acc_full(acc));
+                __syncwarp();
             }
         }
     } else {

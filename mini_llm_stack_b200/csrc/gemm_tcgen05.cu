@@ -16,6 +16,10 @@
 //             cut over gridDim.z CTAs whose partial sums go to float32 scratch.
 //
 // Warp roles: 0 = TMA producer, 1 = TMEM allocation and MMA issue, 2..5 = epilogue.
+// The instructions are issued under elect.sync by a warp whose loop is uniform.  From a branch that one lane takes,
+// the four of a k-block took some 600 cycles to prepare, more than a pair needs to run them (512): 707 x 2,048 x
+// 2,048 with SwiGLU 15.9 -> 12.9 us on tiles of 128 x 128, 2,048 x 28,672 x 4,096 369 -> 318, a decoded token of the 1b
+// shape 774 -> 743.
 // Every wait is bounded; a wait that runs out sets MLS_STATUS_TIMEOUT and the
 // kernel still frees its tensor memory and returns.
 #include "common.cuh"
@@ -197,7 +201,9 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
     auto acc_empty = [&](int a) { return base + L::BARS + 8u * (2 * STAGES + 2 + a); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::TMEM_SLOT);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from which the
+    // instructions take their operands)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int m_tiles = (p.mm + BM - 1) / BM, n_tiles = (p.nn + BN - 1) / BN;
     const int tile_count = m_tiles * n_tiles * p.splits;
     const int kblocks = (p.k + BK - 1) / BK;
@@ -273,7 +279,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
     } else if (warp == 1) {
         chain_wait();
         // --------------------------------------------------------------- MMA issue
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = umma_idesc(BN);
             int g = 0, it = 0;
             for (int tile = blockIdx.x; tile < tile_count && !timed_out; tile += gridDim.x, ++it) {
@@ -294,13 +300,17 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
                     }
                     tc_fence_after();
                     const uint32_t a_src = base + slot * L::STAGE, b_src = a_src + L::A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                        umma(tmem_d, umma_desc(a_src + kk * UMMA_K * 2),
-                             umma_desc(b_src + kk * UMMA_K * 2), idesc, (i | kk) ? 1u : 0u);
-                    umma_commit(empty(slot));       // the stage is free when these are done
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            umma(tmem_d, umma_desc(a_src + kk * UMMA_K * 2),
+                                 umma_desc(b_src + kk * UMMA_K * 2), idesc, (i | kk) ? 1u : 0u);
+                        umma_commit(empty(slot));   // the stage is free when these are done
+                    }
+                    __syncwarp();
                 }
-                umma_commit(acc_full(acc));         // the accumulator is complete
+                if (elect_one()) umma_commit(acc_full(acc));         // the accumulator is complete
+                __syncwarp();
             }
         }
     } else {
@@ -439,7 +449,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     auto acc_empty = [&](int a) { return base + L::BARS + 8u * (2 * STAGES + 2 + a); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::TMEM_SLOT);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();                    // 0: issues the instructions
     const int m_pairs = (p.mm + 2 * BM - 1) / (2 * BM), n_tiles = (p.nn + BN - 1) / BN;
     const int tile_count = m_pairs * n_tiles;
@@ -496,7 +506,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // ----------------------------------------------- MMA issue for the pair
             constexpr uint32_t idesc = umma_idesc_pair(BN);
             int g = 0, it = 0;
@@ -517,14 +527,18 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     }
                     tc_fence_after();
                     const uint32_t a_src = base + slot * L::STAGE, b_src = a_src + L::A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                        umma_pair(tmem_d, umma_desc(a_src + kk * UMMA_K * 2),
-                                  umma_desc(b_src + kk * UMMA_K * 2), idesc,
-                                  (i > w.kb0 || kk) ? 1u : 0u);
-                    umma_commit_pair(empty(slot), 3);        // both CTAs' stage is free
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            umma_pair(tmem_d, umma_desc(a_src + kk * UMMA_K * 2),
+                                      umma_desc(b_src + kk * UMMA_K * 2), idesc,
+                                      (i > w.kb0 || kk) ? 1u : 0u);
+                        umma_commit_pair(empty(slot), 3);    // both CTAs' stage is free
+                    }
+                    __syncwarp();
                 }
-                umma_commit_pair(acc_full(acc), 3);          // both CTAs' accumulator is complete
+                if (elect_one()) umma_commit_pair(acc_full(acc), 3); // both CTAs' accumulator is complete
+                __syncwarp();
             }
         }
     } else {
