@@ -1008,6 +1008,11 @@ static int gemm_bf16(const void* act, const void* w, void* out, int out_f32, int
     p.mm = m;
     p.nn = n;
     p.transposed = 0;
+    // Where 128 x 128 tiles have an SM each, a round of them is shorter than one of larger tiles on some of the SMs (with
+    // SwiGLU, us, 256 x 256 on pairs / 128 x 128: 130 x 2,048 x 2,048 15.9 / 13.4, 707 17.5 / 15.9, 300 x 5,632 x 4,096 27.7 /
+    // 26.3; now 10.7, 12.9 and 20.8).
+    const long long tiles128 = (long long)((m + BM - 1) / BM) * ((n + 127) / 128);
+    if (tiles128 <= sm_count()) return launch<128, 6>(p, act, w, 1, stream);
     if (g_prompt_kernel == 1 && m > BM) return launch_pair<6>(p, act, w, stream);
     return launch<256, 4>(p, act, w, 1, stream);
 }
