@@ -7,15 +7,6 @@
 namespace mls_chunk {
 constexpr int C = CHUNK;
 
-__device__ __forceinline__ float4 load4(const void* base, int dtype, size_t i) {
-    if (dtype == MLS_BF16) {
-        const uint2 raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)base + i);
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-        return make_float4(lo.x, lo.y, hi.x, hi.y);
-    }
-    return *reinterpret_cast<const float4*>((const float*)base + i);
-}
 __device__ __forceinline__ float silu1(float z) { return times_sigmoid(z, z); }
 __device__ __forceinline__ float4 times(float4 v, float f) {
     return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
@@ -76,7 +67,7 @@ __device__ __forceinline__ bool locate(const Args& a, const Part& p, int z, Wher
     return j < w.chunks;
 }
 
-// Four entries of operand row t (zeros past the chunk and past the head's size).
+// Quads of an operand's rows (zeros past the chunk and past the head's size).
 struct Reader {
     const void* base;
     size_t row, at;                  // elements between tokens; the head's first entry
@@ -86,23 +77,18 @@ struct Reader {
     __device__ __forceinline__ Reader(const Rows& r, int silu_, const Where& w, int head, size_t t0)
         : base(r.base), row(r.row), at(t0 * r.row + r.off + (size_t)head * r.width),
           dtype(r.dtype), silu(silu_), n(w.n), size(r.width) {}
-    __device__ __forceinline__ float4 operator()(int t, int i) const {
-        if (t >= n || i >= size) return make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v = load4(base, dtype, at + (size_t)t * row + i);
-        if (silu) v = make_float4(silu1(v.x), silu1(v.y), silu1(v.z), silu1(v.w));
-        return v;
-    }
-    // Quads at i, i + step, ..: the type is asked once, so that their loads are under way together.
-    template <int N>
-    __device__ __forceinline__ void many(int t, int i, int step, float4 (&v)[N]) const {
-        const size_t from = at + (size_t)t * row;
+    // N quads, the x-th at (token, entry) = place(x): the type is asked once, so that their loads are under way
+    // together (a load that is asked for inside a branch on its type is waited for there).
+    template <int N, typename Place>
+    __device__ __forceinline__ void quads(Place place, float4 (&v)[N]) const {
         if (dtype == MLS_BF16) {
             uint2 raw[N];
 #pragma unroll
             for (int x = 0; x < N; ++x) {
-                const bool there = t < n && i + x * step < size;
-                raw[x] = there ? *reinterpret_cast<const uint2*>((const __nv_bfloat16*)base + from + i + x * step)
-                               : make_uint2(0u, 0u);
+                const int2 p = place(x);
+                raw[x] = p.x < n && p.y < size ? *reinterpret_cast<const uint2*>((const __nv_bfloat16*)base + at +
+                                                                                 (size_t)p.x * row + p.y)
+                                               : make_uint2(0u, 0u);
             }
 #pragma unroll
             for (int x = 0; x < N; ++x) {
@@ -113,9 +99,10 @@ struct Reader {
         } else {
 #pragma unroll
             for (int x = 0; x < N; ++x) {
-                const bool there = t < n && i + x * step < size;
-                v[x] = there ? *reinterpret_cast<const float4*>((const float*)base + from + i + x * step)
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
+                const int2 p = place(x);
+                v[x] = p.x < n && p.y < size
+                           ? *reinterpret_cast<const float4*>((const float*)base + at + (size_t)p.x * row + p.y)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         if (silu)

@@ -57,27 +57,39 @@ __device__ __forceinline__ float2 halves(f32x2 v) {
 // eight quads of k a warp) nor the reads of four rows at a time meet a bank twice.
 __device__ __forceinline__ int turn(int k) { return 4 * ((k >> 2) & 7); }
 
-template <int THREADS, typename Get>
-__device__ __forceinline__ void fill_transposed(float (*T)[C], Get get) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll 8
-    for (int u = threadIdx.x >> 5; u < 32; u += THREADS / 32) {
-        const int r = 4 * (u & 15) + (lane & 3), q = (lane >> 2) + 8 * (u >> 4);
-        const float4 v = get(r, 4 * q);
-        const int col = r ^ (4 * (q & 7));
-        T[4 * q][col] = v.x;
-        T[4 * q + 1][col] = v.y;
-        T[4 * q + 2][col] = v.z;
-        T[4 * q + 3][col] = v.w;
-    }
+// A thread's quads of such a tile: row and first of the four k of its y-th.
+template <int THREADS>
+constexpr int QUADS_OF = C * (C / 4) / THREADS;
+template <int THREADS>
+__device__ __forceinline__ int2 transposed_at(int y) {
+    const int u = (threadIdx.x >> 5) + y * (THREADS / 32), lane = threadIdx.x & 31;
+    return make_int2(4 * (u & 15) + (lane & 3), 4 * ((lane >> 2) + 8 * (u >> 4)));
 }
-// 64 rows (of k) of W values, as they are.
-template <int THREADS, int W, typename Get>
-__device__ __forceinline__ void fill_rows(float (*T)[W], Get get) {
-#pragma unroll 8
-    for (int u = threadIdx.x; u < C * (W / 4); u += THREADS) {
-        const int k = u / (W / 4), x = 4 * (u % (W / 4));
-        *reinterpret_cast<float4*>(&T[k][x]) = get(k, x);
+__device__ __forceinline__ void put_transposed(float (*T)[C], int2 p, float4 v) {
+    const int col = p.x ^ turn(p.y);
+    T[p.y][col] = v.x;
+    T[p.y + 1][col] = v.y;
+    T[p.y + 2][col] = v.z;
+    T[p.y + 3][col] = v.w;
+}
+// 64 rows (of k) of W values, as they are, from entry x0 of the operand's rows on; each(row, quad) as it goes by.
+template <int THREADS, int W, typename Each>
+__device__ __forceinline__ void fill_rows(float (*T)[W], const Reader& from, int x0, Each each) {
+    constexpr int ALL = C * (W / 4) / THREADS, N = ALL < 8 ? ALL : 8;
+    static_assert(ALL % N == 0, "whole batches");
+#pragma unroll 1
+    for (int y0 = 0; y0 < ALL; y0 += N) {
+        float4 v[N];
+        auto at = [&](int y) {
+            const int u = threadIdx.x + (y0 + y) * THREADS;
+            return make_int2(u / (W / 4), 4 * (u % (W / 4)));
+        };
+        from.quads<N>([&](int y) { const int2 p = at(y); return make_int2(p.x, x0 + p.y); }, v);
+#pragma unroll
+        for (int y = 0; y < N; ++y) {
+            const int2 p = at(y);
+            *reinterpret_cast<float4*>(&T[p.x][p.y]) = each(p.x, v[y]);
+        }
     }
 }
 
@@ -161,8 +173,16 @@ chunk_scores_kernel(const Args a, const Scratch s, const Part part) {
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = sum[i][0] = sum[i][1] = 0ull;
     for (int i0 = 0; i0 < a.e; i0 += C) {
         __syncthreads();
-        fill_transposed<256>(A, [&](int r, int i) { return q(r, i0 + i); });
-        fill_transposed<256>(B, [&](int r, int i) { return k(r, i0 + i); });
+        constexpr int N = QUADS_OF<256>;
+        float4 x[N], y[N];
+        auto place = [&](int g) { const int2 p = transposed_at<256>(g); return make_int2(p.x, i0 + p.y); };
+        q.quads<N>(place, x);
+        k.quads<N>(place, y);
+#pragma unroll
+        for (int g = 0; g < N; ++g) {
+            put_transposed(A, transposed_at<256>(g), x[g]);
+            put_transposed(B, transposed_at<256>(g), y[g]);
+        }
         __syncthreads();
         if (idle) continue;
 #pragma unroll 16
@@ -258,15 +278,29 @@ chunk_scores_token_kernel(const Args a, const Scratch s, const Part part) {
     const int tid = threadIdx.x;
     const Reader q(a.q, a.silu, w, head), k(a.k, a.silu, w, head);
     float* P = s.scores + (w.idx * a.n_heads + head) * C * C;
-#pragma unroll 4
-    for (int u = tid; u < C * quads; u += 256) {
-        const int t = u / quads, i = 4 * (u - t * quads);
-        float4 d = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (t < w.n)
-            d = *reinterpret_cast<const float4*>(a.decay + ((size_t)(w.t0 + t) * a.n_heads + head) * e + i);
-        *reinterpret_cast<float4*>(r_s + t * pad + i) = q(t, i);
-        *reinterpret_cast<float4*>(k_s + t * pad + i) = k(t, i);
-        *reinterpret_cast<float4*>(w_s + t * pad + i) = d;
+    for (int u0 = tid; u0 < C * quads; u0 += 4 * 256) {
+        float4 rq[4], rk[4], d[4];
+        auto place = [&](int x) {                        // (past the last quad: a token past the chunk)
+            const int u = u0 + 256 * x, t = u / quads;
+            return make_int2(u < C * quads ? t : C, 4 * (u - t * quads));
+        };
+        q.quads<4>(place, rq);
+        k.quads<4>(place, rk);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int2 p = place(x);
+            d[x] = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (p.x < w.n)
+                d[x] = *reinterpret_cast<const float4*>(a.decay + ((size_t)(w.t0 + p.x) * a.n_heads + head) * e + p.y);
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int2 p = place(x);
+            if (p.x >= C) continue;
+            *reinterpret_cast<float4*>(r_s + p.x * pad + p.y) = rq[x];
+            *reinterpret_cast<float4*>(k_s + p.x * pad + p.y) = rk[x];
+            *reinterpret_cast<float4*>(w_s + p.x * pad + p.y) = d[x];
+        }
     }
     for (int i = tid; i < e; i += 256)
         bonus_s[i] = a.bonus ? load_as_float(a.bonus, (size_t)head * e + i, a.bonus_dtype) : 0.f;
@@ -498,8 +532,8 @@ chunk_update_kernel(const Args a, const Scratch s, const Part part) {
     if (MODE == TOKEN_DECAY) kr = Rows{s.rows_k, MLS_F32, a.n_heads * a.e, 0, a.e};
     const Reader k(kr, MODE == TOKEN_DECAY ? 0 : a.silu, w, head, MODE == TOKEN_DECAY ? w.idx * C : (size_t)w.t0);
     const Reader v(a.v, a.silu, w, head);
-    fill_rows<THREADS, C>(A, [&](int t, int i) { return times(k(t, i0 + i), factor[t]); });
-    fill_rows<THREADS, BN>(B, [&](int t, int j) { return v(t, j0 + j); });
+    fill_rows<THREADS, C>(A, k, i0, [&](int t, float4 x) { return times(x, factor[t]); });
+    fill_rows<THREADS, BN>(B, v, j0, [&](int, float4 x) { return x; });
     __syncthreads();
     const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
     f32x2 sum[8][TN / 2], acc[8][TN / 2];                  // (the factors are rounded already: short chains)
@@ -612,7 +646,6 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
     const float* S = s.states + unit * state_floats(MODE, a.e, a.f);
     const float* P = s.scores + unit * C * C;
     const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool with_n = MODE == MLSTM && j0 == 0;
     const int blocks = 1 + (a.e + C - 1) / C;
     // rows i0 .. of S0 into buffer x (what is not there as zeros)
@@ -629,10 +662,15 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     float4 next[QA];
-    fill_transposed<THREADS>(A[0], [&](int t, int x) { return *reinterpret_cast<const float4*>(P + t * C + x); });
+#pragma unroll
+    for (int y = 0; y < QA; ++y) {
+        const int2 p = transposed_at<THREADS>(y);
+        next[y] = *reinterpret_cast<const float4*>(P + p.x * C + p.y);
+    }
+#pragma unroll
+    for (int y = 0; y < QA; ++y) put_transposed(A[0], transposed_at<THREADS>(y), next[y]);
     bool odd = false;                                          // a value that is not a number, or infinite
-    fill_rows<THREADS, BN>(B[0], [&](int t, int j) {
-        const float4 x = v(t, j0 + j);
+    fill_rows<THREADS, BN>(B[0], v, j0, [&](int, float4 x) {
         odd |= !((x.x + x.y + x.z + x.w) * 0.f == 0.f);        // (a sum that overflows: no harm)
         return x;
     });
@@ -648,11 +686,7 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
         float n_next = 0.f;
         if (more) {
             ask_rows(i0, x ^ 1);
-#pragma unroll
-            for (int y = 0; y < QA; ++y) {
-                const int u = warp + y * (THREADS / 32);
-                next[y] = q(4 * (u & 15) + (lane & 3), i0 + 4 * ((lane >> 2) + 8 * (u >> 4)));
-            }
+            q.quads<QA>([&](int y) { const int2 p = transposed_at<THREADS>(y); return make_int2(p.x, i0 + p.y); }, next);
             if (with_n && threadIdx.x < C && i0 + (int)threadIdx.x < a.e)
                 n_next = S[(size_t)a.e * a.f + i0 + threadIdx.x];
         }
@@ -670,13 +704,8 @@ chunk_output_kernel(const Args a, const Scratch s, const Part part) {
         if (more) {
 #pragma unroll
             for (int y = 0; y < QA; ++y) {
-                const int u = warp + y * (THREADS / 32), r = 4 * (u & 15) + (lane & 3),
-                          k = 4 * ((lane >> 2) + 8 * (u >> 4)), col = r ^ turn(k);
-                const float4 z = times(next[y], factor[r]);
-                A[x ^ 1][k][col] = z.x;
-                A[x ^ 1][k + 1][col] = z.y;
-                A[x ^ 1][k + 2][col] = z.z;
-                A[x ^ 1][k + 3][col] = z.w;
+                const int2 p = transposed_at<THREADS>(y);
+                put_transposed(A[x ^ 1], p, times(next[y], factor[p.x]));
             }
             if (with_n && threadIdx.x < C) n_s[x ^ 1][threadIdx.x] = n_next;
         }

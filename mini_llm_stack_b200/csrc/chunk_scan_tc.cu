@@ -478,7 +478,7 @@ chunk_output_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Pa
             for (int g = 0; g < 4; ++g)
                 z[g] = i0 + 4 * PER * g < a.e ? *reinterpret_cast<const float4*>(n + i0 + 4 * PER * g)
                                               : make_float4(0.f, 0.f, 0.f, 0.f);
-            q.template many<4>(t, i0, 4 * PER, y);
+            q.template quads<4>([&](int g) { return make_int2(t, i0 + 4 * PER * g); }, y);
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 d[0] = fmaf(y[g].x, z[g].x, d[0]), d[1] = fmaf(y[g].y, z[g].y, d[1]);

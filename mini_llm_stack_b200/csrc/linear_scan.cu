@@ -253,7 +253,7 @@ scan_finish_kernel(const float* __restrict__ o, const void* __restrict__ gate, i
 
 // The same for heads of up to 128 * QUADS values whose rows can be read four entries at a time: a
 // lane keeps its quads in registers, and all loads are under way before the sum is taken.  (51 ->
-// 35 us for 2,048 tokens of 32 heads of 256 values.  Which of the two runs depends on the sizes
+// 30 us for 2,048 tokens of 32 heads of 256 values; 35 with the gate's type asked quad by quad.  Which of the two runs depends on the sizes
 // alone.)
 template <typename T, int QUADS>
 __global__ void __launch_bounds__(256)
@@ -269,12 +269,35 @@ scan_finish_quads_kernel(const float* __restrict__ o, const void* __restrict__ g
     const size_t at = (size_t)t * n_heads * f + (size_t)head * f;
     float4 v[QUADS], z[QUADS];
     float ss = 0.f;
+    const size_t gate_at = (size_t)t * gate_row + gate_off + head * f;
+    // (a load that is asked for inside a branch on its type is waited for there: one branch for all of them)
+#pragma unroll
+    for (int x = 0; x < QUADS; ++x)
+        if (4 * (lane + 32 * x) < f) v[x] = *reinterpret_cast<const float4*>(o + at + 4 * (lane + 32 * x));
+    if (QUADS == 1) {
+        if (4 * lane < f) z[0] = load4(gate, gate_dtype, gate_at + 4 * lane);
+    } else if (gate_dtype == MLS_BF16) {
+        uint2 raw[QUADS];
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x)
+            if (4 * (lane + 32 * x) < f)
+                raw[x] = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)gate + gate_at + 4 * (lane + 32 * x));
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x) {
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[x].x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[x].y));
+            z[x] = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    } else {
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x)
+            if (4 * (lane + 32 * x) < f)
+                z[x] = *reinterpret_cast<const float4*>((const float*)gate + gate_at + 4 * (lane + 32 * x));
+    }
 #pragma unroll
     for (int x = 0; x < QUADS; ++x) {
         const int j = 4 * (lane + 32 * x);
         if (j >= f) continue;
-        v[x] = *reinterpret_cast<const float4*>(o + at + j);
-        z[x] = load4(gate, gate_dtype, (size_t)t * gate_row + gate_off + head * f + j);
         ss = fmaf(v[x].x, v[x].x, ss);
         ss = fmaf(v[x].y, v[x].y, ss);
         ss = fmaf(v[x].z, v[x].z, ss);
