@@ -933,7 +933,7 @@ int launch_pair(const GemmParams& p, const void* a, const void* b, cudaStream_t 
 }
 
 // Which kernel takes prompts of more than 128 rows: MLS_B200_GEMM_KERNEL = pair (default: two
-// CTAs a tile of 256 x 256) or tiles (one CTA a tile of 128 x 256).  Measured at 2,048 rows of
+// CTAs a tile of 256 x 256; small products one CTA a tile of 128 x 128) or tiles (one CTA a tile of 128 x 256).  Measured at 2,048 rows of
 // the Llama-3-8B products the pairs run at 1.33-1.39 PFLOP/s against 1.26-1.30 (with the
 // SwiGLU epilogue 1.45 against 1.43; at 512 rows 1.12 against 1.07).
 int g_prompt_kernel = [] {
@@ -1010,10 +1010,13 @@ static int gemm_bf16(const void* act, const void* w, void* out, int out_f32, int
     p.transposed = 0;
     // Where 128 x 128 tiles have an SM each, a round of them is shorter than one of larger tiles on some of the SMs (with
     // SwiGLU, us, 256 x 256 on pairs / 128 x 128: 130 x 2,048 x 2,048 15.9 / 13.4, 707 17.5 / 15.9, 300 x 5,632 x 4,096 27.7 /
-    // 26.3; now 10.7, 12.9 and 20.8).
+    // 26.3; now 10.7, 12.9 and 20.8).  A product whose K the pairs cut is left to them: its parts fill the SMs too, and a long K
+    // is drawn from L2 less often by larger tiles (300 x 2,048 x 14,336 40 on pairs, 61 here; 707 x 2,048 x 8,192 36 and 41).
     const long long tiles128 = (long long)((m + BM - 1) / BM) * ((n + 127) / 128);
-    if (tiles128 <= sm_count()) return launch<128, 6>(p, act, w, 1, stream);
-    if (g_prompt_kernel == 1 && m > BM) return launch_pair<6>(p, act, w, stream);
+    const bool pairs = g_prompt_kernel == 1 && m > BM;
+    if (g_prompt_kernel == 1 && tiles128 <= sm_count() && !(pairs && tail_plan(m, n, k).parts > 1))
+        return launch<128, 6>(p, act, w, 1, stream);
+    if (pairs) return launch_pair<6>(p, act, w, stream);
     return launch<256, 4>(p, act, w, 1, stream);
 }
 

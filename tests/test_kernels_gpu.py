@@ -231,6 +231,38 @@ def test_gate_up_projection_with_swiglu_epilogue(rts, m, inter, k):
     assert (out.float().cpu() - want).abs().max().item() <= 8e-3 * want.abs().max().item() + 1e-6
 
 
+@pytest.mark.parametrize("out_dtype", DTYPES)
+@pytest.mark.parametrize("m, n, k, swiglu", [
+    (65, 1000, 72, False), (129, 96, 3080, True), (257, 1056, 136, True), (128, 18944, 64, False),   # 148 tiles
+    (128, 18976, 64, True),                                                                          # 149
+    (700, 136, 4096, False), (300, 2048, 8192, True)])                                    # K cut by the pairs
+def test_products_of_a_tile_an_sm(rts, m, n, k, swiglu, out_dtype):
+    """Products whose tiles of 128 x 128 have an SM each, and their neighbours on larger tiles, against
+    float64: float32 sums differ from it by K roundings of the sum of magnitudes at most."""
+    ops = rts[torch.bfloat16].ops
+    a, w = rand((m, k), torch.bfloat16, 43), rand((n, k), torch.bfloat16, 44, 0.05)
+    both, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    ops.gemm_impl = "tcgen05"
+    try:
+        if swiglu:
+            out = torch.full((m, n // 2), float("nan"), dtype=out_dtype, device=DEV)
+            ops.linear_swiglu(a, w, out)
+            both, size = both.view(m, n // 32, 2, 16), size.view(m, n // 32, 2, 16)
+            g, u = both[:, :, 0].reshape(m, -1), both[:, :, 1].reshape(m, -1)
+            want = torch.nn.functional.silu(g) * u
+            # |d silu| <= 1.1 |dg|, and |silu(g)| <= |g|
+            bound = 1.1 * size[:, :, 0].reshape(m, -1) * u.abs() + g.abs() * size[:, :, 1].reshape(m, -1)
+        else:
+            out = torch.full((m, n), float("nan"), dtype=out_dtype, device=DEV)
+            ops.linear(a, ops.prepare_weight(w), out)
+            want, bound = both, size
+    finally:
+        ops.gemm_impl = "auto"
+    ops.check_status()
+    eps = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -20
+    assert ((out.double() - want).abs() <= eps * want.abs() + k * 2.0 ** -24 * bound + 1e-6).all()
+
+
 @pytest.mark.parametrize("mode", ["always", "auto"])
 @pytest.mark.parametrize("m, n, k, swiglu", [
     (600, 1000, 4096, False),      # twelve ragged tiles, no whole round, in six parts each
