@@ -11,7 +11,8 @@ constexpr int SKINNY_N = 256;        // up to so many columns the product is by 
 constexpr int FEWEST_N = 64;
 constexpr long long FEWEST_SIZE = 1 << 18;
 // From so much of K on the tensor cores pay whatever M is (us, FFMA / tensor cores: 1 x 300 x 2,048 18.4 / 16.4,
-// 1 x 2,048 x 2,048 20.5 / 18.4, 9 x 2,048 x 2,048 82 / 18; but 1 x 4,096 x 1,024 16.4 / 18.4), from a quarter of it
+// 1 x 2,048 x 2,048 20.5 / 18.4, 9 x 2,048 x 2,048 82 / 18; but 1 x 4,096 x 1,024 16.4 / 18.4; those with eight
+// groups of K, with sixteen 1 x 2,048 x 2,048 is at 10.5), from a quarter of it
 // where the weights are so many that their way from memory counts (1 x 16,384 x 1,024 39 / 31, 1 x 16,384 x 512
 // 22.6 both).
 constexpr int TC_K = 2048;
