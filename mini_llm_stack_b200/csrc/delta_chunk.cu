@@ -410,10 +410,12 @@ delta_chunk_scan_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
                 load_t(c + 1);
                 if (!mbar_wait(bar(QS2), c & 1)) timed_out = true;
                 load_q(c + 1);
-                if (!mbar_wait(bar(KU), c & 1)) timed_out = true;
-                if (c + 2 < w.chunks) load_k(c + 2), k_last = c + 2;
+                // (PU ends behind U_PUT, ahead of which lies every read of the factors that come with k; behind KU alone
+                // the columns may still read them, and KU may end once more before this warp looks: all that chunk
+                // c + 1 needs for it is there)
                 if (!mbar_wait(bar(PU), c & 1)) timed_out = true;
                 load_p(c + 1);
+                if (c + 2 < w.chunks) load_k(c + 2), k_last = c + 2;
                 last = c + 1;
                 if (timed_out) break;
             }
