@@ -87,7 +87,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __global__ void __launch_bounds__(THREADS)
 attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                            const __grid_constant__ CUtensorMap kmap_wide) {
-    chain_release();
     chain_wait();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t base = smem_u32(smem_raw);
@@ -138,7 +137,10 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
         mbar_init(bar(B_Q_FULL), ROWS);
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        chain_release();                 // (not before: see there)
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -112,7 +112,6 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                     const __grid_constant__ CUtensorMap vmap,
                     const __grid_constant__ CUtensorMap kmap_wide,
                     const __grid_constant__ CUtensorMap vmap_wide) {
-    chain_release();
     chain_wait();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ float2 chain_state[2][CHAIN_ROWS];    // (maximum, sum) of a row, per chain
@@ -216,7 +215,10 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
         mbar_init(bar(B_Q_FULL), SOFTMAX_THREADS);
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        chain_release();                 // (not before: see there)
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

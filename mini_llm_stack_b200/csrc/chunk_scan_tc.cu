@@ -182,7 +182,6 @@ __device__ __noinline__ float update_chain(const Args& a, const Where w, int hea
 template <int MODE, int GROUPS>
 __global__ void __launch_bounds__(128 * GROUPS, 2)
 chunk_update_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Part part, const int cols) {
-    chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
@@ -200,7 +199,10 @@ chunk_update_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Pa
         for (int g = 0; g < GROUPS; ++g) mbar_init(smem_u32(&bars[g]), 1);
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot_s), cols);
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&tmem_slot_s), cols);
+        chain_release();                 // (not before: see there)
+    }
     if (threadIdx.x < C)
         factor[threadIdx.x] = row_factor<MODE>(a, s.rows_k, w, head, threadIdx.x, w.n - 1 - (int)threadIdx.x);
     Rows kr = a.k;
@@ -327,7 +329,6 @@ __device__ __noinline__ float output_chain(const Args& a, const Where w, int hea
 template <int MODE, int GROUPS>
 __global__ void __launch_bounds__(128 * GROUPS, GROUPS == 4 ? 1 : 2)
 chunk_output_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Part part) {
-    chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
@@ -345,7 +346,10 @@ chunk_output_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Pa
         for (int g = 0; g < GROUPS; ++g) mbar_init(smem_u32(&bars[g]), 1);
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot_s), COLS);
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&tmem_slot_s), COLS);
+        chain_release();                 // (not before: see there)
+    }
     if (threadIdx.x < C)
         factor[threadIdx.x] = row_factor<MODE>(a, s.rows_q, w, head, threadIdx.x, threadIdx.x + 1);
     Rows qr = a.q;

@@ -214,6 +214,9 @@ static inline int launch_status() { return (int)cudaGetLastError(); }
 // which returns once all earlier kernels have finished and their writes are
 // visible.  Between the two a kernel may only touch memory that no kernel writes
 // (weights).  Both are no-ops in a kernel that was launched the plain way.
+// A kernel with tensor memory releases its successors from the warp that allocates, once it has
+// allocated: a successor that is resident earlier could take columns that a block here still waits
+// for, and itself wait for this kernel's end.  One thread's call counts for its block.
 static __device__ __forceinline__ void chain_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

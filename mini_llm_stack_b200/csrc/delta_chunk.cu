@@ -94,7 +94,6 @@ constexpr int PREP_THREADS = 256, PAD = C + 4, MAX_RATIO = 4;
 
 __global__ void __launch_bounds__(PREP_THREADS, 2)
 delta_chunk_prep_kernel(const ChunkArgs a, const __grid_constant__ Args where, const Part part, const Place to) {
-    chain_release();
     chain_wait();
     Where w;
     if (!locate<false>(where, part, blockIdx.x, w)) return;
@@ -111,7 +110,10 @@ delta_chunk_prep_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
         mbar_init(bar, 1);
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot_s), 256);
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&tmem_slot_s), 256);
+        chain_release();                 // (not before: see there)
+    }
     const Prepared rows(a.n_tokens, a.H, a.G, a.er, a.fr);
     // q and k as parts, to shared memory for their products and to scratch for the scan
     {
@@ -345,7 +347,6 @@ delta_chunk_scan_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
     static_assert(ACC + 128 <= 512 && EH % 16 == 0 && EH <= 64, "tensor memory");
     constexpr int K_BYTES = E_TILES * 3 * TILE, Q_AT = 2 * K_BYTES, T_AT = Q_AT + K_BYTES, P_AT = T_AT + 3 * TILE,
                   F_AT = P_AT + 3 * TILE;
-    chain_release();
     chain_wait();
     Where w;
     const int head = blockIdx.y;
@@ -366,7 +367,10 @@ delta_chunk_scan_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
         fence_barrier_init();
     }
     if (threadIdx.x < 2 * UMMA_M) dead_s[threadIdx.x / UMMA_M][threadIdx.x % UMMA_M] = C;
-    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot_s), 512);
+    if (warp == 0) {
+        tmem_alloc(smem_u32(&tmem_slot_s), 512);
+        chain_release();                 // (not before: see there)
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -115,7 +115,6 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
     // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from which the
     // instructions take their operands)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    chain_release();
     if (threadIdx.x == 0) {
         for (int s = 0; s < L::STAGES; ++s) {
             mbar_init(full(s), 1);
@@ -127,7 +126,10 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
         }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), L::COLS);
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), L::COLS);
+        chain_release();                 // (not before: see there)
+    }
     chain_wait();
     if (warp == 0) {
         // start[e]: row tiles of the experts before e.  A lane takes neighbouring experts, whose loads are

@@ -124,7 +124,6 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
     // (the warp's number from a shuffle: what follows from it alone may stay in uniform registers, from
     // which the instructions take their operands)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    chain_release();
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(full(s), 1);
@@ -140,7 +139,10 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
         }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot_s), COLS);
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&tmem_slot_s), COLS);
+        chain_release();                 // (not before: see there)
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

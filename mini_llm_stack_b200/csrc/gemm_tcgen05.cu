@@ -209,7 +209,6 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
     const int kblocks = (p.k + BK - 1) / BK;
     const int per = (kblocks + p.splits - 1) / p.splits;
 
-    chain_release();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full(s), 1);
@@ -223,6 +222,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        chain_release();                 // (not before: see there)
     }
     tc_fence_before();
     __syncthreads();
@@ -458,7 +458,6 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
     const int cut = p.tail_parts > 1 ? (tile_count - p.tail_full) * p.tail_parts : 0;
     const int unit_count = cut ? cut + p.tail_full : tile_count;
 
-    chain_release();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full(s), 1);
@@ -470,7 +469,10 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
         }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+    if (warp == 1) {
+        tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+        chain_release();                 // (not before: see there)
+    }
     tc_fence_before();
     cluster_sync_all();                  // both CTAs' barriers and tensor memory are ready
     tc_fence_after();
