@@ -708,7 +708,7 @@ __device__ __forceinline__ void produce_tiles(const Params& P, const CUtensorMap
         const int slot = t % TSTAGES, round = t / TSTAGES;
         const uint32_t full = bar0 + 8u * slot, empty = bar0 + 8u * (TSTAGES + slot);
         const uint32_t parity = slot == late_slot ? (round & 1) : ((round & 1) ^ 1);
-        if (!mbar_wait(empty, parity)) {
+        if (!mbar_wait_warp(empty, parity)) {
             if (lane == 0 && P.status) atomicOr(P.status, MLS_STATUS_TIMEOUT);
             return;
         }
@@ -980,7 +980,7 @@ attention_split_tma_kernel(const Params P, const Fused F,
     bool timed_out = false;
     for (int t = 0; t < n_tiles; ++t) {
         const int slot = t % TSTAGES, ph = (t / TSTAGES) & 1;
-        if (!mbar_wait(full(slot), ph)) {
+        if (!mbar_wait_warp(full(slot), ph)) {
             timed_out = true;
             break;
         }
@@ -1293,7 +1293,7 @@ attention_tile_tma_kernel(const Params P, const __grid_constant__ CUtensorMap km
     bool timed_out = false;
     for (int t = 0; t < n_tiles; ++t) {
         const int slot = t % TSTAGES, ph = (t / TSTAGES) & 1;
-        if (!mbar_wait(bar0 + 8u * slot, ph)) {
+        if (!mbar_wait_warp(bar0 + 8u * slot, ph)) {
             timed_out = true;
             break;
         }

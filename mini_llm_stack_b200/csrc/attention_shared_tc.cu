@@ -155,7 +155,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
         for (; t < steps; ++t) {
             const int slot = t % STAGES;
             const uint32_t full = bar(B_K_FULL + slot), stage = k_smem + slot * K_STAGE;
-            if (!mbar_wait(bar(B_K_EMPTY + slot), ((t / STAGES) & 1) ^ 1)) {
+            if (!mbar_wait_warp(bar(B_K_EMPTY + slot), ((t / STAGES) & 1) ^ 1)) {
                 timed_out = true;
                 break;
             }
@@ -205,7 +205,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
         }
         // the copies under way land before the block's shared memory goes away
         for (int j = t > STAGES ? t - STAGES : 0; j < t; ++j)
-            if (!mbar_wait(bar(B_K_FULL + j % STAGES), (j / STAGES) & 1)) timed_out = true;
+            if (!mbar_wait_warp(bar(B_K_FULL + j % STAGES), (j / STAGES) & 1)) timed_out = true;
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issue
         {
@@ -215,7 +215,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
             // (the tensor cores run the instructions in the order they were issued)
             auto issue_s = [&](int i) -> bool {
                 const int slot = i % STAGES;
-                if (!mbar_wait(bar(B_K_FULL + slot), (i / STAGES) & 1)) return false;
+                if (!mbar_wait_warp(bar(B_K_FULL + slot), (i / STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint32_t k_src = k_smem + slot * K_STAGE;
                 if (elect_one()) {
@@ -228,11 +228,11 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 __syncwarp();
                 return true;
             };
-            if (!mbar_wait(bar(B_Q_FULL), 0)) timed_out = true;
+            if (!mbar_wait_warp(bar(B_Q_FULL), 0)) timed_out = true;
             for (int i = 0; i < min(steps, 2) && !timed_out; ++i)
                 if (!issue_s(i)) timed_out = true;
             for (int i = 0; i < steps && !timed_out; ++i) {
-                if (!mbar_wait(bar(B_P_FULL + (i & 1)), (i >> 1) & 1)) {
+                if (!mbar_wait_warp(bar(B_P_FULL + (i & 1)), (i >> 1) & 1)) {
                     timed_out = true;
                     break;
                 }
@@ -286,7 +286,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
         for (int i = 0; i < steps && !timed_out; ++i) {
             const int kbase = kbase0 + i * BN;
             const uint32_t s_addr = tmem + lane_base + (i & 1) * 128;
-            if (!mbar_wait(bar(B_S_FULL + (i & 1)), (i >> 1) & 1)) {
+            if (!mbar_wait_warp(bar(B_S_FULL + (i & 1)), (i >> 1) & 1)) {
                 timed_out = true;
                 break;
             }
@@ -323,7 +323,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
                 if (i > 0) {
                     // O must be at rest: the product of the step before has to be done (that of the
                     // one before it is, this step's scores were issued behind it)
-                    if (!mbar_wait(bar(B_O_REST), (i - 1) & 1)) {
+                    if (!mbar_wait_warp(bar(B_O_REST), (i - 1) & 1)) {
                         timed_out = true;
                         break;
                     }
@@ -372,7 +372,7 @@ attention_shared_tc_kernel(const Params P, const __grid_constant__ CUtensorMap k
         // All products are done once the last one is (they run in order).  It has a barrier of its own:
         // behind this thread's last arrival two phases of O_REST could end before it looks, and a parity
         // cannot tell a phase from the one two further on.
-        if (!timed_out && !mbar_wait(bar(B_O_LAST), 0)) timed_out = true;
+        if (!timed_out && !mbar_wait_warp(bar(B_O_LAST), 0)) timed_out = true;
         tc_fence_after();
         if (P.sink && live && m_used != -INFINITY)
             l += exp2f(P.sink[kvh * P.group + g] * LOG2E - m_used);

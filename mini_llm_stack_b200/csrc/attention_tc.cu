@@ -235,7 +235,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
             const int slot = t % stages;
             const uint32_t full = bar((which ? B_V_FULL : B_K_FULL) + slot);
             const uint32_t empty = bar((which ? B_V_EMPTY : B_K_EMPTY) + slot);
-            if (!mbar_wait(empty, ((t / stages) & 1) ^ 1)) return false;
+            if (!mbar_wait_warp(empty, ((t / stages) & 1) ^ 1)) return false;
             const int kb = tile_base(t);
             const uint32_t stage = which ? v_smem + slot * V_STAGE : k_smem + slot * K_STAGE;
             bool valid = false;
@@ -301,7 +301,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
             // run the instructions in the order they were issued)
             auto issue_s = [&](int c, int i) -> bool {
                 const int t = key_tile(c, i), slot = t % K_STAGES;
-                if (!mbar_wait(bar(B_K_FULL + slot), (t / K_STAGES) & 1)) return false;
+                if (!mbar_wait_warp(bar(B_K_FULL + slot), (t / K_STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint32_t k_src = k_smem + slot * K_STAGE;
                 const uint32_t q_src = q_smem + (P.two_tiles ? c * Q_BYTES : 0);
@@ -322,8 +322,8 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
             // O_c += P_c V for chain c's step i, P read from tensor memory
             auto issue_pv = [&](int c, int i) -> bool {
                 const int t = key_tile(c, i), slot = t % V_STAGES;
-                if (!mbar_wait(bar(B_P_FULL + c), i & 1)) return false;
-                if (!mbar_wait(bar(B_V_FULL + slot), (t / V_STAGES) & 1)) return false;
+                if (!mbar_wait_warp(bar(B_P_FULL + c), i & 1)) return false;
+                if (!mbar_wait_warp(bar(B_V_FULL + slot), (t / V_STAGES) & 1)) return false;
                 tc_fence_after();
                 const uint32_t v_src = v_smem + slot * V_STAGE;
                 if (elect_one()) {
@@ -337,7 +337,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                 __syncwarp();
                 return true;
             };
-            if (!mbar_wait(bar(B_Q_FULL), 0)) timed_out = true;
+            if (!mbar_wait_warp(bar(B_Q_FULL), 0)) timed_out = true;
             for (int c = 0; c < chains && !timed_out; ++c)
                 if (n_steps[c] > 0 && !issue_s(c, 0)) timed_out = true;
             const int most = max(n_steps[0], n_steps[1]);
@@ -384,7 +384,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
         const int steps = n_steps[c];
         for (int i = 0; i < steps && !timed_out; ++i) {
             const int kbase = tile_base(key_tile(c, i));
-            if (!mbar_wait(bar(B_S_FULL + c), i & 1)) {
+            if (!mbar_wait_warp(bar(B_S_FULL + c), i & 1)) {
                 timed_out = true;
                 break;
             }
@@ -439,7 +439,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
                 const float cf = (grow && m_used != -INFINITY) ? fast_exp2(m_used - m_new) : 1.0f;
                 if (i > 0) {
                     // O must be at rest: the product of the step before has to be done
-                    if (!mbar_wait(bar(B_O_REST + c), (i - 1) & 1)) {
+                    if (!mbar_wait_warp(bar(B_O_REST + c), (i - 1) & 1)) {
                         timed_out = true;
                         break;
                     }
@@ -485,7 +485,7 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
             mbar_arrive(bar(B_P_FULL + c));
         }
         // the chain's last product (the products end in the order they were issued)
-        if (!timed_out && steps > 0 && !mbar_wait(bar(B_O_REST + c), (steps - 1) & 1))
+        if (!timed_out && steps > 0 && !mbar_wait_warp(bar(B_O_REST + c), (steps - 1) & 1))
             timed_out = true;
         tc_fence_after();
         if (P.two_tiles) {

@@ -206,7 +206,7 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
                 const Unit u = unit_of<NT>(i, m_tiles, start, p.n_experts, p.offsets);
                 const uint32_t idesc = umma_idesc((u.rows + 15) & ~15);
                 const int acc = it % L::ACCS;
-                if (!mbar_wait(acc_empty(acc), ((it / L::ACCS) & 1) ^ 1)) {
+                if (!mbar_wait_warp(acc_empty(acc), ((it / L::ACCS) & 1) ^ 1)) {
                     timed_out = true;
                     break;
                 }
@@ -214,7 +214,7 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
                 const uint32_t d = tmem_base + acc * (L::MATS * NT);
                 for (int kb = 0; kb < kblocks; ++kb, ++g) {
                     const int slot = g % L::STAGES;
-                    if (!mbar_wait(full(slot), (g / L::STAGES) & 1)) {
+                    if (!mbar_wait_warp(full(slot), (g / L::STAGES) & 1)) {
                         timed_out = true;
                         break;
                     }
@@ -244,7 +244,7 @@ expert_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap rows_map,
             const int acc = it % L::ACCS;
             const int n = u.n0 + q * 32 + lane;               // this thread's output
             const bool mine = n < p.N;
-            if (!mbar_wait(acc_full(acc), (it / L::ACCS) & 1)) {
+            if (!mbar_wait_warp(acc_full(acc), (it / L::ACCS) & 1)) {
                 timed_out = true;
                 break;
             }

@@ -200,7 +200,7 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                 for (int kb = u.from; kb < u.to; kb += 2, ++c) {
                     const int acc = c % ACCS, count = min(2, u.to - kb);
                     const uint32_t d = tmem_base + acc * NT;
-                    if (!mbar_wait(acc_empty(acc), ((c / ACCS) & 1) ^ 1)) timed_out = true;
+                    if (!mbar_wait_warp(acc_empty(acc), ((c / ACCS) & 1) ^ 1)) timed_out = true;
                     uint32_t w[2], rows[2];
                     int stage[2];
                     // part x of the weights times part y of the rows, of block b
@@ -213,7 +213,7 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         if (b >= count || timed_out) break;
-                        if (!mbar_wait(full(slot), turn) || !mbar_wait(w_full(g % W_BUFS), (g / W_BUFS) & 1)) {
+                        if (!mbar_wait_warp(full(slot), turn) || !mbar_wait_warp(w_full(g % W_BUFS), (g / W_BUFS) & 1)) {
                             timed_out = true;
                             break;
                         }
@@ -262,7 +262,7 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
             const Unit u = unit_of(p, i);
             for (int kb = u.from; kb < u.to; ++kb, ++g) {
                 const int buf = g % W_BUFS;
-                if (!mbar_wait(w_empty(buf), ((g / W_BUFS) & 1) ^ 1) || !mbar_wait(full(slot), turn)) {
+                if (!mbar_wait_warp(w_empty(buf), ((g / W_BUFS) & 1) ^ 1) || !mbar_wait_warp(full(slot), turn)) {
                     timed_out = true;
                     break;
                 }
@@ -312,7 +312,7 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                 const int k1 = min(k0 + p.group, u.to);
                 for (int kb = k0; kb < k1; kb += 2, ++c) {
                     const int acc = c % ACCS;
-                    if (!mbar_wait(acc_full(acc), (c / ACCS) & 1)) {
+                    if (!mbar_wait_warp(acc_full(acc), (c / ACCS) & 1)) {
                         timed_out = true;
                         break;
                     }

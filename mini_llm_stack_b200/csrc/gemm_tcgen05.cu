@@ -286,7 +286,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
                 const int z = tile / (m_tiles * n_tiles);
                 const int kb0 = z * per, n_kb = max(0, min(kblocks, kb0 + per) - kb0);
                 const int acc = it & 1;
-                if (!mbar_wait(acc_empty(acc), ((it >> 1) & 1) ^ 1)) {
+                if (!mbar_wait_warp(acc_empty(acc), ((it >> 1) & 1) ^ 1)) {
                     timed_out = true;
                     break;
                 }
@@ -294,7 +294,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
                 const uint32_t tmem_d = tmem_base + acc * BN;
                 for (int i = 0; i < n_kb; ++i, ++g) {
                     const int slot = g % STAGES;
-                    if (!mbar_wait(full(slot), (g / STAGES) & 1)) {
+                    if (!mbar_wait_warp(full(slot), (g / STAGES) & 1)) {
                         timed_out = true;
                         break;
                     }
@@ -323,7 +323,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
             const int ni = rest % n_tiles, z = rest / n_tiles;
             const int acc = it & 1;
             const int row = mi * BM + q * 32 + lane;
-            if (!mbar_wait(acc_full(acc), (it >> 1) & 1)) {
+            if (!mbar_wait_warp(acc_full(acc), (it >> 1) & 1)) {
                 timed_out = true;
                 break;
             }
@@ -515,7 +515,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             for (int unit = cluster; unit < unit_count && !timed_out; unit += clusters, ++it) {
                 const PairUnit w = pair_unit(p, unit, cut, kblocks);
                 const int acc = it & 1;
-                if (!mbar_wait_cluster(acc_empty(acc), ((it >> 1) & 1) ^ 1)) {
+                if (!mbar_wait_cluster_warp(acc_empty(acc), ((it >> 1) & 1) ^ 1)) {
                     timed_out = true;
                     break;
                 }
@@ -523,7 +523,7 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                 const uint32_t tmem_d = tmem_base + acc * BN;
                 for (int i = w.kb0; i < w.kb1; ++i, ++g) {
                     const int slot = g % STAGES;
-                    if (!mbar_wait_cluster(full(slot), (g / STAGES) & 1)) {
+                    if (!mbar_wait_cluster_warp(full(slot), (g / STAGES) & 1)) {
                         timed_out = true;
                         break;
                     }
@@ -559,10 +559,8 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
             const int acc = it & 1;
             const int row0 = mi * 2 * BM + (int)rank * BM;
             const int row = row0 + row_in;
-            if (!mbar_wait(acc_full(acc), (it >> 1) & 1)) {
-                timed_out = true;
-                break;
-            }
+            // (a warp whose wait runs out goes on without further ones: the others of its set meet it at theirs)
+            if (!timed_out && !mbar_wait_warp(acc_full(acc), (it >> 1) & 1)) timed_out = true;
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
             if (w.part >= 0) {

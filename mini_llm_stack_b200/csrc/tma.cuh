@@ -91,6 +91,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (global_ns() - t0 > 2000000000ull) return false;
     }
 }
+// The same for a whole warp: true in all of its lanes or in none.  Lanes' tries run out one by one; where a warp
+// leaves a loop by what a wait says and stays in it for instructions that all lanes execute together (elect.sync,
+// tcgen05.ld, votes), those would wait for the lanes that have left.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
 // ---- clusters: rank of this CTA, a barrier over all threads of the cluster, an arrival
 // on the barrier at the same shared-memory offset in another CTA of the cluster, and a
 // bounded wait that sees what such an arrival released.
@@ -137,6 +143,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity)
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (global_ns() - t0 > 2000000000ull) return false;
     }
+}
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity));
 }
 
 // One box of a 2-D tensor map into shared memory; completion is counted in bytes

@@ -32,3 +32,24 @@ def test_successors_start_behind_the_allocation(body):
     columns that the successor holds, and the successor for that kernel's end."""
     assert body.count("chain_release();") == 1
     assert re.search(r"if \(warp == \d\) \{\s*tmem_alloc(_pair)?\([^;]*;\s*chain_release\(\);\s*\}", body)
+
+
+def roles(body):
+    """The parts of a kernel that its warps take by their number."""
+    return re.split(r"(?=\n +(?:if \(warp |\} else if \(warp |\} else \{\n))", body)
+
+
+def waiting_roles():
+    return [pytest.param(role, id=f"{name}-{i}") for path in sorted(CSRC.glob("*.cu")) for name, body in kernels(path)
+            if "tmem_alloc" in body for i, role in enumerate(roles(body)) if re.search(r"mbar_wait\w*\(", role)]
+
+
+@pytest.mark.parametrize("role", waiting_roles())
+def test_lanes_leave_a_loop_together(role):
+    """Where a wait that runs out takes a warp out of a loop, all of its lanes go: those that stayed would wait for
+    the others at the next instruction that a whole warp executes."""
+    together = re.search(r"elect_one|tmem_ld|tmem_st|_sync\(0xffffffffu|__syncwarp", role)
+    leaves = re.search(r"\bbreak;|return false;|&& !timed_out;", role)
+    one_lane = "lane == 0) {\n" in role[:250]
+    if together and leaves and not one_lane:
+        assert not re.search(r"mbar_wait(_cluster)?\(", role), "a wait that each lane judges by itself"
