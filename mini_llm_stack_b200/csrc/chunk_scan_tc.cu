@@ -246,21 +246,22 @@ chunk_update_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Pa
                 if (elect_one()) {
                     constexpr uint32_t idesc = umma_idesc(64, 1);
                     uint32_t accumulate = 0;
-                    // part x of v times part y of k
-                    auto product = [&](int x, int y) {
+                    // part x of v times part y of k; the first of the next kind divides what is there
+                    auto product = [&](int x, int y, bool next_kind) {
                         for (int kk = 0; kk < blocks * (BK / UMMA_K); ++kk) {
-                            umma_ts(acc, A + (kk >> 1) * block_cols + x * (BK / 2) + (kk & 1) * (UMMA_K / 2),
-                                    umma_desc_mn(base + (tile * 3 + y) * TILE + kk * UMMA_K * 128, TILE), idesc,
-                                    accumulate);
+                            const uint32_t v = A + (kk >> 1) * block_cols + x * (BK / 2) + (kk & 1) * (UMMA_K / 2);
+                            const uint64_t k = umma_desc_mn(base + (tile * 3 + y) * TILE + kk * UMMA_K * 128, TILE);
+                            if (next_kind && kk == 0) umma_ts_onto<PART_SHIFT>(acc, v, k, idesc);
+                            else umma_ts(acc, v, k, idesc, accumulate);
                             accumulate = 1;
                         }
                     };
-                    if (!whole) product(1, 1);
-                    product(0, 2);
-                    if (!whole) product(2, 0);
-                    product(0, 1);
-                    if (!whole) product(1, 0);
-                    product(0, 0);
+                    if (!whole) product(1, 1, false);
+                    product(0, 2, false);
+                    if (!whole) product(2, 0, false);
+                    product(0, 1, true);
+                    if (!whole) product(1, 0, false);
+                    product(0, 0, true);
                     umma_commit(bar);
                 }
                 __syncwarp();
@@ -415,21 +416,26 @@ chunk_output_tc_kernel(const __grid_constant__ Args a, const Scratch s, const Pa
                     constexpr uint32_t idesc = umma_idesc(C);
                     const int k = b < s_blocks ? b : 2 * q_tiles + b - s_blocks;      // block of the rows' tiles
                     const uint32_t rows = base + (k >> 1) * 3 * TILE + (k & 1) * BK * 2;
-                    // part x of the state or v times part y of the tokens' rows
-                    auto product = [&](int x, int y, uint32_t accumulate) {
+                    // part x of the state or v times part y of the tokens' rows; the first of the next kind
+                    // divides what is there
+                    enum { FIRST, ONTO, NEXT_KIND };
+                    auto product = [&](int x, int y, int how) {
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                            umma_ts(acc, A + x * (BK / 2) + kk * (UMMA_K / 2),
-                                    umma_desc(rows + y * TILE + kk * UMMA_K * 2), idesc, kk ? 1u : accumulate);
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                            const uint32_t s = A + x * (BK / 2) + kk * (UMMA_K / 2);
+                            const uint64_t r = umma_desc(rows + y * TILE + kk * UMMA_K * 2);
+                            if (how == NEXT_KIND && kk == 0) umma_ts_onto<PART_SHIFT>(acc, s, r, idesc);
+                            else umma_ts(acc, s, r, idesc, how != FIRST || kk ? 1u : 0u);
+                        }
                     };
-                    product(0, 2, 0);
+                    product(0, 2, FIRST);
                     if (!whole) {
-                        product(1, 1, 1);
-                        product(2, 0, 1);
+                        product(1, 1, ONTO);
+                        product(2, 0, ONTO);
                     }
-                    product(0, 1, 1);
-                    if (!whole) product(1, 0, 1);
-                    product(0, 0, 1);
+                    product(0, 1, NEXT_KIND);
+                    if (!whole) product(1, 0, ONTO);
+                    product(0, 0, NEXT_KIND);
                     umma_commit(bar);
                 }
                 __syncwarp();

@@ -184,21 +184,24 @@ delta_chunk_prep_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
             for (int a32 = 0; a32 < 2 * to.e_tiles; ++a32) {
                 const int tile = a32 >> 1, k0 = 2 * (a32 & 1);
                 uint32_t accumulate = 0;
-                // part x of [q; k] times part y of k, 32 of e an accumulator
-                auto product = [&](int x, int y) {
+                // part x of [q; k] times part y of k, 32 of e an accumulator; the first of the next kind divides
+                // what is there
+                auto product = [&](int x, int y, bool next_kind) {
 #pragma unroll
                     for (int kk = k0; kk < k0 + 2; ++kk) {
-                        umma(tmem + a32 * C, umma_desc(base + (tile * 6 + x * 2) * TILE + kk * UMMA_K * 2),
-                             umma_desc(base + (tile * 6 + y * 2 + 1) * TILE + kk * UMMA_K * 2), idesc, accumulate);
+                        const uint64_t qk = umma_desc(base + (tile * 6 + x * 2) * TILE + kk * UMMA_K * 2),
+                                       k = umma_desc(base + (tile * 6 + y * 2 + 1) * TILE + kk * UMMA_K * 2);
+                        if (next_kind && kk == k0) umma_onto<PART_SHIFT>(tmem + a32 * C, qk, k, idesc);
+                        else umma(tmem + a32 * C, qk, k, idesc, accumulate);
                         accumulate = 1;
                     }
                 };
-                product(1, 1);
-                product(0, 2);
-                product(2, 0);
-                product(0, 1);
-                product(1, 0);
-                product(0, 0);
+                product(1, 1, false);
+                product(0, 2, false);
+                product(2, 0, false);
+                product(0, 1, true);
+                product(1, 0, false);
+                product(0, 0, true);
             }
             umma_commit(bar);
         }
@@ -441,20 +444,21 @@ delta_chunk_scan_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
         // 16, the small products first
         auto multiply = [&](uint32_t d, uint32_t A, int apart, uint32_t B, uint32_t idesc, int k0, int k1, bool mn) {
             uint32_t accumulate = 0;
-            auto product = [&](int x, int y) {
+            auto product = [&](int x, int y, bool next_kind) {      // (its first divides what is there)
                 for (int kk = k0; kk < k1; ++kk) {
                     const uint64_t desc = mn ? umma_desc_mn(B + y * TILE + kk * UMMA_K * 128, 3 * TILE)
                                              : umma_desc(B + ((kk >> 2) * 3 + y) * TILE + (kk & 3) * 32);
-                    umma_ts(d, A + x * apart + kk * 8, desc, idesc, accumulate);
+                    if (next_kind && kk == k0) umma_ts_onto<PART_SHIFT>(d, A + x * apart + kk * 8, desc, idesc);
+                    else umma_ts(d, A + x * apart + kk * 8, desc, idesc, accumulate);
                     accumulate = 1;
                 }
             };
-            product(1, 1);
-            product(0, 2);
-            product(2, 0);
-            product(0, 1);
-            product(1, 0);
-            product(0, 0);
+            product(1, 1, false);
+            product(0, 2, false);
+            product(2, 0, false);
+            product(0, 1, true);
+            product(1, 0, false);
+            product(0, 0, true);
         };
         constexpr uint32_t id = umma_idesc(C), id_mn = umma_idesc(ER, 1);
         for (int c = 0; c < w.chunks; ++c) {

@@ -2,7 +2,7 @@
 // out[M, N] = A[M, K] * W[N, K]^T, both operands float32 (A may be bfloat16).
 //
 // Every operand is the sum of three bfloat16 (8 + 8 + 8 bits of the 24 that a float32 has; the
-// second and third round what the ones before left), and of the nine products of such parts the
+// second and third round what the ones before left; bf16_parts.cuh), and of the nine products of such parts the
 // six that reach 2^-24 of the whole are added up:
 //
 //     a w ~ a1 w1 + (a1 w2 + a2 w1) + (a2 w2 + a1 w3 + a3 w1)
@@ -203,12 +203,17 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                     if (!mbar_wait_warp(acc_empty(acc), ((c / ACCS) & 1) ^ 1)) timed_out = true;
                     uint32_t w[2], rows[2];
                     int stage[2];
-                    // part x of the weights times part y of the rows, of block b
-                    auto product = [&](int b, int x, int y, uint32_t accumulate) {
+                    // part x of the weights times part y of the rows, of block b: onto nothing, onto what the
+                    // accumulator holds, or onto that divided by 2^PART_SHIFT
+                    enum { FIRST, ONTO, NEXT_KIND };
+                    auto product = [&](int b, int x, int y, int how) {
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                            umma_ts(d, w[b] + x * (BK / 2) + kk * (UMMA_K / 2),
-                                    rows_desc(rows[b] + y * part + kk * UMMA_K * 2), idesc, kk ? 1u : accumulate);
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                            const uint32_t a = w[b] + x * (BK / 2) + kk * (UMMA_K / 2);
+                            const uint64_t r = rows_desc(rows[b] + y * part + kk * UMMA_K * 2);
+                            if (how == NEXT_KIND && kk == 0) umma_ts_onto<PART_SHIFT>(d, a, r, idesc);
+                            else umma_ts(d, a, r, idesc, how != FIRST || kk ? 1u : 0u);
+                        }
                     };
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
@@ -223,25 +228,29 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                         rows[b] = base + slot * p.stage_bytes + W_BYTES;
                         if (elect_one()) {
                             if (p.parts == 3) {
-                                product(b, 1, 1, b);
-                                product(b, 0, 2, 1);
-                                product(b, 2, 0, 1);
-                                product(b, 0, 1, 1);
+                                product(b, 1, 1, b ? ONTO : FIRST);
+                                product(b, 0, 2, ONTO);
+                                product(b, 2, 0, ONTO);
                             } else {
-                                product(b, 2, 0, b);
+                                product(b, 2, 0, b ? ONTO : FIRST);
                             }
-                            product(b, 1, 0, 1);
                         }
                         ++g;
                         if (++slot == p.stages) slot = 0, turn ^= 1;
                     }
                     if (timed_out) break;
                     if (elect_one()) {
-                        product(0, 0, 0, 1);
+                        product(0, 1, 0, NEXT_KIND);
+                        if (p.parts == 3) product(0, 0, 1, ONTO);
+                        if (count == 2) {
+                            product(1, 1, 0, ONTO);
+                            if (p.parts == 3) product(1, 0, 1, ONTO);
+                        }
+                        product(0, 0, 0, NEXT_KIND);
                         umma_commit(empty(stage[0]));
                         umma_commit(w_empty((g - count) % W_BUFS));
                         if (count == 2) {
-                            product(1, 0, 0, 1);
+                            product(1, 0, 0, ONTO);
                             umma_commit(empty(stage[1]));
                             umma_commit(w_empty((g - 1) % W_BUFS));
                         }

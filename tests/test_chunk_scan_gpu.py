@@ -378,3 +378,25 @@ def test_no_number_reaches_earlier_tokens_or_other_requests(ops, always, kind, w
 def test_wide_heads_on_tensor_cores(ops, always, e, f, heads, kind):
     """Heads of one, two and four groups of 128 columns a block, with remainders of 64 rows and of 128 columns."""
     test_linear_scan(ops, always, [130, 1, 7, 128], e, f, heads, kind)
+
+
+def test_small_values_keep_their_bits(ops, always):
+    """Values (and so the state) whose lower bfloat16 parts lie below bfloat16's smallest number: the outputs
+    are those of ordinary values times a power of two."""
+    heads, e, f, lens = 2, 128, 256, [130, 64]
+    g = torch.Generator().manual_seed(11)
+    t = sum(lens)
+    q, k = (torch.randn(t, heads * e, generator=g).cuda() for _ in range(2))
+    v = torch.randn(t, heads * f, generator=g).cuda()
+    decay = torch.tensor([0.97, 0.6]).cuda()
+    outs, states = [], []
+    for power in (0, -116):
+        step, _, _ = a_step(lens, True)
+        state, out = torch.zeros(2, heads * e * f, device="cuda"), torch.empty(t, heads * f, device="cuda")
+        ops.linear_scan((q, 0), (k, 0), (torch.ldexp(v, torch.tensor(power)), 0), state, step, heads, e, f, out,
+                        decay_head=decay)
+        for to, x in ((outs, out), (states, state)):
+            to.append(torch.ldexp(x.double(), torch.tensor(-power)))
+    # (float32's smallest, 2^-149, is 2^-33 of the values)
+    assert (outs[1] - outs[0]).norm() <= 2.0 ** -23 * outs[0].norm()
+    assert (states[1] - states[0]).norm() <= 2.0 ** -23 * states[0].norm()

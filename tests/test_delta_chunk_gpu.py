@@ -96,3 +96,25 @@ def test_no_number_reaches_earlier_tokens_or_columns(ops, what, odd):
     tokens, _ = walk(ops, case, [(0, 0, 200)], [0], case.new_state(ops, 1), chunked=False)
     assert torch.equal(got[:bad], clean[:bad])
     assert torch.equal(got.isfinite(), tokens.isfinite())
+
+
+def test_small_values_keep_their_bits(ops):
+    """Values (and so R, U and the state) whose lower bfloat16 parts lie below bfloat16's smallest number: the
+    outputs are those of ordinary values times a power of two."""
+    nh, nk, e, f = sizes = (2, 1, 128, 128)
+    case, t = DeltaCase(*sizes, 4, (200,), seed=9), 200
+    step = fake_step([t], [0], [0])
+    p, state = case.rows_of([(0, 0, t)]), case.new_state(ops, 1)
+    rows = torch.zeros(t, ops.delta_rows(*sizes), device="cuda")
+    ops.delta_prep(p, case.cols, case.dev["conv"], case.taps, case.dev["a_exp"], case.dev["dt"], state, step, nh, nk, e, f,
+                   rows)
+    v_at = t * nk * 2 * e                                # (delta_rule.h: q and k, then the values)
+    got = []
+    for power in (0, -116):
+        small, state = rows.clone(), case.new_state(ops, 1)
+        small.view(-1)[v_at:v_at + t * nh * f] *= 2.0 ** power
+        out = torch.empty(t, nh * f, device="cuda")
+        ops.delta_scan(small, p, case.cols[0], case.taps, state, step, nh, nk, e, f, out)
+        got.append([torch.ldexp(x.double(), torch.tensor(-power)) for x in (out, state[:, :nh * e * f])])
+    for small, plain in zip(got[1], got[0]):
+        assert (small - plain).norm() <= 2.0 ** -22 * plain.norm()

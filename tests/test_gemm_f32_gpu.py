@@ -99,3 +99,24 @@ def test_odd_values_on_tensor_cores(ops, m):
     sure[1:] = False
     assert (out[sure] == torch.where(a[0, 5] * w[:, 5] > 0, float("inf"), float("-inf")).expand(m, n)[sure]).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m", [3, 200])
+@pytest.mark.parametrize("power_a, power_w", [(-112, 100), (-120, 100), (-138, 120), (100, -112), (100, -120), (120, -140),
+                                              (-60, -62), (60, 62)])
+def test_small_operands_on_tensor_cores(ops, a_type, m, power_a, power_w):
+    """Operands whose lower parts lie below bfloat16's smallest number, down to float32's own smallest, against large
+    ones (the products are ordinary numbers): all 24 bits count."""
+    n, k = 300, 2048
+    g = torch.Generator(device="cuda").manual_seed(m + power_a)
+    a = torch.ldexp(torch.randn(m, k, device="cuda", generator=g), torch.tensor(power_a)).to(a_type)
+    w = torch.ldexp(torch.randn(n, k, device="cuda", generator=g), torch.tensor(power_w))
+    assert a.any() and w.any()
+    out = torch.empty(m, n, device="cuda")
+    ops.linear(a, w, out)
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # as in test_product_on_tensor_cores: 4 steps a 64 of k of 2^-23, k / 64 / 8 and 8 of 2^-24
+    assert ((out.double() - want).abs() <= 2.0 ** -24 * (2 + 8 + k / 512 + 8) * size).all()
+    assert (out.double() - want).norm() <= 2e-7 * want.norm()
+    ops.check_status()
