@@ -301,12 +301,12 @@ class Ops:
             _need(a.dtype in (torch.float32, torch.bfloat16), f"linear: input dtype {a.dtype}")
             o32 = out if out.dtype == torch.float32 else torch.empty(
                 (m, n), dtype=torch.float32, device=out.device)
-            # rows as bfloat16 parts, and sums of a product cut along K
-            floats = self._gemm_f32_scratch(_ptr(a), _code(a.dtype), _ptr(w), m, n, k)
-            held = self.scratch("gemm_f32", floats) if floats else None
-            self.launches += 1
-            _check(self._gemm_f32(_ptr(a), _code(a.dtype), _ptr(w), _ptr(o32), m, n, k, _ptr(held),
-                                  _ptr(self.status), self._stream()), "gemm_f32")
+            rows, held = self._f32_rows(a, w, m, n, k)
+            for at in range(0, m, rows):
+                some, to = (a, o32) if rows >= m else (a[at:at + rows], o32[at:at + rows])
+                self.launches += 1
+                _check(self._gemm_f32(_ptr(some), _code(a.dtype), _ptr(w), _ptr(to), some.shape[0], n, k, _ptr(held),
+                                      _ptr(self.status), self._stream()), "gemm_f32")
             if o32 is not out:
                 out.copy_(o32)
             return
@@ -323,6 +323,36 @@ class Ops:
             torch.mm(a16, held[1], out_dtype=torch.float32, out=out)
         else:
             torch.mm(a16, held[1], out=out)
+
+    F32_SCRATCH = 1 << 26         # floats that a float32 product may take (fewer once memory ran out)
+
+    def _f32_rows(self, a, w, m: int, n: int, k: int):
+        """How many rows a float32 product takes at a time (a row's bits do not depend on the others), and its
+        scratch: the rows as bfloat16 parts, and the sums of a product cut along K.  All rows as long as that
+        is at most ``F32_SCRATCH`` and there is memory for it."""
+        def floats_of(rows):
+            return max(self._gemm_f32_scratch(_ptr(a), _code(a.dtype), _ptr(w), r, n, k)
+                       for r in {rows, m % rows or rows})
+
+        rows = m
+        while True:
+            floats = floats_of(rows)
+            if not floats:
+                return rows, None
+            if floats > self.F32_SCRATCH and rows > 16:
+                rows = -(-rows // 32) * 16
+                continue
+            held = self._scratch.get("gemm_f32")
+            if held is not None and held.numel() >= floats:
+                return rows, held
+            try:
+                # (a power of two: scratch that grows drops the captured graphs)
+                return rows, self.scratch("gemm_f32", max(floats, min(1 << (floats - 1).bit_length(), self.F32_SCRATCH)))
+            except torch.cuda.OutOfMemoryError:
+                if rows <= 16:
+                    raise
+                # fewer rows at a time, from now on: as many as what there is already holds, or half as much
+                self.F32_SCRATCH = max(held.numel() if held is not None else 0, floats // 2)
 
     def _use_own_gemm(self, m: int, n: int, k: int) -> bool:
         """The tcgen05 kernel takes rows that are whole 16-byte chunks; the choice

@@ -120,3 +120,37 @@ def test_small_operands_on_tensor_cores(ops, a_type, m, power_a, power_w):
     assert ((out.double() - want).abs() <= 2.0 ** -24 * (2 + 8 + k / 512 + 8) * size).all()
     assert (out.double() - want).norm() <= 2e-7 * want.norm()
     ops.check_status()
+
+
+@pytest.mark.parametrize("a_type, m, n, k", [(torch.float32, 700, 300, 2048), (torch.bfloat16, 333, 300, 2052),
+                                             (torch.float32, 40, 2048, 8192)])
+def test_scratch_has_a_bound_and_memory_may_run_out(ops, monkeypatch, a_type, m, n, k):
+    """Rows in parts give the same bits: by the bound, and after the allocator has refused what the whole takes."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k, device="cuda", generator=g).to(a_type)
+    w = torch.randn(n, k, device="cuda", generator=g)
+    whole, out = torch.empty(m, n, device="cuda"), torch.full((m, n), float("nan"), device="cuda")
+    monkeypatch.setattr(ops, "_scratch", {})
+    ops.linear(a, w, whole)
+    most = ops._scratch["gemm_f32"].numel()
+    assert most & (most - 1) == 0                         # grows by powers of two
+    # a bound
+    limit = most // 8
+    monkeypatch.setattr(ops, "F32_SCRATCH", limit, raising=False)
+    monkeypatch.setattr(ops, "_scratch", {})
+    ops.linear(a, w, out)
+    assert torch.equal(out, whole) and ops._scratch["gemm_f32"].numel() <= max(limit, 1 << 16)
+    # an allocator that has less than the whole takes
+    monkeypatch.setattr(ops, "F32_SCRATCH", 1 << 26, raising=False)
+    monkeypatch.setattr(ops, "_scratch", {})
+    real = ops.scratch
+
+    def scratch(tag, floats):
+        if floats > limit:
+            raise torch.cuda.OutOfMemoryError("none left")
+        return real(tag, floats)
+    monkeypatch.setattr(ops, "scratch", scratch)
+    out.fill_(float("nan"))
+    ops.linear(a, w, out)
+    assert torch.equal(out, whole) and ops.F32_SCRATCH < most
+    ops.check_status()
