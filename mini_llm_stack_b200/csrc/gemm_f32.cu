@@ -501,6 +501,12 @@ MLS_API int mls_gemm_f32(const void* A, int a_dtype, const float* W, float* out,
     return MLS_ERR_UNSUPPORTED;
 }
 
+// Kernels that such a call launches.
+MLS_API int mls_gemm_f32_launches(const void* A, int a_dtype, const float* W, int M, int N, int K) {
+    if (M <= 0 || N <= 0) return 0;
+    return takes_tc(a_dtype, W, N, K) ? tc_launches(A, a_dtype, M, N, K) : 1;
+}
+
 MLS_API long long mls_gemm_f32_scratch_floats(const void* A, int a_dtype, const float* W, int M, int N, int K) {
     return M > 0 && takes_tc(a_dtype, W, N, K) ? tc_scratch_floats(A, a_dtype, M, N, K) : 0;
 }

@@ -28,6 +28,7 @@ constexpr int CHAIN_K0 = 4096, CHAIN_K1 = 8192;
 // bits do not depend on the rows it is computed with.
 bool takes_tc(int a_dtype, const float* W, int N, int K);
 long long tc_scratch_floats(const void* A, int a_dtype, int M, int N, int K);
+int tc_launches(const void* A, int a_dtype, int M, int N, int K);
 int product_tc(const void* A, int a_dtype, const float* W, float* out, int M, int N, int K, float* scratch,
                int* status, cudaStream_t stream);
 }  // namespace mls_f32

@@ -531,6 +531,10 @@ long long tc_scratch_floats(const void* A, int a_dtype, int M, int N, int K) {
     return parts_floats(A, a_dtype, M, K) + (c.cut ? (long long)c.groups * M * N : 0);
 }
 
+int tc_launches(const void* A, int a_dtype, int M, int N, int K) {
+    return 1 + (rows_are_their_part(A, a_dtype, K) ? 0 : 1) + cut_of(M, N, K).cut;
+}
+
 int product_tc(const void* A, int a_dtype, const float* W, float* out, int M, int N, int K, float* scratch,
                int* status, cudaStream_t stream) {
     const Cut c = cut_of(M, N, K);

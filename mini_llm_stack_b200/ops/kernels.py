@@ -131,6 +131,7 @@ class Ops:
         self._gemm_f32 = _decl(core, "mls_gemm_f32", [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P])
         self._gemm_f32_scratch = _decl(core, "mls_gemm_f32_scratch_floats",
                                        [_P, _I, _P, _I, _I, _I], restype=ctypes.c_longlong)
+        self._gemm_f32_launches = _decl(core, "mls_gemm_f32_launches", [_P, _I, _P, _I, _I, _I])
         self._rope_store = _decl(core, "mls_rope_store",
                                  [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                                   _LL, _I, _P, _I, _LL, _P, _P])
@@ -304,7 +305,9 @@ class Ops:
             rows, held = self._f32_rows(a, w, m, n, k)
             for at in range(0, m, rows):
                 some, to = (a, o32) if rows >= m else (a[at:at + rows], o32[at:at + rows])
-                self.launches += 1
+                # (with scratch its rows are split first, or its groups' sums added up behind, or both)
+                self.launches += 1 if held is None else self._gemm_f32_launches(
+                    _ptr(some), _code(a.dtype), _ptr(w), some.shape[0], n, k)
                 _check(self._gemm_f32(_ptr(some), _code(a.dtype), _ptr(w), _ptr(to), some.shape[0], n, k, _ptr(held),
                                       _ptr(self.status), self._stream()), "gemm_f32")
             if o32 is not out:

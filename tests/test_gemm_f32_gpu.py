@@ -154,3 +154,22 @@ def test_scratch_has_a_bound_and_memory_may_run_out(ops, monkeypatch, a_type, m,
     ops.linear(a, w, out)
     assert torch.equal(out, whole) and ops.F32_SCRATCH < most
     ops.check_status()
+
+
+@pytest.mark.parametrize("a_type, m, n, k, count", [
+    (torch.float32, 700, 3000, 2048, 2),       # rows split, product
+    (torch.float32, 1, 2048, 2048, 3),         # and sums of the groups of a cut product
+    (torch.bfloat16, 1, 64, 4096, 2),          # rows that are their own part
+    (torch.bfloat16, 3000, 4000, 2048, 1),
+    (torch.float32, 5, 300, 64, 1)])           # CUDA cores
+def test_launches_are_counted(ops, a_type, m, n, k, count):
+    """As many as a captured call has nodes."""
+    from cuda.bindings import runtime
+    a = torch.ones(m, k, device="cuda", dtype=a_type)
+    w, out = torch.ones(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+    ops.linear(a, w, out)
+    before, graph = ops.launches, torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        ops.linear(a, w, out)
+    error, _, nodes = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
+    assert int(error) == 0 and ops.launches - before == count == nodes
