@@ -347,12 +347,15 @@ template <int UNIT, int NT>
 int launch_nt(const TcParams& p, const void* rows, const void* W, int n_slots, cudaStream_t stream) {
     using L = Plan<UNIT, NT>;
     const int smem = L::FIXED + 4 * (p.n_experts + 1);
-    static int configured = 0;
-    if (configured < smem) {
+    static bool configured = false;
+    if (!configured) {
+        // (one limit for all tables: with each product's own, a thread with a smaller table could lower what
+        // another had just raised)
         const cudaError_t e = cudaFuncSetAttribute(expert_tc_kernel<UNIT, NT>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   L::FIXED + 4 * (TC_EXPERTS + 1));
         if (e != cudaSuccess) return (int)e;
-        configured = smem;
+        configured = true;
     }
     CUtensorMap rows_map, w_map;
     if (!operand_map(rows, n_slots, p.K, L::BOX, &rows_map) ||

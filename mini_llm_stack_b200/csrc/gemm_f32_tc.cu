@@ -503,12 +503,14 @@ long long parts_floats(const void* A, int a_dtype, int M, int K) {
 template <int NT>
 int launch_nt(const TcParams& p, const CUtensorMap& rows_map, const CUtensorMap& w_map, cudaStream_t stream) {
     const int smem = p.stages * p.stage_bytes + 1024;
-    static int configured = 0;
-    if (configured < smem) {
+    static bool configured = false;
+    if (!configured) {
+        // (one limit for all rings: with each product's own, a thread with a smaller ring could lower what
+        // another had just raised)
         const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<NT>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024);
         if (e != cudaSuccess) return (int)e;
-        configured = smem;
+        configured = true;
     }
     const long long units = (long long)(p.N + UMMA_M - 1) / UMMA_M * p.m_tiles * (p.cut ? p.groups : 1);
     const int grid = (int)(units < sm_count() ? units : sm_count());

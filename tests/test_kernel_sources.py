@@ -53,3 +53,10 @@ def test_lanes_leave_a_loop_together(role):
     one_lane = "lane == 0) {\n" in role[:250]
     if together and leaves and not one_lane:
         assert not re.search(r"mbar_wait(_cluster)?\(", role), "a wait that each lane judges by itself"
+
+
+@pytest.mark.parametrize("path", sorted(CSRC.glob("*.cu")), ids=lambda p: p.stem)
+def test_shared_memory_limits_never_fall(path):
+    """A launcher that remembers what limit it set a kernel sets one and the same each time: with a limit for every
+    launch, two threads could leave the lower one behind and the memory of the higher."""
+    assert not re.search(r"static int \w*configured", path.read_text())
