@@ -393,10 +393,10 @@ def test_small_values_keep_their_bits(ops, always):
     for power in (0, -116):
         step, _, _ = a_step(lens, True)
         state, out = torch.zeros(2, heads * e * f, device="cuda"), torch.empty(t, heads * f, device="cuda")
-        ops.linear_scan((q, 0), (k, 0), (torch.ldexp(v, torch.tensor(power)), 0), state, step, heads, e, f, out,
+        ops.linear_scan((q, 0), (k, 0), (v * 2.0 ** power, 0), state, step, heads, e, f, out,
                         decay_head=decay)
         for to, x in ((outs, out), (states, state)):
-            to.append(torch.ldexp(x.double(), torch.tensor(-power)))
+            to.append(x.double() * 2.0 ** -power)
     # (float32's smallest, 2^-149, is 2^-33 of the values)
     assert (outs[1] - outs[0]).norm() <= 2.0 ** -23 * outs[0].norm()
     assert (states[1] - states[0]).norm() <= 2.0 ** -23 * states[0].norm()

@@ -110,8 +110,8 @@ def test_small_operands_on_tensor_cores(ops, a_type, m, power_a, power_w):
     ones (the products are ordinary numbers): all 24 bits count."""
     n, k = 300, 2048
     g = torch.Generator(device="cuda").manual_seed(m + power_a)
-    a = torch.ldexp(torch.randn(m, k, device="cuda", generator=g), torch.tensor(power_a)).to(a_type)
-    w = torch.ldexp(torch.randn(n, k, device="cuda", generator=g), torch.tensor(power_w))
+    a = (torch.randn(m, k, device="cuda", generator=g) * 2.0 ** power_a).to(a_type)
+    w = torch.randn(n, k, device="cuda", generator=g) * 2.0 ** power_w
     assert a.any() and w.any()
     out = torch.empty(m, n, device="cuda")
     ops.linear(a, w, out)
