@@ -45,8 +45,8 @@ __device__ __forceinline__ void put_parts(uint8_t* tiles, int r, int x, float4 v
 #pragma unroll
     for (int y = 0; y < 3; ++y) {
         uint2 two;
-        two.x = bf16_part(v.x, v.y);
-        two.y = bf16_part(v.z, v.w);
+        two.x = bf16_part_up(v.x, v.y);
+        two.y = bf16_part_up(v.z, v.w);
         *reinterpret_cast<uint2*>(at + y * TILE) = two;
     }
 }
@@ -109,7 +109,7 @@ __device__ __forceinline__ void put_lane(uint32_t taddr, float (&v)[BK], bool wh
             if (y && whole) break;
             uint32_t two[8];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) two[x] = bf16_part(v[16 * h + 2 * x], v[16 * h + 2 * x + 1]);
+            for (int x = 0; x < 8; ++x) two[x] = bf16_part_up(v[16 * h + 2 * x], v[16 * h + 2 * x + 1]);
             tmem_st8(taddr + y * (BK / 2) + h * 8, two);
         }
 }

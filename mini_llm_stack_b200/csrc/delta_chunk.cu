@@ -80,8 +80,8 @@ struct Place {
 __device__ __forceinline__ int swizzled(int r, int x) { return r * 128 + (((x >> 3) ^ (r & 7)) << 4) + (x & 7) * 2; }
 __device__ __forceinline__ uint2 part4(float4& v) {
     uint2 two;
-    two.x = bf16_part(v.x, v.y);
-    two.y = bf16_part(v.z, v.w);
+    two.x = bf16_part_up(v.x, v.y);
+    two.y = bf16_part_up(v.z, v.w);
     return two;
 }
 // exp(d) for a float64 d <= 0: of the nearest float32, times one plus what that leaves.
@@ -556,7 +556,7 @@ delta_chunk_scan_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
             for (int y = 0; y < 3; ++y) {
                 uint32_t two[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) two[i] = bf16_part(x[2 * i], x[2 * i + 1]);
+                for (int i = 0; i < 8; ++i) two[i] = bf16_part_up(x[2 * i], x[2 * i + 1]);
                 tmem_st8(at + lanes + y * apart, two);
             }
         };

@@ -2,7 +2,7 @@
 // out[M, N] = A[M, K] * W[N, K]^T, both operands float32 (A may be bfloat16).
 //
 // Every operand is the sum of three bfloat16 (8 + 8 + 8 bits of the 24 that a float32 has; the
-// second and third round what the ones before left; bf16_parts.cuh), and of the nine products of such parts the
+// second and third round what the ones before left), and of the nine products of such parts the
 // six that reach 2^-24 of the whole are added up:
 //
 //     a w ~ a1 w1 + (a1 w2 + a2 w1) + (a2 w2 + a1 w3 + a3 w1)
@@ -14,8 +14,10 @@
 // computed with, and whether a CTA walks all of K or one group (few rows), whose sum it then leaves to
 // gemm_f32_parts_kernel.  Distance from float64 (2-norm over 2-norm, normal values) against one chain of fmaf
 // over K: 0.92e-7 / 4.1e-7 at 512, 1.04e-7 / 8.1e-7 at 2,048, 1.23e-7 / 16.2e-7 at 8,192.
-// A sum that is not finite (an operand that is infinite, not a number or beyond bfloat16's largest
-// value, or a sum beyond float32's) is computed again as that chain.
+// Float32 operands are multiplied by 2^16 before they are split (bf16_parts.cuh says why), and the sums by what takes
+// that back out, which rounds nothing but what becomes smaller than float32's normal numbers (2^-149 at most).
+// A sum that is not finite (an operand that is infinite, not a number or 2^112 and more, or a sum of 2^96 and more)
+// is computed again as that chain.
 //
 // The weights take the 128-row side of the instruction: tiles of 128 x 32 come by TMA, a thread a row
 // splits them in registers and puts the parts into tensor memory, from where the instruction reads
@@ -55,6 +57,7 @@ constexpr int THREADS = 512;
 constexpr int SUM_WARPS = 8, SPLIT_WARPS = 4;
 constexpr int W_COLS = 3 * BK / 2, W_BUFS = 4;        // tensor memory of a block's parts; such blocks
 constexpr int GROUPS = 16, GROUP_MIN = 128;
+constexpr float UP = 65536.f;                         // of float32 operands
 constexpr int MAX_STAGES = 12, RING_BYTES = 200 * 1024;
 
 struct TcParams {
@@ -66,6 +69,7 @@ struct TcParams {
     int blocks, group, groups;     // blocks of K, blocks of a group, groups
     int cut;                       // a unit is one group of a tile
     int parts;                     // of a row's values: three, or the one that a bfloat16 is
+    float down;                    // takes the operands' UP out of a sum
     int stages, stage_bytes;
     int* status;
 };
@@ -203,17 +207,12 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                     if (!mbar_wait_warp(acc_empty(acc), ((c / ACCS) & 1) ^ 1)) timed_out = true;
                     uint32_t w[2], rows[2];
                     int stage[2];
-                    // part x of the weights times part y of the rows, of block b: onto nothing, onto what the
-                    // accumulator holds, or onto that divided by 2^PART_SHIFT
-                    enum { FIRST, ONTO, NEXT_KIND };
-                    auto product = [&](int b, int x, int y, int how) {
+                    // part x of the weights times part y of the rows, of block b
+                    auto product = [&](int b, int x, int y, uint32_t accumulate) {
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                            const uint32_t a = w[b] + x * (BK / 2) + kk * (UMMA_K / 2);
-                            const uint64_t r = rows_desc(rows[b] + y * part + kk * UMMA_K * 2);
-                            if (how == NEXT_KIND && kk == 0) umma_ts_onto<PART_SHIFT>(d, a, r, idesc);
-                            else umma_ts(d, a, r, idesc, how != FIRST || kk ? 1u : 0u);
-                        }
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            umma_ts(d, w[b] + x * (BK / 2) + kk * (UMMA_K / 2),
+                                    rows_desc(rows[b] + y * part + kk * UMMA_K * 2), idesc, kk ? 1u : accumulate);
                     };
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
@@ -228,29 +227,25 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                         rows[b] = base + slot * p.stage_bytes + W_BYTES;
                         if (elect_one()) {
                             if (p.parts == 3) {
-                                product(b, 1, 1, b ? ONTO : FIRST);
-                                product(b, 0, 2, ONTO);
-                                product(b, 2, 0, ONTO);
+                                product(b, 1, 1, b);
+                                product(b, 0, 2, 1);
+                                product(b, 2, 0, 1);
+                                product(b, 0, 1, 1);
                             } else {
-                                product(b, 2, 0, b ? ONTO : FIRST);
+                                product(b, 2, 0, b);
                             }
+                            product(b, 1, 0, 1);
                         }
                         ++g;
                         if (++slot == p.stages) slot = 0, turn ^= 1;
                     }
                     if (timed_out) break;
                     if (elect_one()) {
-                        product(0, 1, 0, NEXT_KIND);
-                        if (p.parts == 3) product(0, 0, 1, ONTO);
-                        if (count == 2) {
-                            product(1, 1, 0, ONTO);
-                            if (p.parts == 3) product(1, 0, 1, ONTO);
-                        }
-                        product(0, 0, 0, NEXT_KIND);
+                        product(0, 0, 0, 1);
                         umma_commit(empty(stage[0]));
                         umma_commit(w_empty((g - count) % W_BUFS));
                         if (count == 2) {
-                            product(1, 0, 0, ONTO);
+                            product(1, 0, 0, 1);
                             umma_commit(empty(stage[1]));
                             umma_commit(w_empty((g - 1) % W_BUFS));
                         }
@@ -278,19 +273,20 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                 tc_fence_after();
                 const uint32_t w = tmem_base + ACCS * NT + buf * W_COLS + lanes;
                 const uint32_t src = base + slot * p.stage_bytes + row * (BK * 4);
+                unsigned long long v[16];                 // two values each: all loads first
+#pragma unroll
+                for (int x = 0; x < 8; ++x)              // 16 bytes x of the row, where the swizzle put them
+                    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[2 * x]), "=l"(v[2 * x + 1])
+                                 : "r"(src + ((x ^ (row & 7)) << 4)) : "memory");
+#pragma unroll
+                for (int x = 0; x < 16; ++x) v[x] = both_times(v[x], UP);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    float v[16];
-#pragma unroll
-                    for (int x = 0; x < 4; ++x)          // 16 bytes x of the row, where the swizzle put them
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                     : "=f"(v[4 * x]), "=f"(v[4 * x + 1]), "=f"(v[4 * x + 2]), "=f"(v[4 * x + 3])
-                                     : "r"(src + (((4 * h + x) ^ (row & 7)) << 4)) : "memory");
 #pragma unroll
                     for (int y = 0; y < 3; ++y) {
                         uint32_t two[8];
 #pragma unroll
-                        for (int x = 0; x < 8; ++x) two[x] = bf16_part(v[2 * x], v[2 * x + 1]);
+                        for (int x = 0; x < 8; ++x) two[x] = bf16_part(v[8 * h + x]);
                         tmem_st8(w + y * (BK / 2) + h * 8, two);
                     }
                 }
@@ -358,7 +354,7 @@ gemm_f32_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ C
                     const int m = half * 16 + 32 * r + x;
                     if (m >= rows) break;
                     float v = all[r][x];
-                    if (!p.cut && !finite(v)) v = chain_of(p, u.m0 + m, n);
+                    if (!p.cut) v = finite(v) ? v * p.down : chain_of(p, u.m0 + m, n);
                     out[(size_t)m * p.N] = v;
                 }
         }
@@ -384,8 +380,7 @@ gemm_f32_parts_kernel(const __grid_constant__ TcParams p, const float* __restric
 #pragma unroll
     for (int g = 0; g < GROUPS; ++g)
         if (g < p.groups) s += v[g];
-    if (!finite(s)) s = chain_of(p, (int)(i / p.N), (int)(i % p.N));
-    out[i] = s;
+    out[i] = finite(s) ? s * p.down : chain_of(p, (int)(i / p.N), (int)(i % p.N));
 }
 
 // The three parts of a float32 matrix (the one of a bfloat16 one): [parts, M, width] bfloat16, zeros past K.
@@ -408,15 +403,21 @@ split_rows_kernel(const T* __restrict__ A, int M, int K, int width, __nv_bfloat1
 #pragma unroll
         for (int x = 0; x < 8; ++x) v[x] = k + x < K ? Elem<T>::load(src + x) : 0.f;
     }
+    unsigned long long two[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        two[x] = beside(__float_as_uint(v[2 * x]), __float_as_uint(v[2 * x + 1]));
+        if (sizeof(T) == 4) two[x] = both_times(two[x], UP);
+    }
     uint4* dst = reinterpret_cast<uint4*>(parts + (size_t)m * width + k);
     const size_t apart = (size_t)M * per;
 #pragma unroll
     for (int y = 0; y < (sizeof(T) == 4 ? 3 : 1); ++y) {
         uint4 out;
-        out.x = bf16_part(v[0], v[1]);
-        out.y = bf16_part(v[2], v[3]);
-        out.z = bf16_part(v[4], v[5]);
-        out.w = bf16_part(v[6], v[7]);
+        out.x = bf16_part(two[0]);
+        out.y = bf16_part(two[1]);
+        out.z = bf16_part(two[2]);
+        out.w = bf16_part(two[3]);
         dst[y * apart] = out;
     }
 }
@@ -562,6 +563,7 @@ int product_tc(const void* A, int a_dtype, const float* W, float* out, int M, in
     p.A = A, p.W = W, p.M = M, p.N = N, p.K = K, p.a_f32 = a_dtype == MLS_F32;
     p.nt = c.nt, p.m_tiles = c.m_tiles, p.blocks = c.blocks, p.group = c.group, p.groups = c.groups, p.cut = c.cut;
     p.parts = a_dtype == MLS_F32 ? 3 : 1;
+    p.down = a_dtype == MLS_F32 ? 1.f / (UP * UP) : 1.f / UP;
     p.out = c.cut ? scratch + floats : out;
     p.stage_bytes = W_BYTES + p.parts * c.nt * ROW_BYTES;
     p.stages = RING_BYTES / p.stage_bytes < MAX_STAGES ? RING_BYTES / p.stage_bytes : MAX_STAGES;

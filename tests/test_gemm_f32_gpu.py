@@ -103,28 +103,30 @@ def test_odd_values_on_tensor_cores(ops, m):
 
 @pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("m", [3, 200])
-@pytest.mark.parametrize("power_a, power_w", [(-112, 100), (-120, 100), (-138, 120), (100, -112), (100, -120), (120, -140),
-                                              (-60, -62), (60, 62)])
-def test_small_operands_on_tensor_cores(ops, a_type, m, power_a, power_w):
-    """Operands whose lower parts lie below bfloat16's smallest number, down to float32's own smallest, against large
-    ones (the products are ordinary numbers): all 24 bits count."""
+@pytest.mark.parametrize("power_a, power_w, chain", [
+    (-112, 100, False), (-120, 100, False), (-130, 100, False), (100, -112, False), (100, -120, False), (100, -140, False),
+    (-60, -62, False), (30, 40, False), (-130, 120, True), (60, 60, True)])   # from 2^112, sums from 2^96 on
+def test_operands_of_all_sizes_on_tensor_cores(ops, a_type, m, power_a, power_w, chain):
+    """Operands whose lower parts would lie below bfloat16's smallest number, down to float32's own smallest, against
+    large ones (the products are ordinary numbers): all 24 bits count.  What is too large goes to a chain over k."""
     n, k = 300, 2048
     g = torch.Generator(device="cuda").manual_seed(m + power_a)
     a = (torch.randn(m, k, device="cuda", generator=g) * 2.0 ** power_a).to(a_type)
     w = torch.randn(n, k, device="cuda", generator=g) * 2.0 ** power_w
-    assert a.any() and w.any()
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert a.any() and w.any() and want.abs().max() < 3e38
     out = torch.empty(m, n, device="cuda")
     ops.linear(a, w, out)
-    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
-    # as in test_product_on_tensor_cores: 4 steps a 64 of k of 2^-23, k / 64 / 8 and 8 of 2^-24
-    assert ((out.double() - want).abs() <= 2.0 ** -24 * (2 + 8 + k / 512 + 8) * size).all()
-    assert (out.double() - want).norm() <= 2e-7 * want.norm()
+    # as in test_product_on_tensor_cores (4 steps a 64 of k of 2^-23, k / 64 / 8 and 8 of 2^-24); a chain's k roundings
+    steps = k + 2 if chain else 2 + 8 + k / 512 + 8
+    assert ((out.double() - want).abs() <= 2.0 ** -24 * steps * size).all()
+    assert chain or (out.double() - want).norm() <= 2e-7 * want.norm()
     ops.check_status()
 
 
-@pytest.mark.parametrize("a_type, m, n, k", [(torch.float32, 700, 300, 2048), (torch.bfloat16, 333, 300, 2052),
-                                             (torch.float32, 40, 2048, 8192)])
-def test_scratch_has_a_bound_and_memory_may_run_out(ops, monkeypatch, a_type, m, n, k):
+@pytest.mark.parametrize("a_type, m, n, k, share", [(torch.float32, 700, 300, 2048, 8), (torch.bfloat16, 333, 300, 2052, 8),
+                                                    (torch.float32, 40, 2048, 8192, 2)])
+def test_scratch_has_a_bound_and_memory_may_run_out(ops, monkeypatch, a_type, m, n, k, share):
     """Rows in parts give the same bits: by the bound, and after the allocator has refused what the whole takes."""
     g = torch.Generator(device="cuda").manual_seed(m)
     a = torch.randn(m, k, device="cuda", generator=g).to(a_type)
@@ -135,7 +137,7 @@ def test_scratch_has_a_bound_and_memory_may_run_out(ops, monkeypatch, a_type, m,
     most = ops._scratch["gemm_f32"].numel()
     assert most & (most - 1) == 0                         # grows by powers of two
     # a bound
-    limit = most // 8
+    limit = most // share
     monkeypatch.setattr(ops, "F32_SCRATCH", limit, raising=False)
     monkeypatch.setattr(ops, "_scratch", {})
     ops.linear(a, w, out)
