@@ -175,3 +175,38 @@ def test_launches_are_counted(ops, a_type, m, n, k, count):
         ops.linear(a, w, out)
     error, _, nodes = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
     assert int(error) == 0 and ops.launches - before == count == nodes
+
+
+@pytest.mark.parametrize("what", ["every value", "one value a row", "one row of weights"])
+@pytest.mark.parametrize("m, n, k", [(515, 2048, 2048), (16, 2048, 8192)])
+def test_values_that_are_no_numbers_do_not_hold_a_product_up(ops, what, m, n, k):
+    """Right, and at most sixty times the time of ordinary values (an output at a time took two hundred)."""
+    a, w = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")
+    odd, odd_w = a.clone(), w.clone()
+    if what == "every value":
+        odd[:] = float("nan")
+    elif what == "one value a row":
+        odd[:, k // 2] = float("inf")
+    else:
+        odd_w[5, 7] = float("nan")
+    out = torch.empty(m, n, device="cuda")
+
+    def time(a, w):
+        best = float("inf")
+        for _ in range(4):
+            begin, end = torch.cuda.Event(True), torch.cuda.Event(True)
+            begin.record()
+            ops.linear(a, w, out)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        return best
+    plain = time(a, w)
+    assert time(odd, odd_w) <= 60 * plain
+    if what == "every value":
+        assert out.isnan().all()
+    elif what == "one value a row":
+        assert (out == torch.where(w[:, k // 2] > 0, float("inf"), float("-inf"))).all()
+    else:
+        assert out[:, 5].isnan().all() and out[:, :5].isfinite().all() and out[:, 6:].isfinite().all()
+    ops.check_status()
