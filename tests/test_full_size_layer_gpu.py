@@ -13,6 +13,7 @@ context ends above 8,000 tokens.
 import pytest
 import torch
 
+import plain_llama
 from engine_helpers import Replayer, assert_close, plain_logits, tokens_for
 from mini_llm_stack_b200.config import config_from_dict
 from mini_llm_stack_b200.weights import write_random_model
@@ -143,9 +144,21 @@ def replay_on(model, num_blocks, max_requests=4):
     return rp
 
 
-def test_float32_at_full_layer_sizes(true_float32_products):
+def exact_logits(w, cfg, tokens, monkeypatch):
+    """The plain implementation in float64 (its rotary tables as they are defined, in float32)."""
+    tables = plain_llama.plain_rotary_tables(cfg["head_dim"], cfg["max_seq_len"], cfg["rope_theta"])
+    with monkeypatch.context() as m:
+        m.setattr(plain_llama, "plain_rotary_tables", lambda *a: tuple(t.double() for t in tables))
+        m.setattr(torch.Tensor, "float", torch.Tensor.double)
+        logits = plain_llama.plain_forward(w, cfg, tokens)
+    assert logits.dtype == torch.float64
+    return logits
+
+
+def test_float32_at_full_layer_sizes(true_float32_products, monkeypatch):
     """The true 32-bit path at hidden 4096, feed-forward 14336 and 32 / 8 heads of 128:
-    a prompt in portions, a second request beside it, decoded tokens."""
+    a prompt in portions, a second request beside it, decoded tokens.  Against float64: at this width the plain
+    implementation in float32 lies up to 5.2e-6 of the largest logit from it itself, beyond the limit."""
     model, cfg, w = device_model(BIG, "float32", seed=6)
     toks = {"a": tokens_for(1000, 300, 11), "b": tokens_for(1000, 45, 12)}
     rp = replay_on(model, num_blocks=32)
@@ -155,7 +168,7 @@ def test_float32_at_full_layer_sizes(true_float32_products):
         rp.step([("a", 1), ("b", 1)], toks)
     rp.step([("a", 25)], toks, end=["a", "b"])
     for r in "ab":
-        want = plain_logits(w, cfg, toks[r], "float32").cpu()
+        want = exact_logits(w, cfg, toks[r], monkeypatch).cpu()
         assert_close(rp.logits(r), want, "float32", f"float32 full-size layer, request {r}")
 
 
