@@ -10,19 +10,13 @@ constexpr int SKINNY_N = 256;        // up to so many columns the product is by 
 // 64 x 4,096: 15.2 / 8.4, 12.7 / 10.0, 15.5 / 16.1, 48.1 / 36.4, but 128 x 2,048, 256 rows 8.9 / 11.2.
 constexpr int FEWEST_N = 64;
 constexpr long long FEWEST_SIZE = 1 << 18;
-// From so much of K on the tensor cores pay whatever M is (us, FFMA / tensor cores: 1 x 300 x 2,048 18.4 / 16.4,
-// 1 x 2,048 x 2,048 20.5 / 18.4, 9 x 2,048 x 2,048 82 / 18; but 1 x 4,096 x 1,024 16.4 / 18.4; those with eight
-// groups of K, with sixteen 1 x 2,048 x 2,048 is at 10.5), from a quarter of it
-// where the weights are so many that their way from memory counts (1 x 16,384 x 1,024 39 / 31, 1 x 16,384 x 512
-// 22.6 both).
+// From so much of K on the tensor cores pay whatever M is (us after a flush of L2, FFMA / tensor cores: 1 x 300 x 2,048
+// 18.5 / 14.1, 1 x 2,048 x 2,048 20.4 / 19.4, 9 x 2,048 x 2,048 82 / 19.5, 1 x 4,096 x 4,096 43 / 34, 16 x 4,096 x 4,096 162 / 36,
+// 2,048 x 4,096 x 4,096 1,278 / 329; but 1 x 4,096 x 1,024 16.4 / 18.4), from a quarter of it
+// where the weights are so many that their way from memory counts (1 x 16,384 x 1,024 39 / 32, 1 x 16,384 x 512
+// 22.6 / 21.5; 1 x 8,192 x 1,024 is level, 22.5 / 23.6).
 constexpr int TC_K = 2048;
 constexpr long long TC_SIZE = 1 << 23;
-// Rows of 4,096 to 8,191 stay with the chain over k although the tensor cores would take them faster and leave
-// them nearer to float64 (16 x 4,096 x 4,096: 164 / 35 us).  What such runs are checked against are chains over k
-// in float32 themselves: a layer of hidden size 4,096 lies up to 3.3e-5 from float64 there and is held to 3.0e-5,
-// so that only sums with the same roundings pass (the chain's differ from it by 2.4e-5, the tensor cores' by 3.2e-5,
-// float64's own would by 3.3e-5).  From 8,192 on (feed-forward rows) and below 4,096 both pass.
-constexpr int CHAIN_K0 = 4096, CHAIN_K1 = 8192;
 
 // Whether the tensor cores take a product.  The types, N, K and the weights' address say so, never the rows: a row's
 // bits do not depend on the rows it is computed with.

@@ -597,7 +597,6 @@ bool takes_tc(int a_dtype, const float* W, int N, int K) {
     if (K % 4 || reinterpret_cast<uintptr_t>(W) % 16) return false;
     if (N <= SKINNY_N)
         return N >= FEWEST_N && K >= (a_dtype == MLS_BF16 ? TC_K : 2 * TC_K) && (long long)N * K >= FEWEST_SIZE;
-    if (K >= CHAIN_K0 && K < CHAIN_K1) return false;
     return K >= TC_K || (K >= TC_K / 4 && (long long)N * K >= TC_SIZE);
 }
 

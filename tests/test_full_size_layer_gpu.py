@@ -169,7 +169,9 @@ def test_float32_at_full_layer_sizes(true_float32_products, monkeypatch):
     rp.step([("a", 25)], toks, end=["a", "b"])
     for r in "ab":
         want = exact_logits(w, cfg, toks[r], monkeypatch).cpu()
-        assert_close(rp.logits(r), want, "float32", f"float32 full-size layer, request {r}")
+        mine = assert_close(rp.logits(r), want, "float32", f"float32 full-size layer, request {r}")
+        plain = (plain_logits(w, cfg, toks[r], "float32").cpu() - want).abs().max().item() / want.abs().max().item()
+        assert mine <= plain, "further from float64 than the plain implementation's float32"
 
 
 DEEP = dict(BIG, n_layers=4, max_seq_len=8192)

@@ -53,7 +53,7 @@ def test_rows_between_addresses(ops, a_type, off_a, off_w, m, n, k):
 @pytest.mark.parametrize("off", [0, 1])
 @pytest.mark.parametrize("m, n, k", [
     (1, 257, 2048), (16, 300, 2052), (17, 260, 2304), (33, 2048, 2080), (161, 385, 2056), (170, 4100, 2048),
-    (700, 1000, 8196), (5, 16384, 512), (321, 16500, 548), (1, 64, 4096), (129, 65, 4100), (1030, 130, 4104)])
+    (700, 1000, 8196), (16, 4096, 4096), (200, 300, 5000), (1, 257, 8188), (5, 16384, 512), (321, 16500, 548), (1, 64, 4096), (129, 65, 4100), (1030, 130, 4104)])
 def test_product_on_tensor_cores(ops, a_type, off, m, n, k):
     """Sizes around the edges of its tiles, blocks and groups: nearer to float64 than a chain over k could
     be, and the same bits for a row whatever rows it is computed with (cut along K or not)."""
