@@ -21,7 +21,7 @@
 // and half of the tokens of R, U and o; S0, R and U go into tensor memory as parts, K, Q, T and P come from
 // shared memory (K serves as K-major operand for S0^T k and as MN-major one for sum k u^T), copied ahead by
 // a warp of its own.  Ratios G_t / G_s come from differences of float64 sums of logarithms, never from a
-// quotient.  Accumulators hold at most 64 of k (P U: 32), small products first.
+// quotient.  Accumulators hold at most 64 of k (P U: 32, q k^T and k k^T: 16), small products first.
 //
 // A value that is infinite or not a number counts as zero for the tokens before it; from its token on the
 // column's outputs and state are no numbers (token by token they are not finite from there on either).
@@ -32,10 +32,12 @@
 // ask for at once 8,000 cycles of 40,000, the ratios 4,000 and T 5,500 a value head.
 //
 // Measured (the two kernels together against token by token): 32 heads of 128 x 128, requests of 341 and 683 tokens
-// 202 -> 105 us, one of 2,048 389 -> 272, four of 512 and 64 heads 515 -> 240.  Products issued by a warp that also owns
+// 202 -> 108 us, one of 2,048 389 -> 276.  Products issued by a warp that also owns
 // columns held it up for 3,700 cycles a chunk (181 us for the first).  Distance from float64 as a multiple of token by
-// token's (16 heads of 128 x 128): 0.98 at 192 tokens, 1.00 at 256, 0.97 at 512, 0.93 at 1,024; with the unit diagonal
-// in T, q S0 in one accumulator and dots over 64 1.1 to 1.2.
+// token's (2-norms over all outputs; 8 to 32 heads of 64 x 128 to 128 x 256, 256 to 1,501 tokens, six seeds): outputs 0.91 to
+// 1.09, 0.99 on average (heads of 64 0.94, of 96 0.97, of 128 1.02), states 0.59 to 0.72.  With q k^T and k k^T over 32 and
+// expf's ratios outputs 0.94 to 1.11 (1.01), states 0.61 to 0.75, 3 us less; with q S0 in four accumulators of 32 instead
+// of two of 64 outputs 0.91 to 1.07 (0.98), 12 us more; T R over 32 and P U over 16 change nothing.
 #include "bf16_parts.cuh"
 #include "chunk_common.cuh"
 #include "delta_rule.h"
@@ -84,11 +86,8 @@ __device__ __forceinline__ uint2 part4(float4& v) {
     two.y = bf16_part_up(v.z, v.w);
     return two;
 }
-// exp(d) for a float64 d <= 0: of the nearest float32, times one plus what that leaves.
-__device__ __forceinline__ float exp_of(double d) {
-    const float near = (float)d, e = expf(near);
-    return fmaf(e, (float)(d - (double)near), e);
-}
+// exp(d) for a float64 d <= 0, rounded once (expf's own 2 ulp showed in outputs and states).
+__device__ __forceinline__ float exp_of(double d) { return (float)exp(d); }
 
 constexpr int PREP_THREADS = 256, PAD = C + 4, MAX_RATIO = 4;
 
@@ -178,59 +177,62 @@ delta_chunk_prep_kernel(const ChunkArgs a, const __grid_constant__ Args where, c
         F_s[own][2 * lane] = l[0] + (sum - l[1]);
         F_s[own][2 * lane + 1] = sum;
     };
-    if (warp == 0) {
-        if (elect_one()) {
-            constexpr uint32_t idesc = umma_idesc(C);
-            for (int a32 = 0; a32 < 2 * to.e_tiles; ++a32) {
-                const int tile = a32 >> 1, k0 = 2 * (a32 & 1);
-                uint32_t accumulate = 0;
-                // part x of [q; k] times part y of k, 32 of e an accumulator; the first of the next kind divides
-                // what is there
-                auto product = [&](int x, int y, bool next_kind) {
+    // q k^T and k k^T, 16 of e an accumulator, a tile of e at a time
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    float sum[C];
 #pragma unroll
-                    for (int kk = k0; kk < k0 + 2; ++kk) {
-                        const uint64_t qk = umma_desc(base + (tile * 6 + x * 2) * TILE + kk * UMMA_K * 2),
-                                       k = umma_desc(base + (tile * 6 + y * 2 + 1) * TILE + kk * UMMA_K * 2);
-                        if (next_kind && kk == k0) umma_onto<PART_SHIFT>(tmem + a32 * C, qk, k, idesc);
-                        else umma(tmem + a32 * C, qk, k, idesc, accumulate);
-                        accumulate = 1;
-                    }
-                };
-                product(1, 1, false);
-                product(0, 2, false);
-                product(2, 0, false);
-                product(0, 1, true);
-                product(1, 0, false);
-                product(0, 0, true);
-            }
-            umma_commit(bar);
+    for (int x = 0; x < C; ++x) sum[x] = 0.f;
+    for (int tile = 0; tile < to.e_tiles; ++tile) {
+        if (tile) {                                    // the sums of the tile before have been read
+            tc_fence_before();
+            __syncthreads();
+            tc_fence_after();
         }
-        __syncwarp();
+        if (warp == 0) {
+            if (elect_one()) {
+                constexpr uint32_t idesc = umma_idesc(C);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    const uint32_t d = tmem + kk * C, at = base + tile * 6 * TILE + kk * UMMA_K * 2;
+                    // part x of [q; k] times part y of k; the first of the next kind divides what is there
+                    auto qk = [&](int x) { return umma_desc(at + x * 2 * TILE); };
+                    auto k = [&](int y) { return umma_desc(at + (y * 2 + 1) * TILE); };
+                    umma(d, qk(1), k(1), idesc, 0);
+                    umma(d, qk(0), k(2), idesc, 1);
+                    umma(d, qk(2), k(0), idesc, 1);
+                    umma_onto<PART_SHIFT>(d, qk(0), k(1), idesc);
+                    umma(d, qk(1), k(0), idesc, 1);
+                    umma_onto<PART_SHIFT>(d, qk(0), k(0), idesc);
+                }
+                umma_commit(bar);
+            }
+            __syncwarp();
+        }
+        if (tile == 0) decays(0);
+        if (!timed_out && !mbar_wait(bar, tile & 1)) timed_out = true;
+        tc_fence_after();
+        if (warp < 4) {
+#pragma unroll
+            for (int c0 = 0; c0 < C; c0 += 16)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t x[16];
+                    tmem_ld16(tmem + lanes + kk * C + c0, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[c0 + i] += __uint_as_float(x[i]);
+                }
+        }
     }
-    decays(0);
-    if (!mbar_wait(bar, 0)) timed_out = true;      // (all: the tiles' room serves for what follows)
-    tc_fence_after();
-    float* dots = reinterpret_cast<float*>(tiles);     // [q k^T; k k^T]: [128][PAD]
+    float* dots = reinterpret_cast<float*>(tiles);     // (all products are done: the tiles' room) [q k^T; k k^T]: [128][PAD]
     float* L = dots + 2 * C * PAD;                     // [64][PAD]
     float* T = L + C * PAD;                            // [64][PAD]
     float* M = T + C * PAD;                            // [3][16][20]
     if (warp < 4) {
-        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
         float* dst = dots + (warp * 32 + lane) * PAD;
 #pragma unroll
-        for (int c0 = 0; c0 < C; c0 += 16) {
-            float sum[16];
-            for (int a32 = 0; a32 < 2 * to.e_tiles; ++a32) {
-                uint32_t x[16];
-                tmem_ld16(tmem + lanes + a32 * C + c0, x);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 16; ++i) sum[i] = a32 ? sum[i] + __uint_as_float(x[i]) : __uint_as_float(x[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < 16; i += 4)
-                *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
-        }
+        for (int i = 0; i < C; i += 4)
+            *reinterpret_cast<float4*>(dst + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
     }
     tc_fence_before();
     for (int h = 0; h < ratio; ++h) {

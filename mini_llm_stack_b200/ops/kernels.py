@@ -1137,8 +1137,7 @@ class Ops:
     CHUNKED_FROM = {"head": 48, "token": 192, "mlstm": 128}
     # The delta rule's: its chunk-wise scan costs 39 us and 4.1 a chunk, however few blocks of a head and 128 columns
     # there are, the other one a time per token that falls with them.  32 heads of 128 x 128, one request of 256 tokens 56
-    # us against 67 (192: 50 / 52, but errors of outputs 0.98 at 192 and 1.03 at 128 of its); 16 heads 55 / 44, at
-    # 512 79 / 83.
+    # us against 67 (192: 50 / 52); 16 heads 55 / 44, at 512 79 / 83.  (Distances from float64: delta_chunk.cu.)
     DELTA_CHUNKED_FROM = {"few": 512, "many": 256}
     DELTA_MANY = 32               # blocks of a head and 128 columns
     CHUNK_SCRATCH = 1 << 27       # floats of scratch that the chunks under way may take (at least one does)
