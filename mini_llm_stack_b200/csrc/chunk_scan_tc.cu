@@ -10,7 +10,9 @@
 // straight from memory, its warp's 32 columns side by side, splits them in registers and puts the parts into
 // its lane of tensor memory; and it finds U[.., j] or o[.., j] there, whose stores are whole lines again.  No
 // operand of the wide side passes through shared memory.  A group of four warps walks its 128 columns by itself:
-// convert a block of k, multiply, add up; two or four groups an SM hide each other's waits.
+// convert a block of k, multiply, add up; two or four groups an SM hide each other's waits.  (Updates whose values are
+// not bfloat16 as they lie, with silu or float32, take 160 columns of tensor memory a group, 512 for two: one such block
+// has an SM at a time, the next waits for its columns.)
 //
 // A value that is infinite or not a number: in v it counts as zero for the tokens before it (P is lower
 // triangular, but 0 x inf is not 0), and outputs from its token on are computed again as chains of fmaf, as is

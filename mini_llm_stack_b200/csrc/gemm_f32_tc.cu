@@ -16,7 +16,8 @@
 // over K: 0.92e-7 / 4.1e-7 at 512, 1.04e-7 / 8.1e-7 at 2,048, 1.23e-7 / 16.2e-7 at 8,192.
 // Float32 operands are multiplied by 2^16 before they are split (bf16_parts.cuh says why), and the sums by what takes
 // that back out, which rounds nothing but what becomes smaller than float32's normal numbers (2^-149 at most).
-// A sum that is not finite (an operand that is infinite, not a number or 2^112 and more, or a sum of 2^96 and more)
+// A sum that is not finite (an operand that is infinite, not a number or 2^112 and more, or a sum of 2^96 and more,
+// 2^112 with bfloat16 rows)
 // is computed again as that chain.
 //
 // The weights take the 128-row side of the instruction: tiles of 128 x 32 come by TMA, a thread a row
@@ -29,8 +30,8 @@
 // The instructions are issued by one elected thread of a warp whose loop is uniform: from a branch that a
 // single lane takes each cost some 50 cycles to prepare, which bounded every size (851 us for 651, 431 for 235).
 //
-// Measured against FFMA (us): 2,048 x 16,384 x 2,048 2,460 -> 651 (211 TFLOP/s), 515 x 16,384 x 2,048 721 -> 211,
-// 515 x 2,048 x 8,192 510 -> 127, 16 x 2,048 x 8,192 250 -> 25, 3 x 128,256 x 2,048 393 -> 236 (1.05 GB: 4.5 TB/s),
+// Measured against FFMA (us): 2,048 x 16,384 x 2,048 2,460 -> 648 (212 TFLOP/s), 515 x 16,384 x 2,048 721 -> 213,
+// 515 x 2,048 x 8,192 510 -> 115, 16 x 2,048 x 8,192 250 -> 25, 3 x 128,256 x 2,048 393 -> 250 (1.05 GB: 4.2 TB/s),
 // 1 x 2,048 x 2,048 22.5 -> 10.5; eight groups of K instead of sixteen leave 16 x 64 x 4,096 at 11.3 instead of 7.9.
 //
 // Warp roles: 0 = TMA producer, 1 = tensor memory and instructions, 4..7 = splitting the weights (a
