@@ -404,7 +404,8 @@ def test_small_values_keep_their_bits(ops, always):
 
 @pytest.mark.parametrize("kind", ["head", "mlstm"])
 def test_a_value_that_is_no_number_does_not_hold_a_prompt_up(ops, kind):
-    """All tokens behind it are taken again: at most twelve times the time (an output at a time took twenty-four)."""
+    """All tokens behind it are taken again: at most nine times the time (four; an output at a time
+    took fourteen and seventeen)."""
     heads, e, f, t = 8, 128, 256, 2048
     rows = torch.randn(t, heads * (2 * e + f), device="cuda").bfloat16()
     odd = rows.clone()
@@ -432,5 +433,5 @@ def test_a_value_that_is_no_number_does_not_hold_a_prompt_up(ops, kind):
         return best
     plain = time(rows, gates)
     assert out.isfinite().all()
-    assert time(odd, odd_gates) <= 12 * plain
+    assert time(odd, odd_gates) <= 9 * plain
     assert out[:10].isfinite().all() and out[10:].isnan().all()

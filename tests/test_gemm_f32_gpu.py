@@ -180,7 +180,7 @@ def test_launches_are_counted(ops, a_type, m, n, k, count):
 @pytest.mark.parametrize("what", ["every value", "one value a row", "one row of weights"])
 @pytest.mark.parametrize("m, n, k", [(515, 2048, 2048), (16, 2048, 8192)])
 def test_values_that_are_no_numbers_do_not_hold_a_product_up(ops, what, m, n, k):
-    """Right, and at most sixty times the time of ordinary values (an output at a time took two hundred)."""
+    """Right, and at most ninety times the time of ordinary values (up to 35; an output at a time took 220)."""
     a, w = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")
     odd, odd_w = a.clone(), w.clone()
     if what == "every value":
@@ -202,7 +202,7 @@ def test_values_that_are_no_numbers_do_not_hold_a_product_up(ops, what, m, n, k)
             best = min(best, begin.elapsed_time(end))
         return best
     plain = time(a, w)
-    assert time(odd, odd_w) <= 60 * plain
+    assert time(odd, odd_w) <= 90 * plain
     if what == "every value":
         assert out.isnan().all()
     elif what == "one value a row":
