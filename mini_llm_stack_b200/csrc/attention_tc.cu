@@ -285,12 +285,18 @@ attention_tc_kernel(const Params P, const __grid_constant__ CUtensorMap kmap,
             }
             return true;
         };
-        for (int t = 0; t < n_tiles; ++t) {
-            if (!load(t, 0) || !load(t, 1)) {
-                timed_out = true;
-                break;
-            }
+        int n_k = 0, n_v = 0;                    // tiles asked for
+        for (int t = 0; t < n_tiles && !timed_out; ++t) {
+            if (load(t, 0)) ++n_k;
+            else timed_out = true;
+            if (!timed_out && load(t, 1)) ++n_v;
+            else timed_out = true;
         }
+        // the copies under way land before the block's shared memory goes away
+        for (int j = max(0, n_k - K_STAGES); j < n_k; ++j)
+            if (!mbar_wait_warp(bar(B_K_FULL + j % K_STAGES), (j / K_STAGES) & 1)) timed_out = true;
+        for (int j = max(0, n_v - V_STAGES); j < n_v; ++j)
+            if (!mbar_wait_warp(bar(B_V_FULL + j % V_STAGES), (j / V_STAGES) & 1)) timed_out = true;
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issue
         {

@@ -274,6 +274,9 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap
                         tma_load_2d(b_dst, &bmap, (kb0 + i) * BK, ni * BN, full(slot));
                 }
             }
+            // the copies under way land before the block's shared memory goes away
+            for (int j = g > STAGES ? g - STAGES : 0; j < g; ++j)
+                if (!mbar_wait(full(j % STAGES), (j / STAGES) & 1)) timed_out = true;
         }
         chain_wait();
     } else if (warp == 1) {
@@ -506,6 +509,11 @@ gemm_tcgen05_pair_kernel(const GemmParams p, const __grid_constant__ CUtensorMap
                     }
                 }
             }
+            // the copies under way land before the pair's shared memory goes away (the first CTA's barriers count both
+            // CTAs' bytes, and both CTAs meet once more)
+            if (rank == 0)
+                for (int j = g > STAGES ? g - STAGES : 0; j < g; ++j)
+                    if (!mbar_wait_cluster(full(j % STAGES), (j / STAGES) & 1)) timed_out = true;
         }
     } else if (warp == 1) {
         if (rank == 0) {

@@ -55,6 +55,15 @@ def test_lanes_leave_a_loop_together(role):
         assert not re.search(r"mbar_wait(_cluster)?\(", role), "a wait that each lane judges by itself"
 
 
+@pytest.mark.parametrize("body", [p for p in with_tensor_memory() if "tma_load_2d" in p.values[0] or "bulk_load" in p.values[0]])
+def test_copies_land_before_the_block_ends(body):
+    """The role that copies waits, behind its last copy, until those under way are there: also where a wait ran out."""
+    parts = re.split(r"\n    (?:if|\} else if) \(warp ", body)
+    role = next(r for r in parts if "tma_load_2d" in r or "load_k(c + 2)" in r)
+    behind = role[max(m.end() for m in re.finditer(r"tma_load_2d\w*\(|load_[kqtp]\(c", role)):]
+    assert re.search(r"for \(int \w+ = [^;]*;[^)]*\)\s*if \(!mbar_wait\w*\([^;]*(full|FULL)[^;]*timed_out = true;", behind)
+
+
 @pytest.mark.parametrize("path", sorted(CSRC.glob("*.cu")), ids=lambda p: p.stem)
 def test_shared_memory_limits_never_fall(path):
     """A launcher that remembers what limit it set a kernel sets one and the same each time: with a limit for every
